@@ -35,33 +35,74 @@ static void launch_bag(const BagParams& p, BagHeader* hdr, int* offsets, cudaStr
 // (the pooling kernel of the row exchange on a second stream) splits the SMs' slots between them.
 static thread_local int t_stream_ctas_per_sm = 0;
 
-template <int LANES, int VW, int VPL, int TILES, int INFLIGHT, int MINB>
+// Lookups per chunk of the lookup-granular kernel.  A group pays about 16 lookups' worth of time
+// to start a chunk and to follow its last bag past the end; the chunk that makes
+// rounds x (chunk + 16) smallest therefore spreads few lookups over all groups (one tile each)
+// and cuts a large batch so that its last round is nearly full.  Measured: one table with 2,700
+// lookups 90 us with chunks of 128 (one block), 15 us with chunks of 8; 4.47 M lookups of dim 64
+// 206 us, capped at chunks of 64 229 us, of 32 249 us.
+static int stream_chunk(long long lookups, int num_tables, int lanes, long long groups) {
+  int best = lanes;
+  long long best_cost = -1;
+  for (int tiles = 1; tiles <= 64; ++tiles) {
+    const long long chunk = (long long)tiles * lanes;
+    const long long chunks = lookups / chunk + num_tables / 2 + 1;
+    const long long rounds = (chunks + groups - 1) / groups;
+    const long long cost = rounds * (chunk + 16);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = (int)chunk;
+    }
+  }
+  return best;
+}
+
+template <int LANES, int VPL, int DEPTH, bool FULL, int MINB>
 static void launch_stream(const BagParams& p, BagHeader* hdr, cudaStream_t s) {
-  static int per_sm[kMaxDevices] = {0};
+  static int per_sm[kMaxDevices] = {0}, sm_count[kMaxDevices] = {0};
   const int slot = device_slot();
   if (!per_sm[slot]) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bag_stream_kernel<LANES, VW, VPL, TILES, INFLIGHT, MINB>,
-                                                      256, 0) != cudaSuccess || n < 1)
+    int n = 0, sms = 148;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bag_stream_kernel<LANES, VPL, DEPTH, FULL, MINB>, 256, 0) !=
+            cudaSuccess || n < 1)
       n = 2;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, slot);
+    sm_count[slot] = sms;
     per_sm[slot] = n;
   }
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, slot);
+  const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, per_sm[slot])
+                                            : std::max(1, per_sm[slot] + t_stream_ctas_per_sm);
+  const long long groups_per_block = (256 / 32) * (32 / LANES);
+  const long long max_blocks = (long long)sm_count[slot] * ctas;
+  long long lookups = 0;
+  for (int t = 0; t < p.num_tables; ++t) lookups += p.t[t].nnz;
   StreamChunks sc;
+  sc.chunk = stream_chunk(lookups, p.num_tables, LANES, max_blocks * groups_per_block);
   long long total = 0;
   for (int t = 0; t < p.num_tables; ++t) {
     sc.first[t] = (int)total;
     const long long n = p.t[t].nnz;
-    total += n > 0 ? (n + LANES * TILES - 1) / (LANES * TILES) : (p.batch + 1023) / 1024;
+    total += n > 0 ? (n + sc.chunk - 1) / sc.chunk : (p.batch + 1023) / 1024;
   }
   sc.first[p.num_tables] = (int)total;
   // a persistent grid, no larger than the chunks there are
-  const long long groups_per_block = (256 / 32) * (32 / LANES);
-  const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, per_sm[slot])
-                                            : std::max(1, per_sm[slot] + t_stream_ctas_per_sm);
-  long long blocks = std::min<long long>((long long)sms * ctas, (total + groups_per_block - 1) / groups_per_block);
-  bag_stream_kernel<LANES, VW, VPL, TILES, INFLIGHT, MINB><<<(unsigned)std::max<long long>(blocks, 1), 256, 0, s>>>(p, sc, hdr);
+  const long long blocks = std::min(max_blocks, (total + groups_per_block - 1) / groups_per_block);
+  bag_stream_kernel<LANES, VPL, DEPTH, FULL, MINB><<<(unsigned)std::max<long long>(blocks, 1), 256, 0, s>>>(p, sc, hdr);
+}
+
+template <int LANES, int VPL, int DEPTH, int MINB>
+static void launch_stream_dim(const BagParams& p, BagHeader* hdr, cudaStream_t s) {
+  if (p.dim == LANES * VPL * 4) launch_stream<LANES, VPL, DEPTH, true, MINB>(p, hdr, s);
+  else launch_stream<LANES, VPL, DEPTH, false, MINB>(p, hdr, s);
+}
+
+// Atomic route for tables whose segment ids were not sorted; returns at once for sorted tables.
+static int run_unsorted_route(const BagParams& p, long long max_nnz, BagHeader* hdr, int* offsets, cudaStream_t s) {
+  ANNC_CUDA(launch_pdl(bag_scatter_kernel, dim3(grid_for(max_nnz, 8, 148 * 8)), dim3(256), 0, s, p, hdr, offsets));
+  if (p.combiner == 1)
+    ANNC_CUDA(launch_pdl(bag_scatter_mean_kernel, dim3(grid_for(p.batch * p.dim, 256, 148 * 4)), dim3(256), 0, s, p,
+                         hdr, offsets));
+  return ANNC_OK;
 }
 
 // Launches the bag kernels (+ the atomic route) for up to kMaxTables tables.
@@ -121,33 +162,23 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
 
   // Lookup-granular route: no prepass, one pass over ids and segment ids.  Taken when every
   // table comes with its index matrix (no caller-supplied offsets), unsharded, 16-byte rows.
-  const bool stream = !any_offsets && shard_count == 1 && vecs >= 4 && batch < (1LL << 31) - 1 &&
-                      (vecs == 4 || vecs == 8 || vecs == 16 || vecs == 32 || vecs == 64 || vecs == 128);
+  const bool stream = !any_offsets && shard_count == 1 && vecs >= 1 && vecs <= 128 && batch < (1LL << 31) - 1 &&
+                      ncols < (1LL << 31) && out_stride < (1LL << 31);
   if (stream) {
     if (ev0) cudaEventRecord(ev0, s);
-    switch (vecs) {
-      case 4: launch_stream<4, 4, 1, 8, 4, 5>(p, hdr, s); break;
-      case 8: launch_stream<8, 4, 1, 8, 4, 5>(p, hdr, s); break;
-      // dim 64 and 128: 32 bytes per lane (8 / 16 lanes per row), two row loads in flight: fewer
-      // lanes repeat the per-lookup control instructions (0.70 ms against 0.79 ms with 16 lanes x
-      // 16 bytes x 4 in flight on the 17.9 M lookups of the DLRM batch)
-      case 16: launch_stream<8, 4, 2, 16, 2, 5>(p, hdr, s); break;
-      case 32: launch_stream<16, 4, 2, 8, 2, 5>(p, hdr, s); break;
-      case 64: launch_stream<32, 4, 2, 4, 4, 4>(p, hdr, s); break;
-      default: launch_stream<32, 4, 4, 4, 2, 3>(p, hdr, s); break;
-    }
+    // the smallest shape whose LANES x VPL vectors hold a row; 32 bytes per lane from dim 64 on:
+    // fewer lanes repeat the per-lookup control instructions
+    if (vecs <= 4) launch_stream_dim<4, 1, 2, 4>(p, hdr, s);
+    else if (vecs <= 8) launch_stream_dim<8, 1, 2, 4>(p, hdr, s);
+    else if (vecs <= 16) launch_stream_dim<8, 2, 2, 4>(p, hdr, s);
+    else if (vecs <= 32) launch_stream_dim<16, 2, 2, 4>(p, hdr, s);
+    else if (vecs <= 64) launch_stream_dim<32, 2, 2, 4>(p, hdr, s);
+    else launch_stream_dim<32, 4, 2, 3>(p, hdr, s);
     if (ev1) cudaEventRecord(ev1, s);
-    dim3 rs_grid(148, num_tables);
-    bag_stream_reset_kernel<<<rs_grid, 256, 0, s>>>(p, hdr, offsets);  // returns at once for sorted tables
-    dim3 sc_grid(grid_for(max_nnz, 8, 148), num_tables);
-    bag_scatter_kernel<<<sc_grid, 256, 0, s>>>(p, hdr, offsets);
-    if (combiner == 1) {
-      dim3 mean_grid(grid_for(batch * dim, 256, 148), num_tables);
-      bag_scatter_mean_kernel<<<mean_grid, 256, 0, s>>>(p, hdr, offsets);
-    }
-    cudaError_t es = cudaGetLastError();
-    if (es != cudaSuccess) return cuda_fail(es, "embedding bag launch");
-    return ANNC_OK;
+    // Programmatic launches: 1.5 us each behind the bag kernel on sorted tables; as plain launches
+    // of a block per (table, slice) they cost 4.5 us (26 tables) to 8 us (64 tables) each.
+    ANNC_CUDA(launch_pdl(bag_stream_reset_kernel, dim3(148 * 4), dim3(256), 0, s, p, hdr, offsets));
+    return run_unsorted_route(p, max_nnz, hdr, offsets, s);
   }
 
   if (need_prepass) {  // tables that brought their offsets are skipped inside the kernel
@@ -171,17 +202,7 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
     }
   }
   if (ev1) cudaEventRecord(ev1, s);
-  // Atomic route for tables whose segment ids were not sorted; the blocks return
-  // at once for sorted tables.
-  dim3 sc_grid(grid_for(max_nnz, 8, 148), num_tables);
-  bag_scatter_kernel<<<sc_grid, 256, 0, s>>>(p, hdr, offsets);
-  if (combiner == 1) {
-    dim3 mean_grid(grid_for(batch * dim, 256, 148), num_tables);
-    bag_scatter_mean_kernel<<<mean_grid, 256, 0, s>>>(p, hdr, offsets);
-  }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "embedding bag launch");
-  return ANNC_OK;
+  return run_unsorted_route(p, max_nnz, hdr, offsets, s);
 }
 
 // Exclusive scan of int32 on the device; *total_dev receives the sum.

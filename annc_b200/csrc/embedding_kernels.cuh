@@ -10,6 +10,7 @@
 #include <cstdint>
 
 #include "emb_device.cuh"
+#include "pdl.cuh"
 
 namespace annc {
 namespace emb {
@@ -22,11 +23,17 @@ constexpr int kErrSegment = 2;          // segment id outside [0, batch)
 // Head of the bag workspace (256 bytes), then int32 offsets[num_tables][batch + 1].
 struct BagHeader {
   int err_bits;
-  int pad[3];
+  int any_unsorted;          // some table of the call is marked below
+  int pad[2];
   int unsorted[kMaxTables];  // per table: segment ids were seen to decrease
 };
 static_assert(sizeof(BagHeader) <= 512, "header layout");
 constexpr size_t kHeaderBytes = 512;
+
+__device__ __forceinline__ void mark_unsorted(BagHeader* hdr, int t) {
+  hdr->unsorted[t] = 1;
+  hdr->any_unsorted = 1;
+}
 
 struct BagTableDev {
   const float* table;
@@ -77,7 +84,7 @@ __global__ void bag_prepass_kernel(BagParams p, BagHeader* hdr, int* offsets) {
     if (prev < -1) prev = -1;
     if (prev > p.batch) prev = p.batch;
     if (cur < prev) {
-      if (i < T.nnz) hdr->unsorted[t] = 1;
+      if (i < T.nnz) mark_unsorted(hdr, t);
       continue;
     }
     for (long long s = prev + 1; s <= cur; ++s) off[s] = (int)i;
@@ -112,7 +119,7 @@ bag_prepass2_kernel(BagParams p, BagHeader* hdr, int* offsets) {
     if (prev < -1) prev = -1;
     if (prev > p.batch) prev = p.batch;
     if (cur < prev) {
-      if (i < T.nnz) hdr->unsorted[t] = 1;
+      if (i < T.nnz) mark_unsorted(hdr, t);
       continue;
     }
     for (long long s = prev + 1; s <= cur; ++s) off[s] = (int)i;
@@ -331,49 +338,69 @@ bag_reduce_generic_kernel(BagParams p, BagHeader* hdr, int* offsets) {
 }
 
 // ---- lookup-granular bag kernel ------------------------------------------------------
-// The same pooling without a prepass: blockIdx.y = table; a group of LANES lanes takes a chunk
-// of TILES * LANES consecutive lookups of the table (tile by tile: one lookup per lane, ids and
-// segment ids read with coalesced loads, the hash-bucket modulo applied by the lane that read
-// the id) and owns the bags whose first lookup lies in the chunk; it follows its last bag past
-// the chunk until the segment id changes.  Bag boundaries inside a tile are one ballot; rows are
-// added in lookup order into a zero accumulator (the reference's order, bit-identical sums),
-// INFLIGHT row loads in flight per group.  Work per group does not depend on the bag lengths and
-// short bags leave no lanes idle.  Bags without lookups are zero-filled by the group that owns
-// the next bag (the first bag's owner fills from 0, the last bag's owner to the end).  A
-// decrease of the segment ids marks the table unsorted: bag_stream_reset_kernel then clears its
-// output and the atomic route below redoes it.
-// Chunk numbering of bag_stream_kernel over all tables of a launch: table t owns the chunks
-// [first[t], first[t + 1]); a table without lookups gets one chunk per 1024 bags to zero.
+// The same pooling without a prepass.  A group of LANES lanes takes a chunk of consecutive
+// lookups of a table, tile by tile (LANES lookups, one per lane: ids and segment ids read with
+// coalesced loads, the hash-bucket modulo applied by the lane that read the id) and owns the
+// bags whose first lookup lies in the chunk; it follows its last bag past the chunk until the
+// segment id changes.  Bag boundaries inside a tile are one ballot; rows are added in lookup
+// order into a zero accumulator (the reference's order, bit-identical sums).  Bags without
+// lookups are zero-filled by the group that owns the next bag (the first bag's owner fills from
+// 0, the last bag's owner to the end).  A decrease of the segment ids marks the table unsorted:
+// bag_stream_reset_kernel then clears its output and the atomic route below redoes it.
+//
+// What bounds it: DRAM for tables beyond L2 (batch 65536 over 26 tables of 100 K rows moves
+// 3.4 GB, 0.67 ms), else the instructions per lookup and the latency of the row loads.  So the loop
+// is an unrolled pipeline: DEPTH - 1 row loads are out before a row is added, across tile borders
+// too, the ids of the next tile are already under way, and what only a bag's start needs (its
+// number, gaps of empty bags) is kept out of the loop.  Measured, 26 tables x 1 M rows x dim 64,
+// batch 16384, 4.47 M lookups: 248 us with the former loop (two loads, then two adds; ids of a
+// tile fetched at its start), 189 us now; 26 x 2,100 lookups: 100 us -> 18 us.  Choices at
+// that size: DEPTH 2 with 64 registers 202 us, DEPTH 4 with 80 216 us, 64 bytes per lane 289 us,
+// groups that drift apart 414 us.
+// The chunk length comes from the launch (stream_chunk): short for few lookups, so that they
+// spread over all SMs, long enough for a batch that fills the chip several times.
+//
+// A row has VPL 16-byte vectors per lane; FULL says that LANES * VPL vectors are exactly a row
+// (otherwise the lanes past the row end load and store nothing).
 struct StreamChunks {
-  int first[kMaxTables + 1];
+  int first[kMaxTables + 1];  // table t owns the chunks [first[t], first[t + 1]); a table without
+                              // lookups gets one chunk per 1024 bags to zero
+  int chunk;                  // lookups per chunk, a multiple of LANES
 };
 
-template <int LANES, int VW, int VPL, int TILES, int INFLIGHT_, int MINB>
+template <int LANES, int VPL, int DEPTH, bool FULL, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 bag_stream_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
   constexpr int GROUPS_PER_WARP = 32 / LANES;
-  constexpr int CHUNK = LANES * TILES;
-  constexpr int INFLIGHT = LANES < INFLIGHT_ ? LANES : INFLIGHT_;
-  constexpr int ROWF = LANES * VW * VPL;  // floats per row
-  using Vec = RowVec<VW>;
-  constexpr unsigned kLaneMask = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u);
+  constexpr int STEPS = LANES < 8 ? LANES : 8;  // unrolled lookups
+  static_assert(STEPS % DEPTH == 0, "the row buffers rotate a whole number of times per round");
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr unsigned kLaneMask = LANES == 32 ? kAll : ((1u << LANES) - 1u);
   constexpr int kNoBag = -3;  // a lookup whose segment id is out of range is added nowhere
   __shared__ int s_first[kMaxTables + 1];
+  // Bags of the last two tiles' lookups: lookup i at i % (2 * LANES).  Read at bag starts only.
+  __shared__ int s_key[256 / LANES][2 * LANES];
+  constexpr int kRing = 2 * LANES - 1;
   for (int i = threadIdx.x; i <= p.num_tables; i += blockDim.x) s_first[i] = sc.first[i];
   __syncthreads();
-  const int batch = (int)p.batch;
-  const int lane_in_warp = threadIdx.x & 31;
-  const int lane = lane_in_warp % LANES;
-  const int shift = (lane_in_warp / LANES) * LANES;
-  const unsigned gmask = kLaneMask << shift;
-  const unsigned group = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * GROUPS_PER_WARP +
-                         lane_in_warp / LANES;
-  const unsigned num_groups = gridDim.x * (blockDim.x >> 5) * GROUPS_PER_WARP;
-  const unsigned total_chunks = (unsigned)s_first[p.num_tables];
+  const int batch = (int)p.batch, ncols = (int)p.ncols, dim = (int)p.dim, out_stride = (int)p.out_stride;
+  const int lane = threadIdx.x % LANES;
+  const int shift = (int)(threadIdx.x & 31) / LANES * LANES;
+  int* const keys = s_key[threadIdx.x / LANES];
+  bool col_ok[VPL];
+#pragma unroll
+  for (int w = 0; w < VPL; ++w) col_ok[w] = FULL || (w * LANES + lane) * 4 < dim;
 
-  // Consecutive groups take consecutive chunks, so the whole grid works through one table
-  // after the other and ends together.
-  for (unsigned gc = group; gc < total_chunks; gc += num_groups) {
+  // The groups of a warp work side by side on consecutive chunks and stay in step: every loop
+  // below has the same trip count for the whole warp (a group that has finished has no rows left
+  // to load), otherwise the groups drift apart and are executed one after the other.
+  // Consecutive warps take consecutive chunks, so the whole grid works through one table after
+  // the other and ends together.
+  const unsigned num_groups = gridDim.x * (256 / LANES);
+  for (unsigned gc0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * GROUPS_PER_WARP; gc0 < (unsigned)s_first[p.num_tables];
+       gc0 += num_groups) {
+    const unsigned gc = gc0 + (threadIdx.x & 31) / LANES;
+    const bool have = gc < (unsigned)s_first[p.num_tables];
     int lo = 0, hi = p.num_tables - 1;  // table of chunk gc: last t with first[t] <= gc
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -381,185 +408,261 @@ bag_stream_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
       else hi = mid - 1;
     }
     const int t = lo;
-    const unsigned chunk = gc - (unsigned)s_first[t];
     const BagTableDev& T = p.t[t];
-    const int n = T.nnz;
-    const float* __restrict__ tab = T.table;
-    float* __restrict__ outp = T.out;
+    const int n = have ? T.nnz : 0;
+    const float* __restrict__ tab = T.table + lane * 4;
+    float* __restrict__ outp = T.out + lane * 4;
 
     // rows [a, b) of the output <- 0 (bags without lookups)
     auto zero_fill = [&](int a, int b) {
-      Vec z;
-      z.zero();
       for (int s = a; s < b; ++s) {
-        float* o = outp + (long long)s * p.out_stride;
+        float* o = outp + (long long)s * out_stride;
 #pragma unroll
-        for (int w = 0; w < VPL; ++w) z.store(o + (w * LANES + lane) * VW);
+        for (int w = 0; w < VPL; ++w)
+          if (col_ok[w]) __stcs(reinterpret_cast<float4*>(o + w * LANES * 4), make_float4(0.f, 0.f, 0.f, 0.f));
       }
     };
-    if (n == 0) {  // a table without lookups: every bag is empty
-      zero_fill((int)min((long long)chunk * 1024, (long long)batch), (int)min((long long)(chunk + 1) * 1024, (long long)batch));
-      continue;
-    }
-    {
-    Vec acc[VPL];
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) acc[v].zero();
-    int cur = kNoBag;   // bag being summed
-    int count = 0;      // its lookups so far (for the mean)
-    bool open = false;
-    const int chunk_end = min(n, (int)(chunk + 1) * CHUNK);
+    const long long chunk = (long long)(gc - (unsigned)s_first[t]);
+    if (have && n == 0)  // a table without lookups: every bag is empty
+      zero_fill((int)min(chunk * 1024, (long long)batch), (int)min((chunk + 1) * 1024, (long long)batch));
 
-    auto flush = [&]() {
-      if (open && cur >= 0) {
-        if (p.combiner == 1 && count > 0) {
-          const float inv = __fdiv_rn(1.0f, (float)count);
-#pragma unroll
-          for (int w = 0; w < VPL; ++w) acc[w].scale(inv);
-        }
-        float* o = outp + (long long)cur * p.out_stride;
-#pragma unroll
-        for (int w = 0; w < VPL; ++w) acc[w].store(o + (w * LANES + lane) * VW);
+    // ---- the tile being added and the raw ids of the tile after it
+    int base = n > 0 ? (int)chunk * sc.chunk : 0;  // below nnz < 2^31
+    const int chunk_end = (int)min((long long)n, (long long)base + sc.chunk);
+    long long raw_seg = 0;
+    unsigned long long raw_id = 0;
+    // Ids and outputs pass through once: they leave L2 to the table rows (evict-first).
+    auto load_raw = [&](int b) {
+      if (b < n - lane) {
+        const int i = b + lane;
+        raw_seg = __ldcs(reinterpret_cast<const long long*>(T.seg) + (long long)i * ncols + p.col);
+        if (p.id_kind == 0) raw_id = (unsigned long long)(long long)__ldcs((const int*)T.ids + i);
+        else raw_id = __ldcs((const unsigned long long*)T.ids + i);
       }
     };
-
-    for (int base = (int)chunk * CHUNK; base < n; base += LANES) {
-      const int i = base + lane;
-      int key = kNoBag, row = -1;
-      if (i < n) {
-        const long long seg = T.seg[(long long)i * p.ncols + p.col];
-        const long long r64 = load_row_id(T.ids, p.id_kind, i, T.num_buckets, T.magic);
-        if (seg < 0 || seg >= batch) atomicOr(&hdr->err_bits, kErrSegment);
-        else key = (int)seg;
+    int row = -1;
+    int to = 0;              // the tile's lookups before `to` can belong to this group's bags
+    unsigned smask = 0;      // bag starts among them
+    bool open = false;       // a bag is open after the tile
+    bool more = n > 0;       // there is a tile after this one
+    // The tile at `base` from its raw ids (a group without one: no rows).
+    auto decode = [&]() {
+      const bool in = more && base < n - lane;
+      int k = kNoBag, r = -1;
+      if (in) {
+        if (raw_seg < 0 || raw_seg >= batch) atomicOr(&hdr->err_bits, kErrSegment);
+        else k = (int)raw_seg;
+        const long long r64 = p.id_kind == 2 ? (long long)fast_mod_u64(raw_id, T.num_buckets, T.magic) : (long long)raw_id;
         if (r64 < 0 || r64 >= T.rows) atomicOr(&hdr->err_bits, kErrRow);
-        else row = (int)r64;
+        else r = (int)r64;
       }
-      int prev_key = __shfl_up_sync(gmask, key, 1, LANES);
-      if (lane == 0) {
-        prev_key = -1;  // before the first lookup: bags 0 .. key-1 are empty
-        if (base > 0) {
-          const long long ps = T.seg[(long long)(base - 1) * p.ncols + p.col];
-          prev_key = (ps < 0 || ps >= batch) ? kNoBag : (int)ps;
-        }
-      }
-      const bool starts = (i < n) && (key != prev_key);
-      if (starts && key >= 0 && prev_key >= 0 && key < prev_key) hdr->unsorted[t] = 1;
-      const unsigned smask = (__ballot_sync(gmask, starts) >> shift) & kLaneMask;
+      if (more) keys[(base + lane) & kRing] = k;
+      __syncwarp();
+      const int pk = keys[(base + lane - 1) & kRing];
+      const bool starts = in && k != pk;
+      const unsigned all = (__ballot_sync(kAll, starts) >> shift) & kLaneMask;
       const int tile_n = min(LANES, n - base);
-      int from = 0, to = tile_n;
       const bool inside = base < chunk_end;
-      if (!open) {
-        if (!inside) break;
-        if (smask == 0) continue;
-        from = __ffs(smask) - 1;
-      } else if (!inside) {
-        if (smask != 0) to = __ffs(smask) - 1;
+      const int first = all ? __ffs(all) - 1 : tile_n;
+      const int from = open ? 0 : (inside ? first : tile_n);
+      const int end = inside ? tile_n : (open ? first : 0);
+      const bool mine = more && lane >= from && lane < end;
+      row = mine ? r : -1;
+      smask = more && end > from ? (all & (kLaneMask >> (LANES - end))) : 0u;
+      // lookups whose segment id is not the previous one or its successor: unsorted segment ids,
+      // or empty bags in between (the owner of the next bag zeroes them)
+      const bool odd = mine && starts && k >= 0 && pk >= -1 && k != pk + 1;
+      unsigned gaps = __ballot_sync(kAll, odd);
+      if (gaps) {
+        if (odd && k < pk) mark_unsorted(hdr, t);
+        gaps = (gaps >> shift) & kLaneMask;
+        while (gaps) {
+          const int i = base + __ffs(gaps) - 1;
+          gaps &= gaps - 1;
+          zero_fill(keys[(i - 1) & kRing] + 1, keys[i & kRing]);
+        }
+        __syncwarp();
       }
-      for (int j0 = from; j0 < to; j0 += INFLIGHT) {
-        Vec v[INFLIGHT][VPL];
-        bool has[INFLIGHT];
+      if (more) {
+        to = end;
+        open = open || smask != 0;
+        // the table ends here, the open bag ended, or no bag starts in the rest of the chunk
+        more = !(base >= n - LANES || (inside ? (!open && base >= chunk_end - LANES) : end < tile_n));
+      }
+    };
+
+    float4 acc[VPL];
 #pragma unroll
-        for (int k = 0; k < INFLIGHT; ++k) {
-          const int j = j0 + k;
-          has[k] = false;
-          if (j < to) {
-            const int rw = __shfl_sync(gmask, row, j, LANES);
-            has[k] = rw >= 0;
-            if (has[k]) {
-              const float* src = tab + (long long)rw * ROWF + lane * VW;
+    for (int v = 0; v < VPL; ++v) acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int bag = kNoBag;    // bag being summed
+    int bag_start = 0;   // its first lookup (the mean's count)
+    float4 v[DEPTH][VPL];  // rows on their way
+    int vr[DEPTH];         // their numbers (negative: none)
+
+    auto issue = [&](int slot, int j) {
+      vr[slot] = __shfl_sync(kAll, row, j, LANES);
+      if (vr[slot] >= 0) {
+        const float* src = tab + (long long)vr[slot] * dim;
 #pragma unroll
-              for (int w = 0; w < VPL; ++w) v[k][w].load(src + w * LANES * VW);
-            }
+        for (int w = 0; w < VPL; ++w)
+          if (col_ok[w]) v[slot][w] = ldg4(src + w * LANES * 4);
+      }
+    };
+    auto flush = [&](int end) {
+      if (bag >= 0) {
+        if (p.combiner == 1) {
+          const float inv = __fdiv_rn(1.0f, (float)(end - bag_start));
+#pragma unroll
+          for (int w = 0; w < VPL; ++w) {
+            acc[w].x = __fmul_rn(acc[w].x, inv);
+            acc[w].y = __fmul_rn(acc[w].y, inv);
+            acc[w].z = __fmul_rn(acc[w].z, inv);
+            acc[w].w = __fmul_rn(acc[w].w, inv);
           }
         }
+        float* o = outp + (long long)bag * out_stride;
 #pragma unroll
-        for (int k = 0; k < INFLIGHT; ++k) {
-          const int j = j0 + k;
-          if (j < to) {
-            if ((smask >> j) & 1u) {
-              flush();
+        for (int w = 0; w < VPL; ++w)
+          if (col_ok[w]) __stcs(reinterpret_cast<float4*>(o + w * LANES * 4), acc[w]);
+      }
+    };
+
+    if (lane == 0) {
+      int before = -1;  // before the first lookup: bags 0 .. key - 1 are empty
+      if (base > 0) {
+        const long long ps = __ldcs(reinterpret_cast<const long long*>(T.seg) + (long long)(base - 1) * ncols + p.col);
+        before = (ps < 0 || ps >= batch) ? kNoBag : (int)ps;
+      }
+      keys[(base - 1) & kRing] = before;
+    }
+    load_raw(base);
+    decode();
+    if (more) load_raw(base + LANES);
 #pragma unroll
-              for (int w = 0; w < VPL; ++w) acc[w].zero();
-              cur = __shfl_sync(gmask, key, j, LANES);
-              const int before = __shfl_sync(gmask, prev_key, j, LANES);
-              // empty bags between the previous lookup's bag and this one (sorted input only)
-              if (cur >= 0 && before >= -1 && before < cur - 1) zero_fill(before + 1, cur);
-              count = 0;
-              open = true;
+    for (int k = 0; k < DEPTH - 1; ++k) issue(k, k);
+    bool go_on = true;
+    while (go_on) {
+      unsigned sm = smask;       // bag starts of the tile, the next lookup's bit first
+      const int tile = base;
+#pragma unroll 1
+      for (int j = 0; j < LANES; j += STEPS) {
+#pragma unroll
+        for (int k = 0; k < STEPS; ++k) {
+          // a row load goes out before the row loaded DEPTH - 1 steps ago is added; the last of a
+          // tile's are those of the next tile
+          if (k + DEPTH - 1 < STEPS || j + STEPS < LANES) {
+            issue((k + DEPTH - 1) % DEPTH, j + k + DEPTH - 1);
+          } else {
+            if (k + DEPTH - 1 == STEPS) {
+              go_on = __any_sync(kAll, more);
+              if (go_on) {
+                if (more) base += LANES;
+                decode();
+                if (more) load_raw(base + LANES);
+              } else {
+                row = -1;
+              }
             }
-            ++count;
-            if (has[k]) {
+            issue((k + DEPTH - 1) % DEPTH, k + DEPTH - 1 - STEPS);
+          }
+          if (sm & (1u << k)) {
+            const int i = tile + j + k;
+            flush(i);
 #pragma unroll
-              for (int w = 0; w < VPL; ++w) acc[w].add(v[k][w]);
-            }
+            for (int w = 0; w < VPL; ++w) acc[w] = make_float4(0.f, 0.f, 0.f, 0.f);
+            bag = keys[i & kRing];
+            bag_start = i;
+          }
+          if (vr[k % DEPTH] >= 0) {
+#pragma unroll
+            for (int w = 0; w < VPL; ++w) add4(acc[w], v[k % DEPTH][w]);
           }
         }
+        sm >>= STEPS;
       }
-      if (!inside && to < tile_n) break;
+    }
+    if (open) {
+      flush(base + to);
       // the table's last lookup: bags after its bag are empty
-      if (base + tile_n >= n && to == tile_n && open && cur >= 0) zero_fill(cur + 1, batch);
+      if (base + to == n && bag >= 0) zero_fill(bag + 1, batch);
     }
-    flush();
-    }
+    __syncwarp();  // the ring is free for the next chunk
   }
+  pdl_trigger();
 }
 
-// Tables marked unsorted: zero the output and the per-bag counters for the atomic route.
+// The kernels for tables marked unsorted.  They follow every call, sorted or not (the host does
+// not know), so their cost on sorted tables is what matters: one grid over all marked tables
+// that leaves after one load, launched while the kernel before it drains (pdl_wait holds until
+// that kernel has finished and its writes are visible).
+
+// Zeroes the output and the per-bag counters for the atomic route.
 __global__ void __launch_bounds__(256)
 bag_stream_reset_kernel(BagParams p, BagHeader* hdr, int* offsets) {
-  const int t = blockIdx.y;
-  if (!hdr->unsorted[t]) return;
-  const BagTableDev& T = p.t[t];
-  int* counts = offsets + (long long)t * (p.batch + 1);
+  pdl_wait();
+  pdl_trigger();
+  if (!*(volatile int*)&hdr->any_unsorted) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long total = p.batch * p.dim;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
-    const long long s = e / p.dim, c = e - s * p.dim;
-    T.out[s * p.out_stride + c] = 0.f;
-    if (c == 0) counts[s] = 0;
+  for (int t = 0; t < p.num_tables; ++t) {
+    if (!hdr->unsorted[t]) continue;
+    const BagTableDev& T = p.t[t];
+    int* counts = offsets + (long long)t * (p.batch + 1);
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
+      const long long s = e / p.dim, c = e - s * p.dim;
+      T.out[s * p.out_stride + c] = 0.f;
+      if (c == 0) counts[s] = 0;
+    }
   }
 }
 
-// ---- unsorted route: atomic scatter (sum order not defined; within 1e-5 rel) ----
+// Atomic scatter (sum order not defined; within 1e-5 rel).
 __global__ void __launch_bounds__(256)
 bag_scatter_kernel(BagParams p, BagHeader* hdr, int* offsets) {
-  const int t = blockIdx.y;
-  if (!hdr->unsorted[t]) return;
-  const BagTableDev& T = p.t[t];
-  int* counts = offsets + (long long)t * (p.batch + 1);
+  pdl_wait();
+  pdl_trigger();
+  if (!*(volatile int*)&hdr->any_unsorted) return;
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < T.nnz;
-       i += warps) {
-    long long seg = T.seg[i * p.ncols + p.col];
-    long long r = shard_row(load_row_id(T.ids, p.id_kind, i, T.num_buckets, T.magic), p.shard_count,
-                            p.shard_rank);
-    if (seg < 0 || seg >= p.batch) continue;  // flagged by the prepass
-    if (lane == 0) atomicAdd(&counts[seg], 1);  // bag length counts every rank's lookups
-    if (r == kNotMine) continue;
-    if (r < 0 || r >= T.rows) {
-      if (lane == 0) atomicOr(&hdr->err_bits, kErrRow);
-      continue;
+  for (int t = 0; t < p.num_tables; ++t) {
+    if (!hdr->unsorted[t]) continue;
+    const BagTableDev& T = p.t[t];
+    int* counts = offsets + (long long)t * (p.batch + 1);
+    for (long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < T.nnz;
+         i += warps) {
+      long long seg = T.seg[i * p.ncols + p.col];
+      long long r = shard_row(load_row_id(T.ids, p.id_kind, i, T.num_buckets, T.magic), p.shard_count,
+                              p.shard_rank);
+      if (seg < 0 || seg >= p.batch) continue;  // flagged by the prepass
+      if (lane == 0) atomicAdd(&counts[seg], 1);  // bag length counts every rank's lookups
+      if (r == kNotMine) continue;
+      if (r < 0 || r >= T.rows) {
+        if (lane == 0) atomicOr(&hdr->err_bits, kErrRow);
+        continue;
+      }
+      float* orow = T.out + seg * p.out_stride;
+      for (long long c = lane; c < p.dim; c += 32) atomicAdd(orow + c, __ldg(T.table + r * p.dim + c));
     }
-    float* orow = T.out + seg * p.out_stride;
-    for (long long c = lane; c < p.dim; c += 32) atomicAdd(orow + c, __ldg(T.table + r * p.dim + c));
   }
 }
 
 __global__ void __launch_bounds__(256)
 bag_scatter_mean_kernel(BagParams p, BagHeader* hdr, int* offsets) {
-  const int t = blockIdx.y;
-  if (!hdr->unsorted[t]) return;
-  const BagTableDev& T = p.t[t];
-  const int* counts = offsets + (long long)t * (p.batch + 1);
+  pdl_wait();
+  if (!*(volatile int*)&hdr->any_unsorted) return;
   const long long total = p.batch * p.dim;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
-    const long long s = e / p.dim, c = e - s * p.dim;
-    const int n = counts[s];
-    if (n > 0) {
-      float* q = T.out + s * p.out_stride + c;
-      *q = __fmul_rn(*q, __fdiv_rn(1.0f, (float)n));
+  for (int t = 0; t < p.num_tables; ++t) {
+    if (!hdr->unsorted[t]) continue;
+    const BagTableDev& T = p.t[t];
+    const int* counts = offsets + (long long)t * (p.batch + 1);
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
+      const long long s = e / p.dim, c = e - s * p.dim;
+      const int n = counts[s];
+      if (n > 0) {
+        float* q = T.out + s * p.out_stride + c;
+        *q = __fmul_rn(*q, __fdiv_rn(1.0f, (float)n));
+      }
     }
   }
 }

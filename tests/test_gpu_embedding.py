@@ -356,3 +356,43 @@ def test_division_free_modulo_is_exact(num_buckets):
         got = m.mask.cpu().numpy().view(np.uint32)
         want = np.array([1 << (int(b) % g) for b in want_bucket], dtype=np.uint32)
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("dim,stride_slots", [(4, 1), (20, 2), (48, 3), (64, 3), (128, 2), (132, 1), (264, 1), (516, 1)])
+@pytest.mark.parametrize("combiner", [0, 1])
+@pytest.mark.parametrize("id_kind", [0, 1, 2])
+def test_bag_plan_tile_and_chunk_edges(dim, stride_slots, combiner, id_kind):
+    """Grouped bags at the lengths where the lookup-granular kernel can go wrong: lookups around a
+    tile and a chunk, one bag over many chunks, runs of empty bags at either end and in between, a
+    table without lookups, widths that fill the lanes of a row only partly.  Bit-exact: both sides
+    add a bag's rows in lookup order."""
+    rng = np.random.default_rng(dim + 10 * combiner + id_kind)
+    rows, batch = 211, 1300
+    cases = [np.bincount([5], minlength=batch), np.bincount([batch - 1] * 7, minlength=batch),
+             np.bincount([0] * 8 + [1299], minlength=batch), np.bincount([700] * 2000, minlength=batch),
+             np.zeros(batch, np.int64), rng.integers(0, 3, batch) * rng.integers(0, 9, batch),
+             np.full(batch, 1), np.where(np.arange(batch) % 100 == 50, 31, 0), np.full(batch, 17)]
+    tabs, ids, segs, want = [], [], [], []
+    for lens in cases:
+        n = int(lens.sum())
+        data = rng.standard_normal((rows, dim)).astype(np.float32)
+        raw = rng.integers(0, 1 << 62, n) if id_kind == 2 else rng.integers(0, rows, n)
+        row = raw % rows
+        seg = np.stack([np.repeat(np.arange(batch), lens), rng.integers(0, 9, n)], 1).astype(np.int64)
+        ref = np.zeros((batch, dim), np.float32)
+        np.add.at(ref, seg[:, 0], data[row])
+        if combiner:
+            ref *= (np.float32(1) / np.maximum(lens, 1).astype(np.float32))[:, None]
+        tabs.append(_dev(data))
+        ids.append(_dev(raw.astype(np.int32 if id_kind == 0 else np.int64)))
+        segs.append(_dev(seg.reshape(n, 2)))
+        want.append(ref)
+    slots = len(cases) + stride_slots
+    out = torch.full((batch, slots, dim), -7.0, device="cuda")
+    plan = BagPlan(tabs, ids, segs, out, stride_slots, batch, id_kind=id_kind, combiner=combiner)
+    plan.run()
+    got = out.cpu().numpy()
+    assert plan.error_bits() == 0
+    assert (got[:, :stride_slots] == -7.0).all()
+    for t, ref in enumerate(want):
+        np.testing.assert_array_equal(got[:, stride_slots + t], ref, err_msg=f"table {t}")
