@@ -1,16 +1,15 @@
 // fp32 GEMM on the CUDA cores: the route for shapes the tensor-core kernel does
 // not take (tiny or unaligned problems, transposed A, fp32-exact requests such
 // as KPFusedBatchMatMulAddSigmoid whose reference tolerance is 1e-5).
-// 64x64x16 block tile, 4x4 register tile, strided batch on blockIdx.z.
+// Register-tiled blocks with packed fp32x2 multiply-adds, strided batch on blockIdx.z.
 #include "common.h"
 #include "gemm.h"
 #include "kn4.h"
+#include "tc_ptx.cuh"
 
 namespace annc {
 namespace gemm {
 namespace {
-
-constexpr int BM = 64, BN = 64, BK = 16;
 
 __device__ __forceinline__ float apply_act(float v, int act) {
   if (act == ANNC_ACT_RELU) return fmaxf(v, 0.0f);
@@ -18,93 +17,237 @@ __device__ __forceinline__ float apply_act(float v, int act) {
   return v;
 }
 
-__global__ void __launch_bounds__(256) sgemm_simt_kernel(annc_gemm_desc d, int bias_mode,
-                                                        long long bias_s0, long long bias_s1,
-                                                        long long bias_s2) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  const long long bz = blockIdx.z;
-  const float* A = d.a + bz * d.stride_a;
-  const float* B = d.b + bz * d.stride_b;
-  float* C = d.c + bz * d.stride_c;
-  const float* Add = d.addend ? d.addend + bz * d.stride_addend : nullptr;
-  const long long m0 = (long long)blockIdx.y * BM, n0 = (long long)blockIdx.x * BN;
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;  // 16 x 16 threads, 4 x 4 outputs each
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+// Two independent fp32 multiply-adds in one instruction; each half rounds like fmaf.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
 
-  for (long long k0 = 0; k0 < d.k; k0 += BK) {
-    // A tile: BM x BK, element (i, kk) = op(A)[m0+i, k0+kk]
-    for (int e = tid; e < BM * BK; e += 256) {
-      int i, kk;
-      if (d.trans_a) {  // A stored [k, m]: consecutive threads walk m
-        i = e % BM;
-        kk = e / BM;
-      } else {  // A stored [m, k]: consecutive threads walk k
-        kk = e % BK;
-        i = e / BK;
-      }
-      const long long gm = m0 + i, gk = k0 + kk;
-      float v = 0.f;
-      if (gm < d.m && gk < d.k) v = d.trans_a ? A[gk * d.lda + gm] : A[gm * d.lda + gk];
-      As[kk][i] = v;
-    }
-    for (int e = tid; e < BN * BK; e += 256) {
-      int j, kk;
-      if (d.trans_b) {  // B stored [n, k]
-        kk = e % BK;
-        j = e / BK;
-      } else {  // B stored [k, n]
-        j = e % BN;
-        kk = e / BN;
-      }
-      const long long gn = n0 + j, gk = k0 + kk;
-      float v = 0.f;
-      if (gn < d.n && gk < d.k) {
-        if (d.b_format == ANNC_B_KN4) {
-          v = B[kn4::offset(d.k, d.n, gk, gn)];
+// Block tile BM x BN, k-steps of BK, TM x TN outputs per thread (TM as packed pairs); every output
+// is one chain of fmaf over ascending k.  Both operands sit k-major in shared memory, two stages;
+// the next k-step's global loads are in registers while this one is multiplied.  An operand whose
+// k runs along the row is transposed on its way into shared memory.  A thread's rows and columns
+// are groups of four, BM / (TM / 4) and BN / (TN / 4) apart, so that its shared-memory reads are
+// 16 bytes wide and free of conflicts.  The finished tile goes through shared memory, so that the
+// epilogue is one short loop over rows of 16-byte pieces: a small product is bound by the fetch of
+// instructions that run once, and unrolled over the accumulators the epilogue was most of the code.
+// Bound by instruction issue and, at small k, by the load latency of the first stages.  256 x
+// [50 x 128] x [128 x 256] with bias and sigmoid: 80 us with the former tile (64 x 64, 4 x 4
+// scalar multiply-adds and scalar loads per thread), 34 us now; pairs along n 41 us (twice as many
+// values to double), 8 x 8 outputs per thread 36 us and 47 us with a batched B.  1 x 2048 x 2048:
+// 228 us, 19 us with k split over a cluster.
+//   KC: the operand's k is contiguous ([m,k] A, [n,k] B), else its m / n is ([k,m], [k,n], kn4).
+//   VEC: 16-byte loads (bases and pitches allow them and no piece straddles an edge), else one
+//   float at a time.  Idx: 64-bit where n or k needs it.
+//   ranks > 1 (few tiles): the CTAs of a cluster along z share one tile and split its k range; each
+//   leaves its partial tile in shared memory and rank r adds, for the rows i with i % ranks == r, the
+//   ranks' parts in rank order (deterministic) before the epilogue.
+template <int ROWS, int BK, int THREADS, bool KC, bool VEC, typename Idx>
+struct OperandTile {
+  static constexpr int PER = ROWS * BK / 4 / THREADS;  // pieces of four elements per thread
+  static_assert(ROWS * BK / 4 % THREADS == 0, "every thread loads whole pieces");
+  float4 r[PER];
+
+  // Stage k0 of the operand into registers.  `x0` first row of the tile along m / n, `lim` its extent.
+  __device__ __forceinline__ void load(const float* __restrict__ p, long long ld, Idx x0, Idx lim, Idx k0, Idx kdim,
+                                       bool kn4_fmt) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int e = threadIdx.x + i * THREADS;
+      const Idx x = x0 + (KC ? e / (BK / 4) : (e % (ROWS / 4)) * 4);
+      const Idx k = k0 + (KC ? (e % (BK / 4)) * 4 : e / (ROWS / 4));
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (x < lim && k < kdim) {
+        const float* q = p + (KC ? x * ld + k : kn4_fmt ? kn4::offset(kdim, lim, k, x) : k * ld + x);
+        if (VEC) {  // kn4: n % 4 == 0, four aligned columns never straddle a panel
+          const float4 t = __ldg(reinterpret_cast<const float4*>(q));
+          v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
         } else {
-          v = d.trans_b ? B[gn * d.ldb + gk] : B[gk * d.ldb + gn];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (KC ? k + c < kdim : x + c < lim)
+              v[c] = __ldg(!KC && kn4_fmt ? p + kn4::offset(kdim, lim, k, x + c) : q + c);
+          }
         }
       }
-      Bs[kk][j] = v;
+      r[i] = make_float4(v[0], v[1], v[2], v[3]);
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
   }
+  // LD: floats between two k rows of the stage.
+  template <int LD>
+  __device__ __forceinline__ void store(float* __restrict__ s) const {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long gm = m0 + ty * 4 + i;
-    if (gm >= d.m) continue;
+    for (int i = 0; i < PER; ++i) {
+      const int e = threadIdx.x + i * THREADS;
+      if (KC) {
+        const int x = e / (BK / 4), k = (e % (BK / 4)) * 4;
+        s[(k + 0) * LD + x] = r[i].x;
+        s[(k + 1) * LD + x] = r[i].y;
+        s[(k + 2) * LD + x] = r[i].z;
+        s[(k + 3) * LD + x] = r[i].w;
+      } else {
+        const int k = e / (ROWS / 4), x = (e % (ROWS / 4)) * 4;
+        *reinterpret_cast<float4*>(s + k * LD + x) = r[i];
+      }
+    }
+  }
+};
+
+struct SimtArgs {
+  annc_gemm_desc d;
+  int bias_mode;  // 0: bias[n]; 1: the numpy-style broadcast strides below
+  long long bias_s0, bias_s1, bias_s2;
+  int ranks;      // CTAs of a cluster along z that share a tile
+  int vec_c;      // 16-byte stores of C are possible
+};
+
+template <int BM, int BN, int BK, int TM, int TN, bool A_KC, bool B_KC, bool VEC, typename Idx>
+__global__ void __launch_bounds__(BM * BN / (TM * TN), BM == 64 ? 4 : 8) sgemm_simt_kernel(SimtArgs args) {
+  constexpr int THREADS = BM * BN / (TM * TN);
+  constexpr int TX = BN / TN;  // threads along n
+  constexpr int LDA = BM + 4, LDB = BN + 4;
+  constexpr int RG = TM / 4, CG = TN / 4;  // groups of four rows / columns
+  constexpr int LDP = BN + 4;              // finished (or partial) tile
+  constexpr int STAGES = 2 * BK * (LDA + LDB), PART = BM * LDP;
+  __shared__ __align__(16) float smem[STAGES > PART ? STAGES : PART];
+  auto As = reinterpret_cast<float(*)[BK * LDA]>(smem);
+  auto Bs = reinterpret_cast<float(*)[BK * LDB]>(smem + 2 * BK * LDA);
+  const annc_gemm_desc& d = args.d;
+  const Idx M = (Idx)d.m, N = (Idx)d.n, K = (Idx)d.k;
+  const int ranks = args.ranks;
+  const int rank = ranks > 1 ? (int)blockIdx.z : 0;  // of the cluster (one batch then)
+  const long long bz = ranks > 1 ? 0 : blockIdx.z;
+  const Idx k_per = ranks > 1 ? (K + ranks * BK - 1) / (ranks * BK) * BK : K;
+  const Idx k_first = rank * k_per;
+  const Idx k_end = min(K, k_first + k_per);
+  const float* A = d.a + bz * d.stride_a;
+  const float* B = d.b + bz * d.stride_b;
+  const Idx m0 = (Idx)blockIdx.y * BM, n0 = (Idx)blockIdx.x * BN;
+  const bool kn4_fmt = !B_KC && d.b_format == ANNC_B_KN4;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+
+  // rows in pairs: A's pairs come out of shared memory as they are, only B's values are doubled
+  unsigned long long acc[TM / 2][TN];
+#pragma unroll
+  for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;  // two +0.0f
+
+  OperandTile<BM, BK, THREADS, A_KC, VEC, Idx> ta;
+  OperandTile<BN, BK, THREADS, B_KC, VEC, Idx> tb;
+  int cur = 0;
+#pragma unroll 1
+  for (Idx k0 = k_first - BK; k0 < k_end; k0 += BK) {  // round -1 only loads
+    const bool next = k0 + BK < k_end;
+    if (next) {
+      ta.load(A, d.lda, m0, M, k0 + BK, K, false);
+      tb.load(B, d.ldb, n0, N, k0 + BK, K, kn4_fmt);
+    }
+    if (k0 >= k_first) {
+      // k rows past the end are zero in both operands; a short last stage ends at a multiple of 4
+      const int kn = (int)min((Idx)BK, (k_end - k0 + 3) & ~(Idx)3);
+#pragma unroll 1
+      for (int k4 = 0; k4 < kn; k4 += 4) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          unsigned long long a[TM / 2];
+          float b[TN];
+#pragma unroll
+          for (int g = 0; g < RG; ++g) {
+            const ulonglong2 v =
+                *reinterpret_cast<const ulonglong2*>(&As[cur][(k4 + kk) * LDA + g * (BM / RG) + ty * 4]);
+            a[2 * g] = v.x; a[2 * g + 1] = v.y;
+          }
+#pragma unroll
+          for (int g = 0; g < CG; ++g) {
+            const float4 v = *reinterpret_cast<const float4*>(&Bs[cur][(k4 + kk) * LDB + g * (BN / CG) + tx * 4]);
+            b[4 * g] = v.x; b[4 * g + 1] = v.y; b[4 * g + 2] = v.z; b[4 * g + 3] = v.w;
+          }
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            const unsigned long long b2 = pack2(b[j], b[j]);
+#pragma unroll
+            for (int i = 0; i < TM / 2; ++i) fma2(acc[i][j], a[i], b2);
+          }
+        }
+      }
+    }
+    if (next) {
+      cur ^= 1;
+      ta.template store<LDA>(As[cur]);
+      tb.template store<LDB>(Bs[cur]);
+      __syncthreads();
+    }
+  }
+
+  __syncthreads();  // the stages become the finished tile
+#pragma unroll
+  for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+    for (int g = 0; g < CG; ++g) {
+      float lo[4], hi[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) unpack2(acc[i][4 * g + j], lo[j], hi[j]);
+      float* q = smem + ((i / 2) * (BM / RG) + ty * 4 + (i & 1) * 2) * LDP + g * (BN / CG) + tx * 4;
+      *reinterpret_cast<float4*>(q) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<float4*>(q + LDP) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    }
+  if (ranks > 1) tc::cluster_sync_all();
+  else __syncthreads();
+
+  float* C = d.c + bz * d.stride_c;
+  const float* Add = d.addend ? d.addend + bz * d.stride_addend : nullptr;
+  const float* bias = d.bias ? d.bias + bz * args.bias_s0 : nullptr;
+  const long long bs1 = args.bias_mode ? args.bias_s1 : 0, bs2 = args.bias_mode ? args.bias_s2 : 1;
+  const uint32_t part = tc::smem_u32(smem);
+#pragma unroll 1
+  for (int e = threadIdx.x; e < BM / ranks * (BN / 4); e += THREADS) {
+    const int lm = rank + ranks * (e / (BN / 4)), ln = (e % (BN / 4)) * 4;
+    const Idx gm = m0 + lm, gn = n0 + ln;
+    if (gm >= M || gn >= N) continue;
+    float v[4];
+    if (ranks > 1) {
+      v[0] = v[1] = v[2] = v[3] = 0.f;
+      for (int r = 0; r < ranks; ++r) {
+        float4 t;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
+                     : "r"(tc::mapa_u32(part + (uint32_t)((lm * LDP + ln) * sizeof(float)), (uint32_t)r))
+                     : "memory");
+        v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+      }
+    } else {
+      const float4 t = *reinterpret_cast<const float4*>(smem + lm * LDP + ln);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
+    float* c = C + gm * d.ldc + gn;
+    const float* add = Add ? Add + gm * d.ld_addend + gn : nullptr;
+    const float* bp = bias ? bias + gm * bs1 + gn * bs2 : nullptr;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const long long gn = n0 + tx * 4 + j;
-      if (gn >= d.n) continue;
-      float v = d.alpha * acc[i][j];
-      if (d.beta != 0.f) v += d.beta * C[gm * d.ldc + gn];
-      if (Add) v += Add[gm * d.ld_addend + gn];
-      if (d.bias) {
-        v += bias_mode ? d.bias[bz * bias_s0 + gm * bias_s1 + gn * bias_s2] : d.bias[gn];
-      }
-      C[gm * d.ldc + gn] = apply_act(v, d.activation);
+      if (gn + j >= N) continue;
+      v[j] = d.alpha * v[j];
+      if (d.beta != 0.f) v[j] += d.beta * c[j];
+      if (add) v[j] += add[j];
+      if (bp) v[j] += bp[j * bs2];
+      v[j] = apply_act(v[j], d.activation);
+    }
+    if (args.vec_c && gn + 3 < N) {
+      *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (gn + j < N) c[j] = v[j];
     }
   }
+  if (ranks > 1) tc::cluster_sync_all();  // nobody leaves while a peer may still read its part
 }
 
 // n == 1 with row-major A: one warp per output row (a GEMV with the GEMM epilogue).
@@ -179,6 +322,70 @@ __global__ void __launch_bounds__(128) sgemm_smallk_kernel(annc_gemm_desc d) {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+template <int BM, int BN, int BK, int TM, int TN, bool VEC, typename Idx = int>
+cudaError_t launch_tile(const SimtArgs& a, dim3 grid, cudaStream_t s) {
+  const bool ak = !a.d.trans_a, bk = a.d.trans_b != 0;
+  auto kernel = ak ? (bk ? sgemm_simt_kernel<BM, BN, BK, TM, TN, true, true, VEC, Idx>
+                         : sgemm_simt_kernel<BM, BN, BK, TM, TN, true, false, VEC, Idx>)
+                   : (bk ? sgemm_simt_kernel<BM, BN, BK, TM, TN, false, true, VEC, Idx>
+                         : sgemm_simt_kernel<BM, BN, BK, TM, TN, false, false, VEC, Idx>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(BM * BN / (TM * TN));
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = a.ranks;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.ranks > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// 64 x 64 tiles of 8 x 4 outputs per thread when they fill the SMs at least once, else 32 x 32
+// tiles of 4 x 4 (few rows or columns, small products: more blocks, less padding), with K split
+// over clusters of up to 8 CTAs while the tiles leave SMs idle and every rank keeps two k-steps.
+int launch_simt(SimtArgs& a, cudaStream_t s) {
+  const annc_gemm_desc& d = a.d;
+  const bool huge = d.n >= (1LL << 31) - 64 || d.k >= (1LL << 31) - 64;  // 64-bit indices
+  const long long big = ((d.m + 63) / 64) * ((d.n + 63) / 64) * d.batch;
+  const bool wide = big >= 148 && d.n > 32 && d.m > 32 && !huge;
+  const int bm = wide ? 64 : 32, bn = bm;
+  const long long gx = (d.n + bn - 1) / bn, gy = (d.m + bm - 1) / bm;
+  const bool many = d.batch > 1;
+  const bool vec_a = aligned16(d.a) && (d.lda & 3) == 0 && (!many || (d.stride_a & 3) == 0) &&
+                     ((d.trans_a ? d.m : d.k) & 3) == 0;
+  const bool vec_b = aligned16(d.b) && (!many || (d.stride_b & 3) == 0) && ((d.trans_b ? d.k : d.n) & 3) == 0 &&
+                     (d.b_format == ANNC_B_KN4 || (d.ldb & 3) == 0);
+  a.vec_c = aligned16(d.c) && (d.ldc & 3) == 0 && (!many || (d.stride_c & 3) == 0);
+  a.ranks = 1;
+  if (!wide && !many)
+    while (a.ranks < 8 && gx * gy * a.ranks * 2 <= 148 * 4 && d.k >= 32 * a.ranks * 4) a.ranks *= 2;
+  // blockIdx.y and .z are limited to 65535: walk tall products and long batches in slabs.
+  for (long long b0 = 0; b0 < d.batch; b0 += 65535) {
+    const long long nb = d.batch - b0 < 65535 ? d.batch - b0 : 65535;
+    for (long long y0 = 0; y0 < gy; y0 += 65535) {
+      const long long ny = gy - y0 < 65535 ? gy - y0 : 65535;
+      SimtArgs e = a;
+      e.d.batch = nb;
+      e.d.m = d.m - y0 * bm < ny * bm ? d.m - y0 * bm : ny * bm;
+      e.d.a = d.a + b0 * d.stride_a + y0 * bm * (d.trans_a ? 1 : d.lda);
+      e.d.b = d.b + b0 * d.stride_b;
+      e.d.c = d.c + b0 * d.stride_c + y0 * bm * d.ldc;
+      if (d.addend) e.d.addend = d.addend + b0 * d.stride_addend + y0 * bm * d.ld_addend;
+      if (d.bias && a.bias_mode) e.d.bias = d.bias + b0 * a.bias_s0 + y0 * bm * a.bias_s1;
+      const dim3 grid((unsigned)gx, (unsigned)ny, (unsigned)(a.ranks > 1 ? a.ranks : nb));
+      if (wide && vec_a && vec_b) ANNC_CUDA((launch_tile<64, 64, 16, 8, 4, true>(e, grid, s)));
+      else if (wide) ANNC_CUDA((launch_tile<64, 64, 16, 8, 4, false>(e, grid, s)));
+      else if (huge) ANNC_CUDA((launch_tile<32, 32, 32, 4, 4, false, long long>(e, grid, s)));
+      else if (vec_a && vec_b) ANNC_CUDA((launch_tile<32, 32, 32, 4, 4, true>(e, grid, s)));
+      else ANNC_CUDA((launch_tile<32, 32, 32, 4, 4, false>(e, grid, s)));
+    }
+  }
+  return ANNC_OK;
+}
+
 }  // namespace
 
 int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
@@ -199,23 +406,23 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
     ANNC_CUDA(cudaGetLastError());
     return ANNC_OK;
   }
-  const long long gx = (d.n + BN - 1) / BN, gy = (d.m + BM - 1) / BM;
-  if (gy > 65535) return fail(ANNC_ERR_UNSUPPORTED, "simt gemm: more than 4M rows");
-  // blockIdx.z is limited to 65535: walk the batch in slabs.
-  for (long long b0 = 0; b0 < d.batch; b0 += 65535) {
-    annc_gemm_desc e = d;
-    e.batch = d.batch - b0 < 65535 ? d.batch - b0 : 65535;
-    e.a = d.a + b0 * d.stride_a;
-    e.b = d.b + b0 * d.stride_b;
-    e.c = d.c + b0 * d.stride_c;
-    if (d.addend) e.addend = d.addend + b0 * d.stride_addend;
-    if (d.bias && bb) e.bias = d.bias + b0 * bb->s0;
-    dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)e.batch);
-    sgemm_simt_kernel<<<grid, 256, 0, s>>>(e, bb ? 1 : 0, bb ? bb->s0 : 0, bb ? bb->s1 : 0,
-                                           bb ? bb->s2 : 0);
+  if ((d.m + 63) / 64 > 65535) return fail(ANNC_ERR_UNSUPPORTED, "simt gemm: more than 4M rows");
+  SimtArgs args;
+  args.d = d;
+  args.bias_mode = bb ? 1 : 0;
+  args.bias_s0 = bb ? bb->s0 : 0;
+  args.bias_s1 = bb ? bb->s1 : 0;
+  args.bias_s2 = bb ? bb->s2 : 0;
+  // A batch whose B is shared and whose A and C slabs follow one another is one tall product: no
+  // tile is left part empty by a slab's last rows (50 of 64).
+  annc_gemm_desc& e = args.d;
+  if (e.batch > 1 && e.stride_b == 0 && !e.trans_a && e.stride_a == e.m * e.lda && e.stride_c == e.m * e.ldc &&
+      (!e.addend || e.stride_addend == e.m * e.ld_addend) &&
+      (!e.bias || !bb || (bb->s0 == 0 && bb->s1 == 0))) {
+    e.m *= e.batch;
+    e.batch = 1;
   }
-  ANNC_CUDA(cudaGetLastError());
-  return ANNC_OK;
+  return launch_simt(args, s);
 }
 
 }  // namespace gemm

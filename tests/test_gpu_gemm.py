@@ -193,3 +193,40 @@ def test_strided_batch_on_tensor_cores(shared_b, trans_b):
                        stride_b=0 if shared_b else k * n, stride_c=m * n)
     assert name in ("tcgen05_tf32", "tcgen05_pair_tf32") and not device.gemm_timed_out()
     assert nerr(c, want) <= 2e-3
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (1, 33, 512), (31, 32, 33), (33, 31, 128), (63, 260, 1000), (64, 65, 31),
+                                   (65, 64, 17), (70, 2000, 96), (1000, 1030, 20)])
+@pytest.mark.parametrize("trA,trB,kn4", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (1, 1, 0), (0, 0, 1), (1, 0, 1)])
+def test_fp32_route_tile_edges(m, n, k, trA, trB, kn4):
+    """The fp32 tiles at their edges, both loads (16-byte and one float at a time), every operand
+    order and K split over a cluster.  Bound: a chain of k rounded multiply-adds, and three more
+    roundings for alpha, beta * C and bias, is within (k + 4) ulp of the sum of magnitudes."""
+    rng = np.random.default_rng(m + 3 * n + 7 * k + trA)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    b = rng.standard_normal((k, n)).astype(np.float32)
+    c0 = rng.standard_normal((m, n)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    bd = oracle.kn4_pack(b) if kn4 else (b.T if trB else b)
+    c = _dev(c0)
+    name = device.gemm(_dev(a.T if trA else a), _dev(bd), c, m=m, n=n, k=k, trans_a=bool(trA), trans_b=bool(trB),
+                       alpha=0.5, beta=2.0, bias=_dev(bias), b_format=_lib.B_KN4 if kn4 else _lib.B_PLAIN,
+                       math=_lib.MATH_FP32)
+    assert name == "simt_fp32"
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    want = 0.5 * (a64 @ b64) + 2.0 * c0 + bias
+    size = 0.5 * (abs(a64) @ abs(b64)) + 2.0 * abs(c0) + abs(bias)
+    assert (abs(c.cpu().numpy() - want) <= (k + 4) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("bias_shape", [(1,), (24,), (1, 24), (50, 1), (50, 24), (7, 1, 1), (7, 50, 24), (1, 1, 24)])
+@pytest.mark.parametrize("batched", [False, True])
+def test_batch_matmul_add_sigmoid_bias_broadcast(bias_shape, batched):
+    """A shared right-hand side is multiplied as one tall product when the bias allows it."""
+    rng = np.random.default_rng(len(bias_shape))
+    lhs = rng.standard_normal((7, 50, 36)).astype(np.float32)
+    rhs = rng.standard_normal((7, 36, 24) if batched else (36, 24)).astype(np.float32)
+    bias = rng.standard_normal(bias_shape).astype(np.float32)
+    got = ops.kp_fused_batch_matmul_add_sigmoid(_dev(lhs), _dev(rhs), _dev(bias)).cpu().numpy()
+    want = 1 / (1 + np.exp(-(np.matmul(lhs.astype(np.float64), rhs.astype(np.float64)) + bias)))
+    np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-7)
