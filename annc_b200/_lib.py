@@ -64,6 +64,7 @@ def _load() -> C.CDLL:
     lib.annc_lookup_custom_call.argtypes = [C.c_char_p]
     lib.annc_select_gemm_target.restype = C.c_char_p
     lib.annc_gemm_kernel_name.restype = C.c_char_p
+    lib.annc_gemm_run.argtypes = [C.POINTER(GemmDesc), C.c_void_p]
     lib.annc_embed_bag_workspace_bytes.restype = C.c_size_t
     lib.annc_embed_bag_workspace_bytes.argtypes = [C.c_int, C.c_int64]
     lib.annc_kn4_offset.restype = C.c_int64

@@ -13,8 +13,15 @@ import torch
 from ._lib import (ACT_NONE, B_PLAIN, MATH_AUTO, BagTable, GemmDesc, check, lib)
 
 
+def raw_stream() -> int:
+    """Handle of torch's current stream, without the Stream object around it (0.2 us, not 3 us)."""
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(raw_stream())
 
 
 class BagPlan:
@@ -72,26 +79,24 @@ def gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, *, m: int, n: int, k
          ld_addend: Optional[int] = None, stride_addend: int = 0,
          bias: Optional[torch.Tensor] = None, activation: int = ACT_NONE,
          b_format: int = B_PLAIN, math: int = MATH_AUTO,
-         workspace: Optional[torch.Tensor] = None, io_flags: int = 0) -> str:
-    """annc_gemm_run; returns the name of the kernel family that ran."""
-    d = GemmDesc()
-    d.trans_a, d.trans_b = int(trans_a), int(trans_b)
-    d.m, d.n, d.k, d.batch = m, n, k, batch
-    d.lda = lda if lda is not None else (m if trans_a else k)
-    d.ldb = ldb if ldb is not None else (k if trans_b else n)
-    d.ldc = ldc if ldc is not None else n
-    d.ld_addend = ld_addend if ld_addend is not None else n
-    d.stride_a, d.stride_b, d.stride_c, d.stride_addend = stride_a, stride_b, stride_c, stride_addend
-    d.alpha, d.beta = alpha, beta
-    d.a, d.b, d.c = a.data_ptr(), b.data_ptr(), c.data_ptr()
-    d.addend = addend.data_ptr() if addend is not None else None
-    d.bias = bias.data_ptr() if bias is not None else None
-    d.activation, d.b_format, d.math = activation, b_format, math
-    d.io_flags = io_flags
+         workspace: Optional[torch.Tensor] = None, io_flags: int = 0,
+         stream: Optional[int] = None) -> str:
+    """annc_gemm_run on the current stream (or the one whose handle is given); returns the name of
+    the kernel family that ran."""
+    d = GemmDesc(trans_a, trans_b, m, n, k, batch,
+                 (m if trans_a else k) if lda is None else lda,
+                 (k if trans_b else n) if ldb is None else ldb,
+                 n if ldc is None else ldc, n if ld_addend is None else ld_addend,
+                 stride_a, stride_b, stride_c, stride_addend, alpha, beta,
+                 a.data_ptr(), b.data_ptr(), c.data_ptr(),
+                 None if addend is None else addend.data_ptr(), None if bias is None else bias.data_ptr(),
+                 activation, b_format, math, io_flags)
     if workspace is not None:
         d.workspace, d.workspace_bytes = workspace.data_ptr(), workspace.numel() * workspace.element_size()
     name = lib.annc_gemm_kernel_name(C.byref(d)).decode()
-    check(lib.annc_gemm_run(C.byref(d), _stream()))
+    rc = lib.annc_gemm_run(C.byref(d), raw_stream() if stream is None else stream)
+    if rc:
+        check(rc)
     return name
 
 

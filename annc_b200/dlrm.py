@@ -97,6 +97,8 @@ class DlrmPipeline:
         self._sum_done = [torch.cuda.Event() for _ in range(2)]
         self._bottom_done = [torch.cuda.Event() for _ in range(2)]
         self._begin_done = torch.cuda.Event()
+        self._forked = torch.cuda.Event()
+        self._side_done = torch.cuda.Event()
         self._pooled = torch.cuda.Event()
         self.split_finish = False  # embed() = embed_pool() + embed_finish(), the latter movable
         self._pstep = 0
@@ -164,28 +166,35 @@ class DlrmPipeline:
         return bits
 
     # ------------------------------------------------------------------ one step
-    def _sparse_part(self, names, lookahead: bool = False) -> None:
-        """Bottom MLP (second stream) beside the embedding pooling; z is complete afterwards."""
+    def _bottom_mlp(self, names) -> None:
+        """Bottom MLP, queued on the second stream."""
         B, F, D = self.batch, self.F, self.dim
+        side = self.side_stream.cuda_stream
         x = self.dense
         nb = len(self.bottom)
+        for i, (w, b) in enumerate(self.bottom):
+            last = i == nb - 1
+            y = self.z if last else self.acts_b[i]
+            names.append(dev.gemm(x, w, y, m=B, n=w.shape[1], k=w.shape[0], bias=b,
+                                  activation=ACT_RELU, ldc=(F * D if last else None),
+                                  math=self.math, stream=side))
+            x = y
+
+    def _sparse_part(self, names, lookahead: bool = False) -> None:
+        """Bottom MLP (second stream) beside the embedding pooling; z is complete afterwards."""
         main = torch.cuda.current_stream()
         self.embed_prefetch()
-        self.side_stream.wait_stream(main)  # this step's inputs, and the previous readers of z
-        with torch.cuda.stream(self.side_stream):
-            for i, (w, b) in enumerate(self.bottom):
-                last = i == nb - 1
-                y = self.z if last else self.acts_b[i]
-                names.append(dev.gemm(x, w, y, m=B, n=w.shape[1], k=w.shape[0], bias=b,
-                                      activation=ACT_RELU, ldc=(F * D if last else None),
-                                      math=self.math))
-                x = y
-            if lookahead:
+        self._forked.record(main)
+        self.side_stream.wait_event(self._forked)  # this step's inputs, and the previous readers of z
+        self._bottom_mlp(names)
+        if lookahead:
+            with torch.cuda.stream(self.side_stream):
                 # after a step issued with split=True the previous sum ran on the dense stream
                 self.side_stream.wait_event(self._sum_done[1 - self._buf])
                 self.embed_prefetch_next()
         self.embed()
-        main.wait_stream(self.side_stream)
+        self._side_done.record(self.side_stream)
+        main.wait_event(self._side_done)
 
     def _dense_part(self, names) -> None:
         """Interaction + top MLP on the current stream."""
@@ -204,7 +213,10 @@ class DlrmPipeline:
         self.launches_per_step = self.embed_launches + 1 + len(names)
 
     def forward(self) -> torch.Tensor:
-        self.sync_pipeline()
+        if self._pstep:
+            self.sync_pipeline()
+        else:  # nothing was ever queued on the dense stream
+            torch.cuda.current_stream().wait_event(self._side_done)
         self._select(0)
         names = []
         self._sparse_part(names)
@@ -223,19 +235,10 @@ class DlrmPipeline:
         main = torch.cuda.current_stream()
         main.wait_event(self._dense_done[buf])  # the step before last has finished with this set
         names = []
-        B, F, D = self.batch, self.F, self.dim
         self.embed_prefetch()                   # first step only: nothing has been split ahead
         self.side_stream.wait_stream(main)
+        self._bottom_mlp(names)
         with torch.cuda.stream(self.side_stream):
-            x = self.dense
-            nb = len(self.bottom)
-            for i, (w, b) in enumerate(self.bottom):
-                last = i == nb - 1
-                y = self.z if last else self.acts_b[i]
-                names.append(dev.gemm(x, w, y, m=B, n=w.shape[1], k=w.shape[0], bias=b,
-                                      activation=ACT_RELU, ldc=(F * D if last else None),
-                                      math=self.math))
-                x = y
             self.embed_side()                   # embedding work that needs no peer (writes z too)
             self._bottom_done[buf].record(self.side_stream)
             # the next step's split reuses the masks and lists of the step before this one

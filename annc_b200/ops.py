@@ -13,6 +13,7 @@ shape-info vector [dims..., minor_to_major...] per operand
 from __future__ import annotations
 
 import ctypes as C
+from functools import lru_cache
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -24,6 +25,8 @@ try:  # torch is plumbing for device memory only
     import torch
 except Exception:  # pragma: no cover
     torch = None
+else:
+    from . import device
 
 _NP_DTYPE = {ANNC_F32: np.float32, ANNC_I32: np.int32, ANNC_I64: np.int64, ANNC_BOOL: np.bool_,
              ANNC_U64: np.uint64}
@@ -33,13 +36,20 @@ def _is_torch(x) -> bool:
     return torch is not None and isinstance(x, torch.Tensor)
 
 
+_CODE = {np.dtype(np.float32): ANNC_F32, np.dtype(np.int32): ANNC_I32,
+         np.dtype(np.int64): ANNC_I64, np.dtype(np.bool_): ANNC_BOOL,
+         np.dtype(np.uint8): ANNC_BOOL, np.dtype(np.uint64): ANNC_U64}
+if torch is not None:
+    _CODE.update({torch.float32: ANNC_F32, torch.int32: ANNC_I32, torch.int64: ANNC_I64,
+                  torch.bool: ANNC_BOOL, torch.uint8: ANNC_BOOL, torch.uint64: ANNC_U64})
+
+
 def _code(x) -> int:
-    if _is_torch(x):
-        return {torch.float32: ANNC_F32, torch.int32: ANNC_I32, torch.int64: ANNC_I64,
-                torch.bool: ANNC_BOOL, torch.uint8: ANNC_BOOL, torch.uint64: ANNC_U64}[x.dtype]
-    return {np.dtype(np.float32): ANNC_F32, np.dtype(np.int32): ANNC_I32,
-            np.dtype(np.int64): ANNC_I64, np.dtype(np.bool_): ANNC_BOOL,
-            np.dtype(np.uint8): ANNC_BOOL, np.dtype(np.uint64): ANNC_U64}[x.dtype]
+    return _CODE[x.dtype]
+
+
+def _use_current_stream() -> None:
+    lib.annc_set_stream(device.raw_stream())
 
 
 def _ptr(x) -> int:
@@ -57,16 +67,10 @@ def _contig(x):
 
 
 def as_tensor(x, dtype_code: Optional[int] = None) -> Tensor:
-    t = Tensor()
-    t.data = _ptr(x)
-    t.dtype = _code(x) if dtype_code is None else dtype_code
     shape = tuple(x.shape)
     if len(shape) > 4:
         raise ValueError("rank > 4 not supported")
-    t.rank = len(shape)
-    for i, d in enumerate(shape):
-        t.dims[i] = int(d)
-    return t
+    return Tensor(_ptr(x), _code(x) if dtype_code is None else dtype_code, len(shape), shape)
 
 
 class _Outputs:
@@ -96,7 +100,7 @@ class _Outputs:
 
 def _outputs_for(x) -> _Outputs:
     if _is_torch(x) and x.is_cuda:
-        lib.annc_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        _use_current_stream()
         return _Outputs(True, x.device)
     return _Outputs(False)
 
@@ -187,7 +191,7 @@ def sparse_embedding2(ids, table, lo, hi, dflt):
     ids, table = _contig(ids), _contig(table)
     n = int(np.prod(ids.shape))
     if _is_torch(table) and table.is_cuda:
-        lib.annc_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        _use_current_stream()
         out = torch.empty((n, table.shape[1]), dtype=torch.float32, device=table.device)
     else:
         out = np.empty((n, table.shape[1]), np.float32)
@@ -205,16 +209,34 @@ def shape_info(x) -> np.ndarray:
     return np.array(list(x.shape) + list(range(r - 1, -1, -1)), np.int64)
 
 
+@lru_cache(maxsize=1024)
+def _info_of(shape) -> np.ndarray:
+    info = np.array(list(shape) + list(range(len(shape) - 1, -1, -1)), np.int64)
+    info.setflags(write=False)  # shared by the calls of this shape
+    return info
+
+
+def _info(x) -> np.ndarray:
+    """shape_info for a call made here: nobody else gets to see the array."""
+    return _info_of(tuple(x.shape))
+
+
+_TARGET = C.CFUNCTYPE(None, C.c_void_p, C.POINTER(C.c_void_p))
+_targets = {}  # the registered targets never change (the flags are read once)
+
+
 def _call_custom(target: str, out, operands: List):
-    fn_addr = lib.annc_lookup_custom_call(target.encode())
-    if not fn_addr:
-        raise _lib.AnncError(102, f"custom-call target {target} is not registered "
-                                  "(flag annc-pass off?)")
-    fn = C.CFUNCTYPE(None, C.c_void_p, C.POINTER(C.c_void_p))(fn_addr)
+    fn = _targets.get(target)
+    if fn is None:
+        fn_addr = lib.annc_lookup_custom_call(target.encode())
+        if not fn_addr:
+            raise _lib.AnncError(102, f"custom-call target {target} is not registered "
+                                      "(flag annc-pass off?)")
+        fn = _targets[target] = _TARGET(fn_addr)
     arr = (C.c_void_p * len(operands))(*[_ptr(o) for o in operands])
     if any(_is_torch(o) and o.is_cuda for o in operands):
-        lib.annc_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
-    fn(C.c_void_p(_ptr(out)), arr)
+        _use_current_stream()
+    fn(_ptr(out), arr)
     return out
 
 
@@ -228,7 +250,7 @@ def xla_matmul(lhs, rhs):
     """custom-call "__matmul": in = {lhs, rhs, info(lhs), info(rhs)}."""
     lhs, rhs = _contig(lhs), _contig(rhs)
     out = _new_like(lhs, (lhs.shape[0], rhs.shape[1]))
-    return _call_custom("__matmul", out, [lhs, rhs, shape_info(lhs), shape_info(rhs)])
+    return _call_custom("__matmul", out, [lhs, rhs, _info(lhs), _info(rhs)])
 
 
 def xla_layout_matmul(lhs, rhs_packed):
@@ -236,21 +258,21 @@ def xla_layout_matmul(lhs, rhs_packed):
     lhs, rhs_packed = _contig(lhs), _contig(rhs_packed)
     out = _new_like(lhs, (lhs.shape[0], rhs_packed.shape[1]))
     return _call_custom("__layout_matmul", out,
-                        [lhs, rhs_packed, shape_info(lhs), shape_info(rhs_packed)])
+                        [lhs, rhs_packed, _info(lhs), _info(rhs_packed)])
 
 
 def xla_batch_matmul(lhs, rhs):
     lhs, rhs = _contig(lhs), _contig(rhs)
     out = _new_like(lhs, (lhs.shape[0], lhs.shape[1], rhs.shape[2]))
-    return _call_custom("__batch_matmul", out, [lhs, rhs, shape_info(lhs), shape_info(rhs)])
+    return _call_custom("__batch_matmul", out, [lhs, rhs, _info(lhs), _info(rhs)])
 
 
 def xla_matmul_add(addend, lhs, rhs):
     """in = {addend, lhs, rhs, info(addend), info(lhs), info(rhs)}."""
     addend, lhs, rhs = _contig(addend), _contig(lhs), _contig(rhs)
     out = _new_like(lhs, (lhs.shape[0], rhs.shape[1]))
-    return _call_custom("__matmul_add", out, [addend, lhs, rhs, shape_info(addend),
-                                              shape_info(lhs), shape_info(rhs)])
+    return _call_custom("__matmul_add", out, [addend, lhs, rhs, _info(addend),
+                                              _info(lhs), _info(rhs)])
 
 
 def xla_matmul_add_relu(max_operand, addend, lhs, rhs):
@@ -258,8 +280,8 @@ def xla_matmul_add_relu(max_operand, addend, lhs, rhs):
     max_operand, addend, lhs, rhs = (_contig(v) for v in (max_operand, addend, lhs, rhs))
     out = _new_like(lhs, (lhs.shape[0], rhs.shape[1]))
     return _call_custom("__matmul_add_relu", out,
-                        [max_operand, addend, lhs, rhs, shape_info(max_operand),
-                         shape_info(addend), shape_info(lhs), shape_info(rhs)])
+                        [max_operand, addend, lhs, rhs, _info(max_operand),
+                         _info(addend), _info(lhs), _info(rhs)])
 
 
 def xla_pooling(arg, mul_out, slice_starts, slice_limits):
@@ -268,8 +290,8 @@ def xla_pooling(arg, mul_out, slice_starts, slice_limits):
     ss = np.ascontiguousarray(slice_starts, np.int64)
     sl = np.ascontiguousarray(slice_limits, np.int64)
     out = _new_like(mul_out, (arg.shape[0], mul_out.shape[2]))
-    return _call_custom("__pooling", out, [arg, mul_out, ss, sl, shape_info(arg),
-                                           shape_info(mul_out)])
+    return _call_custom("__pooling", out, [arg, mul_out, ss, sl, _info(arg),
+                                           _info(mul_out)])
 
 
 def xla_reduce_mean(value, m, n):
@@ -287,7 +309,7 @@ def xla_softmax(x):
     ch = x.shape[-1]
     out = _new_like(x, tuple(x.shape))
     if _is_torch(x) and x.is_cuda:
-        lib.annc_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        _use_current_stream()
     n = int(np.prod(x.shape))
     lib.__xla_cpu_runtime_XnnPackSoftMaxND(None, C.c_void_p(_ptr(x)), C.c_void_p(_ptr(out)),
                                            C.c_int64(n // ch), C.c_int64(ch))
