@@ -38,13 +38,18 @@ static thread_local int t_stream_ctas_per_sm = 0;
 // Lookups per chunk of the lookup-granular kernel.  A group pays about 16 lookups' worth of time
 // to start a chunk and to follow its last bag past the end; the chunk that makes
 // rounds x (chunk + 16) smallest therefore spreads few lookups over all groups (one tile each)
-// and cuts a large batch so that its last round is nearly full.  Measured: one table with 2,700
-// lookups 90 us with chunks of 128 (one block), 15 us with chunks of 8; 4.47 M lookups of dim 64
-// 206 us, capped at chunks of 64 229 us, of 32 249 us.
+// and cuts a batch of a few rounds so that the last one is nearly full.  One table with 2,700
+// lookups: 90 us with chunks of 128 (one block), 15 us with chunks of 8.  Where the tables are
+// long enough that chunks of 128 in flight stay within four of them, longer ones would spread
+// over more tables and their rows no longer share L2: 17.9 M lookups of dim 64 over 26 tables
+// of 144 K rows 608 us with chunks up to 128, 645 us up to 256, 701 us up to 512, 659 us up to
+// 64.  With short tables the limit only costs: 64 tables x 50 K lookups of dim 128 199 us against
+// 183 us.
 static int stream_chunk(long long lookups, int num_tables, int lanes, long long groups) {
+  const int limit = groups * 128 <= 4 * (lookups / num_tables) ? 128 : 64 * lanes;
   int best = lanes;
   long long best_cost = -1;
-  for (int tiles = 1; tiles <= 64; ++tiles) {
+  for (int tiles = 1; tiles * lanes <= limit; ++tiles) {
     const long long chunk = (long long)tiles * lanes;
     const long long chunks = lookups / chunk + num_tables / 2 + 1;
     const long long rounds = (chunks + groups - 1) / groups;
@@ -94,6 +99,11 @@ template <int LANES, int VPL, int DEPTH, int MINB>
 static void launch_stream_dim(const BagParams& p, BagHeader* hdr, cudaStream_t s) {
   if (p.dim == LANES * VPL * 4) launch_stream<LANES, VPL, DEPTH, true, MINB>(p, hdr, s);
   else launch_stream<LANES, VPL, DEPTH, false, MINB>(p, hdr, s);
+}
+
+// Between two groups of tables of one call: the marks and the chunk counter start again.
+static cudaError_t reset_marks(BagHeader* hdr, cudaStream_t s) {
+  return cudaMemsetAsync(&hdr->next_chunks, 0, sizeof(int) + sizeof(hdr->unsorted), s);
 }
 
 // Atomic route for tables whose segment ids were not sorted; returns at once for sorted tables.
@@ -295,7 +305,7 @@ int annc_embed_bags_dev(const annc_bag_table* tables, int num_tables, int64_t di
   ANNC_CUDA(cudaMemsetAsync(hdr, 0, kHeaderBytes, s));
   for (int t0 = 0; t0 < num_tables; t0 += kMaxTables) {
     const int nt = std::min(kMaxTables, num_tables - t0);
-    if (t0 > 0) ANNC_CUDA(cudaMemsetAsync(hdr->unsorted, 0, sizeof(hdr->unsorted), s));
+    if (t0 > 0) ANNC_CUDA(reset_marks(hdr, s));
     ANNC_TRY(run_bags(tables + t0, nt, dim, id_kind, ncols, col, combiner, batch, out_stride, hdr,
                       offsets + (size_t)t0 * (size_t)(batch + 1), s));
   }
@@ -325,7 +335,7 @@ static int bags_sharded(const annc_bag_table* tables, int num_tables, int64_t di
   ANNC_CUDA(cudaMemsetAsync(hdr, 0, kHeaderBytes, s));
   for (int t0 = 0; t0 < num_tables; t0 += kMaxTables) {
     const int nt = std::min(kMaxTables, num_tables - t0);
-    if (t0 > 0) ANNC_CUDA(cudaMemsetAsync(hdr->unsorted, 0, sizeof(hdr->unsorted), s));
+    if (t0 > 0) ANNC_CUDA(reset_marks(hdr, s));
     ANNC_TRY(run_bags(tables + t0, nt, dim, id_kind, ncols, col, combiner, batch, out_stride, hdr,
                       offsets + (size_t)t0 * (size_t)(batch + 1), s, shard_count, shard_rank,
                       skip_empty));
@@ -490,7 +500,7 @@ int annc_embed_bags_static_dev(const annc_bag_table* tables, int num_tables, int
   ANNC_CUDA(cudaMemsetAsync(hdr, 0, kHeaderBytes, s));
   for (int t0 = 0; t0 < num_tables; t0 += kMaxTables) {
     const int nt = std::min(kMaxTables, num_tables - t0);
-    if (t0 > 0) ANNC_CUDA(cudaMemsetAsync(hdr->unsorted, 0, sizeof(hdr->unsorted), s));
+    if (t0 > 0) ANNC_CUDA(reset_marks(hdr, s));
     ANNC_TRY(run_bags(tables + t0, nt, dim, id_kind, ncols, col, combiner, batch, out_stride, hdr,
                       offsets + (size_t)t0 * (size_t)(batch + 1), s));
   }
