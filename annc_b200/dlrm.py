@@ -33,6 +33,8 @@ from .synth import DlrmModel
 
 
 class DlrmPipeline:
+    embed_first = True  # forward() queues the pooling kernel before the bottom MLP
+
     def __init__(self, model: DlrmModel, device: torch.device, math: int = MATH_AUTO,
                  keep_host_inputs: bool = False):
         self.device = device
@@ -166,10 +168,9 @@ class DlrmPipeline:
         return bits
 
     # ------------------------------------------------------------------ one step
-    def _bottom_mlp(self, names) -> None:
-        """Bottom MLP, queued on the second stream."""
+    def _bottom_mlp(self, names, stream: int) -> None:
+        """Bottom MLP, queued on the stream with this handle."""
         B, F, D = self.batch, self.F, self.dim
-        side = self.side_stream.cuda_stream
         x = self.dense
         nb = len(self.bottom)
         for i, (w, b) in enumerate(self.bottom):
@@ -177,7 +178,7 @@ class DlrmPipeline:
             y = self.z if last else self.acts_b[i]
             names.append(dev.gemm(x, w, y, m=B, n=w.shape[1], k=w.shape[0], bias=b,
                                   activation=ACT_RELU, ldc=(F * D if last else None),
-                                  math=self.math, stream=side))
+                                  math=self.math, stream=stream))
             x = y
 
     def _sparse_part(self, names, lookahead: bool = False) -> None:
@@ -186,13 +187,20 @@ class DlrmPipeline:
         self.embed_prefetch()
         self._forked.record(main)
         self.side_stream.wait_event(self._forked)  # this step's inputs, and the previous readers of z
-        self._bottom_mlp(names)
+        # The pooling kernel goes out first: queued behind a layer of the MLP that still holds the
+        # SMs it starts with a quarter of its blocks, and the next layer, waiting for whole SMs,
+        # keeps the others out (batch 65536: 1.4 ms instead of 0.6 ms whenever the host is slow).
+        first = self.embed_first and not lookahead
+        if first:
+            self.embed()
+        self._bottom_mlp(names, self.side_stream.cuda_stream)
         if lookahead:
             with torch.cuda.stream(self.side_stream):
                 # after a step issued with split=True the previous sum ran on the dense stream
                 self.side_stream.wait_event(self._sum_done[1 - self._buf])
                 self.embed_prefetch_next()
-        self.embed()
+        if not first:
+            self.embed()
         self._side_done.record(self.side_stream)
         main.wait_event(self._side_done)
 
@@ -237,7 +245,7 @@ class DlrmPipeline:
         names = []
         self.embed_prefetch()                   # first step only: nothing has been split ahead
         self.side_stream.wait_stream(main)
-        self._bottom_mlp(names)
+        self._bottom_mlp(names, self.side_stream.cuda_stream)
         with torch.cuda.stream(self.side_stream):
             self.embed_side()                   # embedding work that needs no peer (writes z too)
             self._bottom_done[buf].record(self.side_stream)

@@ -357,6 +357,8 @@ def _make_pipeline(model, device, mode: str, math=None, keep_host_inputs: bool =
     world, rank = dist.get_world_size(), dist.get_rank()
 
     class _Pipe(DlrmPipeline):
+        embed_first = False  # the exchange waits for its peers: the bottom MLP runs in that time
+
         def _setup_embedding(self, m) -> None:
             emb = m.emb
             T, B, D = self.T, self.batch, self.dim
