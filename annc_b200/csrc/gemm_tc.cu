@@ -117,6 +117,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const bool b_n_major = p.b_mode != B_TMA_NK;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&tmap_a);
+    prefetch_tensormap(&tmap_b);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1 + (b_by_loader ? LOADER_THREADS : 0));
       mbar_init(bar_empty + 8 * s, 1);
@@ -298,26 +300,27 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tc_fence_after();
     if (done) {
       // Phase 1: this warp's 32 x 128 accumulator slab, scaled by alpha, goes to shared
-      // memory (the stage ring is idle once `done` has fired), rows padded to 132 floats.
+      // memory (the stage ring is idle once `done` has fired), rows padded to 132 floats; two
+      // tensor-memory loads in flight.
       float* slab = reinterpret_cast<float*>(gen_base) + (size_t)q * 32 * LD;
+      const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        uint32_t r[32];
+      for (int c0 = 0; c0 < BN; c0 += 64) {
+        uint32_t r[2][32];
         if (KT > 0) {
-          tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+          tmem_ld32(trow + (uint32_t)c0, r[0]);
+          tmem_ld32(trow + (uint32_t)c0 + 32u, r[1]);
           tmem_ld_wait();
         } else {  // a split-K rank without k-steps contributes zeros
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = 0u;
+          for (int j = 0; j < 64; ++j) r[j >> 5][j & 31] = 0u;
         }
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          float4 v;
-          v.x = p.alpha * __uint_as_float(r[j]);
-          v.y = p.alpha * __uint_as_float(r[j + 1]);
-          v.z = p.alpha * __uint_as_float(r[j + 2]);
-          v.w = p.alpha * __uint_as_float(r[j + 3]);
-          *reinterpret_cast<float4*>(slab + lane * LD + c0 + j) = v;
+        for (int j = 0; j < 64; j += 4) {
+          const uint32_t* rj = &r[j >> 5][j & 31];
+          *reinterpret_cast<float4*>(slab + lane * LD + c0 + j) =
+              make_float4(p.alpha * __uint_as_float(rj[0]), p.alpha * __uint_as_float(rj[1]),
+                          p.alpha * __uint_as_float(rj[2]), p.alpha * __uint_as_float(rj[3]));
         }
       }
       __syncwarp();
@@ -334,74 +337,98 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (done) {
       const float* slab = reinterpret_cast<const float*>(gen_base) + (size_t)q * 32 * LD;
       const uint32_t slab_s = base + (uint32_t)((size_t)q * 32 * LD * sizeof(float));
-      // Phase 2: one output row per step, the 32 lanes cover its 128 columns with
+      // Phase 2: one output row per instruction, the 32 lanes cover its 128 columns with
       // 16-byte accesses, so C, the addend and the bias are read and written coalesced.
       // Under split K rank c takes the rows rr with rr % split == c and adds the ranks'
-      // partial rows in rank order.
-      const bool vec = ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
-      const bool add_vec = p.addend && ((p.ld_addend & 3) == 0) &&
-                           ((reinterpret_cast<uintptr_t>(p.addend) & 15) == 0);
+      // partial rows in rank order.  Two rows go together: their reads of C, the addend and
+      // the partial tiles are all out before the first is used.  One row at a time, behind
+      // ordered volatile loads, paid the memory latency for every row: 512 x 1024 x 1024 with an
+      // addend 12.7 us against 11.1 us, 1024^3 17.0 / 14.6, 2000 x 500 x 400 13.5 / 11.1 (four
+      // rows: 11.7, 14.3, 11.0, but 200 x 256 x 512 8.9 against 7.6).
+      constexpr int RB = 2;
       const int col = n0 + lane * 4;
-      float bias4[4] = {0.f, 0.f, 0.f, 0.f};
-      if (p.bias) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (col + e < p.N) bias4[e] = __ldg(p.bias + col + e);
-      }
-      const int rows_here = min(32, p.M - (m0 + q * 32));
+      const bool vec = col + 3 < p.N && ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+      const bool add_vec = col + 3 < p.N && p.addend && ((p.ld_addend & 3) == 0) &&
+                           ((reinterpret_cast<uintptr_t>(p.addend) & 15) == 0);
+      // four columns of a row, those past the edge read as zero
+      auto load4 = [&](const float* q4, bool wide) {
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (wide) return *reinterpret_cast<const float4*>(q4);
+        if (col < p.N) t.x = q4[0];
+        if (col + 1 < p.N) t.y = q4[1];
+        if (col + 2 < p.N) t.z = q4[2];
+        if (col + 3 < p.N) t.w = q4[3];
+        return t;
+      };
+      float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.bias) bias4 = load4(p.bias + col, false);
+      const int rows_here = col < p.N ? min(32, p.M - (m0 + q * 32)) : 0;
       const int rstep = p.split > 1 ? p.split : 1;
-      for (int rr = crank; rr < rows_here; rr += rstep) {
-        if (col >= p.N) break;
-        const long long grow = (long long)(m0 + q * 32 + rr);
-        float v[4];
-        if (p.split > 1) {
-          v[0] = v[1] = v[2] = v[3] = 0.f;
-          const uint32_t off = slab_s + (uint32_t)((rr * LD + lane * 4) * sizeof(float));
-          for (int r = 0; r < p.split; ++r) {
-            float4 a4;
-            const uint32_t ra = mapa_u32(off, (uint32_t)r);
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(a4.x), "=f"(a4.y), "=f"(a4.z), "=f"(a4.w)
-                         : "r"(ra)
-                         : "memory");
-            v[0] += a4.x; v[1] += a4.y; v[2] += a4.z; v[3] += a4.w;
+      const long long row0 = m0 + q * 32;
+      const bool reads_rows = p.beta != 0.f || p.addend;
+#pragma unroll 1
+      for (int rr0 = crank; rr0 < rows_here; rr0 += rstep * RB) {
+        float4 v[RB], old[RB], add[RB];
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+          const int rr = rr0 + i * rstep;
+          if (reads_rows && rr < rows_here) {
+            if (p.beta != 0.f) old[i] = load4(p.C + zb * p.stride_c + (row0 + rr) * p.ldc + col, vec);
+            if (p.addend) add[i] = load4(p.addend + zb * p.stride_addend + (row0 + rr) * p.ld_addend + col, add_vec);
           }
-        } else {
-          const float4 a4 = *reinterpret_cast<const float4*>(slab + rr * LD + lane * 4);
-          v[0] = a4.x; v[1] = a4.y; v[2] = a4.z; v[3] = a4.w;
         }
-        float* crow = p.C + zb * p.stride_c + grow * p.ldc + col;
-        const float* arow =
-            p.addend ? p.addend + zb * p.stride_addend + grow * p.ld_addend + col : nullptr;
-        if (vec && col + 3 < p.N) {
-          if (p.beta != 0.f) {
-            const float4 o = *reinterpret_cast<const float4*>(crow);
-            v[0] += p.beta * o.x; v[1] += p.beta * o.y; v[2] += p.beta * o.z; v[3] += p.beta * o.w;
-          }
-          if (arow) {
-            if (add_vec) {
-              const float4 a = __ldg(reinterpret_cast<const float4*>(arow));
-              v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-            } else {
+        if (p.split > 1) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) v[e] += __ldg(arow + e);
+          for (int i = 0; i < RB; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int r = 0; r < p.split; r += 2) {  // (split is even) four partial pieces in flight
+            float4 t[2][RB];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t peer = mapa_u32(slab_s, (uint32_t)(r + h));
+#pragma unroll
+              for (int i = 0; i < RB; ++i) {
+                const int rr = min(rr0 + i * rstep, 31);
+                // volatile keeps it behind the cluster barrier; no memory clobber, so that the
+                // loads are issued back to back
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(t[h][i].x), "=f"(t[h][i].y), "=f"(t[h][i].z), "=f"(t[h][i].w)
+                             : "r"(peer + (uint32_t)((rr * LD + lane * 4) * sizeof(float))));
+              }
             }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int i = 0; i < RB; ++i) {
+                v[i].x += t[h][i].x; v[i].y += t[h][i].y; v[i].z += t[h][i].z; v[i].w += t[h][i].w;
+              }
           }
-          float4 o;
-          o.x = act_apply(v[0] + bias4[0], p.act);
-          o.y = act_apply(v[1] + bias4[1], p.act);
-          o.z = act_apply(v[2] + bias4[2], p.act);
-          o.w = act_apply(v[3] + bias4[3], p.act);
-          *reinterpret_cast<float4*>(crow) = o;
         } else {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (col + e < p.N) {
-              float x = v[e];
-              if (p.beta != 0.f) x += p.beta * crow[e];
-              if (arow) x += __ldg(arow + e);
-              crow[e] = act_apply(x + bias4[e], p.act);
-            }
+          for (int i = 0; i < RB; ++i)
+            v[i] = *reinterpret_cast<const float4*>(slab + min(rr0 + i, 31) * LD + lane * 4);
+        }
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+          const int rr = rr0 + i * rstep;
+          if (rr >= rows_here) break;
+          float* crow = p.C + zb * p.stride_c + (row0 + rr) * p.ldc + col;
+          float o[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+          if (p.beta != 0.f) {
+            o[0] += p.beta * old[i].x; o[1] += p.beta * old[i].y; o[2] += p.beta * old[i].z; o[3] += p.beta * old[i].w;
+          }
+          if (p.addend) {
+            o[0] += add[i].x; o[1] += add[i].y; o[2] += add[i].z; o[3] += add[i].w;
+          }
+          o[0] = act_apply(o[0] + bias4.x, p.act);
+          o[1] = act_apply(o[1] + bias4.y, p.act);
+          o[2] = act_apply(o[2] + bias4.z, p.act);
+          o[3] = act_apply(o[3] + bias4.w, p.act);
+          if (vec) {
+            *reinterpret_cast<float4*>(crow) = make_float4(o[0], o[1], o[2], o[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (col + e < p.N) crow[e] = o[e];
           }
         }
       }
