@@ -26,18 +26,21 @@ static int validate(const annc_gemm_desc& d) {
   return ANNC_OK;
 }
 
-// The CTA-pair kernel works on 256 x 256 tiles with a long main loop per tile: it takes the
-// compute-bound GEMMs.  Skinny layers (small K, output-bound) stay on the single-CTA kernel,
-// whose two resident CTAs per SM and staged, coalesced epilogue stream C faster.
+// Pair kernel (256 x 256 tiles per two SMs, persistent) or single-CTA kernel (128 x 128 tiles, two
+// per SM or split K inside a cluster).  With its TMA-store epilogue the pair kernel wins from
+// about 32 tiles on, measured in us pair / single: 65536 x 512 x 416 61 / 111, 4096 x 512 x 416 (32
+// tiles) 13.6 / 14.4, 2048 x 1000 x 500 (32) 15.2 / 15.7, 64 x [256 x 256 x 64] 9.4 / 11.5; 1024^3 (16)
+// 21 / 15.  A narrow C pays for 256 columns of multiplications: from n = 64 on that still hides
+// under the memory traffic when K is short and the rows fill every pair (65536 x 64 x 256 24 / 28).
+// Its general epilogue (beta * C, addend) is slow per tile and needs a long main loop to hide in.
 static bool use_pair(const annc_gemm_desc& d, int math) {
   if (!pair_supported(d, math)) return false;
   if (math == ANNC_MATH_BF16 || (d.io_flags & (ANNC_IO_SOFTMAX | ANNC_IO_PAIR))) return true;
   if (!tc_supported(d, math)) return true;
-  // 256 x 256 pair tiles pay off when there are enough of them to occupy the SM pairs; a
-  // smaller product runs on the single-CTA kernel (128 x 128 tiles, split K inside a cluster
-  // when even those are few).
   const long long pair_tiles = ((d.m + 255) / 256) * ((d.n + 255) / 256) * d.batch;
-  return d.m >= 256 && d.n >= 192 && d.k >= 1024 && pair_tiles >= 74;
+  if (d.m >= 256 && d.n >= 192 && d.k >= 1024 && pair_tiles >= 74) return true;
+  if (!pair_stores_by_tma(d)) return false;
+  return (d.n >= 192 && d.m >= 192 && pair_tiles >= 32) || (d.n >= 64 && d.k <= 512 && pair_tiles >= 148);
 }
 
 // AUTO: tensor cores (TF32) when the shape fits a tcgen05 kernel, else CUDA cores.

@@ -14,11 +14,12 @@
 //   warp 1   allocates tensor memory for the pair; in the leader one thread issues the MMAs
 //            (UMMA 256 x 256 x {8,16}), commits to the "empty" barrier of both CTAs and, after
 //            the last k-step of a tile, to the "accumulator full" barrier of both CTAs
-//   warps 2-9  epilogue, two warps per 32 accumulator rows (128 columns each): tcgen05.ld of a
-//            32 x 32 chunk (the next chunk's load already in flight), transpose through a
-//            swizzled shared-memory tile, then scale / addend / bias / activation and stores
-//            in whole 128-byte lines; or a thread-per-row softmax.  Each warp then releases
-//            the accumulator to the leader
+//   warps 2-9  epilogue, two warps per 32 accumulator rows (128 columns each), in one of three
+//            forms, picked by the launch (Epilogue below): scale / bias / activation in
+//            registers and a TMA store of every 32-row chunk; the general form with beta * C and
+//            addend, transposed through a swizzled shared-memory tile for accesses in whole
+//            128-byte lines; a thread-per-row softmax.  Each warp then releases the
+//            accumulator to the leader
 //
 // The kernel is persistent (one pair per two SMs, tiles taken round robin) and the accumulator
 // is double-buffered in the 512 tensor-memory columns, so the epilogue of tile i runs under
@@ -55,7 +56,9 @@ constexpr int P_THREADS = 320;      // producer, MMA issuer, eight epilogue warp
 constexpr int P_TMEM_COLS = 512;
 constexpr int P_EPI_WARPS = 8;                       // two per TMEM lane quadrant, 128 columns each
 constexpr int P_STG_BYTES = P_EPI_WARPS * 32 * 32 * 4;  // one swizzled 32 x 32 chunk per epilogue warp
-constexpr size_t P_SMEM = 1024 + (size_t)P_STAGES * P_STAGE + 256 + P_STG_BYTES;
+constexpr size_t P_SMEM = 1024 + (size_t)P_STAGES * P_STAGE + P_STG_BYTES + 256;
+
+enum Epilogue { EPI_GENERAL = 0, EPI_SOFTMAX = 1, EPI_TMA_STORE = 2 };
 
 struct PairParams {
   int M, N, K;
@@ -256,21 +259,24 @@ __device__ __forceinline__ void stage_row(float* stg, int lane, const uint32_t (
 }
 
 // DT 0: TF32 (fp32 elements, 32 per 128-byte k-step, UMMA K = 8); DT 1: BF16 (64, K = 16).
-template <int DT, bool SOFTMAX>
+template <int DT, int EPI>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                         const __grid_constant__ CUtensorMap tmap_b, PairParams p) {
+                         const __grid_constant__ CUtensorMap tmap_b,
+                         const __grid_constant__ CUtensorMap tmap_c /* EPI_TMA_STORE */, PairParams p) {
+  constexpr bool SOFTMAX = EPI == EPI_SOFTMAX;
   constexpr int KELTS = DT == 0 ? 32 : 64;  // elements per 128-byte k-step row
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - raw);
-  const uint32_t bars = base + P_STAGES * P_STAGE;
+  // stages, staging tiles (1024-byte aligned, as the swizzle of a TMA store wants), barriers
+  const uint32_t bars = base + P_STAGES * P_STAGE + P_STG_BYTES;
   const uint32_t bar_full = bars, bar_empty = bars + 8 * P_STAGES;
   const uint32_t bar_tfull = bars + 16 * P_STAGES, bar_tempty = bar_tfull + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + P_STAGES * P_STAGE + 16 * P_STAGES + 32);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + P_STAGES * P_STAGE + P_STG_BYTES + 16 * P_STAGES + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* staging = reinterpret_cast<float*>(gen_base + P_STAGES * P_STAGE + 256);
+  float* staging = reinterpret_cast<float*>(gen_base + P_STAGES * P_STAGE);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -279,6 +285,9 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int KT = (p.K + KELTS - 1) / KELTS;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&tmap_a);
+    prefetch_tensormap(&tmap_b);
+    if (EPI == EPI_TMA_STORE) prefetch_tensormap(&tmap_c);
     for (int s = 0; s < P_STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1);   // the leader's expect_tx arrival; bytes come from both CTAs
       mbar_init(bar_empty + 8 * s, 1);  // one commit
@@ -406,7 +415,90 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (!ok) break;
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * (uint32_t)PN;
-        if (!SOFTMAX) {
+        if (EPI == EPI_TMA_STORE) {
+          // Values finished in registers (a lane holds 32 or 64 columns of its row), one 4 KB
+          // staging tile per warp, one TMA store per chunk; the next chunk is read from tensor
+          // memory meanwhile.  The general form below spends about 800 instructions a chunk on
+          // addresses, edges and the transposition, with two warps per scheduler to hide them:
+          // it bounded every product with K below 1024 (65536 x 512 x 416: 121 us, 17 us a tile
+          // of which the MMAs are 5).
+          uint32_t ra[32];
+          const uint32_t tcol = taddr + (uint32_t)(half * WCOLS);
+          const uint32_t stg_s = smem_u32(stg);
+          float* const bias_f = &bias_w.x;
+          auto finish = [&](const uint32_t (&r)[32], float (&v)[32], int first_lane) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              v[j] = p.alpha * __uint_as_float(r[j]) + __shfl_sync(0xffffffffu, bias_f[j & 3], first_lane + (j >> 2));
+            if (p.act == ANNC_ACT_RELU) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+            } else if (p.act == ANNC_ACT_SIGMOID) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = act_apply(v[j], ANNC_ACT_SIGMOID);
+            }
+          };
+          auto send = [&](int c0) {  // staging tile -> C
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+              if (row0 < p.M) {
+                if (p.batched) tma_store_3d(&tmap_c, c0, (int)row0, (int)bz, stg_s);
+                else tma_store_2d(&tmap_c, c0, (int)row0, stg_s);
+              }
+              bulk_commit();
+            }
+          };
+          auto staging_free = [&]() {
+            if (lane == 0) bulk_wait_read<0>();
+            __syncwarp();
+          };
+          if (nb < p.N) tmem_ld32(tcol, ra);
+          if (!p.c_bf16) {
+#pragma unroll 1
+            for (int i = 0; i < WCOLS / 32; ++i) {
+              const int c0 = nb + 32 * i;
+              if (c0 >= p.N) break;  // warp-uniform
+              float v[32];
+              tmem_ld_wait();
+              finish(ra, v, 8 * i);
+              if (i + 1 < WCOLS / 32 && c0 + 32 < p.N) tmem_ld32(tcol + 32u * (i + 1), ra);
+              staging_free();
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<float4*>(stg_at(stg, lane, j)) =
+                    make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+              send(c0);
+            }
+          } else {
+#pragma unroll 1
+            for (int i = 0; i < WCOLS / 64; ++i) {
+              const int c0 = nb + 64 * i;
+              if (c0 >= p.N) break;
+              uint32_t w[32];  // 64 bf16 columns: one 128-byte row of the staging tile
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                float v[32];
+                tmem_ld_wait();
+                finish(ra, v, 16 * i + 8 * h);
+                // (columns past N hold zeros and are clipped by the store)
+                if (h == 0 || i + 1 < WCOLS / 64) tmem_ld32(tcol + 64u * i + 32u * (h + 1), ra);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                  w[16 * h + j] = *reinterpret_cast<uint32_t*>(&b2);
+                }
+              }
+              staging_free();
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<uint4*>(stg_at(stg, lane, j)) =
+                    make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+              send(c0);
+            }
+            tmem_ld_wait();
+          }
+        } else if (!SOFTMAX) {
           // chunk i + 1 is read from tensor memory (into the registers staging has just
           // freed) while chunk i goes from the staging tile to global memory
           uint32_t ra[32];
@@ -472,6 +564,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_u32(bar_tempty + 8 * acc, 0));
       }
+      if (EPI == EPI_TMA_STORE && lane == 0) bulk_wait_all();  // the stores read this CTA's shared memory
     }
   }
   tc_fence_before();
@@ -533,19 +626,34 @@ bool pair_supported(const annc_gemm_desc& d, int math) {
   return true;
 }
 
+// The TMA store takes every C whose rows are 16-byte aligned and whole 16-byte pieces long (it clips
+// at the tensor's edge in such pieces), without beta * C and addend.
+bool pair_stores_by_tma(const annc_gemm_desc& d) {
+  const int per16 = (d.io_flags & ANNC_IO_C_BF16) ? 8 : 4;
+  return !(d.io_flags & ANNC_IO_SOFTMAX) && d.beta == 0.f && !d.addend && al16(d.c) && d.ldc >= d.n &&
+         d.n % per16 == 0 && d.ldc % per16 == 0 && (d.batch == 1 || (d.stride_c % per16 == 0 && d.stride_c > 0));
+}
+
 int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   if (!pair_supported(d, math)) return fail(ANNC_ERR_UNSUPPORTED, "tcgen05 pair gemm: unsupported shape");
   const bool bf16 = math == ANNC_MATH_BF16;
   static int max_pairs_dev[kMaxDevices][2] = {};
   int (&max_pairs)[2] = max_pairs_dev[device_slot()];
   const bool softmax = (d.io_flags & ANNC_IO_SOFTMAX) != 0;
-  auto kern = bf16 ? (softmax ? gemm_pair_tcgen05_kernel<1, true> : gemm_pair_tcgen05_kernel<1, false>)
-                   : (softmax ? gemm_pair_tcgen05_kernel<0, true> : gemm_pair_tcgen05_kernel<0, false>);
-  static bool attr_done_dev[kMaxDevices][2][2] = {};
-  bool (&attr_done)[2][2] = attr_done_dev[device_slot()];
-  if (!attr_done[bf16][softmax]) {
+  const bool c_bf16 = (d.io_flags & ANNC_IO_C_BF16) != 0;
+  const bool tma_store = pair_stores_by_tma(d);
+  const int epi = softmax ? EPI_SOFTMAX : tma_store ? EPI_TMA_STORE : EPI_GENERAL;
+  auto kern = bf16 ? (softmax     ? gemm_pair_tcgen05_kernel<1, EPI_SOFTMAX>
+                      : tma_store ? gemm_pair_tcgen05_kernel<1, EPI_TMA_STORE>
+                                  : gemm_pair_tcgen05_kernel<1, EPI_GENERAL>)
+                   : (softmax     ? gemm_pair_tcgen05_kernel<0, EPI_SOFTMAX>
+                      : tma_store ? gemm_pair_tcgen05_kernel<0, EPI_TMA_STORE>
+                                  : gemm_pair_tcgen05_kernel<0, EPI_GENERAL>);
+  static bool attr_done_dev[kMaxDevices][2][3] = {};
+  bool (&attr_done)[2][3] = attr_done_dev[device_slot()];
+  if (!attr_done[bf16][epi]) {
     ANNC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM));
-    attr_done[bf16][softmax] = true;
+    attr_done[bf16][epi] = true;
   }
   if (max_pairs[bf16] == 0) {
     ANNC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM));
@@ -568,7 +676,7 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   }
   const int kelts = bf16 ? 64 : 32;
   const bool batched = d.batch > 1, b_batched = batched && d.stride_b > 0;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, tc;
   ANNC_TRY(make_map_any(&ta, d.a, bf16, batched ? d.batch : 1, d.m, d.k, d.lda, d.stride_a, kelts, PM, false));
   PairParams p;
   memset(&p, 0, sizeof(p));
@@ -579,6 +687,10 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
     p.b_n_major = 1;
     ANNC_TRY(make_map_any(&tb, d.b, false, b_batched ? d.batch : 1, d.k, d.n, d.ldb, d.stride_b, 32, 32, true));
   }
+  if (tma_store)
+    ANNC_TRY(make_map_any(&tc, d.c, c_bf16, batched ? d.batch : 1, d.m, d.n, d.ldc, d.stride_c, c_bf16 ? 64 : 32, 32,
+                          false));
+  else tc = ta;
   p.M = (int)d.m;
   p.N = (int)d.n;
   p.K = (int)d.k;
@@ -591,7 +703,7 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   p.beta = d.beta;
   p.act = d.activation;
   p.softmax = (d.io_flags & ANNC_IO_SOFTMAX) ? 1 : 0;
-  p.c_bf16 = (d.io_flags & ANNC_IO_C_BF16) ? 1 : 0;
+  p.c_bf16 = c_bf16 ? 1 : 0;
   p.batched = batched;
   p.b_batched = b_batched;
   p.stride_c = batched ? d.stride_c : 0;
@@ -615,7 +727,7 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ANNC_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
+  ANNC_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p));
   return ANNC_OK;
 }
 

@@ -127,3 +127,32 @@ def test_pair_batch_matmul_softmax(n):
     assert np.abs(probs.cpu().numpy() - own).max() <= 1e-6
     ref = oracle.softmax(np.matmul(q, kt).reshape(-1, n)).reshape(bsz, m, n)
     assert np.abs(probs.cpu().numpy() - ref).max() <= 2e-3
+
+
+@pytest.mark.parametrize("m,n,k,ldc,batch", [(1, 8, 32, 8, 1), (31, 40, 64, 48, 1), (257, 64, 256, 1728, 1),
+                                             (300, 200, 64, 200, 3), (129, 255, 96, 260, 1), (513, 600, 36, 601, 1),
+                                             (1500, 264, 512, 264, 1)])
+@pytest.mark.parametrize("dt", ["tf32", "bf16", "bf16_out"])
+@pytest.mark.parametrize("act", [ACT_NONE, ACT_RELU])
+def test_pair_store_edges(m, n, k, ldc, batch, dt, act):
+    """Epilogue with TMA stores at the edges of its 32-row chunks, with padded rows that must stay
+    untouched and, where a row is not made of whole 16-byte pieces, its general form.  Against fp64: products
+    of operands cut to 11 (TF32) or rounded to 8 bits, hence 2e-3 / 1e-2 of the largest value."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn((batch, m, k), device="cuda", generator=g)
+    b = torch.randn((batch, n, k), device="cuda", generator=g)
+    bias = torch.randn(n, device="cuda", generator=g)
+    io, math = IO_PAIR, MATH_TF32
+    if dt != "tf32":
+        if k % 8:
+            pytest.skip("bf16 rows of 16 bytes")
+        a, b = a.bfloat16(), b.bfloat16()
+        io, math = IO_A_BF16 | IO_B_BF16 | (IO_C_BF16 if dt == "bf16_out" else 0), MATH_BF16
+    c = torch.full((batch, m, ldc), -7.0, device="cuda", dtype=torch.bfloat16 if dt == "bf16_out" else torch.float32)
+    device.gemm(a, b, c, m=m, n=n, k=k, batch=batch, trans_b=True, ldc=ldc, stride_a=m * k, stride_b=n * k,
+                stride_c=m * ldc, alpha=0.5, bias=bias, activation=act, math=math, io_flags=io)
+    assert not device.gemm_timed_out()
+    want = 0.5 * (a.double() @ b.double().transpose(1, 2)) + bias
+    want = want.relu() if act == ACT_RELU else want
+    assert nerr(c[:, :, :n], want.float().cpu().numpy()) <= (2e-3 if dt == "tf32" else 1e-2)
+    assert (c[:, :, n:] == -7.0).all()
