@@ -451,6 +451,32 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 // ---------------------------------------------------------------- host side
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// Clusters of `size` CTAs of the six-stage kernel (one CTA per SM) that the device holds at once.
+int max_clusters(int size) {
+  static int known[kMaxDevices][4] = {};
+  int& n = known[device_slot()][size == 2 ? 1 : size == 4 ? 2 : 3];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)size;
+    cfg.gridDim = dim3(1, 1, (unsigned)size);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = smem_bytes(6);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int got = 0;
+    if (cudaOccupancyMaxActiveClusters(&got, gemm_tf32_tcgen05_kernel<6>, &cfg) != cudaSuccess || got < 1) {
+      cudaGetLastError();
+      got = 148 / size / 2;
+    }
+    n = got;
+  }
+  return n;
+}
+
 }  // namespace
 
 bool tc_supported(const annc_gemm_desc& d, int math) {
@@ -520,9 +546,11 @@ int run_tc(const annc_gemm_desc& d, int math, cudaStream_t s) {
   // Few tiles and a long K: a cluster of 2, 4 or 8 CTAs shares each tile and splits its K range,
   // so that a 512 x 1024 x 1024 product occupies 128 SMs instead of 32.
   const int kt_all = (int)((d.k + BK - 1) / BK);
+  // All clusters have to be resident at once: one more round costs more than the split gives
+  // (192 x 1024 x 1024, 16 tiles: 14.5 us in clusters of 8, of which 15 fit, 10.0 us in clusters of 4; 128 x 2304 x 1024 16.5 / 10.1).
   int split = 1;
   if (d.batch == 1 && ctas * 2 <= 148 && kt_all >= 8) {
-    while (split < 8 && ctas * split * 2 <= 148 && kt_all / (split * 2) >= 2) split *= 2;
+    while (split < 8 && ctas <= max_clusters(split * 2) && kt_all / (split * 2) >= 2) split *= 2;
   }
   p.split = split;
   if (split > 1) {
