@@ -343,11 +343,22 @@ size_t dtype_size(int32_t dtype) {
   }
 }
 
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {  // legacy stream beside a capture
+    cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 Call::Call() : stream_(g_stream), device_(device_slot()) {
   g_arenas.per_device[device_].reset();
   // A previous call of this thread that returned without synchronising (device pointers only)
   // may still use the arena's scratch on another stream: order this call's stream after it.
-  if (g_unsynced[device_] && g_last_event[device_] && g_last_stream[device_] != stream_)
+  // (A call being captured takes no scratch without a wait of its own, and may not depend on work
+  // outside the capture.)
+  if (g_unsynced[device_] && g_last_event[device_] && g_last_stream[device_] != stream_ && !capturing(stream_))
     cudaStreamWaitEvent(stream_, g_last_event[device_], 0);
 }
 Call::~Call() {
@@ -490,6 +501,16 @@ void* Call::scratch(size_t bytes) {
   void* d = g_arenas.per_device[device_].alloc(bytes);
   if (!d) status_ = fail(ANNC_ERR_CUDA, "device scratch allocation of %zu bytes failed", bytes);
   used_scratch_ = true;
+  return d;
+}
+
+void* Call::optional_scratch(size_t bytes) {
+  if (status_ != ANNC_OK || bytes > kMaxOptionalScratch || capturing(stream_)) return nullptr;
+  size_t cap = size_t(1) << 20;
+  while (cap < bytes) cap <<= 1;
+  void* d = g_arenas.per_device[device_].alloc(cap);
+  if (!d) cudaGetLastError();
+  else used_scratch_ = true;
   return d;
 }
 

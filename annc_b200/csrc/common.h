@@ -91,6 +91,12 @@ class Call {
   }
   // Device scratch valid until the next call of this thread on this device.
   void* scratch(size_t bytes);
+  // The same for a large buffer the call can do without: nullptr (and no error) when the stream is
+  // being captured (a replay would use the arena behind the back of later calls), beyond
+  // kMaxOptionalScratch or without memory.  Sizes are rounded to powers of two, so that the arena
+  // holds at most twice the limit of them however the sizes vary.
+  static constexpr size_t kMaxOptionalScratch = size_t(256) << 20;
+  void* optional_scratch(size_t bytes);
   // A re-laid form (`tag`) of host operand p whose mirror is reusable: the cached buffer, or a
   // new one of out_bytes with *fresh set (the caller fills it).  nullptr when p has no reusable
   // mirror (device pointer, cache off) or memory is short: the caller then works without it.

@@ -230,3 +230,38 @@ def test_batch_matmul_add_sigmoid_bias_broadcast(bias_shape, batched):
     got = ops.kp_fused_batch_matmul_add_sigmoid(_dev(lhs), _dev(rhs), _dev(bias)).cpu().numpy()
     want = 1 / (1 + np.exp(-(np.matmul(lhs.astype(np.float64), rhs.astype(np.float64)) + bias)))
     np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 16, 32), (200, 140, 352), (300, 264, 353), (130, 4100, 100), (70, 260, 1061),
+                                   (2100, 1000, 704)])
+def test_layout_matmul_device_weight(m, n, k):
+    """A packed weight on the device is re-laid into scratch by each call (K chunks of 352 and the two
+    that share the rest, panels of 12 and 4 columns, tiles of 128 x 32)."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn((m, k), device="cuda", generator=g)
+    w = torch.randn((k, n), device="cuda", generator=g)
+    got = ops.xla_layout_matmul(a, device.kn4_pack(w))
+    want = (a.double() @ w.double()).cpu().numpy()
+    assert nerr(got, want) <= 2e-3  # TF32
+
+
+def test_layout_matmul_device_weight_streams_and_capture():
+    """The scratch is safe across streams of a thread, and a captured call does without it."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a = torch.randn((256, 512), device="cuda", generator=g)
+    packed = [device.kn4_pack(torch.randn((512, 768), device="cuda", generator=g)) for _ in range(2)]
+    want = [ops.xla_layout_matmul(a, p) for p in packed]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = []
+    for i in range(40):
+        with torch.cuda.stream(streams[i % 2]):
+            outs.append(ops.xla_layout_matmul(a, packed[i % 2]))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = ops.xla_layout_matmul(a, packed[0])
+    graph.replay()
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        assert torch.equal(o, want[i % 2])
+    assert nerr(captured, want[0].cpu().numpy()) <= 1e-5  # the same products, summed in another tiling
