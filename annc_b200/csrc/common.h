@@ -103,6 +103,8 @@ class Call {
   void* derived(const void* p, size_t bytes, int tag, size_t out_bytes, bool* fresh);
   // Small host read of possibly-device memory (synchronous).
   int read_host(const void* p, size_t bytes, void* dst);
+  // Waits for the call's stream (an operator whose outputs are complete when it returns).
+  int wait();
   // True when p is device (or managed) memory.
   bool is_device(const void* p);
   // True when the call waited for its stream (then device-side error words can be read).

@@ -115,11 +115,12 @@ static int run_unsorted_route(const BagParams& p, long long max_nnz, BagHeader* 
   return ANNC_OK;
 }
 
-// Launches the bag kernels (+ the atomic route) for up to kMaxTables tables.
+// Launches the bag kernels (+ the atomic route, unless the caller knows the segment ids to be
+// sorted) for up to kMaxTables tables.
 static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, int id_kind,
                     int64_t ncols, int32_t col, int combiner, int64_t batch, int64_t out_stride,
                     BagHeader* hdr, int* offsets, cudaStream_t s, int shard_count = 1,
-                    int shard_rank = 0, int skip_empty = 0) {
+                    int shard_rank = 0, int skip_empty = 0, bool known_sorted = false) {
   BagParams p;
   memset(&p, 0, sizeof(p));
   p.shard_count = shard_count;
@@ -185,6 +186,10 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
     else if (vecs <= 64) launch_stream_dim<32, 2, 2, 4>(p, hdr, s);
     else launch_stream_dim<32, 4, 2, 3>(p, hdr, s);
     if (ev1) cudaEventRecord(ev1, s);
+    if (known_sorted) {
+      ANNC_CUDA(cudaGetLastError());
+      return ANNC_OK;
+    }
     // Programmatic launches: 1.5 us each behind the bag kernel on sorted tables; as plain launches
     // of a block per (table, slice) they cost 4.5 us (26 tables) to 8 us (64 tables) each.
     ANNC_CUDA(launch_pdl(bag_stream_reset_kernel, dim3(148 * 4), dim3(256), 0, s, p, hdr, offsets));
@@ -212,6 +217,10 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
     }
   }
   if (ev1) cudaEventRecord(ev1, s);
+  if (known_sorted) {
+    ANNC_CUDA(cudaGetLastError());
+    return ANNC_OK;
+  }
   return run_unsorted_route(p, max_nnz, hdr, offsets, s);
 }
 
@@ -231,39 +240,42 @@ static size_t scan_scratch_ints(long long n) {
 
 // First-appearance unique of column `col` of src[n, ncols] (device).  Produces the
 // number of unique keys (host), and optionally the unique keys, the int32 inverse
-// map and an int64 copy of it.
+// map and an int64 copy of it; with rows >= 0 also whether every key is below it.
 struct UniqueResult {
   long long count = 0;
+  int err_bits = 0;
 };
 
 static int unique_first_appearance(Call& call, const int64_t* src, long long n, long long ncols,
                                    int col, long long* out_unique /*[n] or null*/,
-                                   int* inverse32, long long* inverse64, UniqueResult* res) {
+                                   int* inverse32, long long* inverse64, UniqueResult* res,
+                                   long long rows = -1) {
   cudaStream_t s = call.stream();
+  if (n <= 0) return call.status();
   long long cap = 16;
   while (cap < 2 * n + 2) cap <<= 1;
   auto* keys = static_cast<long long*>(call.scratch((cap + 1) * sizeof(long long)));
   auto* first = static_cast<int*>(call.scratch((cap + 1) * sizeof(int)));
-  auto* slot_of = static_cast<int*>(call.scratch(std::max<long long>(n, 1) * sizeof(int)));
-  auto* flag = static_cast<int*>(call.scratch(std::max<long long>(n, 1) * sizeof(int)));
-  auto* rank = static_cast<int*>(call.scratch(std::max<long long>(n, 1) * sizeof(int)));
+  auto* slot_of = static_cast<int*>(call.scratch(n * sizeof(int)));
   auto* tiles = static_cast<int*>(call.scratch(scan_scratch_ints(n) * sizeof(int)));
-  auto* total = static_cast<int*>(call.scratch(sizeof(int)));
+  auto* total_err = static_cast<int*>(call.scratch(3 * sizeof(int)));  // count, error bits, (scan total)
   if (call.status() != ANNC_OK) return call.status();
-  unique_init_kernel<<<grid_for(cap + 1, 256), 256, 0, s>>>(keys, first, cap);
-  if (n > 0) {
-    const int g = grid_for(n, 256);
-    unique_insert_kernel<<<g, 256, 0, s>>>(src, n, ncols, col, keys, first, cap, slot_of);
-    unique_flag_kernel<<<g, 256, 0, s>>>(slot_of, first, n, flag);
-    exclusive_scan(flag, n, rank, tiles, total, s);
-    unique_emit_kernel<<<g, 256, 0, s>>>(src, n, ncols, col, slot_of, flag, rank, first, out_unique);
-    unique_inverse_kernel<<<g, 256, 0, s>>>(slot_of, first, n, inverse32, inverse64);
-    int h = 0;
-    ANNC_TRY(call.read_host(total, sizeof(int), &h));
-    res->count = h;
-  } else {
-    res->count = 0;
-  }
+  unique_init_kernel<<<grid_for(cap + 1, 256), 256, 0, s>>>(keys, first, cap, total_err);
+  const int g = grid_for(n, 256);
+  unique_insert_kernel<<<g, 256, 0, s>>>(src, n, ncols, col, keys, first, cap, slot_of, rows, total_err + 1);
+  const long long ntiles = (n + kScanTile - 1) / kScanTile;
+  unique_count_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(slot_of, first, n, tiles);
+  // every block adds up the tiles before it: up to 2048 tiles (4 M keys) that is at most four loads
+  // a thread, cheaper than a pass of its own
+  const int scanned = ntiles > 2048;
+  if (scanned) scan_tile_offsets_kernel<<<1, kScanThreads, 0, s>>>(tiles, ntiles, total_err + 2);
+  unique_emit_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(src, n, ncols, col, slot_of, first, tiles, scanned,
+                                                               out_unique, total_err);
+  unique_inverse_kernel<<<g, 256, 0, s>>>(slot_of, first, n, inverse32, inverse64);
+  int h[2] = {0, 0};
+  ANNC_TRY(call.read_host(total_err, sizeof(h), h));
+  res->count = h[0];
+  res->err_bits = h[1];
   return ANNC_OK;
 }
 
@@ -539,15 +551,21 @@ int annc_KPFusedSparseSegmentReduce(const annc_tensor* data, const annc_tensor* 
   const float* d_data = call.in_constant((const float*)data->data, (size_t)numel(*data));
   const void* d_idx = call.in(indices->data, (size_t)nnz * dtype_size(indices->dtype));
   const int64_t* d_seg = call.in((const int64_t*)slice_input->data, (size_t)(nnz * ncols));
-  auto* d_max = static_cast<long long*>(call.scratch(sizeof(long long)));
+  // the scan's result and the bag header side by side: one memset starts both
+  char* ctrl = static_cast<char*>(call.scratch(kHeaderBytes + sizeof(SegScan)));
   if (call.status() != ANNC_OK) return call.status();
+  auto* hdr = reinterpret_cast<BagHeader*>(ctrl);
+  auto* d_scan = reinterpret_cast<SegScan*>(ctrl + kHeaderBytes);
 
   // batch = max segment id + 1 (max starts at 0), needed on the host to size output 0.
-  ANNC_CUDA(cudaMemsetAsync(d_max, 0, sizeof(long long), s));
-  if (nnz > 0) seg_max_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(d_seg, nnz, ncols, col, d_max);
-  long long max_seg = 0;
-  ANNC_TRY(call.read_host(d_max, sizeof(long long), &max_seg));
-  const int64_t batch = max_seg + 1;
+  const int id_kind = indices->dtype == ANNC_I64 ? 1 : 0;
+  ANNC_CUDA(cudaMemsetAsync(ctrl, 0, kHeaderBytes + sizeof(SegScan), s));
+  if (nnz > 0)
+    seg_scan_kernel<<<grid_for(nnz, 256, 148 * 4), 256, 0, s>>>(d_seg, d_idx, id_kind, nnz, ncols, col, data->dims[0],
+                                                                d_scan);
+  SegScan scan;
+  ANNC_TRY(call.read_host(d_scan, sizeof(scan), &scan));
+  const int64_t batch = scan.max_seg + 1;
 
   const int64_t dims0[2] = {batch, dim};
   float* out0 = static_cast<float*>(alloc(ctx, 0, ANNC_F32, 2, dims0));
@@ -566,23 +584,20 @@ int annc_KPFusedSparseSegmentReduce(const annc_tensor* data, const annc_tensor* 
   tb.nnz = nnz;
   tb.out = d_out;
   tb.offsets = nullptr;
-  auto* hdr = static_cast<BagHeader*>(ws);
-  ANNC_CUDA(cudaMemsetAsync(hdr, 0, kHeaderBytes, s));
-  ANNC_TRY(run_bags(&tb, 1, dim, indices->dtype == ANNC_I64 ? 1 : 0, ncols, col, combiner, batch,
-                    dim, hdr, reinterpret_cast<int*>(static_cast<char*>(ws) + kHeaderBytes), s));
+  ANNC_TRY(run_bags(&tb, 1, dim, id_kind, ncols, col, combiner, batch, dim, hdr,
+                    reinterpret_cast<int*>(static_cast<char*>(ws) + kHeaderBytes), s, 1, 0, 0, !scan.unsorted));
   // Second output: begin_1[0] == 0 ? batch : embedding size (reference :81-83).
   const int32_t slice_out = (b1 == 0) ? (int32_t)batch : (int32_t)dim;
   if (call.is_device(out1)) {
-    ANNC_CUDA(cudaMemcpyAsync(out1, &slice_out, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    ANNC_CUDA(cudaStreamSynchronize(s));
+    store_i32_kernel<<<1, 1, 0, s>>>(out1, slice_out);
+    ANNC_CUDA(cudaGetLastError());
   } else {
     *out1 = slice_out;
   }
-  int bits = 0;
-  ANNC_TRY(check_err_word(call, &hdr->err_bits, &bits));
+  ANNC_TRY(call.wait());
   ANNC_TRY(call.finish());
-  if (bits & kErrRow) return fail(ANNC_ERR_INVALID_ARGUMENT, "indices out of range of input rows");
-  if (bits & kErrSegment) return fail(ANNC_ERR_INVALID_ARGUMENT, "segment ids must be >= 0");
+  if (scan.err_bits & kErrRow) return fail(ANNC_ERR_INVALID_ARGUMENT, "indices out of range of input rows");
+  if (scan.err_bits & kErrSegment) return fail(ANNC_ERR_INVALID_ARGUMENT, "segment ids must be >= 0");
   return ANNC_OK;
 }
 
@@ -715,11 +730,9 @@ int annc_KPFusedGather(const annc_tensor* data, const annc_tensor* keys, const a
   const int64_t* d_keys = call.in((const int64_t*)keys->data, (size_t)(nnz * ncols));
   int32_t* d_inv = nnz > 0 ? call.out(out_inv, (size_t)nnz) : nullptr;
   auto* d_unique = static_cast<long long*>(call.scratch(std::max<int64_t>(nnz, 1) * sizeof(long long)));
-  auto* d_err = static_cast<int*>(call.scratch(sizeof(int)));
   if (call.status() != ANNC_OK) return call.status();
-  ANNC_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), s));
   UniqueResult ur;
-  ANNC_TRY(unique_first_appearance(call, d_keys, nnz, ncols, col, d_unique, d_inv, nullptr, &ur));
+  ANNC_TRY(unique_first_appearance(call, d_keys, nnz, ncols, col, d_unique, d_inv, nullptr, &ur, data->dims[0]));
   const int64_t nu = ur.count;
 
   const int64_t u_dims[1] = {nu};
@@ -728,20 +741,23 @@ int annc_KPFusedGather(const annc_tensor* data, const annc_tensor* keys, const a
   float* out_rows = static_cast<float*>(alloc(ctx, 2, ANNC_F32, 2, d_dims));
   ANNC_REQUIRE((out_unique && out_rows) || nu == 0, ANNC_ERR_INTERNAL, "output allocation failed");
   if (nu > 0) {
-    if (call.is_device(out_unique)) {
-      ANNC_CUDA(cudaMemcpyAsync(out_unique, d_unique, nu * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
-    } else {
+    const bool keys_on_device = call.is_device(out_unique);
+    if (!keys_on_device)
       ANNC_CUDA(cudaMemcpyAsync(out_unique, d_unique, nu * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    }
     float* d_rows = call.out(out_rows, (size_t)(nu * dim));
     if (call.status() != ANNC_OK) return call.status();
-    unique_rows_kernel<<<grid_for(nu, 8), 256, 0, s>>>(d_data, data->dims[0], dim, d_unique, nu,
-                                                       d_rows, d_err);
+    const int vec = dim % 4 == 0 && aligned16(d_data) && aligned16(d_rows);
+    const long long pieces = vec ? dim / 4 : dim;
+    long long* d_keys_out = keys_on_device ? (long long*)out_unique : nullptr;
+    auto rows_kernel = pieces <= 4 ? unique_rows_kernel<4> : pieces <= 8 ? unique_rows_kernel<8>
+                     : pieces <= 16 ? unique_rows_kernel<16> : unique_rows_kernel<32>;
+    const int lanes = pieces <= 4 ? 4 : pieces <= 8 ? 8 : pieces <= 16 ? 16 : 32;
+    rows_kernel<<<grid_for(nu, 4 * 256 / lanes), 256, 0, s>>>(d_data, data->dims[0], (int)dim, vec, d_unique, nu,
+                                                              d_rows, d_keys_out);
   }
-  int bits = 0;
-  ANNC_TRY(check_err_word(call, d_err, &bits));
+  ANNC_TRY(call.wait());
   ANNC_TRY(call.finish());
-  if (bits & kErrRow) return fail(ANNC_ERR_INTERNAL, "idx out of table range");
+  if (ur.err_bits & kErrRow) return fail(ANNC_ERR_INTERNAL, "idx out of table range");
   return ANNC_OK;
 }
 

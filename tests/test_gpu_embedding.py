@@ -396,3 +396,39 @@ def test_bag_plan_tile_and_chunk_edges(dim, stride_slots, combiner, id_kind):
     assert (got[:, :stride_slots] == -7.0).all()
     for t, ref in enumerate(want):
         np.testing.assert_array_equal(got[:, stride_slots + t], ref, err_msg=f"table {t}")
+
+
+@pytest.mark.parametrize("n,distinct,dim", [(1, 1, 4), (2047, 3, 5), (2048, 2048, 8), (2049, 700, 20), (10_000, 1, 64),
+                                            (70_001, 30_000, 16), (4_300_000, 9_000, 1)])
+def test_gather_unique_tiles(n, distinct, dim):
+    """Unique keys in first-appearance order at the edges of the counting tiles, with one key that
+    holds most positions, and beyond the size where the tiles are summed in a pass of their own."""
+    rng = np.random.default_rng(n)
+    rows = distinct + 5
+    pool = rng.permutation(rows)[:distinct]
+    keys = np.where(rng.random(n) < 0.5, pool[0], pool[rng.integers(0, distinct, n)])
+    keys[rng.permutation(n)[:min(n, distinct)]] = pool[:min(n, distinct)]
+    data = rng.standard_normal((rows, dim)).astype(np.float32)
+    col = np.stack([np.arange(n), keys], 1).astype(np.int64)
+    uniq, inv, got = ops.kp_fused_gather(_dev(data), _dev(col), np.array([0, 1], np.int32))
+    u, first, idx = np.unique(keys, return_index=True, return_inverse=True)
+    order = np.argsort(first, kind="stable")
+    rank = np.empty(len(u), np.int64)
+    rank[order] = np.arange(len(u))
+    np.testing.assert_array_equal(uniq.cpu().numpy(), u[order])
+    np.testing.assert_array_equal(inv.cpu().numpy(), rank[idx])
+    np.testing.assert_array_equal(got.cpu().numpy(), data[u[order]])
+
+
+@pytest.mark.parametrize("bad", [-1, 50])
+def test_gather_and_reduce_report_rows_outside_the_table(bad):
+    data = _dev(np.ones((50, 8), np.float32))
+    keys = np.stack([np.zeros(300, np.int64), np.arange(300) % 50], 1)
+    keys[299, 1] = bad
+    with pytest.raises(AnncError) as e:
+        ops.kp_fused_gather(data, _dev(keys), np.array([0, 1], np.int32))
+    assert "idx out of table range" in e.value.message
+    with pytest.raises(AnncError) as e:
+        ops.kp_fused_sparse_segment_reduce(data, _dev(keys[:, 1].copy()), _dev(np.sort(keys.clip(0), axis=0)),
+                                           np.zeros(2, np.int32), np.zeros(1, np.int32), 0)
+    assert "indices out of range" in e.value.message
