@@ -77,10 +77,11 @@ __device__ int g_gemm_error = 0;  // 1: an mbarrier wait ran out
 
 using namespace annc::tc;
 
-__device__ __forceinline__ float act_apply(float v, int act) {
-  if (act == ANNC_ACT_RELU) return fmaxf(v, 0.0f);
-  if (act == ANNC_ACT_SIGMOID) return __fdiv_rn(1.0f, 1.0f + expf(-v));
-  return v;
+// Four sigmoids, out of line: they would fill the instruction cache of an epilogue that hardly ever
+// takes them.
+__device__ __noinline__ float4 sigmoid4(float4 v) {
+  return make_float4(__fdiv_rn(1.0f, 1.0f + expf(-v.x)), __fdiv_rn(1.0f, 1.0f + expf(-v.y)),
+                     __fdiv_rn(1.0f, 1.0f + expf(-v.z)), __fdiv_rn(1.0f, 1.0f + expf(-v.w)));
 }
 
 // ---------------------------------------------------------------- kernel
@@ -419,10 +420,14 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (p.addend) {
             o[0] += add[i].x; o[1] += add[i].y; o[2] += add[i].z; o[3] += add[i].w;
           }
-          o[0] = act_apply(o[0] + bias4.x, p.act);
-          o[1] = act_apply(o[1] + bias4.y, p.act);
-          o[2] = act_apply(o[2] + bias4.z, p.act);
-          o[3] = act_apply(o[3] + bias4.w, p.act);
+          o[0] += bias4.x; o[1] += bias4.y; o[2] += bias4.z; o[3] += bias4.w;
+          if (p.act == ANNC_ACT_RELU) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = fmaxf(o[e], 0.0f);
+          } else if (p.act == ANNC_ACT_SIGMOID) {
+            const float4 t = sigmoid4(make_float4(o[0], o[1], o[2], o[3]));
+            o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
+          }
           if (vec) {
             *reinterpret_cast<float4*>(crow) = make_float4(o[0], o[1], o[2], o[3]);
           } else {

@@ -196,7 +196,8 @@ def test_strided_batch_on_tensor_cores(shared_b, trans_b):
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (1, 33, 512), (31, 32, 33), (33, 31, 128), (63, 260, 1000), (64, 65, 31),
-                                   (65, 64, 17), (70, 2000, 96), (1000, 1030, 20)])
+                                   (65, 64, 17), (70, 2000, 96), (1000, 1030, 20), (65, 64, 16), (130, 516, 13),
+                                   (64, 4, 1), (1001, 8, 8)])
 @pytest.mark.parametrize("trA,trB,kn4", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (1, 1, 0), (0, 0, 1), (1, 0, 1)])
 def test_fp32_route_tile_edges(m, n, k, trA, trB, kn4):
     """The fp32 tiles at their edges, both loads (16-byte and one float at a time), every operand
