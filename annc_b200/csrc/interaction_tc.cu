@@ -9,14 +9,17 @@
 // Rows R..127 of a stage are never written; whatever they hold only reaches accumulator
 // rows and columns that are not read.
 //
-// Persistent CTAs (one per SM): warp 0 TMA producer over a 2-stage ring, warp 1 MMA
+// Persistent CTAs (one per SM): warp 0 TMA producer over a 5-stage ring, warp 1 MMA
 // issuer with two TMEM accumulators in ping-pong, warps 2-9 two epilogue groups of four
-// warps, group g taking the tiles that use accumulator g: tcgen05.ld of the needed column
-// chunks into the group's padded shared-memory copy of the accumulator, then the group's four
-// warps together write the tile's output rows contiguously (row 0 of every sample comes
-// from global memory unrounded, the products are TF32 x TF32 with fp32 sums).  The epilogue
-// is the longest stage of a tile, so two of them run side by side.
-// The kernel is bound by HBM (F*64*4 bytes read and (64 + F(F-1)/2)*4 written per sample).
+// warps, group g taking the tiles that use accumulator g.  A lane holds one accumulator row, of
+// which the columns below the diagonal of its sample's block are one run of the output row: it
+// drops them there in a shared-memory image of the tile's output (row offsets are triangular
+// numbers, 32 in a row of which differ modulo 32: no bank conflicts), and one bulk copy sends the
+// image off while the next tile is worked on.  Row 0 of every sample comes from global memory
+// unrounded; the products are TF32 x TF32 with fp32 sums.
+// Bound by HBM (F*64*4 bytes read and (64 + F(F-1)/2)*4 written per sample).  65536 x 27: 86 us (85 at the copy rate); 140 us
+// with two stages and an epilogue that went through a copy of the whole accumulator and wrote
+// the output one float per thread, a division's worth of index work each.
 // All mbarrier waits are bounded (tc_ptx.cuh).
 #include <cstring>
 
@@ -30,15 +33,15 @@ namespace {
 using namespace annc::tc;
 
 constexpr int ID = 64;              // embedding dim
-constexpr int I_STAGES = 2;
+constexpr int I_STAGES = 5;
 constexpr int I_BOX = 128 * 128;    // bytes reserved per 32-float half (128 rows x 128 B)
 constexpr int I_STAGE = 2 * I_BOX;
-constexpr int I_LD = 132;           // padded accumulator row in shared memory (floats)
 constexpr int I_THREADS = 320;     // producer, MMA issuer, two epilogue groups of 128
 // Row-0 floats each epilogue thread carries per tile: samples_per_tile * 64 / 128, rounded up
 // to the template instance (2 covers F >= 26, the DLRM case; 32 covers F = 2).
-constexpr int I_DSM = 128 * I_LD * 4;  // one group's accumulator copy
-constexpr size_t I_SMEM = 1024 + (size_t)I_STAGES * I_STAGE + 2 * I_DSM + 1024 + 256;
+// Output image of a tile: spt rows of 64 + F(F-1)/2 floats rounded up to four; largest for F = 2.
+constexpr int I_IMG = 64 * 68 * 4;
+constexpr size_t I_SMEM = 1024 + (size_t)I_STAGES * I_STAGE + 2 * I_IMG + 256;
 
 __device__ int g_inter_error = 0;
 
@@ -47,6 +50,8 @@ struct InterParams {
   float* out;
   long long batch, out_stride;
   int F, spt, rows, tri;
+  int img_row;  // floats per row of the output image: 64 + tri, rounded up to four
+  int bulk;     // the output rows are 16-byte aligned: bulk copies
   long long tiles;
 };
 
@@ -64,14 +69,12 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - raw);
-  float* dsm_all = reinterpret_cast<float*>(gen + I_STAGES * I_STAGE);
-  uint8_t* pair_i = gen + I_STAGES * I_STAGE + 2 * I_DSM;
-  uint8_t* pair_j = pair_i + 512;
-  const uint32_t bars = base + I_STAGES * I_STAGE + 2 * I_DSM + 1024;
+  float* img_all = reinterpret_cast<float*>(gen + I_STAGES * I_STAGE);
+  const uint32_t bars = base + I_STAGES * I_STAGE + 2 * I_IMG;
   const uint32_t bar_full = bars, bar_empty = bars + 8 * I_STAGES;
   const uint32_t bar_tfull = bars + 16 * I_STAGES, bar_tempty = bar_tfull + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + I_STAGES * I_STAGE + 2 * I_DSM +
-                                                    1024 + 16 * I_STAGES + 32);
+  uint32_t* tmem_slot =
+      reinterpret_cast<uint32_t*>(gen + I_STAGES * I_STAGE + 2 * I_IMG + 16 * I_STAGES + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* epi_fail_all = reinterpret_cast<volatile int*>(tmem_slot + 2);  // one word per group
 
@@ -79,6 +82,7 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&tmap);
     for (int s = 0; s < I_STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
@@ -92,11 +96,11 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
     epi_fail_all[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int e = threadIdx.x; e < p.tri; e += I_THREADS) {  // pair e -> (i, j), j < i, row-major
-    int i = 1, rem = e;
-    while (rem >= i) { rem -= i; ++i; }
-    pair_i[e] = (uint8_t)i;
-    pair_j[e] = (uint8_t)rem;
+  // padding inside the image rows: zero for good
+  const int img_pad = p.img_row - ID - p.tri;
+  for (int e = threadIdx.x; e < 2 * p.spt * img_pad; e += I_THREADS) {
+    const int row = e / img_pad, g = row / p.spt;
+    img_all[g * (I_IMG / 4) + (row - g * p.spt) * p.img_row + ID + p.tri + (e - row * img_pad)] = 0.f;
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -146,7 +150,7 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
   } else {
     const int group = (warp - 2) >> 2;                // accumulator and tiles of this group
     const int q = warp & 3, te = (threadIdx.x - 64) & 127;
-    float* dsm = dsm_all + group * (I_DSM / 4);
+    float* img = img_all + group * (I_IMG / 4);
     volatile int* epi_fail = epi_fail_all + group;
     const int row_lo = 32 * q;
     // columns this warp's rows need: the diagonal blocks of the samples they belong to
@@ -156,67 +160,81 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
       c_lo = (row_lo / p.F) * p.F;
       c_hi = (row_hi / p.F + 1) * p.F;
     }
+    // this lane's accumulator row: feature fi of sample fs; it keeps the columns first .. first + fi - 1
+    const int row = row_lo + lane;
+    const int fs = row / p.F, first = fs * p.F, fi = row < p.rows ? row - first : 0;
+    float* const my_img = img + fs * p.img_row + ID + fi * (fi - 1) / 2;
     long long li = group;
     for (long long t = blockIdx.x + (long long)group * gridDim.x; t < p.tiles;
          t += 2LL * gridDim.x, li += 2) {
       const int buf = group;
       const uint32_t tph = (uint32_t)(li >> 1) & 1u;
       const long long b0 = t * p.spt;
+      const int samples = (int)min((long long)p.spt, p.batch - b0);
       float row0[ROW0_PER_THREAD];
 #pragma unroll
       for (int r = 0; r < ROW0_PER_THREAD; ++r) {  // unrounded copy of Z[b, 0, :]
         const int idx = te + 128 * r;
         const int s = idx / ID, col = idx - s * ID;
-        row0[r] = (s < p.spt && b0 + s < p.batch) ? __ldg(p.z + (b0 + s) * p.F * ID + col) : 0.f;
+        row0[r] = s < samples ? __ldg(p.z + (b0 + s) * p.F * ID + col) : 0.f;
       }
       // All four warps leave together: a warp that gave up still joins the barrier.
       const bool ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * buf, tph, abort_flag,
                                                         &g_inter_error)) != 0;
       if (!ok) *epi_fail = 1;
+      if (te == 0) bulk_wait_read<0>();  // the image of the group's last tile has been read
       epi_sync(group);
       if (*epi_fail) break;  // written before the barrier by epilogue warps only: same answer for all
       tc_fence_after();
 #pragma unroll 1
-      for (int c0 = 0; c0 < 128; c0 += 32) {
-        if (c0 + 32 <= c_lo || c0 >= c_hi) continue;  // warp-uniform
+      for (int c0 = c_lo & ~31; c0 < c_hi; c0 += 32) {  // warp-uniform
         uint32_t r[32];
         tmem_ld32(tmem_base + buf * 128 + ((uint32_t)row_lo << 16) + (uint32_t)c0, r);
         tmem_ld_wait();
-        float* drow = dsm + (row_lo + lane) * I_LD + c0;
+        const int d = c0 - first;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(drow + j) =
-              make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                          __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+        for (int j = 0; j < 32; ++j)
+          if ((unsigned)(d + j) < (unsigned)fi) my_img[d + j] = __uint_as_float(r[j]);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);  // accumulator may be overwritten
-      epi_sync(group);
-      // Output rows of the tile's samples.  Triangle: pair index outer (its (i, j) is read
-      // once), sample inner; for one sample consecutive threads write consecutive floats.
-      for (int pe = te; pe < p.tri; pe += 128) {
-        const int pi = pair_i[pe], pj = pair_j[pe];
-        for (int s = 0; s < p.spt; ++s) {
-          const long long b = b0 + s;
-          if (b >= p.batch) break;
-          p.out[b * p.out_stride + ID + pe] = dsm[(s * p.F + pi) * I_LD + s * p.F + pj];
-        }
-      }
-      // Row 0 of every sample (loaded before the wait on the accumulator) and the padding.
 #pragma unroll
       for (int r = 0; r < ROW0_PER_THREAD; ++r) {
         const int idx = te + 128 * r;
         const int s = idx / ID, col = idx - s * ID;
-        if (s < p.spt && b0 + s < p.batch) p.out[(b0 + s) * p.out_stride + col] = row0[r];
+        if (s < p.spt) img[s * p.img_row + col] = row0[r];
       }
-      const int pad = (int)p.out_stride - ID - p.tri;
-      for (int e = te; e < p.spt * pad; e += 128) {
-        const int s = e / pad, col = ID + p.tri + (e - s * pad);
-        if (b0 + s < p.batch) p.out[(b0 + s) * p.out_stride + col] = 0.f;
+      if (p.bulk) fence_proxy_async();
+      epi_sync(group);
+      if (p.bulk) {
+        if (te == 0) {
+          const uint32_t src = smem_u32(img);
+          const uint32_t row_bytes = (uint32_t)p.img_row * 4u;
+          if (p.out_stride == p.img_row) {
+            bulk_store(p.out + b0 * p.out_stride, src, (uint32_t)samples * row_bytes);
+          } else {
+            for (int s = 0; s < samples; ++s)
+              bulk_store(p.out + (b0 + s) * p.out_stride, src + (uint32_t)s * row_bytes, row_bytes);
+          }
+          bulk_commit();
+        }
+      } else {
+        const int w = ID + p.tri;
+        for (int e = te; e < samples * w; e += 128) {
+          const int s = e / w;
+          p.out[(b0 + s) * p.out_stride + (e - s * w)] = img[s * p.img_row + (e - s * w)];
+        }
       }
-      epi_sync(group);  // dsm is rewritten by the next tile
+      // zeros behind the part the image holds
+      const int have = p.bulk ? p.img_row : ID + p.tri;
+      const int pad = (int)p.out_stride - have;
+      for (int e = te; e < samples * pad; e += 128) {
+        const int s = e / pad;
+        p.out[(b0 + s) * p.out_stride + have + (e - s * pad)] = 0.f;
+      }
     }
+    if (te == 0) bulk_wait_all();  // the copies read this CTA's shared memory
   }
   tc_fence_before();
   __syncthreads();
@@ -258,6 +276,8 @@ int dot_interaction_tc(const float* z, int64_t batch, int F, int dim, int64_t z_
   p.rows = p.spt * F;
   p.tri = F * (F - 1) / 2;
   p.tiles = (batch + p.spt - 1) / p.spt;
+  p.img_row = (ID + p.tri + 3) & ~3;
+  p.bulk = out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   CUtensorMap tm;
   ANNC_TRY(tc::make_map(&tm, z, batch * F, ID, ID, p.rows, false));
   int dev = 0, sms = 148;

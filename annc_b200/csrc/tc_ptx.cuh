@@ -85,6 +85,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int 
                "r"(y), "r"(z), "r"(src)
                : "memory");
 }
+// `bytes` contiguous bytes, shared to global memory: both addresses and the size in multiples of 16.
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // All but this thread's newest N committed groups have read their shared memory / are complete.
 template <int N>

@@ -131,3 +131,26 @@ def test_masked_sum_of_slot_major_parts_with_output_slots(use_map, bf16):
         assert np.array_equal(got, ref)
     else:
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("F", [2, 3, 7, 16, 26, 27, 31, 32])
+@pytest.mark.parametrize("batch", [1, 5, 1203])
+@pytest.mark.parametrize("extra", [0, 1, 4, 21])
+def test_dot_interaction_image_rows(F, batch, extra):
+    """Tensor-core interaction at every way a row can end: image rows padded to four floats, output
+    rows that are not 16-byte aligned, padding behind the image, a last tile with few samples.
+    Operands cut to 11 significant bits: each product is off by at most 2^-9 of its size, and the fp32
+    sums by far less; row 0 is a copy."""
+    tri = F * (F - 1) // 2
+    stride = 64 + tri + extra
+    g = torch.Generator(device="cuda").manual_seed(F * 100 + batch)
+    z = torch.randn((batch, F, 64), device="cuda", generator=g)
+    out = torch.full((batch + 1, stride), -7.0, device="cuda")
+    device.dot_interaction(z, out[:batch], 2)
+    assert not device.gemm_timed_out()
+    i, j = torch.tril_indices(F, F, offset=-1, device="cuda")
+    want = torch.bmm(z.double(), z.double().transpose(1, 2))[:, i, j]
+    size = torch.bmm(z.double().abs(), z.double().abs().transpose(1, 2))[:, i, j]
+    assert torch.equal(out[:batch, :64], z[:, 0])
+    assert ((out[:batch, 64:64 + tri] - want).abs() <= 2.0 ** -9 * size + 1e-5).all()
+    assert (out[:batch, 64 + tri:] == 0).all() and (out[batch] == -7.0).all()
