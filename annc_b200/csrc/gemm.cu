@@ -32,7 +32,9 @@ static int validate(const annc_gemm_desc& d) {
 // tiles) 13.6 / 14.4, 2048 x 1000 x 500 (32) 15.2 / 15.7, 64 x [256 x 256 x 64] 9.4 / 11.5; 1024^3 (16)
 // 21 / 15.  A narrow C pays for 256 columns of multiplications: from n = 64 on that still hides
 // under the memory traffic when K is short and the rows fill every pair (65536 x 64 x 256 24 / 28).
-// Its general epilogue (beta * C, addend) is slow per tile and needs a long main loop to hide in.
+// With an addend: 8192 x 1024 x 512 31 / 59, 3000 x 1000 x 1000 (48 tiles) 25 / 43, 4096 x 512 x 416 (32)
+// 17 / 20.  Its general epilogue (beta * C, rows not of whole 16-byte pieces) is slow per tile and
+// needs a long main loop to hide in.
 static bool use_pair(const annc_gemm_desc& d, int math) {
   if (!pair_supported(d, math)) return false;
   if (math == ANNC_MATH_BF16 || (d.io_flags & (ANNC_IO_SOFTMAX | ANNC_IO_PAIR))) return true;

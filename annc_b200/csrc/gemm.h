@@ -24,7 +24,7 @@ int run_tc(const annc_gemm_desc& d, int math, cudaStream_t s);
 // Persistent CTA-pair tcgen05 kernel (TF32 with fp32 operands, BF16 with bf16 operands).
 bool pair_supported(const annc_gemm_desc& d, int math);
 int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s);
-// Whether its epilogue for this descriptor is the TMA store (no beta * C, addend or softmax).
+// Whether its epilogue for this descriptor stores by TMA (no beta * C or softmax, aligned rows).
 bool pair_stores_by_tma(const annc_gemm_desc& d);
 
 // A kn4-packed B re-laid into `ws` (4*K*N bytes): relaid_desc returns 0 when that does not

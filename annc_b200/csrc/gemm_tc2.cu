@@ -58,7 +58,7 @@ constexpr int P_EPI_WARPS = 8;                       // two per TMEM lane quadra
 constexpr int P_STG_BYTES = P_EPI_WARPS * 32 * 32 * 4;  // one swizzled 32 x 32 chunk per epilogue warp
 constexpr size_t P_SMEM = 1024 + (size_t)P_STAGES * P_STAGE + P_STG_BYTES + 256;
 
-enum Epilogue { EPI_GENERAL = 0, EPI_SOFTMAX = 1, EPI_TMA_STORE = 2 };
+enum Epilogue { EPI_GENERAL = 0, EPI_SOFTMAX = 1, EPI_TMA_STORE = 2, EPI_TMA_ADD = 3 /* and an addend */ };
 
 struct PairParams {
   int M, N, K;
@@ -263,8 +263,9 @@ template <int DT, int EPI>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                          const __grid_constant__ CUtensorMap tmap_b,
-                         const __grid_constant__ CUtensorMap tmap_c /* EPI_TMA_STORE */, PairParams p) {
+                         const __grid_constant__ CUtensorMap tmap_c /* TMA stores */, PairParams p) {
   constexpr bool SOFTMAX = EPI == EPI_SOFTMAX;
+  constexpr bool TMA_STORE = EPI == EPI_TMA_STORE || EPI == EPI_TMA_ADD;
   constexpr int KELTS = DT == 0 ? 32 : 64;  // elements per 128-byte k-step row
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -287,7 +288,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tmap_a);
     prefetch_tensormap(&tmap_b);
-    if (EPI == EPI_TMA_STORE) prefetch_tensormap(&tmap_c);
+    if (TMA_STORE) prefetch_tensormap(&tmap_c);
     for (int s = 0; s < P_STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1);   // the leader's expect_tx arrival; bytes come from both CTAs
       mbar_init(bar_empty + 8 * s, 1);  // one commit
@@ -415,7 +416,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (!ok) break;
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * (uint32_t)PN;
-        if (EPI == EPI_TMA_STORE) {
+        if (TMA_STORE) {
           // Values finished in registers (a lane holds 32 or 64 columns of its row), one 4 KB
           // staging tile per warp, one TMA store per chunk; the next chunk is read from tensor
           // memory meanwhile.  The general form below spends about 800 instructions a chunk on
@@ -426,10 +427,24 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const uint32_t tcol = taddr + (uint32_t)(half * WCOLS);
           const uint32_t stg_s = smem_u32(stg);
           float* const bias_f = &bias_w.x;
+          // EPI_TMA_ADD: the lane's 32 addend values of a chunk, in registers before the accumulator is
+          // waited for; a lane reads whole lines of its own row, eight times from L1.
+          float4 add[8];
+          auto load_addend = [&](int c0) {
+            if (EPI != EPI_TMA_ADD) return;
+            const float* a = p.addend + bz * p.stride_addend + grow * p.ld_addend + c0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              add[j] = row_ok && c0 + 4 * j < p.N ? __ldg(reinterpret_cast<const float4*>(a + 4 * j))
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+          };
           auto finish = [&](const uint32_t (&r)[32], float (&v)[32], int first_lane) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              v[j] = p.alpha * __uint_as_float(r[j]) + __shfl_sync(0xffffffffu, bias_f[j & 3], first_lane + (j >> 2));
+            for (int j = 0; j < 32; ++j) {
+              v[j] = p.alpha * __uint_as_float(r[j]);
+              if (EPI == EPI_TMA_ADD) v[j] += (&add[j >> 2].x)[j & 3];
+              v[j] += __shfl_sync(0xffffffffu, bias_f[j & 3], first_lane + (j >> 2));
+            }
             if (p.act == ANNC_ACT_RELU) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
@@ -453,13 +468,17 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (lane == 0) bulk_wait_read<0>();
             __syncwarp();
           };
-          if (nb < p.N) tmem_ld32(tcol, ra);
+          if (nb < p.N) {
+            load_addend(nb);
+            tmem_ld32(tcol, ra);
+          }
           if (!p.c_bf16) {
 #pragma unroll 1
             for (int i = 0; i < WCOLS / 32; ++i) {
               const int c0 = nb + 32 * i;
               if (c0 >= p.N) break;  // warp-uniform
               float v[32];
+              if (i > 0) load_addend(c0);
               tmem_ld_wait();
               finish(ra, v, 8 * i);
               if (i + 1 < WCOLS / 32 && c0 + 32 < p.N) tmem_ld32(tcol + 32u * (i + 1), ra);
@@ -479,6 +498,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 float v[32];
+                if (i + h > 0) load_addend(c0 + 32 * h);
                 tmem_ld_wait();
                 finish(ra, v, 16 * i + 8 * h);
                 // (columns past N hold zeros and are clipped by the store)
@@ -564,7 +584,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_u32(bar_tempty + 8 * acc, 0));
       }
-      if (EPI == EPI_TMA_STORE && lane == 0) bulk_wait_all();  // the stores read this CTA's shared memory
+      if (TMA_STORE && lane == 0) bulk_wait_all();  // the stores read this CTA's shared memory
     }
   }
   tc_fence_before();
@@ -627,10 +647,12 @@ bool pair_supported(const annc_gemm_desc& d, int math) {
 }
 
 // The TMA store takes every C whose rows are 16-byte aligned and whole 16-byte pieces long (it clips
-// at the tensor's edge in such pieces), without beta * C and addend.
+// at the tensor's edge in such pieces), without beta * C; an addend has to be 16-byte aligned too.
 bool pair_stores_by_tma(const annc_gemm_desc& d) {
   const int per16 = (d.io_flags & ANNC_IO_C_BF16) ? 8 : 4;
-  return !(d.io_flags & ANNC_IO_SOFTMAX) && d.beta == 0.f && !d.addend && al16(d.c) && d.ldc >= d.n &&
+  if (d.addend && (!al16(d.addend) || (d.ld_addend & 3) || (d.batch > 1 && (d.stride_addend & 3)) || (d.n & 3)))
+    return false;
+  return !(d.io_flags & ANNC_IO_SOFTMAX) && d.beta == 0.f && al16(d.c) && d.ldc >= d.n &&
          d.n % per16 == 0 && d.ldc % per16 == 0 && (d.batch == 1 || (d.stride_c % per16 == 0 && d.stride_c > 0));
 }
 
@@ -642,15 +664,16 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   const bool softmax = (d.io_flags & ANNC_IO_SOFTMAX) != 0;
   const bool c_bf16 = (d.io_flags & ANNC_IO_C_BF16) != 0;
   const bool tma_store = pair_stores_by_tma(d);
-  const int epi = softmax ? EPI_SOFTMAX : tma_store ? EPI_TMA_STORE : EPI_GENERAL;
-  auto kern = bf16 ? (softmax     ? gemm_pair_tcgen05_kernel<1, EPI_SOFTMAX>
-                      : tma_store ? gemm_pair_tcgen05_kernel<1, EPI_TMA_STORE>
-                                  : gemm_pair_tcgen05_kernel<1, EPI_GENERAL>)
-                   : (softmax     ? gemm_pair_tcgen05_kernel<0, EPI_SOFTMAX>
-                      : tma_store ? gemm_pair_tcgen05_kernel<0, EPI_TMA_STORE>
-                                  : gemm_pair_tcgen05_kernel<0, EPI_GENERAL>);
-  static bool attr_done_dev[kMaxDevices][2][3] = {};
-  bool (&attr_done)[2][3] = attr_done_dev[device_slot()];
+  const int epi = softmax ? EPI_SOFTMAX : !tma_store ? EPI_GENERAL : d.addend ? EPI_TMA_ADD : EPI_TMA_STORE;
+  using Kernel = decltype(&gemm_pair_tcgen05_kernel<0, EPI_GENERAL>);
+  static const Kernel kernels[2][4] = {
+      {gemm_pair_tcgen05_kernel<0, EPI_GENERAL>, gemm_pair_tcgen05_kernel<0, EPI_SOFTMAX>,
+       gemm_pair_tcgen05_kernel<0, EPI_TMA_STORE>, gemm_pair_tcgen05_kernel<0, EPI_TMA_ADD>},
+      {gemm_pair_tcgen05_kernel<1, EPI_GENERAL>, gemm_pair_tcgen05_kernel<1, EPI_SOFTMAX>,
+       gemm_pair_tcgen05_kernel<1, EPI_TMA_STORE>, gemm_pair_tcgen05_kernel<1, EPI_TMA_ADD>}};
+  const Kernel kern = kernels[bf16][epi];
+  static bool attr_done_dev[kMaxDevices][2][4] = {};
+  bool (&attr_done)[2][4] = attr_done_dev[device_slot()];
   if (!attr_done[bf16][epi]) {
     ANNC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM));
     attr_done[bf16][epi] = true;
