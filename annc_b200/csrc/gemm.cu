@@ -77,11 +77,12 @@ __global__ void kn4_convert_kernel(const float* src, float* dst, long long K, lo
   }
 }
 
-// kn4 -> [K,N], or [N,K] (the K-major layout the TMA route likes best), N % 4 == 0: a block moves
-// a tile of 128 (k) x 32 (n).  A thread reads 16-byte pieces of one panel (a piece never straddles
+// Between kn4 and [K,N], or from kn4 to [N,K] (the K-major layout the TMA route likes best), N % 4 ==
+// 0: a block moves a tile of 128 (k) x 32 (n).  A thread reads 16-byte pieces of one panel (a piece never straddles
 // two), whose place it works out once; for [N,K] the tile turns in shared memory (rows of 129
 // floats: neither side conflicts).  Bound by memory: 2048 x 4096 in 8 to 13 us (of which 10 at the copy rate from DRAM), 38 us with one element
 // and one 64-bit place computation per thread and step.
+enum Relay { RELAY_KN = 0, RELAY_NK = 1, RELAY_PACK = 2 /* [K,N] -> kn4 */ };
 constexpr int kRelayK = 128, kRelayN = 32;
 struct RelayParams {
   const float* src;
@@ -90,8 +91,9 @@ struct RelayParams {
   // k-chunks: 352 rows each (len0 if there is only one) up to k_uniform, then the two that share the rest
   int k_uniform, k_split, len0;
 };
-template <bool TRANSPOSED>
+template <int MODE>
 __global__ void __launch_bounds__(256) kn4_relay_kernel(RelayParams p) {
+  constexpr bool TRANSPOSED = MODE == RELAY_NK;
   __shared__ float tile[TRANSPOSED ? kRelayN : 1][kRelayK + 1];
   const int n0 = blockIdx.x * kRelayN, k0 = blockIdx.y * kRelayK;
   const int c = threadIdx.x & 7, kk = threadIdx.x >> 3;
@@ -116,9 +118,12 @@ __global__ void __launch_bounds__(256) kn4_relay_kernel(RelayParams p) {
         start = p.k_split;
         len = p.K - p.k_split;
       }
-      v[i] = __ldg(reinterpret_cast<const float4*>(p.src + (long long)start * p.N + (long long)len * term +
-                                                   (long long)(k - start) * width + in0));
+      const long long packed = (long long)start * p.N + (long long)len * term + (long long)(k - start) * width + in0;
+      if (MODE == RELAY_PACK)
+        *reinterpret_cast<float4*>(p.dst + packed) = __ldg(reinterpret_cast<const float4*>(p.src + (long long)k * p.N + n));
+      else v[i] = __ldg(reinterpret_cast<const float4*>(p.src + packed));
     }
+    if (MODE == RELAY_PACK) return;
 #pragma unroll
     for (int i = 0; i < kRelayK / 32; ++i) {
       const int k = k0 + kk + 32 * i;
@@ -198,16 +203,39 @@ int relaid_desc(const annc_gemm_desc& d, void* ws, size_t ws_bytes, annc_gemm_de
   return 2;
 }
 
-void relay_kn4(const float* packed, float* ws, long long k, long long n, int form, cudaStream_t s) {
+static RelayParams relay_params(const float* src, float* dst, long long k, long long n) {
   constexpr int tk = (int)kn4::kTileK;
-  RelayParams p{packed, ws, (int)k, (int)n, (int)k, (int)k, k < tk ? (int)k : tk};
+  RelayParams p{src, dst, (int)k, (int)n, (int)k, (int)k, k < tk ? (int)k : tk};
   if (k >= tk && k % tk != 0) {  // the first of the last two chunks, as kn4::axis_chunk cuts them
     p.k_uniform = (int)(k / tk - 1) * tk;
     p.k_split = p.k_uniform + (int)kn4::axis_chunk(k, tk, p.k_uniform).len;
   }
-  const dim3 grid((unsigned)((n + kRelayN - 1) / kRelayN), (unsigned)((k + kRelayK - 1) / kRelayK));
-  if (form == 1) kn4_relay_kernel<true><<<grid, 256, 0, s>>>(p);
-  else kn4_relay_kernel<false><<<grid, 256, 0, s>>>(p);
+  return p;
+}
+static dim3 relay_grid(long long k, long long n) {
+  return dim3((unsigned)((n + kRelayN - 1) / kRelayN), (unsigned)((k + kRelayK - 1) / kRelayK));
+}
+
+void relay_kn4(const float* packed, float* ws, long long k, long long n, int form, cudaStream_t s) {
+  const RelayParams p = relay_params(packed, ws, k, n);
+  if (form == 1) kn4_relay_kernel<RELAY_NK><<<relay_grid(k, n), 256, 0, s>>>(p);
+  else kn4_relay_kernel<RELAY_KN><<<relay_grid(k, n), 256, 0, s>>>(p);
+}
+
+// kn4 <-> [K,N], any extents: 16-byte pieces where they exist (2048 x 4096: 11 and 9 us against 56 us one
+// element at a time).
+static void convert_kn4(const float* src, float* dst, long long k, long long n, bool pack, cudaStream_t s) {
+  const bool pieces = n % 4 == 0 && n < (1LL << 31) && (k + kRelayK - 1) / kRelayK <= 65535 &&
+                      ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+  if (pieces) {
+    const RelayParams p = relay_params(src, dst, k, n);
+    if (pack) kn4_relay_kernel<RELAY_PACK><<<relay_grid(k, n), 256, 0, s>>>(p);
+    else kn4_relay_kernel<RELAY_KN><<<relay_grid(k, n), 256, 0, s>>>(p);
+    return;
+  }
+  long long g = (k * n + 255) / 256;
+  if (g > 148 * 32) g = 148 * 32;
+  kn4_convert_kernel<<<(unsigned)g, 256, 0, s>>>(src, dst, k, n, pack ? 1 : 0);
 }
 
 static bool unpack_kn4_into_workspace(const annc_gemm_desc& d, cudaStream_t s, annc_gemm_desc* plain) {
@@ -273,10 +301,7 @@ int annc_bf16_weight_dev(const float* b_kn, int64_t ldb, void* b_nk_bf16, int64_
 int annc_kn4_pack_dev(const float* b_kn, float* b_packed, int64_t k, int64_t n, void* stream) {
   ANNC_REQUIRE(b_kn && b_packed && b_kn != b_packed, ANNC_ERR_INVALID_ARGUMENT, "kn4: bad buffers");
   if (k * n <= 0) return ANNC_OK;
-  long long g = (k * n + 255) / 256;
-  if (g > 148 * 32) g = 148 * 32;
-  gemm::kn4_convert_kernel<<<(unsigned)g, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      b_kn, b_packed, k, n, 1);
+  gemm::convert_kn4(b_kn, b_packed, k, n, true, static_cast<cudaStream_t>(stream));
   ANNC_CUDA(cudaGetLastError());
   return ANNC_OK;
 }
@@ -284,10 +309,7 @@ int annc_kn4_pack_dev(const float* b_kn, float* b_packed, int64_t k, int64_t n, 
 int annc_kn4_unpack_dev(const float* b_packed, float* b_kn, int64_t k, int64_t n, void* stream) {
   ANNC_REQUIRE(b_kn && b_packed && b_kn != b_packed, ANNC_ERR_INVALID_ARGUMENT, "kn4: bad buffers");
   if (k * n <= 0) return ANNC_OK;
-  long long g = (k * n + 255) / 256;
-  if (g > 148 * 32) g = 148 * 32;
-  gemm::kn4_convert_kernel<<<(unsigned)g, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      b_packed, b_kn, k, n, 0);
+  gemm::convert_kn4(b_packed, b_kn, k, n, false, static_cast<cudaStream_t>(stream));
   ANNC_CUDA(cudaGetLastError());
   return ANNC_OK;
 }

@@ -241,7 +241,10 @@ def test_layout_matmul_device_weight(m, n, k):
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     a = torch.randn((m, k), device="cuda", generator=g)
     w = torch.randn((k, n), device="cuda", generator=g)
-    got = ops.xla_layout_matmul(a, device.kn4_pack(w))
+    packed = device.kn4_pack(w)
+    np.testing.assert_array_equal(packed.cpu().numpy(), oracle.kn4_pack(w.cpu().numpy()))
+    assert torch.equal(device.kn4_unpack(packed), w)
+    got = ops.xla_layout_matmul(a, packed)
     want = (a.double() @ w.double()).cpu().numpy()
     assert nerr(got, want) <= 2e-3  # TF32
 
