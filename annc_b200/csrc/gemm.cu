@@ -28,10 +28,12 @@ static int validate(const annc_gemm_desc& d) {
 
 // Pair kernel (256 x 256 tiles per two SMs, persistent) or single-CTA kernel (128 x 128 tiles, two
 // per SM or split K inside a cluster).  With its TMA-store epilogue the pair kernel wins from
-// about 32 tiles on, measured in us pair / single: 65536 x 512 x 416 61 / 111, 4096 x 512 x 416 (32
-// tiles) 13.6 / 14.4, 2048 x 1000 x 500 (32) 15.2 / 15.7, 64 x [256 x 256 x 64] 9.4 / 11.5; 1024^3 (16)
-// 21 / 15.  A narrow C pays for 256 columns of multiplications: from n = 64 on that still hides
-// under the memory traffic when K is short and the rows fill every pair (65536 x 64 x 256 24 / 28).
+// about 32 tiles on, measured in us pair / single: 65536 x 512 x 416 62 / 111, 4096 x 512 x 416 (32
+// tiles) 11.6 / 14.4, 2048 x 1000 x 500 (32) 12.8 / 15.7, 64 x [256 x 256 x 64] 9.5 / 11.5.  Below, split K
+// decides: 1500 x 1100 x 700 (30) 15.1 / 16.6, 20 x [256 x 256 x 100] 8.1 / 9.2, but 2048 x 512 x 416 (16)
+// 11.2 / 11.0 and 1024^3 (16) 17.7 / 14.6.  A narrow C pays for 256 columns of multiplications: from
+// n = 64 on that still hides under the memory traffic when K is short and the rows fill every
+// pair (65536 x 64 x 256 24 / 28).
 // With an addend: 8192 x 1024 x 512 31 / 59, 3000 x 1000 x 1000 (48 tiles) 25 / 43, 4096 x 512 x 416 (32)
 // 17 / 20.  Its general epilogue (beta * C, rows not of whole 16-byte pieces) is slow per tile and
 // needs a long main loop to hide in.
@@ -42,7 +44,7 @@ static bool use_pair(const annc_gemm_desc& d, int math) {
   const long long pair_tiles = ((d.m + 255) / 256) * ((d.n + 255) / 256) * d.batch;
   if (d.m >= 256 && d.n >= 192 && d.k >= 1024 && pair_tiles >= 74) return true;
   if (!pair_stores_by_tma(d)) return false;
-  return (d.n >= 192 && d.m >= 192 && pair_tiles >= 32) || (d.n >= 64 && d.k <= 512 && pair_tiles >= 148);
+  return (d.n >= 192 && d.m >= 192 && pair_tiles >= (d.k <= 704 ? 20 : 32)) || (d.n >= 64 && d.k <= 512 && pair_tiles >= 148);
 }
 
 // AUTO: tensor cores (TF32) when the shape fits a tcgen05 kernel, else CUDA cores.

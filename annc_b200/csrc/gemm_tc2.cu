@@ -75,7 +75,8 @@ struct PairParams {
   int batched, b_batched;
   long long stride_c, stride_addend;
   int tiles_m, tiles_n;
-  long long tiles;
+  long long whole;  // work items 0 .. whole - 1 are whole tiles, the others up to `items` are half tiles:
+  long long items;  // the tiles of a last round that fills at most half of the pairs are cut in two
   int* error_word;
 };
 
@@ -84,16 +85,26 @@ struct PairParams {
 // tiles: every A and B panel they stream is shared through L2 by several pairs instead of
 // being fetched from DRAM once per column (or row) tile.
 constexpr int P_BAND = 8;
-__device__ __forceinline__ void tile_coords(const PairParams& p, long long tile, long long* bz, int* tm,
-                                            int* tn) {
+// Work item: batch, row tile, first column and width (256, or 128 for half a tile).  False for a half
+// that lies beyond N.
+// CUT: the launch has half tiles at all (without, widths are constants in the loops below: the whole
+// tiles of 8192 x 4096 x 2048 ran 1.5 % slower with run-time widths).
+template <bool CUT>
+__device__ __forceinline__ bool item_coords(const PairParams& p, long long item, long long* bz, int* tm, int* n0,
+                                            int* width) {
+  const long long over = CUT ? item - p.whole : -1;
+  const long long tile = over < 0 ? item : p.whole + (over >> 1);
   const long long per_batch = (long long)p.tiles_m * p.tiles_n;
   *bz = tile / per_batch;
   const int t2 = (int)(tile - *bz * per_batch);
   const int band = t2 / (P_BAND * p.tiles_n);
   const int rem = t2 - band * (P_BAND * p.tiles_n);
   const int rows = min(P_BAND, p.tiles_m - band * P_BAND);
-  *tn = rem / rows;
-  *tm = band * P_BAND + (rem - *tn * rows);
+  const int tn = rem / rows;
+  *tm = band * P_BAND + (rem - tn * rows);
+  *width = over < 0 ? PN : PN / 2;
+  *n0 = tn * PN + (over < 0 ? 0 : (int)(over & 1) * (PN / 2));
+  return !CUT || *n0 < p.N;
 }
 
 __device__ __forceinline__ float act_apply(float v, int act) {
@@ -259,10 +270,11 @@ __device__ __forceinline__ void stage_row(float* stg, int lane, const uint32_t (
 }
 
 // DT 0: TF32 (fp32 elements, 32 per 128-byte k-step, UMMA K = 8); DT 1: BF16 (64, K = 16).
-template <int DT, int EPI>
+template <int DT, int EPI, bool CUT>
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                          const __grid_constant__ CUtensorMap tmap_b,
+                         const __grid_constant__ CUtensorMap tmap_bh /* [N,K] B, half as many rows */,
                          const __grid_constant__ CUtensorMap tmap_c /* TMA stores */, PairParams p) {
   constexpr bool SOFTMAX = EPI == EPI_SOFTMAX;
   constexpr bool TMA_STORE = EPI == EPI_TMA_STORE || EPI == EPI_TMA_ADD;
@@ -314,12 +326,13 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (lane == 0) {
         uint32_t kit = 0;
         bool ok = true;
-        for (long long tile = pair; tile < p.tiles && ok; tile += pairs) {
+        for (long long item = pair; item < p.items && ok; item += pairs) {
           long long bz;
-          int tm, tn;
-          tile_coords(p, tile, &bz, &tm, &tn);
+          int tm, n0, width;
+          if (!item_coords<CUT>(p, item, &bz, &tm, &n0, &width)) continue;
           const int m0 = tm * (2 * PM) + (int)rank * PM;
-          const int n0 = tn * PN + (int)rank * (PN / 2);
+          n0 += (int)rank * (width / 2);
+          const uint32_t stage_bytes = P_A_BYTES + (uint32_t)width * (P_B_BYTES / PN);
           for (int kt = 0; kt < KT; ++kt, ++kit) {
             const int s = kit % P_STAGES;
             const uint32_t ph = (kit / P_STAGES) & 1u;
@@ -327,16 +340,18 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (!ok) break;
             const uint32_t sa = base + s * P_STAGE, sb = sa + P_A_BYTES;
             const uint32_t full_leader = mapa_u32(bar_full + 8 * s, 0);
-            if (leader) mbar_expect_tx(bar_full + 8 * s, 2 * P_STAGE);
+            if (leader) mbar_expect_tx(bar_full + 8 * s, 2 * stage_bytes);
             const int k0 = kt * KELTS;
             if (p.batched) tma_load_3d_pair(sa, &tmap_a, k0, m0, (int)bz, full_leader);
             else tma_load_2d_pair(sa, &tmap_a, k0, m0, full_leader);
             if (!p.b_n_major) {
-              if (p.b_batched) tma_load_3d_pair(sb, &tmap_b, k0, n0, (int)bz, full_leader);
-              else tma_load_2d_pair(sb, &tmap_b, k0, n0, full_leader);
+              const CUtensorMap* map = width == PN ? &tmap_b : &tmap_bh;
+              if (p.b_batched) tma_load_3d_pair(sb, map, k0, n0, (int)bz, full_leader);
+              else tma_load_2d_pair(sb, map, k0, n0, full_leader);
             } else {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {  // one 32-column x 32-row box per 4 KB block
+                if (32 * j >= width / 2) break;
                 if (p.b_batched)
                   tma_load_3d_pair(sb + j * 4096, &tmap_b, n0 + 32 * j, k0, (int)bz, full_leader);
                 else
@@ -351,12 +366,17 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (leader && lane == 0) {
         // D fp32; A/B tf32 or bf16; A K-major; B K- or N-major; N = 256; M = 256
         const uint32_t fmt = DT == 0 ? 2u : 1u;
-        const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((p.b_n_major ? 1u : 0u) << 16) |
-                               ((uint32_t)(PN >> 3) << 17) | ((uint32_t)((2 * PM) >> 4) << 24);
+        const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((p.b_n_major ? 1u : 0u) << 16) |
+                                ((uint32_t)((2 * PM) >> 4) << 24);
         uint32_t kit = 0, tcount = 0;
         bool ok = true;
-        for (long long tile = pair; tile < p.tiles && ok; tile += pairs, ++tcount) {
+        for (long long item = pair; item < p.items && ok; item += pairs) {
+          long long bz;
+          int tm, n0, width;
+          if (!item_coords<CUT>(p, item, &bz, &tm, &n0, &width)) continue;
+          const uint32_t idesc = idesc0 | ((uint32_t)(width >> 3) << 17);
           const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
+          ++tcount;
           ok = mbar_wait(bar_tempty + 8 * acc, aph ^ 1u, abort_flag, p.error_word);
           if (!ok) break;
           tc_fence_after();
@@ -388,16 +408,17 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       float* stg = staging + (warp - 2) * (32 * 32);
       uint32_t tcount = 0;
       bool ok = true;
-      for (long long tile = pair; tile < p.tiles && ok; tile += pairs, ++tcount) {
-        const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
+      for (long long item = pair; item < p.items && ok; item += pairs) {
         long long bz;
-        int tm, tn;
-        tile_coords(p, tile, &bz, &tm, &tn);
+        int tm, n0, width;
+        if (!item_coords<CUT>(p, item, &bz, &tm, &n0, &width)) continue;
+        const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
+        ++tcount;
         const long long row0 = (long long)tm * (2 * PM) + rank * PM + q * 32;  // first row of this warp
         const long long grow = row0 + lane;
         const bool row_ok = grow < p.M;
-        constexpr int WCOLS = PN / (P_EPI_WARPS / 4);  // columns per epilogue warp (128)
-        const int nb = tn * PN + half * WCOLS;  // first column of this warp
+        const int wcols = width / (P_EPI_WARPS / 4);  // columns per epilogue warp (128 or 64)
+        const int nb = n0 + half * wcols;             // first column of this warp
         // Bias of the warp's 128 columns, four per lane, fetched once per tile while the MMAs
         // still run: a load per chunk would put an L2 round trip on every chunk's critical path.
         float4 bias_w = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -424,7 +445,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           // it bounded every product with K below 1024 (65536 x 512 x 416: 121 us, 17 us a tile
           // of which the MMAs are 5).
           uint32_t ra[32];
-          const uint32_t tcol = taddr + (uint32_t)(half * WCOLS);
+          const uint32_t tcol = taddr + (uint32_t)(half * wcols);
           const uint32_t stg_s = smem_u32(stg);
           float* const bias_f = &bias_w.x;
           // EPI_TMA_ADD: the lane's 32 addend values of a chunk, in registers before the accumulator is
@@ -474,14 +495,14 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           if (!p.c_bf16) {
 #pragma unroll 1
-            for (int i = 0; i < WCOLS / 32; ++i) {
+            for (int i = 0; i < wcols / 32; ++i) {
               const int c0 = nb + 32 * i;
               if (c0 >= p.N) break;  // warp-uniform
               float v[32];
               if (i > 0) load_addend(c0);
               tmem_ld_wait();
               finish(ra, v, 8 * i);
-              if (i + 1 < WCOLS / 32 && c0 + 32 < p.N) tmem_ld32(tcol + 32u * (i + 1), ra);
+              if (i + 1 < wcols / 32 && c0 + 32 < p.N) tmem_ld32(tcol + 32u * (i + 1), ra);
               staging_free();
 #pragma unroll
               for (int j = 0; j < 8; ++j)
@@ -491,7 +512,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             }
           } else {
 #pragma unroll 1
-            for (int i = 0; i < WCOLS / 64; ++i) {
+            for (int i = 0; i < wcols / 64; ++i) {
               const int c0 = nb + 64 * i;
               if (c0 >= p.N) break;
               uint32_t w[32];  // 64 bf16 columns: one 128-byte row of the staging tile
@@ -502,7 +523,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 tmem_ld_wait();
                 finish(ra, v, 16 * i + 8 * h);
                 // (columns past N hold zeros and are clipped by the store)
-                if (h == 0 || i + 1 < WCOLS / 64) tmem_ld32(tcol + 64u * i + 32u * (h + 1), ra);
+                if (h == 0 || i + 1 < wcols / 64) tmem_ld32(tcol + 64u * i + 32u * (h + 1), ra);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                   __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
@@ -522,11 +543,11 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           // chunk i + 1 is read from tensor memory (into the registers staging has just
           // freed) while chunk i goes from the staging tile to global memory
           uint32_t ra[32];
-          const uint32_t tcol = taddr + (uint32_t)(half * WCOLS);
+          const uint32_t tcol = taddr + (uint32_t)(half * wcols);
           if (nb < p.N) tmem_ld32(tcol, ra);
           // not unrolled: the body is large, and unrolled copies of it thrash the instruction cache
 #pragma unroll 1
-          for (int i = 0; i < WCOLS / 32; ++i) {
+          for (int i = 0; i < wcols / 32; ++i) {
             const int c0 = nb + 32 * i;
             if (c0 < p.N) {  // warp-uniform
               float bias4[4];  // this lane's columns of the chunk, from the lane that fetched them
@@ -537,7 +558,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
               bias4[3] = __shfl_sync(0xffffffffu, bias_w.w, src);
               tmem_ld_wait();
               stage_row(stg, lane, ra, p.alpha);
-              if (i + 1 < WCOLS / 32 && c0 + 32 < p.N) tmem_ld32(tcol + 32u * (i + 1), ra);
+              if (i + 1 < wcols / 32 && c0 + 32 < p.N) tmem_ld32(tcol + 32u * (i + 1), ra);
               __syncwarp();
               chunk_store_staged(p, stg, lane, row0, c0, bz, true, bias4);
               __syncwarp();
@@ -551,7 +572,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll 1
           for (int pass = 0; pass < 3; ++pass) {
 #pragma unroll 1
-            for (int c0 = 0; c0 < PN && c0 < p.N; c0 += 32) {
+            for (int c0 = 0; c0 < PN && c0 < p.N; c0 += 32) {  // (never cut in half)
               uint32_t r[32];
               float v[32];
               tmem_ld32(taddr + (uint32_t)c0, r);
@@ -665,21 +686,23 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   const bool c_bf16 = (d.io_flags & ANNC_IO_C_BF16) != 0;
   const bool tma_store = pair_stores_by_tma(d);
   const int epi = softmax ? EPI_SOFTMAX : !tma_store ? EPI_GENERAL : d.addend ? EPI_TMA_ADD : EPI_TMA_STORE;
-  using Kernel = decltype(&gemm_pair_tcgen05_kernel<0, EPI_GENERAL>);
-  static const Kernel kernels[2][4] = {
-      {gemm_pair_tcgen05_kernel<0, EPI_GENERAL>, gemm_pair_tcgen05_kernel<0, EPI_SOFTMAX>,
-       gemm_pair_tcgen05_kernel<0, EPI_TMA_STORE>, gemm_pair_tcgen05_kernel<0, EPI_TMA_ADD>},
-      {gemm_pair_tcgen05_kernel<1, EPI_GENERAL>, gemm_pair_tcgen05_kernel<1, EPI_SOFTMAX>,
-       gemm_pair_tcgen05_kernel<1, EPI_TMA_STORE>, gemm_pair_tcgen05_kernel<1, EPI_TMA_ADD>}};
-  const Kernel kern = kernels[bf16][epi];
+  using Kernel = decltype(&gemm_pair_tcgen05_kernel<0, EPI_GENERAL, false>);
+#define ANNC_PAIR_KERNELS(DT)                                                                             \
+  {{gemm_pair_tcgen05_kernel<DT, EPI_GENERAL, false>, gemm_pair_tcgen05_kernel<DT, EPI_SOFTMAX, false>,    \
+    gemm_pair_tcgen05_kernel<DT, EPI_TMA_STORE, false>, gemm_pair_tcgen05_kernel<DT, EPI_TMA_ADD, false>}, \
+   {gemm_pair_tcgen05_kernel<DT, EPI_GENERAL, true>, gemm_pair_tcgen05_kernel<DT, EPI_SOFTMAX, false>,     \
+    gemm_pair_tcgen05_kernel<DT, EPI_TMA_STORE, true>, gemm_pair_tcgen05_kernel<DT, EPI_TMA_ADD, true>}}
+  static const Kernel kernels[2][2][4] = {ANNC_PAIR_KERNELS(0), ANNC_PAIR_KERNELS(1)};
+#undef ANNC_PAIR_KERNELS
   static bool attr_done_dev[kMaxDevices][2][4] = {};
   bool (&attr_done)[2][4] = attr_done_dev[device_slot()];
   if (!attr_done[bf16][epi]) {
-    ANNC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM));
+    for (int cut = 0; cut < 2; ++cut)
+      ANNC_CUDA(cudaFuncSetAttribute(kernels[bf16][cut][epi], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)P_SMEM));
     attr_done[bf16][epi] = true;
   }
   if (max_pairs[bf16] == 0) {
-    ANNC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM));
     cudaLaunchConfig_t q;
     memset(&q, 0, sizeof(q));
     cudaLaunchAttribute qa[1];
@@ -693,22 +716,25 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
     q.attrs = qa;
     q.numAttrs = 1;
     int n = 0;
-    ANNC_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &q));
+    ANNC_CUDA(cudaOccupancyMaxActiveClusters(&n, kernels[bf16][0][epi], &q));
     if (n < 1) return fail(ANNC_ERR_CUDA, "no CTA pair fits this device");
     max_pairs[bf16] = n;
   }
   const int kelts = bf16 ? 64 : 32;
   const bool batched = d.batch > 1, b_batched = batched && d.stride_b > 0;
-  CUtensorMap ta, tb, tc;
+  CUtensorMap ta, tb, tbh, tc;
   ANNC_TRY(make_map_any(&ta, d.a, bf16, batched ? d.batch : 1, d.m, d.k, d.lda, d.stride_a, kelts, PM, false));
   PairParams p;
   memset(&p, 0, sizeof(p));
   if (d.trans_b) {
     ANNC_TRY(make_map_any(&tb, d.b, bf16, b_batched ? d.batch : 1, d.n, d.k, d.ldb, d.stride_b, kelts,
                           PN / 2, false));
+    ANNC_TRY(make_map_any(&tbh, d.b, bf16, b_batched ? d.batch : 1, d.n, d.k, d.ldb, d.stride_b, kelts,
+                          PN / 4, false));
   } else {
     p.b_n_major = 1;
     ANNC_TRY(make_map_any(&tb, d.b, false, b_batched ? d.batch : 1, d.k, d.n, d.ldb, d.stride_b, 32, 32, true));
+    tbh = tb;
   }
   if (tma_store)
     ANNC_TRY(make_map_any(&tc, d.c, c_bf16, batched ? d.batch : 1, d.m, d.n, d.ldc, d.stride_c, c_bf16 ? 64 : 32, 32,
@@ -733,10 +759,19 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   p.stride_addend = batched ? d.stride_addend : 0;
   p.tiles_m = (int)((d.m + 2 * PM - 1) / (2 * PM));
   p.tiles_n = (int)((d.n + PN - 1) / PN);
-  p.tiles = (long long)p.tiles_m * p.tiles_n * d.batch;
+  const long long tiles = (long long)p.tiles_m * p.tiles_n * d.batch;
   p.error_word = gemm_error_word();
   if (!p.error_word) return fail(ANNC_ERR_CUDA, "gemm error word is not addressable");
-  const long long pairs = p.tiles < max_pairs[bf16] ? p.tiles : max_pairs[bf16];
+  // Tiles of the last (or only) round, when they fill at most half of the pairs, are cut in two column
+  // halves.  A half tile moves three quarters of the operands of a whole one, so behind whole rounds
+  // of a long main loop, which keep the chip at its power limit, nothing is won: 4096 x 512 x 416 (32
+  // tiles) 13.7 us whole, 11.6 us cut; 65536 x 256 x 512 (3 rounds and 34 tiles) 45.0 / 43.1; 16384 x
+  // 1024 x 8192 bf16 (the same) 211 / 215.
+  const long long last = tiles % max_pairs[bf16];
+  const bool cut = !softmax && d.n > PN / 2 && 2 * last <= max_pairs[bf16] && (tiles == last || d.k <= 64 * kelts);
+  p.whole = cut ? tiles - last : tiles;
+  p.items = p.whole + 2 * (tiles - p.whole);
+  const long long pairs = p.items < max_pairs[bf16] ? p.items : max_pairs[bf16];
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cudaLaunchAttribute attr[1];
@@ -750,7 +785,7 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ANNC_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p));
+  ANNC_CUDA(cudaLaunchKernelEx(&cfg, kernels[bf16][cut][epi], ta, tb, tbh, tc, p));
   return ANNC_OK;
 }
 

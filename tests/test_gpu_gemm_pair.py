@@ -156,3 +156,30 @@ def test_pair_store_edges(m, n, k, ldc, batch, dt, act):
     want = want.relu() if act == ACT_RELU else want
     assert nerr(c[:, :, :n], want.float().cpu().numpy()) <= (2e-3 if dt == "tf32" else 1e-2)
     assert (c[:, :, n:] == -7.0).all()
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(256, 256, 64, 1), (300, 600, 96, 1), (2600, 500, 128, 1), (9500, 500, 160, 2),
+                                         (19200, 260, 64, 1), (256, 129, 64, 5), (256, 140, 2048, 80)])
+@pytest.mark.parametrize("form", ["nk", "kn", "bf16", "add"])
+def test_pair_half_tiles(m, n, k, batch, form):
+    """Tiles of a last round cut in column halves (a half beyond N, a ragged N in either half, whole
+    rounds before them), in every operand form and with beta * C (the general epilogue).  Bounds as
+    in test_pair_store_edges."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn((batch, m, k), device="cuda", generator=g)
+    b = torch.randn((batch, k, n), device="cuda", generator=g)
+    c = torch.randn((batch, m, n), device="cuda", generator=g)
+    add = torch.randn((batch, m, n), device="cuda", generator=g) if form == "add" else None
+    if form in ("kn", "add") and n % 4:
+        pytest.skip("[K,N] rows of 16 bytes")
+    if form == "bf16":
+        a, b = a.bfloat16(), b.bfloat16()
+    beta = 0.0 if form in ("add", "bf16") else 1.0
+    want = a.double() @ b.double() + beta * c.double() + (0 if add is None else add.double())
+    bop = b if form in ("kn", "add") else b.transpose(1, 2).contiguous()
+    device.gemm(a, bop, c, m=m, n=n, k=k, batch=batch, trans_b=form not in ("kn", "add"), stride_a=m * k,
+                stride_b=n * k, stride_c=m * n, addend=add, stride_addend=m * n if add is not None else 0, beta=beta,
+                math=MATH_BF16 if form == "bf16" else MATH_TF32,
+                io_flags=IO_A_BF16 | IO_B_BF16 if form == "bf16" else IO_PAIR)
+    assert not device.gemm_timed_out()
+    assert nerr(c, want.float().cpu().numpy()) <= (1e-2 if form == "bf16" else 2e-3)
