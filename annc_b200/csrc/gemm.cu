@@ -41,6 +41,7 @@ static bool use_pair(const annc_gemm_desc& d, int math) {
   if (!pair_supported(d, math)) return false;
   if (math == ANNC_MATH_BF16 || (d.io_flags & (ANNC_IO_SOFTMAX | ANNC_IO_PAIR))) return true;
   if (!tc_supported(d, math)) return true;
+  if (d.io_flags & ANNC_IO_SINGLE) return false;
   const long long pair_tiles = ((d.m + 255) / 256) * ((d.n + 255) / 256) * d.batch;
   if (d.m >= 256 && d.n >= 192 && d.k >= 1024 && pair_tiles >= 74) return true;
   if (!pair_stores_by_tma(d)) return false;
@@ -51,7 +52,7 @@ static bool use_pair(const annc_gemm_desc& d, int math) {
 static int pick_math(const annc_gemm_desc& d) {
   if (d.math == ANNC_MATH_FP32) return ANNC_MATH_FP32;
   const int want = d.math == ANNC_MATH_AUTO ? ANNC_MATH_TF32 : d.math;
-  if (d.math == ANNC_MATH_AUTO && d.io_flags == 0 && (d.m < 64 || d.n < 16 || d.k < 32))
+  if (d.math == ANNC_MATH_AUTO && (d.io_flags & ~ANNC_IO_SINGLE) == 0 && (d.m < 64 || d.n < 16 || d.k < 32))
     return ANNC_MATH_FP32;  // tiny shapes stay on the CUDA cores
   return (tc_supported(d, want) || pair_supported(d, want)) ? want : ANNC_MATH_FP32;
 }
@@ -262,7 +263,7 @@ int annc_gemm_run(const annc_gemm_desc* desc, void* stream) {
   if (desc->math != ANNC_MATH_AUTO && desc->math != math)
     return fail(ANNC_ERR_UNSUPPORTED, "gemm: shape not supported by the requested math mode");
   if (math == ANNC_MATH_FP32) {
-    if (desc->io_flags != 0)
+    if ((desc->io_flags & ~ANNC_IO_SINGLE) != 0)
       return fail(ANNC_ERR_UNSUPPORTED, "gemm: io_flags need a tensor-core route this shape does not fit");
     return gemm::run_simt(*desc, s);
   }

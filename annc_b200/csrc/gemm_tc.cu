@@ -86,7 +86,9 @@ __device__ __noinline__ float4 sigmoid4(float4 v) {
 
 // ---------------------------------------------------------------- kernel
 template <int STAGES>
-__global__ void __launch_bounds__(NUM_THREADS, STAGES <= 3 ? 2 : 1)
+// (80 registers in the two-per-SM form, although shared memory is what limits it to two: a block then
+// still fits beside four blocks of the row exchange's pooling kernel)
+__global__ void __launch_bounds__(NUM_THREADS, STAGES <= 3 ? 4 : 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                          const __grid_constant__ CUtensorMap tmap_b, TcParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -301,23 +303,23 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tc_fence_after();
     if (done) {
       // Phase 1: this warp's 32 x 128 accumulator slab, scaled by alpha, goes to shared
-      // memory (the stage ring is idle once `done` has fired), rows padded to 132 floats; two
-      // tensor-memory loads in flight.
+      // memory (the stage ring is idle once `done` has fired), rows padded to 132 floats.
       float* slab = reinterpret_cast<float*>(gen_base) + (size_t)q * 32 * LD;
       const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16);
+      constexpr int CW = STAGES <= 3 ? 32 : 64;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 64) {
-        uint32_t r[2][32];
+      for (int c0 = 0; c0 < BN; c0 += CW) {
+        uint32_t r[CW / 32][32];
         if (KT > 0) {
           tmem_ld32(trow + (uint32_t)c0, r[0]);
-          tmem_ld32(trow + (uint32_t)c0 + 32u, r[1]);
+          if (CW == 64) tmem_ld32(trow + (uint32_t)c0 + 32u, r[CW / 32 - 1]);
           tmem_ld_wait();
         } else {  // a split-K rank without k-steps contributes zeros
 #pragma unroll
-          for (int j = 0; j < 64; ++j) r[j >> 5][j & 31] = 0u;
+          for (int j = 0; j < CW; ++j) r[j >> 5][j & 31] = 0u;
         }
 #pragma unroll
-        for (int j = 0; j < 64; j += 4) {
+        for (int j = 0; j < CW; j += 4) {
           const uint32_t* rj = &r[j >> 5][j & 31];
           *reinterpret_cast<float4*>(slab + lane * LD + c0 + j) =
               make_float4(p.alpha * __uint_as_float(rj[0]), p.alpha * __uint_as_float(rj[1]),
@@ -485,7 +487,7 @@ int max_clusters(int size) {
 }  // namespace
 
 bool tc_supported(const annc_gemm_desc& d, int math) {
-  if (math != ANNC_MATH_TF32 || d.io_flags != 0) return false;
+  if (math != ANNC_MATH_TF32 || (d.io_flags & ~ANNC_IO_SINGLE) != 0) return false;
   if (d.trans_a || d.batch < 1 || d.batch > 65535) return false;
   if (d.batch > 1) {  // strided batch: rank-3 tensor maps need 16-byte batch pitches
     if (d.b_format != ANNC_B_PLAIN || (d.stride_a & 3) || (d.stride_b & 3) || d.stride_a <= 0 ||

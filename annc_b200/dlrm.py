@@ -34,6 +34,7 @@ from .synth import DlrmModel
 
 class DlrmPipeline:
     embed_first = True  # forward() queues the pooling kernel before the bottom MLP
+    gemm_flags = 0
 
     def __init__(self, model: DlrmModel, device: torch.device, math: int = MATH_AUTO,
                  keep_host_inputs: bool = False):
@@ -178,7 +179,7 @@ class DlrmPipeline:
             y = self.z if last else self.acts_b[i]
             names.append(dev.gemm(x, w, y, m=B, n=w.shape[1], k=w.shape[0], bias=b,
                                   activation=ACT_RELU, ldc=(F * D if last else None),
-                                  math=self.math, stream=stream))
+                                  math=self.math, stream=stream, io_flags=self.gemm_flags))
             x = y
 
     def _sparse_part(self, names, lookahead: bool = False) -> None:
@@ -214,7 +215,7 @@ class DlrmPipeline:
             y = self.acts_t[i]
             act = ACT_SIGMOID if i == nt - 1 else ACT_RELU
             names.append(dev.gemm(x, w, y, m=B, n=w.shape[1], k=w.shape[0], bias=b, activation=act,
-                                  math=self.math))
+                                  math=self.math, io_flags=self.gemm_flags))
             x = y
         self.kernel_names = names
         # embedding launches + interaction + one kernel per MLP layer
@@ -278,6 +279,13 @@ class DlrmPipeline:
         main = torch.cuda.current_stream()
         main.wait_event(self._dense_done[buf])  # the step before last has finished with this set
         names = []
+        if self.embed_first:
+            # One GPU: no dense kernel fits on an SM beside the pooling kernel, and the two streams only
+            # keep each other's blocks waiting (batch 65536: 1.44 ms a step against 0.90 ms).
+            self._sparse_part(names)
+            self._dense_part(names)
+            self._dense_done[buf].record(main)
+            return self.out
         self._sparse_part(names, lookahead=True)
         self.dense_stream.wait_stream(main)
         with torch.cuda.stream(self.dense_stream):

@@ -351,13 +351,14 @@ def _make_pipeline(model, device, mode: str, math=None, keep_host_inputs: bool =
     import torch.distributed as dist
 
     from . import device as dev
-    from ._lib import MATH_AUTO, lib
+    from ._lib import IO_SINGLE, MATH_AUTO, lib
     from .dlrm import DlrmPipeline
 
     world, rank = dist.get_world_size(), dist.get_rank()
 
     class _Pipe(DlrmPipeline):
         embed_first = False  # the exchange waits for its peers: the bottom MLP runs in that time
+        gemm_flags = IO_SINGLE  # and the layers run beside the pooling kernel
 
         def _setup_embedding(self, m) -> None:
             emb = m.emb
