@@ -38,11 +38,11 @@ UNIT = "samples/s"
 
 # DRAM bytes (read + write) of one bag-kernel launch: a constant, not measured by this run.  It is
 # the dram__bytes_read.sum + dram__bytes_write.sum of a profiler capture of the small case
-# (batch 16384, rows <= 1e6: 0.5465 GB for 4,472,660 lookups) scaled to this workload by the lookups
-# per launch; traffic grows in proportion (the same scaling of the previous kernel's small-case
-# figure matched a full-size capture within 2 %).  Keyed by (batch, max_rows, seed); any other
+# (batch 16384, rows <= 1e6: 0.7148 GB for 4,472,660 lookups) scaled to this workload by the lookups
+# per launch (an upper estimate: the large batch walks its tables in shorter chunks, which share more
+# of L2).  Keyed by (batch, max_rows, seed); any other
 # workload reports null.
-NCU_BAG_TRAFFIC_BYTES = {(65536, 1e7, 0): 0.5465e9 * 17883957 / 4472660}
+NCU_BAG_TRAFFIC_BYTES = {(65536, 1e7, 0): 0.7148e9 * 17883957 / 4472660}
 
 
 def parse_args():
@@ -435,7 +435,7 @@ def run_gpu(args):
                                  input_seed=(1000 + rank) if world > 1 else None)
         emb_bytes = model.emb.algorithmic_bytes()
         nnz = model.emb.nnz
-        bag_kernel = "bag_stream_kernel<8,4,2,16,2,5> (hash-bucket + gather + segment sum, 26 tables in one launch)"
+        bag_kernel = "bag_stream_kernel<8,2,2,true,4> (hash-bucket + gather + segment sum, 26 tables in one launch)"
 
         def build(mode):
             if world == 1:
