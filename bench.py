@@ -39,8 +39,7 @@ UNIT = "samples/s"
 # DRAM bytes (read + write) of one bag-kernel launch: a constant, not measured by this run.  It is
 # the dram__bytes_read.sum + dram__bytes_write.sum of a profiler capture of the small case
 # (batch 16384, rows <= 1e6: 0.7148 GB for 4,472,660 lookups) scaled to this workload by the lookups
-# per launch (an upper estimate: the large batch walks its tables in shorter chunks, which share more
-# of L2).  Keyed by (batch, max_rows, seed); any other
+# per launch (not checked against a capture of the full size).  Keyed by (batch, max_rows, seed); any other
 # workload reports null.
 NCU_BAG_TRAFFIC_BYTES = {(65536, 1e7, 0): 0.7148e9 * 17883957 / 4472660}
 
@@ -460,7 +459,7 @@ def run_gpu(args):
     it = iter(pairs)
 
     # Back-to-back batches may be issued in two orders: one step after the other (forward), or
-    # with the dense part of a step (interaction + top MLP) on a second stream under the next
+    # with the dense part of a step (interaction + top MLP; sharded: on a second stream) under the next
     # step's embedding part and, under row sharding, the split of the next step under this
     # step's pooling (DlrmPipeline.forward_pipelined).  Which one is faster depends on how much
     # of the GPU the embedding part leaves free; five steps of each decide, the same on all ranks.
@@ -636,9 +635,10 @@ def run_gpu(args):
                         "host_cores_local_to_gpu": numa_cores},
                 "ms_per_step_unpipelined": ms_alone,
                 "pipelining": ("the timed steps are issued back to back in the order '%s' (chosen by five "
-                               "calibration steps of each order): work of neighbouring steps overlaps on "
-                               "second and third streams, two sets of intermediate buffers; "
-                               "ms_per_step_unpipelined is one step with nothing overlapping it" % issue_order)
+                               "calibration steps of each order): %s, two sets of intermediate buffers; "
+                               "ms_per_step_unpipelined is one step with nothing overlapping it"
+                               % (issue_order, "one stream" if world == 1 else
+                                  "work of neighbouring steps overlaps on second and third streams"))
                               if issue_order != "none" else "none",
                 "issue_orders_ms_per_step": order_ms,
                 "gpu_launches": pipe.launches_per_step * args.steps,
