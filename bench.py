@@ -599,7 +599,7 @@ def run_gpu(args):
                     "peak_source": peak_source,
                     "label": "algorithmic GB/s (L2-assisted): algorithmic bytes per launch / kernel time; "
                              "Zipf-hot rows are served by L2, so DRAM moves less (dram_frac)",
-                    "limited_by": "instruction issue and L2 / row-gather latency, not DRAM bandwidth",
+                    "limited_by": "row-gather latency (DRAM and L2) and instruction issue",
                     "algorithmic_bytes_per_launch": emb_bytes, "lookups_per_launch": nnz,
                     "kernel_ms": bag_avg_ms, "traffic": traffic,
                     "traffic_source": "constant, not measured by this run: ncu dram__bytes_read.sum + "
