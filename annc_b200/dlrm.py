@@ -270,10 +270,11 @@ class DlrmPipeline:
         return self.out
 
     def forward_pipelined(self, split: bool = False) -> torch.Tensor:
-        """One step of a back-to-back sequence: its dense part is queued on `dense_stream` and
-        overlaps the next step's embedding part.  The returned tensor is valid after
-        sync_pipeline() (or a device synchronize).  split=True (pipelines with split_finish):
-        the closing pass of the embedding part runs on the dense stream too."""
+        """One step of a back-to-back sequence.  One GPU (embed_first): all of it is queued on the
+        current stream.  Otherwise the dense part is queued on `dense_stream` and overlaps the next
+        step's embedding part.  The returned tensor is valid after sync_pipeline() (or a device
+        synchronize).  split=True (pipelines with split_finish): the closing pass of the embedding
+        part runs on the dense stream too."""
         if split and self.split_finish:
             return self._forward_split()
         buf = self._pstep % 2
@@ -297,10 +298,12 @@ class DlrmPipeline:
         return self.out
 
     def sync_pipeline(self) -> None:
-        """Orders the current stream after every queued dense part."""
+        """Orders the current stream after every queued dense part, whichever stream it is on."""
         main = torch.cuda.current_stream()
         main.wait_stream(self.dense_stream)
         main.wait_stream(self.side_stream)
+        for done in self._dense_done:  # the last step of either buffer set; each waited for those before it
+            main.wait_event(done)
 
     def _issue_copy(self, i: int) -> None:
         st = self.sets[i]

@@ -30,6 +30,28 @@ def test_dlrm_step_matches_oracle(math, tol):
     np.testing.assert_array_equal(h.numpy(), got)
 
 
+def test_pipelined_steps_of_another_stream_are_waited_for():
+    """Steps issued under one stream, sync_pipeline() and the reads on another: the results are
+    complete there, and a forward() after it does not write over a buffer set still in use."""
+    model = synth.dlrm_model(seed=4, batch=8192, max_rows=2e4)
+    pipe = DlrmPipeline(model, torch.device("cuda:0"))
+    want = pipe.forward().clone()
+    torch.cuda.synchronize()
+    other = torch.cuda.Stream()
+    for steps in (1, 2, 3):
+        for b in pipe._bufs:
+            b["acts_t"][-1].fill_(-1.0)
+        other.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(other):
+            outs = [pipe.forward_pipelined() for _ in range(steps)]
+        pipe.sync_pipeline()
+        got = [o.clone() for o in outs[-2:]]
+        again = pipe.forward().clone()
+        torch.cuda.synchronize()
+        for o in got + [again]:
+            assert torch.equal(o, want)
+
+
 def test_smoke_entry():
     import __graft_entry__ as g
     g.smoke()
