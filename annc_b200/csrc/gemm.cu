@@ -183,7 +183,8 @@ bf16_weight_kernel(const float* __restrict__ src, long long ldb, __nv_bfloat16* 
 int relaid_desc(const annc_gemm_desc& d, void* ws, size_t ws_bytes, annc_gemm_desc* plain) {
   if (d.b_format != ANNC_B_KN4 || !ws || d.batch != 1) return 0;
   if (ws_bytes < (size_t)d.k * (size_t)d.n * sizeof(float)) return 0;
-  if ((reinterpret_cast<uintptr_t>(ws) & 15) || (d.n & 3) || d.m < 64) return 0;
+  // the packed weight is read in 16-byte pieces too
+  if (((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(d.b)) & 15) || (d.n & 3) || d.m < 64) return 0;
   if (d.k >= (1LL << 31) || d.n >= (1LL << 31) || (d.k + kRelayK - 1) / kRelayK > 65535) return 0;
   *plain = d;
   plain->b = static_cast<const float*>(ws);

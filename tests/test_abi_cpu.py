@@ -204,3 +204,22 @@ def test_kernel_map_resolves_library_symbols(annc):
     arr2 = (C.c_int * 2)(1, 2)
     assert annc.lib.annc_kernel_map_resolve(b"gemv", arr2, 2) is None
     annc.lib.annc_kernel_map_clear()
+
+
+# ---------------------------------------------------------------- when a packed weight is re-laid
+def _relaid_form(annc, m, k, n, weight=1 << 20):
+    """Form the library re-lays a kn4 weight at this (never read) address into for such a product:
+    1 = [N,K], 2 = [K,N], 0 = the weight is taken as it lies."""
+    fn = getattr(annc.lib, "_ZN4annc4gemm11relaid_descERK14annc_gemm_descPvmPS1_")  # gemm::relaid_desc
+    fn.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+    from annc_b200._lib import B_KN4, GemmDesc
+    d = GemmDesc(0, 0, m, n, k, 1, k, n, n, n, 0, 0, 0, 0, 1.0, 0.0, 2 << 20, weight, 3 << 20, None, None, 0, B_KN4)
+    return fn(C.byref(d), 4 << 20, 4 * k * n, C.byref(GemmDesc()))
+
+
+@pytest.mark.parametrize("m,k,n", [(64, 512, 256), (200, 2048, 4096), (8192, 2048, 4096)])
+def test_a_packed_weight_off_16_bytes_is_not_relaid(annc, m, k, n):
+    """The kernel that re-lays a weight reads it in 16-byte pieces."""
+    assert _relaid_form(annc, m, k, n) != 0
+    for off in (4, 8, 12):
+        assert _relaid_form(annc, m, k, n, weight=(1 << 20) + off) == 0

@@ -249,6 +249,20 @@ def test_layout_matmul_device_weight(m, n, k):
     assert nerr(got, want) <= 2e-3  # TF32
 
 
+@pytest.mark.parametrize("off", [1, 2, 3])
+def test_layout_matmul_device_weight_off_16_bytes(off):
+    """A packed weight that is a view at an odd place of a larger buffer."""
+    g = torch.Generator(device="cuda").manual_seed(off)
+    m, k, n = 200, 356, 264
+    a = torch.randn((m, k), device="cuda", generator=g)
+    w = torch.randn((k, n), device="cuda", generator=g)
+    packed = torch.empty(k * n + off, device="cuda")[off:].view(k, n).copy_(device.kn4_pack(w))
+    assert packed.data_ptr() % 16 == 4 * off
+    got = ops.xla_layout_matmul(a, packed)
+    want = (a.double() @ w.double()).cpu().numpy()
+    assert nerr(got, want) <= 2e-5  # the fp32 route
+
+
 def test_layout_matmul_device_weight_streams_and_capture():
     """The scratch is safe across streams of a thread, and a captured call does without it."""
     g = torch.Generator(device="cuda").manual_seed(5)
