@@ -56,12 +56,14 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
   d.b_format = b_format;
   d.math = ANNC_MATH_AUTO;
   if (call.status() != ANNC_OK) return call.status();
-  if (b_format == ANNC_B_KN4 && (n & 3) == 0 && batch == 1) {
-    const size_t ws_bytes = (size_t)k * (size_t)n * sizeof(float);
+  const size_t ws_bytes = (size_t)k * (size_t)n * sizeof(float);
+  annc_gemm_desc plain;
+  // Asked before a buffer is taken, for one that is not filled may not be kept (the place of the buffer
+  // only counts by its alignment: the weight's own stands for it).
+  if (gemm::relaid_desc(d, const_cast<float*>(d.b), ws_bytes, &plain)) {
     bool fresh = false;
     void* ws = call.derived(b, b_count * sizeof(float), /*tag: re-laid kn4*/ 1, ws_bytes, &fresh);
-    annc_gemm_desc plain;
-    if (!ws && gemm::relaid_desc(d, /*any aligned address*/ d.c, ws_bytes, &plain)) {
+    if (!ws) {
       // A weight on the device (or not to be kept): re-laid into scratch by every call.  The pass
       // over the weight costs 8 us at 2048 x 4096 and 2 us at 256 x 512; the loader that takes the
       // packed panels as they lie is further behind at every size: 64 rows 24 us against 21 us in
@@ -69,8 +71,7 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
       ws = call.optional_scratch(ws_bytes);
       fresh = ws != nullptr;
     }
-    const int form = ws ? gemm::relaid_desc(d, ws, ws_bytes, &plain) : 0;
-    if (form) {
+    if (const int form = gemm::relaid_desc(d, ws, ws_bytes, &plain)) {
       if (fresh) gemm::relay_kn4(d.b, static_cast<float*>(ws), k, n, form, call.stream());
       d = plain;
     }

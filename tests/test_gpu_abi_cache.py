@@ -140,6 +140,31 @@ def test_layout_matmul_keeps_the_relaid_weight():
     assert counters()[0] - h1 == 0
 
 
+def _host_layout_matmul(x, packed):
+    out = torch.empty((x.shape[0], packed.shape[1]), device="cuda")
+    ops._call_custom("__layout_matmul", out, [x, packed, ops.shape_info(x), ops.shape_info(packed)])
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _host_weight(k, n):
+    """Device activations of a drawn batch, a packed weight in a host buffer of its own, the weight."""
+    rng = np.random.default_rng(k + n)
+    w = (rng.standard_normal((k, n)) / 16).astype(np.float32)
+    return lambda m: rng.standard_normal((m, k)).astype(np.float32), oracle.kn4_pack(w), w
+
+
+@pytest.mark.parametrize("first", [1, 63])
+def test_layout_matmul_host_weight_first_seen_by_a_small_batch(first):
+    """A batch too small for the re-laid form leaves nothing behind that a larger one would take for it."""
+    k, n = 512, 1028
+    draw, packed, w = _host_weight(k, n)
+    for m in (first, 200, first, 300):
+        x = draw(m)
+        got = _host_layout_matmul(torch.from_numpy(x).cuda(), packed)
+        assert nerr(got, x.astype(np.float64) @ w) <= 2e-3
+
+
 def test_a_wait_that_ran_out_is_reported(capfd):
     rng = np.random.default_rng(3)
     a = rng.standard_normal((256, 256)).astype(np.float32)
