@@ -256,7 +256,7 @@ struct Mirror {
   int users = 0;                 // calls copying into the mirror right now: not to be evicted
   cudaEvent_t ready = nullptr;   // after the last write of the mirror
   cudaEvent_t used = nullptr;    // after the last read of the mirror
-  std::unordered_map<int, std::pair<void*, size_t>> derived;  // re-laid forms of a constant, by tag
+  std::unordered_map<long long, std::pair<void*, size_t>> derived;  // re-laid forms of a constant, by tag
 };
 std::mutex g_mu;
 std::unordered_map<Key, Mirror, KeyHash> g_mirrors;
@@ -539,7 +539,7 @@ void* Call::optional_scratch(size_t bytes) {
 
 // A re-laid form (`tag`) of constant host operand p, kept with its mirror: returns the cached
 // device buffer, or allocates `out_bytes` and sets *fresh so that the caller fills it.
-void* Call::derived(const void* p, size_t bytes, int tag, size_t out_bytes, bool* fresh) {
+void* Call::derived(const void* p, size_t bytes, long long tag, size_t out_bytes, bool* fresh) {
   *fresh = false;
   if (status_ != ANNC_OK) return nullptr;
   std::lock_guard<std::mutex> lk(g_mu);

@@ -100,7 +100,7 @@ class Call {
   // A re-laid form (`tag`) of host operand p whose mirror is reusable: the cached buffer, or a
   // new one of out_bytes with *fresh set (the caller fills it).  nullptr when p has no reusable
   // mirror (device pointer, cache off) or memory is short: the caller then works without it.
-  void* derived(const void* p, size_t bytes, int tag, size_t out_bytes, bool* fresh);
+  void* derived(const void* p, size_t bytes, long long tag, size_t out_bytes, bool* fresh);
   // Small host read of possibly-device memory (synchronous).
   int read_host(const void* p, size_t bytes, void* dst);
   // Waits for the call's stream (an operator whose outputs are complete when it returns).

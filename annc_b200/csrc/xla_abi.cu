@@ -60,9 +60,11 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
   annc_gemm_desc plain;
   // Asked before a buffer is taken, for one that is not filled may not be kept (the place of the buffer
   // only counts by its alignment: the weight's own stands for it).
-  if (gemm::relaid_desc(d, const_cast<float*>(d.b), ws_bytes, &plain)) {
+  if (const int form = gemm::relaid_desc(d, const_cast<float*>(d.b), ws_bytes, &plain)) {
     bool fresh = false;
-    void* ws = call.derived(b, b_count * sizeof(float), /*tag: re-laid kn4*/ 1, ws_bytes, &fresh);
+    // One kept copy per layout: the form goes with the batch, and the same bytes may be a weight of
+    // another shape.
+    void* ws = call.derived(b, b_count * sizeof(float), /*tag*/ 4 * n + form, ws_bytes, &fresh);
     if (!ws) {
       // A weight on the device (or not to be kept): re-laid into scratch by every call.  The pass
       // over the weight costs 8 us at 2048 x 4096 and 2 us at 256 x 512; the loader that takes the
@@ -71,7 +73,7 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
       ws = call.optional_scratch(ws_bytes);
       fresh = ws != nullptr;
     }
-    if (const int form = gemm::relaid_desc(d, ws, ws_bytes, &plain)) {
+    if (ws && gemm::relaid_desc(d, ws, ws_bytes, &plain) == form) {
       if (fresh) gemm::relay_kn4(d.b, static_cast<float*>(ws), k, n, form, call.stream());
       d = plain;
     }

@@ -165,6 +165,22 @@ def test_layout_matmul_host_weight_first_seen_by_a_small_batch(first):
         assert nerr(got, x.astype(np.float64) @ w) <= 2e-3
 
 
+def test_layout_matmul_host_weight_in_both_layouts():
+    """The re-laid layout goes with the batch (column tiles of a large one want [N,K]): each is kept on
+    its own, and a weight of another shape in the same bytes has its own as well."""
+    k, n = 2048, 1024
+    draw, packed, w = _host_weight(k, n)
+    for m in (8192, 200, 8192, 70):
+        x = draw(m)
+        got = _host_layout_matmul(torch.from_numpy(x).cuda(), packed)
+        assert nerr(got, x.astype(np.float64) @ w) <= 2e-3
+    other = packed.reshape(n, k)
+    w2 = oracle.kn4_unpack(other, n, k)
+    x = np.random.default_rng(1).standard_normal((200, n)).astype(np.float32)
+    got = _host_layout_matmul(torch.from_numpy(x).cuda(), other)
+    assert nerr(got, x.astype(np.float64) @ w2) <= 2e-3
+
+
 def test_a_wait_that_ran_out_is_reported(capfd):
     rng = np.random.default_rng(3)
     a = rng.standard_normal((256, 256)).astype(np.float32)
