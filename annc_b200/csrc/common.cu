@@ -246,6 +246,11 @@ struct KeyHash {
     return h ^ (size_t)k.device;
   }
 };
+struct Relaid {
+  void* dev;
+  size_t bytes;
+  cudaEvent_t filled;  // after the pass that filled it
+};
 struct Mirror {
   void* dev = nullptr;
   size_t bytes = 0;
@@ -256,7 +261,7 @@ struct Mirror {
   int users = 0;                 // calls copying into the mirror right now: not to be evicted
   cudaEvent_t ready = nullptr;   // after the last write of the mirror
   cudaEvent_t used = nullptr;    // after the last read of the mirror
-  std::unordered_map<long long, std::pair<void*, size_t>> derived;  // re-laid forms of a constant, by tag
+  std::unordered_map<long long, Relaid> derived;  // re-laid forms of a constant, by tag
 };
 std::mutex g_mu;
 std::unordered_map<Key, Mirror, KeyHash> g_mirrors;
@@ -303,13 +308,21 @@ unsigned long long fingerprint(const void* p, size_t bytes, size_t max_samples =
   return h;
 }
 
+void free_derived(Mirror& m) {
+  for (auto& d : m.derived) {
+    cudaFree(d.second.dev);
+    cudaEventDestroy(d.second.filled);
+    g_mirror_bytes -= d.second.bytes;
+  }
+  m.derived.clear();
+}
+
 void free_mirror(Mirror& m) {
   if (m.dev) cudaFree(m.dev);
-  for (auto& d : m.derived) cudaFree(d.second.first);
+  free_derived(m);
   if (m.ready) cudaEventDestroy(m.ready);
   if (m.used) cudaEventDestroy(m.used);
   g_mirror_bytes -= m.bytes;
-  for (auto& d : m.derived) g_mirror_bytes -= d.second.second;
 }
 
 // Drops least recently used mirrors until `need` more bytes fit under the cap (called with g_mu held).
@@ -464,11 +477,7 @@ void* Call::mirror(const void* p, size_t bytes, bool upload, bool role_constant,
       cudaStreamWaitEvent(stream_, m.used, 0);
       cudaStreamWaitEvent(stream_, m.ready, 0);
       m.valid = false;  // becomes valid again in finish(), once the host copy exists
-      for (auto& d : m.derived) {
-        cudaFree(d.second.first);
-        g_mirror_bytes -= d.second.second;
-      }
-      m.derived.clear();
+      free_derived(m);
     }
   }
   if (need) {  // the copy itself runs outside the lock: other threads' calls go on
@@ -483,11 +492,7 @@ void* Call::mirror(const void* p, size_t bytes, bool upload, bool role_constant,
     g_staged_h2d += bytes;
     mp->valid = may_reuse;
     mp->print = fp;
-    for (auto& d : mp->derived) {  // re-laid forms are stale now
-      cudaFree(d.second.first);
-      g_mirror_bytes -= d.second.second;
-    }
-    mp->derived.clear();
+    free_derived(*mp);  // re-laid forms are stale now
     staged_ = true;
   }
   return mp->dev;
@@ -537,27 +542,33 @@ void* Call::optional_scratch(size_t bytes) {
   return d;
 }
 
-// A re-laid form (`tag`) of constant host operand p, kept with its mirror: returns the cached
-// device buffer, or allocates `out_bytes` and sets *fresh so that the caller fills it.
-void* Call::derived(const void* p, size_t bytes, long long tag, size_t out_bytes, bool* fresh) {
-  *fresh = false;
+// A re-laid form (`tag`) of constant host operand p, kept with its mirror: the cached device buffer, or
+// a new one of `out_bytes`, queued to be filled on this call's stream before the lock is given up;
+// other streams and threads wait for that pass.
+void* Call::derived(const void* p, size_t bytes, long long tag, size_t out_bytes,
+                    const std::function<void(void*)>& fill) {
   if (status_ != ANNC_OK) return nullptr;
   std::lock_guard<std::mutex> lk(g_mu);
   auto it = g_mirrors.find(Key{p, bytes ? bytes : 1, device_});
   if (it == g_mirrors.end() || !it->second.valid) return nullptr;  // not a mirrored, reusable operand
   Mirror& m = it->second;
   auto d = m.derived.find(tag);
-  if (d != m.derived.end() && d->second.second == out_bytes) return d->second.first;
+  if (d != m.derived.end()) {
+    cudaStreamWaitEvent(stream_, d->second.filled, 0);
+    return d->second.dev;
+  }
   make_room(out_bytes, &it->first);
-  void* buf = nullptr;
-  if (cudaMalloc(&buf, out_bytes) != cudaSuccess) {
+  Relaid r{nullptr, out_bytes, nullptr};
+  if (cudaMalloc(&r.dev, out_bytes) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  m.derived[tag] = {buf, out_bytes};
+  cudaEventCreateWithFlags(&r.filled, cudaEventDisableTiming);
+  fill(r.dev);
+  cudaEventRecord(r.filled, stream_);
+  m.derived[tag] = r;
   g_mirror_bytes += out_bytes;
-  *fresh = true;
-  return buf;
+  return r.dev;
 }
 
 int Call::read_host(const void* p, size_t bytes, void* dst) {

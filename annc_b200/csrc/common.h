@@ -7,6 +7,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "annc_b200.h"
@@ -97,10 +98,12 @@ class Call {
   // holds at most twice the limit of them however the sizes vary.
   static constexpr size_t kMaxOptionalScratch = size_t(256) << 20;
   void* optional_scratch(size_t bytes);
-  // A re-laid form (`tag`) of host operand p whose mirror is reusable: the cached buffer, or a
-  // new one of out_bytes with *fresh set (the caller fills it).  nullptr when p has no reusable
-  // mirror (device pointer, cache off) or memory is short: the caller then works without it.
-  void* derived(const void* p, size_t bytes, long long tag, size_t out_bytes, bool* fresh);
+  // A re-laid form (`tag`, which fixes out_bytes) of host operand p whose mirror is reusable: the
+  // cached buffer, or a new one that `fill` is called for (it queues the pass on stream()).  nullptr
+  // when p has no reusable mirror (device pointer, cache off) or memory is short: the caller then
+  // works without it.
+  void* derived(const void* p, size_t bytes, long long tag, size_t out_bytes,
+                const std::function<void(void*)>& fill);
   // Small host read of possibly-device memory (synchronous).
   int read_host(const void* p, size_t bytes, void* dst);
   // Waits for the call's stream (an operator whose outputs are complete when it returns).

@@ -181,6 +181,26 @@ def test_layout_matmul_host_weight_in_both_layouts():
     assert nerr(got, x.astype(np.float64) @ w2) <= 2e-3
 
 
+def test_layout_matmul_host_weight_across_streams():
+    """A stream that finds the re-laid copy of another waits for the pass that fills it."""
+    k, n = 1024, 516
+    draw, packed, w = _host_weight(k, n)
+    _host_layout_matmul(torch.from_numpy(draw(1)).cuda(), packed)  # uploads the weight, re-lays nothing
+    x = [draw(200), draw(200)]
+    xd = [torch.from_numpy(a).cuda() for a in x]
+    out = [torch.empty((200, n), device="cuda") for _ in x]
+    torch.cuda.synchronize()
+    for i, s in enumerate([torch.cuda.Stream(), torch.cuda.Stream()]):
+        with torch.cuda.stream(s):
+            if i == 0:
+                torch.cuda._sleep(100_000_000)  # the first stream is late
+            ops._use_current_stream()
+            ops._call_custom("__layout_matmul", out[i], [xd[i], packed, ops.shape_info(x[i]), ops.shape_info(packed)])
+    torch.cuda.synchronize()
+    for a, o in zip(x, out):
+        assert nerr(o.cpu().numpy(), a.astype(np.float64) @ w) <= 2e-3
+
+
 def test_a_wait_that_ran_out_is_reported(capfd):
     rng = np.random.default_rng(3)
     a = rng.standard_normal((256, 256)).astype(np.float32)
