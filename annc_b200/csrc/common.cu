@@ -669,6 +669,7 @@ int annc_register_constant(const void* ptr, size_t bytes) {
   cudaError_t e = cudaMemcpy(m.dev, ptr, bytes, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(constant)");
   g_staged_h2d += bytes;
+  free_derived(m);  // re-laid forms of the former contents
   m.valid = true;
   m.pinned = true;
   m.print = fingerprint(ptr, bytes);

@@ -201,6 +201,21 @@ def test_layout_matmul_host_weight_across_streams():
         assert nerr(o.cpu().numpy(), a.astype(np.float64) @ w) <= 2e-3
 
 
+def test_layout_matmul_constant_registered_again():
+    """A registered weight whose contents change is registered again: its re-laid copy follows."""
+    k, n = 352, 260
+    draw, packed, w = _host_weight(k, n)
+    x = draw(200)
+    try:
+        for scale in (1.0, -3.0):
+            packed[:] = oracle.kn4_pack((scale * w).astype(np.float32))
+            assert lib.annc_register_constant(packed.ctypes.data, packed.nbytes) == 0
+            got = _host_layout_matmul(torch.from_numpy(x).cuda(), packed)
+            assert nerr(got, scale * (x.astype(np.float64) @ w)) <= 2e-3
+    finally:
+        assert lib.annc_unregister_constant(packed.ctypes.data) == 0
+
+
 def test_a_wait_that_ran_out_is_reported(capfd):
     rng = np.random.default_rng(3)
     a = rng.standard_normal((256, 256)).astype(np.float32)
