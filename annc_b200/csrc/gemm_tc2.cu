@@ -113,37 +113,53 @@ __device__ __forceinline__ float act_apply(float v, int act) {
   return v;
 }
 
+// The parts of the softmax epilogue that a plain batch_matmul + softmax does not use, out of line: its
+// loop body is unrolled over 32 columns, and with these inside it is bound by instruction fetch.
+__device__ __noinline__ float4 sigmoid4(float4 v) {
+  return make_float4(act_apply(v.x, ANNC_ACT_SIGMOID), act_apply(v.y, ANNC_ACT_SIGMOID),
+                     act_apply(v.z, ANNC_ACT_SIGMOID), act_apply(v.w, ANNC_ACT_SIGMOID));
+}
+// v + beta * C + addend + bias at the first `cols` of four columns (null: not added).
+__device__ __noinline__ float4 add_terms(float4 v, const void* c, int c_bf16, float beta, const float* addend,
+                                         const float* bias, int cols) {
+  float t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (e >= cols) break;
+    if (c) t[e] += beta * (c_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(c)[e]) : static_cast<const float*>(c)[e]);
+    if (addend) t[e] += __ldg(addend + e);
+    if (bias) t[e] += __ldg(bias + e);
+  }
+  return make_float4(t[0], t[1], t[2], t[3]);
+}
+
 // Per-row form of the epilogue (the softmax needs whole rows in one thread): values of one
-// 32-column chunk of this thread's row before the activation,
-// alpha * acc (+ beta * C) (+ addend) (+ bias).
+// 32-column chunk of this thread's row, act(alpha * acc (+ beta * C) (+ addend) (+ bias)).
 __device__ __forceinline__ void chunk_values(const PairParams& p, const uint32_t (&r)[32], float (&v)[32],
                                              long long grow, int col0, long long bz, bool row_ok) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = p.alpha * __uint_as_float(r[j]);
-  if (!row_ok) return;
-  if (p.beta != 0.f) {
-    if (p.c_bf16) {
-      const __nv_bfloat16* c = static_cast<const __nv_bfloat16*>(p.C) + bz * p.stride_c + grow * p.ldc + col0;
+  if (row_ok && (p.beta != 0.f || p.addend || p.bias)) {
+    const long long coff = bz * p.stride_c + grow * p.ldc + col0;
+    const char* c = p.beta != 0.f ? static_cast<const char*>(p.C) + coff * (p.c_bf16 ? 2 : 4) : nullptr;
+    const float* addend = p.addend ? p.addend + bz * p.stride_addend + grow * p.ld_addend + col0 : nullptr;
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (col0 + j < p.N) v[j] += p.beta * __bfloat162float(c[j]);
-    } else {
-      const float* c = static_cast<const float*>(p.C) + bz * p.stride_c + grow * p.ldc + col0;
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (col0 + j < p.N) v[j] += p.beta * c[j];
+    for (int j = 0; j < 32; j += 4) {
+      const float4 t = add_terms(make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]), c ? c + j * (p.c_bf16 ? 2 : 4) : nullptr,
+                                 p.c_bf16, p.beta, addend ? addend + j : nullptr,
+                                 p.bias ? p.bias + col0 + j : nullptr, p.N - col0 - j);
+      v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
     }
   }
-  if (p.addend) {
-    const float* a = p.addend + bz * p.stride_addend + grow * p.ld_addend + col0;
+  if (p.act == ANNC_ACT_RELU) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (col0 + j < p.N) v[j] += __ldg(a + j);
-  }
-  if (p.bias) {
+    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+  } else if (p.act == ANNC_ACT_SIGMOID) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (col0 + j < p.N) v[j] += __ldg(p.bias + col0 + j);
+    for (int j = 0; j < 32; j += 4) {
+      const float4 t = sigmoid4(make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+      v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
+    }
   }
 }
 
@@ -566,7 +582,9 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
         } else if (half == 0) {
           // row softmax: one thread per row over all N <= 256 columns, three passes over the
-          // row in tensor memory: max, sum of exp, normalised store (warps of half 1 idle)
+          // row in tensor memory: max, sum of exp, normalised store (warps of half 1 idle).  Bound by
+          // the instructions of these passes: 64 x [256 x 256 x 64] 37 us, 58.5 us with every term
+          // and activation of chunk_values unrolled here.
           const float no_bias[4] = {0.f, 0.f, 0.f, 0.f};
           float mx = -INFINITY, sum = 0.f;
 #pragma unroll 1
@@ -578,8 +596,6 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
               tmem_ld32(taddr + (uint32_t)c0, r);
               tmem_ld_wait();
               chunk_values(p, r, v, grow, c0, bz, row_ok);
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = act_apply(v[j], p.act);
               if (pass == 0) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j)

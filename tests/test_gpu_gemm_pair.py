@@ -183,3 +183,31 @@ def test_pair_half_tiles(m, n, k, batch, form):
                 io_flags=IO_A_BF16 | IO_B_BF16 if form == "bf16" else IO_PAIR)
     assert not device.gemm_timed_out()
     assert nerr(c, want.float().cpu().numpy()) <= (1e-2 if form == "bf16" else 2e-3)
+
+
+@pytest.mark.parametrize("n,m,batch", [(256, 256, 2), (130, 257, 1), (33, 100, 3)])
+@pytest.mark.parametrize("act", [ACT_NONE, ACT_RELU, ACT_SIGMOID])
+@pytest.mark.parametrize("terms", ["", "bias", "addend", "beta", "all"])
+def test_pair_softmax_terms(n, m, batch, act, terms):
+    """Row softmax over act(alpha * A B + beta * C + addend + bias), at row and column remainders.  Against
+    fp64: the products are off by 2^-9 of their size (operands cut to 11 bits), a softmax value by at
+    most twice that error of its exponent."""
+    g = torch.Generator(device="cuda").manual_seed(n + m)
+    k = 64
+    a = torch.randn((batch, m, k), device="cuda", generator=g) / 8
+    b = torch.randn((batch, n, k), device="cuda", generator=g) / 8
+    c = torch.randn((batch, m, n), device="cuda", generator=g)
+    add = torch.randn((batch, m, n), device="cuda", generator=g) if terms in ("addend", "all") else None
+    bias = torch.randn(n, device="cuda", generator=g) if terms in ("bias", "all") else None
+    beta = -0.5 if terms in ("beta", "all") else 0.0
+    want = 0.75 * (a.double() @ b.double().transpose(1, 2)) + beta * c.double()
+    size = 0.75 * (a.double().abs() @ b.double().abs().transpose(1, 2))
+    want = want + (0 if add is None else add.double()) + (0 if bias is None else bias.double())
+    want = want.relu() if act == ACT_RELU else want.sigmoid() if act == ACT_SIGMOID else want
+    want = torch.softmax(want, -1)
+    device.gemm(a, b, c, m=m, n=n, k=k, batch=batch, trans_b=True, stride_a=m * k, stride_b=n * k, stride_c=m * n,
+                alpha=0.75, beta=beta, addend=add, stride_addend=m * n if add is not None else 0, bias=bias,
+                activation=act, math=MATH_TF32, io_flags=IO_SOFTMAX)
+    assert not device.gemm_timed_out()
+    err = 2.0 ** -8 * float(size.max()) + 1e-5
+    assert ((c - want).abs() <= err * want).all()
