@@ -62,27 +62,30 @@ static int stream_chunk(long long lookups, int num_tables, int lanes, long long 
   return best;
 }
 
-template <int LANES, int VPL, int DEPTH, bool FULL, int MINB>
-static void launch_stream(const BagParams& p, BagHeader* hdr, cudaStream_t s) {
-  static int per_sm[kMaxDevices] = {0}, sm_count[kMaxDevices] = {0};
+// A lookup-granular kernel: lanes of a group, and its resident blocks per SM by device (0: not asked).
+struct StreamShape {
+  void (*kernel)(BagParams, StreamChunks, BagHeader*);
+  int lanes;
+  int per_sm[kMaxDevices];
+};
+
+static void launch_stream(StreamShape& shape, const BagParams& p, BagHeader* hdr, cudaStream_t s) {
   const int slot = device_slot();
-  if (!per_sm[slot]) {
-    int n = 0, sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bag_stream_kernel<LANES, VPL, DEPTH, FULL, MINB>, 256, 0) !=
-            cudaSuccess || n < 1)
-      n = 2;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, slot);
-    sm_count[slot] = sms;
-    per_sm[slot] = n;
+  if (!shape.per_sm[slot]) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, shape.kernel, 256, 0) != cudaSuccess || n < 1) n = 2;
+    shape.per_sm[slot] = n;
   }
-  const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, per_sm[slot])
-                                            : std::max(1, per_sm[slot] + t_stream_ctas_per_sm);
-  const long long groups_per_block = (256 / 32) * (32 / LANES);
-  const long long max_blocks = (long long)sm_count[slot] * ctas;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, slot);
+  const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, shape.per_sm[slot])
+                                            : std::max(1, shape.per_sm[slot] + t_stream_ctas_per_sm);
+  const long long groups_per_block = (256 / 32) * (32 / shape.lanes);
+  const long long max_blocks = (long long)sms * ctas;
   long long lookups = 0;
   for (int t = 0; t < p.num_tables; ++t) lookups += p.t[t].nnz;
   StreamChunks sc;
-  sc.chunk = stream_chunk(lookups, p.num_tables, LANES, max_blocks * groups_per_block);
+  sc.chunk = stream_chunk(lookups, p.num_tables, shape.lanes, max_blocks * groups_per_block);
   long long total = 0;
   for (int t = 0; t < p.num_tables; ++t) {
     sc.first[t] = (int)total;
@@ -92,13 +95,27 @@ static void launch_stream(const BagParams& p, BagHeader* hdr, cudaStream_t s) {
   sc.first[p.num_tables] = (int)total;
   // a persistent grid, no larger than the chunks there are
   const long long blocks = std::min(max_blocks, (total + groups_per_block - 1) / groups_per_block);
-  bag_stream_kernel<LANES, VPL, DEPTH, FULL, MINB><<<(unsigned)std::max<long long>(blocks, 1), 256, 0, s>>>(p, sc, hdr);
+  shape.kernel<<<(unsigned)std::max<long long>(blocks, 1), 256, 0, s>>>(p, sc, hdr);
 }
 
 template <int LANES, int VPL, int DEPTH, int MINB>
-static void launch_stream_dim(const BagParams& p, BagHeader* hdr, cudaStream_t s) {
-  if (p.dim == LANES * VPL * 4) launch_stream<LANES, VPL, DEPTH, true, MINB>(p, hdr, s);
-  else launch_stream<LANES, VPL, DEPTH, false, MINB>(p, hdr, s);
+static StreamShape& stream_shape(int vecs) {
+  static StreamShape full{bag_stream_kernel<LANES, VPL, DEPTH, true, MINB>, LANES, {}};
+  static StreamShape part{bag_stream_kernel<LANES, VPL, DEPTH, false, MINB>, LANES, {}};
+  return vecs == LANES * VPL ? full : part;
+}
+
+// The smallest shape whose LANES x VPL vectors hold a row; 32 bytes per lane from dim 64 on: fewer
+// lanes repeat the per-lookup control instructions.
+static StreamShape& stream_shape_for(int vecs, long long max_nnz) {
+  static StreamShape wide{bag_wide_kernel, 32, {}};
+  if (vecs <= 4) return stream_shape<4, 1, 2, 4>(vecs);
+  if (vecs <= 8) return stream_shape<8, 1, 2, 4>(vecs);
+  if (vecs <= 16) return stream_shape<8, 2, 2, 4>(vecs);
+  if (vecs <= 32) return stream_shape<16, 2, 2, 4>(vecs);
+  if (vecs == 64 && max_nnz < kWideLookups) return wide;
+  if (vecs <= 64) return stream_shape<32, 2, 2, 4>(vecs);
+  return stream_shape<32, 4, 2, 3>(vecs);
 }
 
 // Between two groups of tables of one call: the marks and the chunk counter start again.
@@ -177,14 +194,7 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
                       ncols < (1LL << 31) && out_stride < (1LL << 31);
   if (stream) {
     if (ev0) cudaEventRecord(ev0, s);
-    // the smallest shape whose LANES x VPL vectors hold a row; 32 bytes per lane from dim 64 on:
-    // fewer lanes repeat the per-lookup control instructions
-    if (vecs <= 4) launch_stream_dim<4, 1, 2, 4>(p, hdr, s);
-    else if (vecs <= 8) launch_stream_dim<8, 1, 2, 4>(p, hdr, s);
-    else if (vecs <= 16) launch_stream_dim<8, 2, 2, 4>(p, hdr, s);
-    else if (vecs <= 32) launch_stream_dim<16, 2, 2, 4>(p, hdr, s);
-    else if (vecs <= 64) launch_stream_dim<32, 2, 2, 4>(p, hdr, s);
-    else launch_stream_dim<32, 4, 2, 3>(p, hdr, s);
+    launch_stream(stream_shape_for(vecs, max_nnz), p, hdr, s);
     if (ev1) cudaEventRecord(ev1, s);
     if (known_sorted) {
       ANNC_CUDA(cudaGetLastError());

@@ -599,6 +599,155 @@ bag_stream_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
   pdl_trigger();
 }
 
+// The same for rows of 256 floats: a warp per chunk and two vectors per lane.  Row loads go out four at
+// a time and are added when they are back, without the pipeline above: of these long rows that keeps
+// only two on their way in 64 registers, and what it spills is reloaded from behind the rows that
+// stream through L1.  26 tables x 100 K rows, batch 2048: 63 us, 82 us in the pipeline (with four rows
+// on their way 108 us, with 80 registers 83 us); 10 tables x 1 M rows, batch 16384: 151 us / 186 us;
+// batch 100 over 26 tables 19 us / 23 us.  It lives at the edge of its registers (20 bytes spilled): with a
+// launch trigger at its end it spills 44 and the same three take 66, 163 and 21 us.
+// Tables of up to kWideLookups lookups, so that sums with a chunk fit an int.
+constexpr long long kWideLookups = (1LL << 31) - 8192;
+__global__ void __launch_bounds__(256, 4) bag_wide_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
+  constexpr int LANES = 32, VPL = 2, INFLIGHT = 4, DIM = LANES * VPL * 4;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kNoBag = -3;  // a lookup whose segment id is out of range is added nowhere
+  using Vec = RowVec<4>;
+  __shared__ int s_first[kMaxTables + 1];
+  for (int i = threadIdx.x; i <= p.num_tables; i += blockDim.x) s_first[i] = sc.first[i];
+  __syncthreads();
+  const int batch = (int)p.batch;
+  const int lane = threadIdx.x & 31;
+  const unsigned total_chunks = (unsigned)s_first[p.num_tables];
+  const unsigned warps = gridDim.x * (blockDim.x >> 5);
+  for (unsigned gc = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); gc < total_chunks; gc += warps) {
+    int lo = 0, hi = p.num_tables - 1;  // table of chunk gc: last t with first[t] <= gc
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if ((unsigned)s_first[mid] <= gc) lo = mid;
+      else hi = mid - 1;
+    }
+    const int t = lo;
+    const unsigned chunk = gc - (unsigned)s_first[t];
+    const BagTableDev& T = p.t[t];
+    const int n = T.nnz;
+    const float* __restrict__ tab = T.table;
+    float* __restrict__ outp = T.out;
+
+    // rows [a, b) of the output <- 0 (bags without lookups)
+    auto zero_fill = [&](int a, int b) {
+      Vec z;
+      z.zero();
+      for (int s = a; s < b; ++s) {
+        float* o = outp + (long long)s * p.out_stride;
+#pragma unroll
+        for (int w = 0; w < VPL; ++w) z.store(o + (w * LANES + lane) * 4);
+      }
+    };
+    if (n == 0) {  // a table without lookups: every bag is empty
+      zero_fill((int)min((long long)chunk * 1024, (long long)batch), (int)min((long long)(chunk + 1) * 1024, (long long)batch));
+      continue;
+    }
+    Vec acc[VPL];
+#pragma unroll
+    for (int w = 0; w < VPL; ++w) acc[w].zero();
+    int cur = kNoBag;  // bag being summed
+    int count = 0;     // its lookups so far (for the mean)
+    bool open = false;
+    auto flush = [&]() {
+      if (open && cur >= 0) {
+        if (p.combiner == 1 && count > 0) {
+          const float inv = __fdiv_rn(1.0f, (float)count);
+#pragma unroll
+          for (int w = 0; w < VPL; ++w) acc[w].scale(inv);
+        }
+        float* o = outp + (long long)cur * p.out_stride;
+#pragma unroll
+        for (int w = 0; w < VPL; ++w) acc[w].store(o + (w * LANES + lane) * 4);
+      }
+    };
+
+    const int chunk_end = min(n, (int)(chunk + 1) * sc.chunk);
+    for (int base = (int)chunk * sc.chunk; base < n; base += LANES) {
+      const int i = base + lane;
+      int key = kNoBag, row = -1;
+      if (i < n) {
+        const long long seg = T.seg[(long long)i * p.ncols + p.col];
+        const long long r64 = load_row_id(T.ids, p.id_kind, i, T.num_buckets, T.magic);
+        if (seg < 0 || seg >= batch) atomicOr(&hdr->err_bits, kErrSegment);
+        else key = (int)seg;
+        if (r64 < 0 || r64 >= T.rows) atomicOr(&hdr->err_bits, kErrRow);
+        else row = (int)r64;
+      }
+      int prev_key = __shfl_up_sync(kAll, key, 1);
+      if (lane == 0) {
+        prev_key = -1;  // before the first lookup: bags 0 .. key - 1 are empty
+        if (base > 0) {
+          const long long ps = T.seg[(long long)(base - 1) * p.ncols + p.col];
+          prev_key = (ps < 0 || ps >= batch) ? kNoBag : (int)ps;
+        }
+      }
+      const bool starts = i < n && key != prev_key;
+      if (starts && key >= 0 && prev_key >= 0 && key < prev_key) mark_unsorted(hdr, t);
+      const unsigned smask = __ballot_sync(kAll, starts);
+      const int tile_n = min(LANES, n - base);
+      int from = 0, to = tile_n;
+      const bool inside = base < chunk_end;
+      if (!open) {
+        if (!inside) break;
+        if (smask == 0) continue;
+        from = __ffs(smask) - 1;
+      } else if (!inside && smask != 0) {
+        to = __ffs(smask) - 1;
+      }
+      for (int j0 = from; j0 < to; j0 += INFLIGHT) {
+        Vec v[INFLIGHT][VPL];
+        bool has[INFLIGHT];
+#pragma unroll
+        for (int k = 0; k < INFLIGHT; ++k) {
+          const int j = j0 + k;
+          has[k] = false;
+          if (j < to) {
+            const int rw = __shfl_sync(kAll, row, j);
+            has[k] = rw >= 0;
+            if (has[k]) {
+              const float* src = tab + (long long)rw * DIM + lane * 4;
+#pragma unroll
+              for (int w = 0; w < VPL; ++w) v[k][w].load(src + w * LANES * 4);
+            }
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < INFLIGHT; ++k) {
+          const int j = j0 + k;
+          if (j < to) {
+            if ((smask >> j) & 1u) {
+              flush();
+#pragma unroll
+              for (int w = 0; w < VPL; ++w) acc[w].zero();
+              cur = __shfl_sync(kAll, key, j);
+              const int before = __shfl_sync(kAll, prev_key, j);
+              // empty bags between the previous lookup's bag and this one (sorted input only)
+              if (cur >= 0 && before >= -1 && before < cur - 1) zero_fill(before + 1, cur);
+              count = 0;
+              open = true;
+            }
+            ++count;
+            if (has[k]) {
+#pragma unroll
+              for (int w = 0; w < VPL; ++w) acc[w].add(v[k][w]);
+            }
+          }
+        }
+      }
+      if (!inside && to < tile_n) break;
+      // the table's last lookup: bags after its bag are empty
+      if (base + tile_n >= n && to == tile_n && open && cur >= 0) zero_fill(cur + 1, batch);
+    }
+    flush();
+  }
+}
+
 // The kernels for tables marked unsorted.  They follow every call, sorted or not (the host does
 // not know), so their cost on sorted tables is what matters: one grid over all marked tables
 // that leaves after one load, launched while the kernel before it drains (pdl_wait holds until

@@ -358,7 +358,7 @@ def test_division_free_modulo_is_exact(num_buckets):
         np.testing.assert_array_equal(got, want)
 
 
-@pytest.mark.parametrize("dim,stride_slots", [(4, 1), (20, 2), (48, 3), (64, 3), (128, 2), (132, 1), (264, 1), (516, 1)])
+@pytest.mark.parametrize("dim,stride_slots", [(4, 1), (20, 2), (48, 3), (64, 3), (128, 2), (132, 1), (256, 2), (264, 1), (516, 1)])
 @pytest.mark.parametrize("combiner", [0, 1])
 @pytest.mark.parametrize("id_kind", [0, 1, 2])
 def test_bag_plan_tile_and_chunk_edges(dim, stride_slots, combiner, id_kind):
@@ -396,6 +396,39 @@ def test_bag_plan_tile_and_chunk_edges(dim, stride_slots, combiner, id_kind):
     assert (got[:, :stride_slots] == -7.0).all()
     for t, ref in enumerate(want):
         np.testing.assert_array_equal(got[:, stride_slots + t], ref, err_msg=f"table {t}")
+
+
+@pytest.mark.parametrize("dim", [64, 252, 256, 260])
+@pytest.mark.parametrize("combiner", [0, 1])
+def test_bag_plan_marks_unsorted_and_out_of_range(dim, combiner):
+    """A table whose segment ids decrease is redone by the atomic route (sums in any order: as many ulp
+    of the sum of magnitudes as a bag has lookups), its neighbours are not; a row or segment id out of
+    range is reported and added nowhere."""
+    rng = np.random.default_rng(dim + combiner)
+    rows, batch, n = 300, 200, 3000
+    data = rng.standard_normal((rows, dim)).astype(np.float32)
+    row, lens = rng.integers(0, rows, n), rng.multinomial(n, np.ones(batch) / batch)
+    seg = np.repeat(np.arange(batch), lens)
+    shuffled = rng.permutation(seg)
+    out = torch.full((batch, 3, dim), -7.0, device="cuda")
+    pairs = [np.stack([s, s], 1).astype(np.int64) for s in (seg, shuffled, seg)]
+    plan = BagPlan([_dev(data)] * 3, [_dev(row)] * 3, [_dev(p) for p in pairs], out, 0, batch, id_kind=1, combiner=combiner)
+    plan.run()
+    assert plan.error_bits() == 0
+    got = out.cpu().numpy()
+    for t, s in enumerate((seg, shuffled, seg)):
+        ref, size = np.zeros((batch, dim)), np.zeros((batch, dim))
+        np.add.at(ref, s, data[row].astype(np.float64))
+        np.add.at(size, s, np.abs(data[row]).astype(np.float64))
+        div = np.maximum(np.bincount(s, minlength=batch), 1)[:, None] if combiner else 1
+        assert (np.abs(got[:, t] - ref / div) <= (lens.max() + 2) * 2.0 ** -24 * size / div + 1e-30).all()
+    assert np.array_equal(got[:, 0], got[:, 2])
+    bad_row, bad_seg = row.copy(), pairs[0].copy()
+    bad_row[17], bad_seg[n - 1] = rows, batch
+    for ids, sg, bit in ((bad_row, pairs[0], 1), (row, bad_seg, 2)):
+        plan = BagPlan([_dev(data)], [_dev(ids)], [_dev(sg)], out, 1, batch, id_kind=1, combiner=0)
+        plan.run()
+        assert plan.error_bits() == bit
 
 
 @pytest.mark.parametrize("n,distinct,dim", [(1, 1, 4), (2047, 3, 5), (2048, 2048, 8), (2049, 700, 20), (10_000, 1, 64),
