@@ -105,14 +105,24 @@ static StreamShape& stream_shape(int vecs) {
   return vecs == LANES * VPL ? full : part;
 }
 
+// Rows of up to 128 floats for a caller that gave the kernel a share of two or more blocks per SM (0 and 1:
+// the faster shape).  The pooling kernel of the row exchange fits five times on an SM at these widths, and
+// shares of the two kernels that add up to five have to fit together: 48 registers, as that one has,
+// instead of 64 (three blocks of those leave room for one of the pooling kernel).  11 tables x 60 K rows of
+// dim 64, batch 16384, three blocks per SM, alone: 108 us, 79 us with 64 registers (two blocks 130 / 93).
+template <int LANES, int VPL>
+static StreamShape& stream_shape_beside(int vecs) {
+  return t_stream_ctas_per_sm >= 2 ? stream_shape<LANES, VPL, 2, 5>(vecs) : stream_shape<LANES, VPL, 2, 4>(vecs);
+}
+
 // The smallest shape whose LANES x VPL vectors hold a row; 32 bytes per lane from dim 64 on: fewer
 // lanes repeat the per-lookup control instructions.
 static StreamShape& stream_shape_for(int vecs, long long max_nnz) {
   static StreamShape wide{bag_wide_kernel, 32, {}};
-  if (vecs <= 4) return stream_shape<4, 1, 2, 4>(vecs);
-  if (vecs <= 8) return stream_shape<8, 1, 2, 4>(vecs);
-  if (vecs <= 16) return stream_shape<8, 2, 2, 4>(vecs);
-  if (vecs <= 32) return stream_shape<16, 2, 2, 4>(vecs);
+  if (vecs <= 4) return stream_shape_beside<4, 1>(vecs);
+  if (vecs <= 8) return stream_shape_beside<8, 1>(vecs);
+  if (vecs <= 16) return stream_shape_beside<8, 2>(vecs);
+  if (vecs <= 32) return stream_shape_beside<16, 2>(vecs);
   if (vecs == 64 && max_nnz < kWideLookups) return wide;
   if (vecs <= 64) return stream_shape<32, 2, 2, 4>(vecs);
   return stream_shape<32, 4, 2, 3>(vecs);
@@ -309,6 +319,15 @@ size_t annc_embed_bag_workspace_bytes(int num_tables, int64_t batch) {
 }
 
 void annc_embed_bag_set_stream_ctas_per_sm(int ctas_per_sm) { t_stream_ctas_per_sm = ctas_per_sm; }
+
+int annc_embed_bag_stream_registers(int64_t dim, int* registers_per_thread) {
+  ANNC_REQUIRE(registers_per_thread && dim >= 4 && dim <= 512 && dim % 4 == 0, ANNC_ERR_INVALID_ARGUMENT,
+               "bag registers: dim must be a multiple of four up to 512");
+  cudaFuncAttributes attr;
+  ANNC_CUDA(cudaFuncGetAttributes(&attr, stream_shape_for((int)(dim / 4), 0).kernel));
+  *registers_per_thread = attr.numRegs;
+  return ANNC_OK;
+}
 
 int annc_embed_bags_dev(const annc_bag_table* tables, int num_tables, int64_t dim, int id_kind,
                         int64_t ncols, int32_t col, int combiner, int64_t batch,

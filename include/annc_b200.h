@@ -499,8 +499,12 @@ void annc_embed_bag_set_timing_events(void* start, void* stop);
 /* Blocks per SM of the persistent lookup-granular bag kernel for the calls of this thread
  * (0 = as many as fit, the default; n > 0 = at most n; -n = n fewer than fit).  For a caller
  * that runs annc_embed_bags_dev on one stream beside another kernel of its own on a second
- * stream and wants both resident (see annc_row_exchange_set_pool_ctas_per_sm). */
+ * stream and wants both resident (see annc_row_exchange_set_pool_ctas_per_sm): shares of the two
+ * kernels that add up to five per SM fit together for rows of up to 128 floats. */
 void annc_embed_bag_set_stream_ctas_per_sm(int ctas_per_sm);
+/* Registers per thread (256 threads a block) of that kernel for rows of dim floats (a multiple of
+ * four up to 512), under the share set for this thread. */
+int annc_embed_bag_stream_registers(int64_t dim, int* registers_per_thread);
 
 /* GEMM core: C = act(alpha * op(A) * op(B) + beta * C + addend + bias), row-major. */
 enum { ANNC_ACT_NONE = 0, ANNC_ACT_RELU = 1, ANNC_ACT_SIGMOID = 2 };

@@ -1,6 +1,8 @@
 """Parity of the CUDA embedding path with the CPU oracle and with the reference's
 known-answer tests, through the C ABI.  Bit-exact for ids, rows, COO indices and
 for sums over sorted segment ids; 1e-5 relative for the atomic (unsorted) route."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -12,6 +14,7 @@ pytestmark = pytest.mark.gpu
 import torch
 from annc_b200 import ops  # noqa: E402  (no fallback: a missing library fails the collection)
 from annc_b200 import AnncError, synth  # noqa: E402
+from annc_b200._lib import lib  # noqa: E402
 from annc_b200.device import BagPlan  # noqa: E402
 
 
@@ -429,6 +432,33 @@ def test_bag_plan_marks_unsorted_and_out_of_range(dim, combiner):
         plan = BagPlan([_dev(data)], [_dev(ids)], [_dev(sg)], out, 1, batch, id_kind=1, combiner=0)
         plan.run()
         assert plan.error_bits() == bit
+
+
+@pytest.mark.parametrize("dim", [16, 32, 64, 100, 128])
+def test_bag_share_fits_beside_the_pooling_kernel(dim):
+    """A share of n blocks per SM leaves room for 5 - n blocks of the pooling kernel of the row exchange
+    (256 threads of at most 48 registers, by its launch bounds), and gives the same sums."""
+    rng = np.random.default_rng(dim)
+    rows, batch = 500, 3000
+    lens = rng.integers(0, 12, batch)
+    n = int(lens.sum())
+    seg = np.repeat(np.arange(batch), lens)
+    out = torch.empty((batch, 1, dim), device="cuda")
+    plan = BagPlan([_dev(rng.standard_normal((rows, dim)).astype(np.float32))], [_dev(rng.integers(0, rows, n))],
+                   [_dev(np.stack([seg, seg], 1).astype(np.int64))], out, 0, batch, id_kind=1, combiner=1)
+    plan.run()
+    want = out.clone()
+    try:
+        for share in (1, 2, 3, 4, 5):
+            lib.annc_embed_bag_set_stream_ctas_per_sm(share)
+            regs = C.c_int(0)
+            assert lib.annc_embed_bag_stream_registers(dim, C.byref(regs)) == 0
+            assert 256 * (share * regs.value + (5 - share) * 48) <= 65536, (share, regs.value)
+            out.fill_(-7.0)
+            plan.run()
+            assert plan.error_bits() == 0 and torch.equal(out, want)
+    finally:
+        lib.annc_embed_bag_set_stream_ctas_per_sm(0)
 
 
 @pytest.mark.parametrize("n,distinct,dim", [(1, 1, 4), (2047, 3, 5), (2048, 2048, 8), (2049, 700, 20), (10_000, 1, 64),
