@@ -26,6 +26,9 @@ bool pair_supported(const annc_gemm_desc& d, int math);
 int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s);
 // Whether its epilogue for this descriptor stores by TMA (no beta * C or softmax, aligned rows).
 bool pair_stores_by_tma(const annc_gemm_desc& d);
+// How many of its `tiles` 256 x 256 tiles it takes whole on a chip of so many SM pairs; the rest of
+// the last round is cut in halves (and only then the kernel's tile width is a run-time value).
+long long pair_whole_tiles(const annc_gemm_desc& d, int math, long long tiles, long long pairs);
 
 // A kn4-packed B re-laid into `ws` (4*K*N bytes): relaid_desc returns 0 when that does not
 // pay off, else the form the weight takes in ws (1 = [N,K], 2 = [K,N]) and fills `plain`

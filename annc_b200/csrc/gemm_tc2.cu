@@ -693,6 +693,18 @@ bool pair_stores_by_tma(const annc_gemm_desc& d) {
          d.n % per16 == 0 && d.ldc % per16 == 0 && (d.batch == 1 || (d.stride_c % per16 == 0 && d.stride_c > 0));
 }
 
+// Tiles of the last (or only) round, when they fill at most half of the pairs, are cut in two column
+// halves.  A half tile moves three quarters of the operands of a whole one, so behind whole rounds
+// of a long main loop, which keep the chip at its power limit, nothing is won: 4096 x 512 x 416 (32
+// tiles) 13.7 us whole, 11.6 us cut; 65536 x 256 x 512 (3 rounds and 34 tiles) 45.0 / 43.1; 16384 x
+// 1024 x 8192 bf16 (the same) 211 / 215.
+long long pair_whole_tiles(const annc_gemm_desc& d, int math, long long tiles, long long pairs) {
+  const long long last = tiles % pairs;
+  const bool cut = !(d.io_flags & ANNC_IO_SOFTMAX) && d.n > PN / 2 && 2 * last <= pairs &&
+                   (tiles == last || d.k <= (math == ANNC_MATH_BF16 ? 64 * 64 : 64 * 32));
+  return cut ? tiles - last : tiles;
+}
+
 int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   if (!pair_supported(d, math)) return fail(ANNC_ERR_UNSUPPORTED, "tcgen05 pair gemm: unsupported shape");
   const bool bf16 = math == ANNC_MATH_BF16;
@@ -778,14 +790,8 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   const long long tiles = (long long)p.tiles_m * p.tiles_n * d.batch;
   p.error_word = gemm_error_word();
   if (!p.error_word) return fail(ANNC_ERR_CUDA, "gemm error word is not addressable");
-  // Tiles of the last (or only) round, when they fill at most half of the pairs, are cut in two column
-  // halves.  A half tile moves three quarters of the operands of a whole one, so behind whole rounds
-  // of a long main loop, which keep the chip at its power limit, nothing is won: 4096 x 512 x 416 (32
-  // tiles) 13.7 us whole, 11.6 us cut; 65536 x 256 x 512 (3 rounds and 34 tiles) 45.0 / 43.1; 16384 x
-  // 1024 x 8192 bf16 (the same) 211 / 215.
-  const long long last = tiles % max_pairs[bf16];
-  const bool cut = !softmax && d.n > PN / 2 && 2 * last <= max_pairs[bf16] && (tiles == last || d.k <= 64 * kelts);
-  p.whole = cut ? tiles - last : tiles;
+  p.whole = pair_whole_tiles(d, math, tiles, max_pairs[bf16]);
+  const bool cut = p.whole < tiles;
   p.items = p.whole + 2 * (tiles - p.whole);
   const long long pairs = p.items < max_pairs[bf16] ? p.items : max_pairs[bf16];
   cudaLaunchConfig_t cfg;

@@ -223,3 +223,19 @@ def test_a_packed_weight_off_16_bytes_is_not_relaid(annc, m, k, n):
     assert _relaid_form(annc, m, k, n) != 0
     for off in (4, 8, 12):
         assert _relaid_form(annc, m, k, n, weight=(1 << 20) + off) == 0
+
+
+@pytest.mark.parametrize("math,n,k,softmax,tiles,whole", [
+    (2, 512, 64, 0, 37, 0), (2, 512, 64, 0, 38, 38), (2, 512, 64, 0, 1, 0),      # one round: half of the pairs or more
+    (2, 512, 2048, 0, 84, 74), (2, 512, 2049, 0, 84, 84), (2, 512, 64, 0, 112, 112),  # a last round behind whole ones
+    (3, 512, 4096, 0, 84, 74), (3, 512, 4097, 0, 84, 84),
+    (2, 512, 64, 0, 74, 74), (2, 512, 64, 0, 222, 222), (3, 512, 64, 0, 148, 148),    # no last round: nothing to cut
+    (2, 128, 64, 0, 20, 20), (2, 256, 64, 1, 20, 20)])
+def test_tiles_the_pair_gemm_cuts_in_halves(annc, math, n, k, softmax, tiles, whole):
+    """On 74 SM pairs, tiles taken whole and (the rest) in halves.  A product of whole rounds has none of
+    the latter, and says so: the launch then takes the build with constant tile widths."""
+    fn = getattr(annc.lib, "_ZN4annc4gemm16pair_whole_tilesERK14annc_gemm_descixx")  # gemm::pair_whole_tiles
+    fn.argtypes, fn.restype = [C.c_void_p, C.c_int, C.c_longlong, C.c_longlong], C.c_longlong
+    from annc_b200._lib import IO_SOFTMAX, GemmDesc
+    d = GemmDesc(m=1000, n=n, k=k, batch=1, io_flags=IO_SOFTMAX if softmax else 0)
+    assert fn(C.byref(d), math, tiles, 74) == whole
