@@ -26,17 +26,20 @@ static int validate(const annc_gemm_desc& d) {
   return ANNC_OK;
 }
 
-// Pair kernel (256 x 256 tiles per two SMs, persistent) or single-CTA kernel (128 x 128 tiles, two
-// per SM or split K inside a cluster).  With its TMA-store epilogue the pair kernel wins from
-// about 32 tiles on, measured in us pair / single: 65536 x 512 x 416 62 / 111, 4096 x 512 x 416 (32
-// tiles) 11.6 / 14.4, 2048 x 1000 x 500 (32) 12.8 / 15.7, 64 x [256 x 256 x 64] 9.5 / 11.5.  Below, split K
-// decides: 1500 x 1100 x 700 (30) 15.1 / 16.6, 20 x [256 x 256 x 100] 8.1 / 9.2, but 2048 x 512 x 416 (16)
-// 11.2 / 11.0 and 1024^3 (16) 17.7 / 14.6.  A narrow C pays for 256 columns of multiplications: from
-// n = 64 on that still hides under the memory traffic when K is short and the rows fill every
-// pair (65536 x 64 x 256 24 / 28).
-// With an addend: 8192 x 1024 x 512 31 / 59, 3000 x 1000 x 1000 (48 tiles) 25 / 43, 4096 x 512 x 416 (32)
-// 17 / 20.  Its general epilogue (beta * C, rows not of whole 16-byte pieces) is slow per tile and
-// needs a long main loop to hide in.
+// Pair kernel (256 x 256 tiles per two SMs, persistent; few tiles are cut in halves) or single-CTA kernel
+// (128 x 128 tiles, one or two per SM, or split K inside a cluster).  With its TMA-store epilogue the pair
+// kernel wins from 20 tiles on, except where the single one
+//   * splits K (at most 74 tiles of one product, K from 225 on): us pair / single 300 x 3000 x 704 1.18 times,
+//     2600 x 260 x 1024 1.29, 1024 x 1100 x 4096 1.48 times its time, and 1.02 at K = 256; at K = 128, unsplit, 0.89;
+//   * takes the product in one round (at most 148 tiles) and the pair kernel has more tiles than it can
+//     cut (more than 37 on 74 pairs): 300 x 5000 1.09 to 1.12, 2048 x 1100 1.12 to 1.15 from K = 128 to 4096.
+// Otherwise, pair / single over 40 products and batches each at K = 64 to 4096, with and without an addend:
+// up to 37 pair tiles 0.80 to 1.00, more than 148 single tiles 0.53 to 0.75 (149 to 222, two rounds; 10 x [520 x
+// 300 x 64], 60 pair tiles for 150 of them, 1.06) and 0.85 to 1.00 (more, two per SM).  Below 20 pair tiles K is split nearly always (1024^3 17.7 / 14.6).
+// A narrow C pays for 256 columns of multiplications: from n = 64 on that still hides under the memory
+// traffic when K is short and the rows fill every pair (65536 x 64 x 256 24 / 28).
+// Its general epilogue (beta * C, rows not of whole 16-byte pieces) is slow per tile and needs a long
+// main loop to hide in.
 static bool use_pair(const annc_gemm_desc& d, int math) {
   if (!pair_supported(d, math)) return false;
   if (math == ANNC_MATH_BF16 || (d.io_flags & (ANNC_IO_SOFTMAX | ANNC_IO_PAIR))) return true;
@@ -45,7 +48,10 @@ static bool use_pair(const annc_gemm_desc& d, int math) {
   const long long pair_tiles = ((d.m + 255) / 256) * ((d.n + 255) / 256) * d.batch;
   if (d.m >= 256 && d.n >= 192 && d.k >= 1024 && pair_tiles >= 74) return true;
   if (!pair_stores_by_tma(d)) return false;
-  return (d.n >= 192 && d.m >= 192 && pair_tiles >= (d.k <= 704 ? 20 : 32)) || (d.n >= 64 && d.k <= 512 && pair_tiles >= 148);
+  const long long single_tiles = ((d.m + 127) / 128) * ((d.n + 127) / 128) * d.batch;
+  const bool single_splits = d.batch == 1 && single_tiles * 2 <= 148 && d.k > 224;
+  if (d.n >= 192 && d.m >= 192 && pair_tiles >= 20 && !single_splits && (single_tiles > 148 || pair_tiles <= 37)) return true;
+  return d.n >= 64 && d.k <= 512 && pair_tiles >= 148;
 }
 
 // AUTO: tensor cores (TF32) when the shape fits a tcgen05 kernel, else CUDA cores.

@@ -239,3 +239,21 @@ def test_tiles_the_pair_gemm_cuts_in_halves(annc, math, n, k, softmax, tiles, wh
     from annc_b200._lib import IO_SOFTMAX, GemmDesc
     d = GemmDesc(m=1000, n=n, k=k, batch=1, io_flags=IO_SOFTMAX if softmax else 0)
     assert fn(C.byref(d), math, tiles, 74) == whole
+
+
+@pytest.mark.parametrize("m,n,k,batch,pair", [
+    (1024, 1024, 1024, 1, False), (2048, 512, 256, 1, False),                # below 20 tiles
+    (300, 3000, 224, 1, True), (300, 3000, 228, 1, False),                   # 72 single tiles: K is split from 225 on
+    (1024, 1100, 4096, 1, False), (2600, 260, 704, 1, False),
+    (2048, 520, 704, 1, True), (2048, 520, 4096, 1, True),                   # 24 tiles, 80 single ones
+    (2048, 1024, 4096, 1, True), (4 * 256, 9 * 256, 1024, 1, True),          # 32 and 36 tiles
+    (300, 5000, 1024, 1, False), (2048, 1100, 4096, 1, False),               # 40 tiles, at most 148 single ones
+    (512, 5000, 1024, 1, True), (1024, 4096, 1024, 1, True),                 # 40 and 64 tiles, 160 and 256 single ones
+    (256, 256, 512, 20, True), (300, 256, 512, 20, False), (256, 256, 512, 40, True),
+    (65536, 64, 256, 1, True), (65536, 60, 256, 1, False), (65536, 64, 1028, 1, False)])
+def test_gemm_route_by_tiles(annc, m, n, k, batch, pair):
+    """CTA-pair or single-CTA kernel at the borders of the rule that picks one by shape."""
+    from annc_b200._lib import GemmDesc
+    d = GemmDesc(0, 0, m, n, k, batch, k, n, n, n, m * k, k * n, m * n, 0, 1.0, 0.0, 1 << 20, 2 << 20, 3 << 20)
+    name = annc.lib.annc_gemm_kernel_name(C.byref(d)).decode()
+    assert name == ("tcgen05_pair_tf32" if pair else "tcgen05_tf32")
