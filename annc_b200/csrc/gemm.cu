@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(256) kn4_relay_kernel(RelayParams p) {
     const kn4::Chunk nc = kn4::axis_chunk(p.N, kn4::kTileN, n);
     const kn4::Panel pn = kn4::panel_of(nc.len, n - nc.start);
     const int term = (int)(nc.start + pn.start), width = (int)pn.width, in0 = n - term;
-    float4 v[kRelayK / 32];
+    float4 v[kRelayK / 32];  // all on their way before the first is stored
+    long long to[kRelayK / 32];
 #pragma unroll
     for (int i = 0; i < kRelayK / 32; ++i) {
       const int k = k0 + kk + 32 * i;
@@ -128,11 +129,10 @@ __global__ void __launch_bounds__(256) kn4_relay_kernel(RelayParams p) {
         len = p.K - p.k_split;
       }
       const long long packed = (long long)start * p.N + (long long)len * term + (long long)(k - start) * width + in0;
-      if (MODE == RELAY_PACK)
-        *reinterpret_cast<float4*>(p.dst + packed) = __ldg(reinterpret_cast<const float4*>(p.src + (long long)k * p.N + n));
-      else v[i] = __ldg(reinterpret_cast<const float4*>(p.src + packed));
+      const long long plain = (long long)k * p.N + n;
+      to[i] = MODE == RELAY_PACK ? packed : plain;
+      v[i] = __ldg(reinterpret_cast<const float4*>(p.src + (MODE == RELAY_PACK ? plain : packed)));
     }
-    if (MODE == RELAY_PACK) return;
 #pragma unroll
     for (int i = 0; i < kRelayK / 32; ++i) {
       const int k = k0 + kk + 32 * i;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) kn4_relay_kernel(RelayParams p) {
         tile[4 * c + 2][kk + 32 * i] = v[i].z;
         tile[4 * c + 3][kk + 32 * i] = v[i].w;
       } else {
-        *reinterpret_cast<float4*>(p.dst + (long long)k * p.N + n) = v[i];
+        *reinterpret_cast<float4*>(p.dst + to[i]) = v[i];
       }
     }
   }
@@ -232,10 +232,11 @@ void relay_kn4(const float* packed, float* ws, long long k, long long n, int for
   else kn4_relay_kernel<RELAY_KN><<<relay_grid(k, n), 256, 0, s>>>(p);
 }
 
-// kn4 <-> [K,N], any extents: 16-byte pieces where they exist (2048 x 4096: 11 and 9 us against 56 us one
-// element at a time).
+// kn4 <-> [K,N], any extents: 16-byte pieces where they exist (2048 x 4096: 9 us against 54 us one element
+// at a time), except for small matrices with enough rows that a block's threads walk several in turn
+// (128 x 256 2.2 us / 2.0 us; 200 x 256 2.2 / 2.3, 64 x 512 1.9 / 2.0).
 static void convert_kn4(const float* src, float* dst, long long k, long long n, bool pack, cudaStream_t s) {
-  const bool pieces = n % 4 == 0 && n < (1LL << 31) && (k + kRelayK - 1) / kRelayK <= 65535 &&
+  const bool pieces = n % 4 == 0 && n < (1LL << 31) && (k <= 64 || k * n > 32768) && (k + kRelayK - 1) / kRelayK <= 65535 &&
                       ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
   if (pieces) {
     const RelayParams p = relay_params(src, dst, k, n);
