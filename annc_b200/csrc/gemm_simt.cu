@@ -434,6 +434,7 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
     ANNC_CUDA(cudaGetLastError());
     return ANNC_OK;
   }
+  if ((d.m + 63) / 64 > 65535) return fail(ANNC_ERR_UNSUPPORTED, "simt gemm: more than 4M rows");
   // With an addend a thread waits for each row's part of it in turn, which small products do not hide:
   // 200 x 512 x 13 6.8 us, 5.3 us in tiles; 1000 x 512 x 13 7.1 / 5.9; 500 x 2048 x 13 7.2 / 7.8.
   const bool small_add = d.addend && d.m * d.n <= (1 << 19);
@@ -441,7 +442,7 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
       d.b_format == ANNC_B_PLAIN && (d.n & 3) == 0 && (d.ldb & 3) == 0 && (d.ldc & 3) == 0 &&
       aligned16(d.b) && aligned16(d.c) && (!d.bias || aligned16(d.bias)) &&
       (!d.addend || (aligned16(d.addend) && (d.ld_addend & 3) == 0)) &&
-      (d.n / 4 + 127) / 128 <= 65535 && (d.m + SK_ROWS - 1) / SK_ROWS < (1LL << 31)) {
+      (d.n / 4 + 127) / 128 <= 65535) {
     dim3 grid((unsigned)((d.m + SK_ROWS - 1) / SK_ROWS), (unsigned)((d.n / 4 + 127) / 128));
     if (d.k <= 8) sgemm_smallk_kernel<8><<<grid, 128, 0, s>>>(d);
     else if (d.k <= 13) sgemm_smallk_kernel<13><<<grid, 128, 0, s>>>(d);
@@ -449,7 +450,6 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
     ANNC_CUDA(cudaGetLastError());
     return ANNC_OK;
   }
-  if ((d.m + 63) / 64 > 65535) return fail(ANNC_ERR_UNSUPPORTED, "simt gemm: more than 4M rows");
   SimtArgs args;
   args.d = d;
   args.bias_mode = bb ? 1 : 0;

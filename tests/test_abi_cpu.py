@@ -257,3 +257,15 @@ def test_gemm_route_by_tiles(annc, m, n, k, batch, pair):
     d = GemmDesc(0, 0, m, n, k, batch, k, n, n, n, m * k, k * n, m * n, 0, 1.0, 0.0, 1 << 20, 2 << 20, 3 << 20)
     name = annc.lib.annc_gemm_kernel_name(C.byref(d)).decode()
     assert name == ("tcgen05_pair_tf32" if pair else "tcgen05_tf32")
+
+
+@pytest.mark.parametrize("k,trans_b", [(8, 0), (16, 0), (17, 0), (8, 1)])
+def test_fp32_gemm_refuses_more_than_4m_rows(annc, k, trans_b):
+    """On every kernel of the fp32 route but the one for a single column (refused before a launch)."""
+    from annc_b200._lib import MATH_FP32, GemmDesc
+    m, n = 65535 * 64 + 1, 8
+    d = GemmDesc(0, trans_b, m, n, k, 1, k, k if trans_b else n, n, n, 0, 0, 0, 0, 1.0, 0.0,
+                 1 << 20, 2 << 20, 3 << 20, None, None, 0, 0, MATH_FP32)
+    assert annc.lib.annc_gemm_run(C.byref(d), None) != 0
+    annc.lib.annc_last_error.restype = C.c_char_p
+    assert b"more than 4M rows" in annc.lib.annc_last_error()
