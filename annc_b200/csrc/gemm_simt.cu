@@ -444,9 +444,13 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
       (!d.addend || (aligned16(d.addend) && (d.ld_addend & 3) == 0)) &&
       (d.n / 4 + 127) / 128 <= 65535) {
     dim3 grid((unsigned)((d.m + SK_ROWS - 1) / SK_ROWS), (unsigned)((d.n / 4 + 127) / 128));
-    if (d.k <= 8) sgemm_smallk_kernel<8><<<grid, 128, 0, s>>>(d);
-    else if (d.k <= 13) sgemm_smallk_kernel<13><<<grid, 128, 0, s>>>(d);
-    else sgemm_smallk_kernel<SK_MAXK><<<grid, 128, 0, s>>>(d);
+    // One build per K, for its registers and multiply-adds: 65536 x 512 with K = 9 28.7 us, 36 in the build for
+    // 13; with K = 13 36 us, 37.5 us in that for 16.  14 and 15 take 16, whose index arithmetic is shifts:
+    // 200 x 512 x 15 3.9 us, 4.8 us in a build of its own.
+    static void (*const kernels[])(annc_gemm_desc) = {
+        sgemm_smallk_kernel<8>,  sgemm_smallk_kernel<9>,  sgemm_smallk_kernel<10>, sgemm_smallk_kernel<11>,
+        sgemm_smallk_kernel<12>, sgemm_smallk_kernel<13>, sgemm_smallk_kernel<SK_MAXK>};
+    kernels[d.k <= 8 ? 0 : d.k <= 13 ? d.k - 8 : 6]<<<grid, 128, 0, s>>>(d);
     ANNC_CUDA(cudaGetLastError());
     return ANNC_OK;
   }

@@ -283,3 +283,18 @@ def test_layout_matmul_device_weight_streams_and_capture():
     for i, o in enumerate(outs):
         assert torch.equal(o, want[i % 2])
     assert nerr(captured, want[0].cpu().numpy()) <= 1e-5  # the same products, summed in another tiling
+
+
+@pytest.mark.parametrize("k", range(1, 18))
+@pytest.mark.parametrize("m,n", [(64, 4), (79, 516)])
+def test_small_k_product_at_every_k(m, n, k):
+    """Bias, ReLU and beta * C, with ragged rows.  Bound: a chain of k rounded multiply-adds and three more
+    roundings."""
+    rng = np.random.default_rng(k + n)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    c0, bias = rng.standard_normal((m, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    c = _dev(c0)
+    device.gemm(_dev(a), _dev(b), c, m=m, n=n, k=k, beta=-1.0, bias=_dev(bias), activation=1, math=_lib.MATH_FP32)
+    want = np.maximum(a.astype(np.float64) @ b - c0 + bias, 0)
+    size = abs(a).astype(np.float64) @ abs(b) + abs(c0) + abs(bias)
+    assert (abs(c.cpu().numpy() - want) <= (k + 4) * 2.0 ** -24 * size).all()
