@@ -182,22 +182,25 @@ bf16_weight_kernel(const float* __restrict__ src, long long ldb, __nv_bfloat16* 
 
 }  // namespace
 
-// Re-laying a kn4 B into a workspace of 4*K*N bytes.  relaid_desc() says whether that pays off
-// for this descriptor and returns the descriptor of the equivalent plain-layout GEMM over `ws`
-// together with the form the weight has to take there (1 = [N,K], 2 = [K,N]); relay_kn4() runs
-// the conversion.  Kept apart so that a caller that owns a cache of constants converts once.
-int relaid_desc(const annc_gemm_desc& d, void* ws, size_t ws_bytes, annc_gemm_desc* plain) {
-  if (d.b_format != ANNC_B_KN4 || !ws || d.batch != 1) return 0;
-  if (ws_bytes < (size_t)d.k * (size_t)d.n * sizeof(float)) return 0;
-  // the packed weight is read in 16-byte pieces too
-  if (((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(d.b)) & 15) || (d.n & 3) || d.m < 64) return 0;
+// Re-laying a kn4 B into a buffer of 4*K*N bytes, 16-byte aligned.  relaid_desc() says whether that pays off
+// for this descriptor and returns the descriptor of the equivalent plain-layout GEMM, whose `b` the
+// caller sets to that buffer, together with the form the weight has to take there (1 = [N,K], 2 =
+// [K,N]); relay_kn4() runs the conversion.  Kept apart so that a caller that owns a cache of constants
+// converts once (`kept`: then only the products count, not the pass over the weight).
+int relaid_desc(const annc_gemm_desc& d, bool kept, annc_gemm_desc* plain) {
+  if (d.b_format != ANNC_B_KN4 || d.batch != 1 || (d.n & 3) || d.m < 64) return 0;
+  if (reinterpret_cast<uintptr_t>(d.b) & 15) return 0;  // the packed weight is read in 16-byte pieces
   if (d.k >= (1LL << 31) || d.n >= (1LL << 31) || (d.k + kRelayK - 1) / kRelayK > 65535) return 0;
   *plain = d;
-  plain->b = static_cast<const float*>(ws);
+  plain->b = nullptr;
   plain->b_format = ANNC_B_PLAIN;
   plain->ldb = d.n;
   plain->workspace = nullptr;
   plain->workspace_bytes = 0;
+  // The CUDA cores take the packed form as it lies, at a place computation per element: only long K (with
+  // fewer than 16 columns) pays for the pass over the weight.  __layout_matmul, us packed / re-laid: 64 x 16 x 64
+  // 13 / 16, 64 rows of 8 columns K = 1024 13.5 / 15.9, 2048 20.6 / 16.4; 4000 rows 512 15.6 / 16.5, 1024 24.9 / 22.6.
+  if (!kept && pick_math(*plain) == ANNC_MATH_FP32 && d.k * (d.m >= 2048 ? 2 : 1) < 2048) return 0;
   // Re-laid as [N,K] the weight takes the K-major TMA route (one 16 KB box per stage), the
   // fastest one; [K,N] is the fallback when K rows would not be 16-byte pitched.
   if ((d.k & 3) == 0 && (d.k + 31) / 32 <= 65535) {
@@ -250,8 +253,12 @@ static void convert_kn4(const float* src, float* dst, long long k, long long n, 
 }
 
 static bool unpack_kn4_into_workspace(const annc_gemm_desc& d, cudaStream_t s, annc_gemm_desc* plain) {
-  const int form = relaid_desc(d, d.workspace, d.workspace_bytes, plain);
+  if (!d.workspace || (reinterpret_cast<uintptr_t>(d.workspace) & 15) ||
+      d.workspace_bytes < (size_t)d.k * (size_t)d.n * sizeof(float))
+    return false;
+  const int form = relaid_desc(d, /*kept=*/false, plain);
   if (!form) return false;
+  plain->b = static_cast<const float*>(d.workspace);
   relay_kn4(d.b, static_cast<float*>(d.workspace), d.k, d.n, form, s);
   return true;
 }

@@ -30,10 +30,11 @@ bool pair_stores_by_tma(const annc_gemm_desc& d);
 // the last round is cut in halves (and only then the kernel's tile width is a run-time value).
 long long pair_whole_tiles(const annc_gemm_desc& d, int math, long long tiles, long long pairs);
 
-// A kn4-packed B re-laid into `ws` (4*K*N bytes): relaid_desc returns 0 when that does not
-// pay off, else the form the weight takes in ws (1 = [N,K], 2 = [K,N]) and fills `plain`
-// with the equivalent plain-layout descriptor; relay_kn4 runs the conversion.
-int relaid_desc(const annc_gemm_desc& d, void* ws, size_t ws_bytes, annc_gemm_desc* plain);
+// A kn4-packed B re-laid into a 16-byte aligned buffer of 4*K*N bytes: relaid_desc returns 0 when that
+// does not pay off, else the form the weight takes there (1 = [N,K], 2 = [K,N]) and fills `plain`
+// with the equivalent plain-layout descriptor but for `b`; relay_kn4 runs the conversion (`kept`: once
+// for many products).
+int relaid_desc(const annc_gemm_desc& d, bool kept, annc_gemm_desc* plain);
 void relay_kn4(const float* packed, float* ws, long long k, long long n, int form, cudaStream_t s);
 // Device-side error word of the tensor-core kernels (a bounded wait that ran out).
 int read_error_flag(int* flag);

@@ -58,14 +58,13 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
   if (call.status() != ANNC_OK) return call.status();
   const size_t ws_bytes = (size_t)k * (size_t)n * sizeof(float);
   annc_gemm_desc plain;
-  // Asked before a buffer is taken, for one that is not filled may not be kept (the place of the buffer
-  // only counts by its alignment: the weight's own stands for it).
-  if (const int form = gemm::relaid_desc(d, const_cast<float*>(d.b), ws_bytes, &plain)) {
+  // Asked before a buffer is taken, for one that is not filled may not be kept.
+  if (const int form = gemm::relaid_desc(d, /*kept=*/true, &plain)) {
     auto relay = [&](void* ws) { gemm::relay_kn4(d.b, static_cast<float*>(ws), k, n, form, call.stream()); };
     // One kept copy per layout: the form goes with the batch, and the same bytes may be a weight of
     // another shape.
     void* ws = call.derived(b, b_count * sizeof(float), /*tag*/ 4 * n + form, ws_bytes, relay);
-    if (!ws) {
+    if (!ws && gemm::relaid_desc(d, /*kept=*/false, &plain)) {
       // A weight on the device (or not to be kept): re-laid into scratch by every call.  The pass
       // over the weight costs 8 us at 2048 x 4096 and 2 us at 256 x 512; the loader that takes the
       // packed panels as they lie is further behind at every size: 64 rows 24 us against 21 us in
@@ -73,7 +72,10 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
       ws = call.optional_scratch(ws_bytes);
       if (ws) relay(ws);
     }
-    if (ws && gemm::relaid_desc(d, ws, ws_bytes, &plain) == form) d = plain;
+    if (ws) {
+      d = plain;
+      d.b = static_cast<const float*>(ws);
+    }
   }
   ANNC_TRY(annc_gemm_run(&d, call.stream()));
   ANNC_TRY(call.finish());

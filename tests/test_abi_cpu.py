@@ -207,14 +207,14 @@ def test_kernel_map_resolves_library_symbols(annc):
 
 
 # ---------------------------------------------------------------- when a packed weight is re-laid
-def _relaid_form(annc, m, k, n, weight=1 << 20):
+def _relaid_form(annc, m, k, n, weight=1 << 20, out=3 << 20, kept=False):
     """Form the library re-lays a kn4 weight at this (never read) address into for such a product:
     1 = [N,K], 2 = [K,N], 0 = the weight is taken as it lies."""
-    fn = getattr(annc.lib, "_ZN4annc4gemm11relaid_descERK14annc_gemm_descPvmPS1_")  # gemm::relaid_desc
-    fn.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+    fn = getattr(annc.lib, "_ZN4annc4gemm11relaid_descERK14annc_gemm_descbPS1_")  # gemm::relaid_desc
+    fn.argtypes = [C.c_void_p, C.c_bool, C.c_void_p]
     from annc_b200._lib import B_KN4, GemmDesc
-    d = GemmDesc(0, 0, m, n, k, 1, k, n, n, n, 0, 0, 0, 0, 1.0, 0.0, 2 << 20, weight, 3 << 20, None, None, 0, B_KN4)
-    return fn(C.byref(d), 4 << 20, 4 * k * n, C.byref(GemmDesc()))
+    d = GemmDesc(0, 0, m, n, k, 1, k, n, n, n, 0, 0, 0, 0, 1.0, 0.0, 2 << 20, weight, out, None, None, 0, B_KN4)
+    return fn(C.byref(d), kept, C.byref(GemmDesc()))
 
 
 @pytest.mark.parametrize("m,k,n", [(64, 512, 256), (200, 2048, 4096), (8192, 2048, 4096)])
@@ -222,7 +222,17 @@ def test_a_packed_weight_off_16_bytes_is_not_relaid(annc, m, k, n):
     """The kernel that re-lays a weight reads it in 16-byte pieces."""
     assert _relaid_form(annc, m, k, n) != 0
     for off in (4, 8, 12):
-        assert _relaid_form(annc, m, k, n, weight=(1 << 20) + off) == 0
+        assert _relaid_form(annc, m, k, n, weight=(1 << 20) + off, kept=bool(off & 8)) == 0
+
+
+@pytest.mark.parametrize("m,k,n,form", [(64, 28, 512, 0), (64, 32, 512, 2), (1000, 16, 4096, 0), (64, 512, 12, 0),
+                                        (64, 512, 16, 2), (63, 512, 512, 0), (8192, 2048, 4096, 1),
+                                        (64, 2044, 8, 0), (64, 2048, 8, 1), (2048, 1020, 12, 0), (2048, 1024, 12, 1)])
+def test_a_packed_weight_is_relaid_where_it_pays(annc, m, k, n, form):
+    """For the tensor cores, and for the CUDA cores with a long K; where the output lies does not matter."""
+    assert _relaid_form(annc, m, k, n) == form
+    assert _relaid_form(annc, m, k, n, out=(3 << 20) + 4) == form
+    assert _relaid_form(annc, m, k, n, kept=True) == (0 if m < 64 else form or 1)  # once for many products
 
 
 @pytest.mark.parametrize("math,n,k,softmax,tiles,whole", [
