@@ -250,6 +250,7 @@ struct Relaid {
   void* dev;
   size_t bytes;
   cudaEvent_t filled;  // after the pass that filled it
+  bool settled;        // that pass is known to be over
 };
 struct Mirror {
   void* dev = nullptr;
@@ -554,11 +555,15 @@ void* Call::derived(const void* p, size_t bytes, long long tag, size_t out_bytes
   Mirror& m = it->second;
   auto d = m.derived.find(tag);
   if (d != m.derived.end()) {
-    cudaStreamWaitEvent(stream_, d->second.filled, 0);
-    return d->second.dev;
+    Relaid& r = d->second;
+    if (!r.settled && !(r.settled = cudaEventQuery(r.filled) == cudaSuccess)) {
+      cudaGetLastError();
+      cudaStreamWaitEvent(stream_, r.filled, 0);
+    }
+    return r.dev;
   }
   make_room(out_bytes, &it->first);
-  Relaid r{nullptr, out_bytes, nullptr};
+  Relaid r{nullptr, out_bytes, nullptr, false};
   if (cudaMalloc(&r.dev, out_bytes) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;

@@ -63,7 +63,7 @@ int gemm_host(const char* who, float* out, const float* a, const float* b, const
     auto relay = [&](void* ws) { gemm::relay_kn4(d.b, static_cast<float*>(ws), k, n, form, call.stream()); };
     // One kept copy per layout: the form goes with the batch, and the same bytes may be a weight of
     // another shape.
-    void* ws = call.derived(b, b_count * sizeof(float), /*tag*/ 4 * n + form, ws_bytes, relay);
+    void* ws = call.derived(b, b_count * sizeof(float), /*tag*/ 4 * n + form, ws_bytes, std::ref(relay));
     if (!ws && gemm::relaid_desc(d, /*kept=*/false, &plain)) {
       // A weight on the device (or not to be kept): re-laid into scratch by every call.  The pass
       // over the weight costs 8 us at 2048 x 4096 and 2 us at 256 x 512; the loader that takes the
