@@ -25,6 +25,14 @@ namespace {
 thread_local char g_error[512] = "";
 thread_local cudaStream_t g_stream = nullptr;
 
+// Allocations of this library belong to no capture, so they may run while another thread captures a
+// graph in the global mode (which otherwise forbids them to every thread, and is ended by them).
+struct OutsideCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // ---- scratch arena: bump allocator over cudaMalloc'd blocks, one per thread and device.
 // Blocks are kept: a call that outgrows them adds one, reset() only rewinds.
 struct Block {
@@ -36,6 +44,8 @@ struct Arena {
   std::vector<Block> blocks;
   ~Arena() { release(); }
   void release() {
+    if (blocks.empty()) return;
+    OutsideCaptures relaxed;
     for (auto& b : blocks) cudaFree(b.base);
     blocks.clear();
   }
@@ -54,6 +64,7 @@ struct Arena {
     }
     size_t cap = bytes < (size_t(1) << 20) ? (size_t(1) << 20) : bytes;
     char* p = nullptr;
+    OutsideCaptures relaxed;
     if (cudaMalloc(&p, cap) != cudaSuccess) return nullptr;
     blocks.push_back({p, cap, bytes});
     return p;
@@ -167,7 +178,9 @@ struct Mailbox {
   void* p = nullptr;
   bool tried = false;
   ~Mailbox() {
-    if (p) cudaFreeHost(p);
+    if (!p) return;
+    OutsideCaptures relaxed;
+    cudaFreeHost(p);
   }
 };
 thread_local Mailbox g_mailbox;
@@ -176,6 +189,7 @@ void* mailbox() {
   Mailbox& m = g_mailbox;
   if (!m.tried) {
     m.tried = true;
+    OutsideCaptures relaxed;
     if (cudaHostAlloc(&m.p, kMailboxBytes, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
       m.p = nullptr;

@@ -298,3 +298,36 @@ def test_small_k_product_at_every_k(m, n, k):
     want = np.maximum(a.astype(np.float64) @ b - c0 + bias, 0)
     size = abs(a).astype(np.float64) @ abs(b) + abs(c0) + abs(bias)
     assert (abs(c.cpu().numpy() - want) <= (k + 4) * 2.0 ** -24 * size).all()
+
+
+def test_layout_matmul_beside_a_capture_of_another_thread():
+    """A thread whose first call takes scratch, and that ends and gives it back, while another thread
+    captures: the capture goes on."""
+    import threading
+    g = torch.Generator(device="cuda").manual_seed(9)
+    a = torch.randn((200, 512), device="cuda", generator=g)
+    w = torch.randn((512, 1000), device="cuda", generator=g)
+    packed, out = device.kn4_pack(w), torch.empty((200, 1000), device="cuda")
+    x, y = torch.randn((64, 64), device="cuda", generator=g), torch.empty((64, 64), device="cuda")
+    step = lambda: device.gemm(x, x, y, m=64, n=64, k=64)
+    step()
+    ops.xla_layout_matmul(a, packed)  # the kernels are loaded
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def other():
+        with torch.cuda.stream(streams[1]):
+            ops._call_custom("__layout_matmul", out, [a, packed, ops.shape_info(a), ops.shape_info(packed)])
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        step()
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        step()
+    y.fill_(-7.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert nerr(y, (x.double() @ x.double()).cpu().numpy()) <= 2e-3
+    assert nerr(out, (a.double() @ w.double()).cpu().numpy()) <= 2e-3
