@@ -405,21 +405,28 @@ static bool capturing(cudaStream_t s) {
 
 Call::Call() : stream_(g_stream), device_(device_slot()) {
   g_arenas.per_device[device_].reset();
-  // A previous call of this thread that returned without synchronising (device pointers only)
-  // may still use the arena's scratch on another stream: order this call's stream after it.
-  // (A call being captured takes no scratch without a wait of its own, and may not depend on work
-  // outside the capture.)
-  if (g_unsynced[device_] && g_last_event[device_] && g_last_stream[device_] != stream_ && !capturing(stream_))
-    cudaStreamWaitEvent(stream_, g_last_event[device_], 0);
 }
+
+// A previous call of this thread that returned without synchronising (device pointers only) may still
+// use the arena's scratch on another stream: a call that takes some is ordered after it.
+void* Call::take_scratch(size_t bytes) {
+  void* d = g_arenas.per_device[device_].alloc(bytes);
+  if (d && !used_scratch_) {
+    if (g_unsynced[device_] && g_last_event[device_] && g_last_stream[device_] != stream_)
+      cudaStreamWaitEvent(stream_, g_last_event[device_], 0);
+    used_scratch_ = true;
+  }
+  return d;
+}
+
 Call::~Call() {
   if (used_scratch_ && !synced_) {
     if (!g_last_event[device_]) cudaEventCreateWithFlags(&g_last_event[device_], cudaEventDisableTiming);
     if (g_last_event[device_]) cudaEventRecord(g_last_event[device_], stream_);
     g_last_stream[device_] = stream_;
     g_unsynced[device_] = true;
-  } else if (synced_) {
-    g_unsynced[device_] = false;
+  } else if (synced_ && (used_scratch_ || g_last_stream[device_] == stream_)) {
+    g_unsynced[device_] = false;  // what used the scratch is over
   }
 }
 
@@ -541,9 +548,8 @@ void* Call::out(void* p, size_t bytes, bool preload) {
 
 void* Call::scratch(size_t bytes) {
   if (status_ != ANNC_OK) return nullptr;
-  void* d = g_arenas.per_device[device_].alloc(bytes);
+  void* d = take_scratch(bytes);
   if (!d) status_ = fail(ANNC_ERR_CUDA, "device scratch allocation of %zu bytes failed", bytes);
-  used_scratch_ = true;
   return d;
 }
 
@@ -551,9 +557,8 @@ void* Call::optional_scratch(size_t bytes) {
   if (status_ != ANNC_OK || bytes > kMaxOptionalScratch || capturing(stream_)) return nullptr;
   size_t cap = size_t(1) << 20;
   while (cap < bytes) cap <<= 1;
-  void* d = g_arenas.per_device[device_].alloc(cap);
+  void* d = take_scratch(cap);
   if (!d) cudaGetLastError();
-  else used_scratch_ = true;
   return d;
 }
 

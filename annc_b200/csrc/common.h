@@ -126,6 +126,7 @@ class Call {
     size_t bytes;
     int device;
   };
+  void* take_scratch(size_t bytes);
   const void* in_role(const void* p, size_t bytes, bool role_constant);
   void* mirror(const void* p, size_t bytes, bool upload, bool role_constant, bool is_output);
   cudaStream_t stream_;

@@ -300,6 +300,29 @@ def test_small_k_product_at_every_k(m, n, k):
     assert (abs(c.cpu().numpy() - want) <= (k + 4) * 2.0 ** -24 * size).all()
 
 
+def test_a_call_without_scratch_does_not_wait_for_one_with():
+    """Calls of one thread on two streams: only those that take the thread's scratch follow each other."""
+    g = torch.Generator(device="cuda").manual_seed(10)
+    a, w = torch.randn((200, 512), device="cuda", generator=g), torch.randn((512, 1000), device="cuda", generator=g)
+    packed, x = device.kn4_pack(w), torch.randn((64, 64), device="cuda", generator=g)
+    want = [ops.xla_layout_matmul(a, packed), ops.xla_matmul(x, x)]
+    torch.cuda.synchronize()
+    late, other = torch.cuda.Stream(), torch.cuda.Stream()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(late):
+        torch.cuda._sleep(400_000_000)
+        first = ops.xla_layout_matmul(a, packed)
+    with torch.cuda.stream(other):
+        plain = ops.xla_matmul(x, x)
+        done.record(other)
+        done.synchronize()
+        assert not late.query()
+        second = ops.xla_layout_matmul(a, packed)  # waits for the scratch
+        other.synchronize()
+        assert late.query()
+    assert torch.equal(plain, want[1]) and torch.equal(first, want[0]) and torch.equal(second, want[0])
+
+
 def test_layout_matmul_beside_a_capture_of_another_thread():
     """A thread whose first call takes scratch, and that ends and gives it back, while another thread
     captures: the capture goes on."""
