@@ -279,3 +279,13 @@ def test_fp32_gemm_refuses_more_than_4m_rows(annc, k, trans_b):
     assert annc.lib.annc_gemm_run(C.byref(d), None) != 0
     annc.lib.annc_last_error.restype = C.c_char_p
     assert b"more than 4M rows" in annc.lib.annc_last_error()
+
+
+@pytest.mark.parametrize("yes", [True, 1, np.bool_(True), np.int64(1)])
+def test_gemm_takes_transposes_of_any_truth_type(annc, yes):
+    """The binding converts the flags (the call itself is refused: no rows of such a product)."""
+    import torch
+    from annc_b200 import device
+    t = torch.zeros(64, 64)
+    with pytest.raises(annc.AnncError):
+        device.gemm(t, t, t, m=-1, n=64, k=64, trans_a=yes, trans_b=yes, stream=0)
