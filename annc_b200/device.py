@@ -26,7 +26,9 @@ def _stream() -> C.c_void_p:
 
 class BagPlan:
     """Holds the host descriptor array and the device workspace of one grouped
-    embedding-bag call (tables, id buffers, segment matrices and outputs fixed)."""
+    embedding-bag call (tables, id buffers, segment matrices and outputs fixed).  One run() at a
+    time: runs on different streams that may overlap need a plan each (the workspace holds the
+    counter from which the kernel hands out its work)."""
 
     def __init__(self, tables: Sequence[torch.Tensor], ids: Sequence[torch.Tensor],
                  slice_inputs: Sequence[torch.Tensor], out: torch.Tensor, out_slot0: int,

@@ -29,7 +29,13 @@
  * caller that rewrites part of a buffer in place between two calls, leaving every sampled word
  * as it was, must select mode 0 or 1 with annc_set_operand_cache.  One thread keeps one stream,
  * or synchronises before changing it (calls made with device pointers only do not wait for
- * the stream; a later call on another stream is ordered after them by an event).  There is no
+ * the stream; only calls that share the thread's scratch are ordered across streams, by an
+ * event).  Scratch comes from an arena of the calling thread and device, which grows with the
+ * largest call, is kept between calls and is freed when the thread ends or calls
+ * annc_release_device_memory.  __layout_matmul on a device weight of up to 256 MB takes it
+ * too (the weight is re-laid into it, 4 * K * N bytes rounded up to a power of two, so that at
+ * most 512 MB are held for such weights): the first call of a size allocates, and without the
+ * memory, or while its stream is captured, the call takes the weight as it lies.  There is no
  * CPU fallback anywhere: without a CUDA device every compute entry point fails with
  * ANNC_ERR_CUDA.
  *
@@ -84,7 +90,7 @@ int annc_set_operand_cache(int mode, size_t max_bytes);
  * host-to-device bytes that were not copied because the mirror already held them. */
 void annc_staging_counters(uint64_t* h2d_bytes, uint64_t* d2h_bytes, uint64_t* h2d_skipped_bytes);
 
-/* Frees the calling thread's scratch arena and every mirror (synchronises the device). */
+/* Frees the calling thread's scratch arenas and every mirror (synchronises the device). */
 void annc_release_device_memory(void);
 
 /* ---------------------------------------------------------------- gating
@@ -249,7 +255,10 @@ int annc_sparse_embedding2(const annc_tensor* ids, const annc_tensor* table, int
  * Sorted segment ids (the order of a canonical SparseTensor) run bit-exactly in the
  * reference's summation order; unsorted ids are accepted and reduced with atomics.
  * out f32[batch, ...]: row s is written at out + s*out_stride (out_stride >= D floats).
- * workspace: annc_embed_bag_workspace_bytes(batch) bytes of device memory. */
+ * workspace: annc_embed_bag_workspace_bytes(num_tables, batch) bytes of device memory, for one
+ * call at a time: it holds the counter from which the kernel hands out its work, so two calls
+ * that can overlap on the GPU (different streams, no ordering) take one each, or bags are left
+ * unwritten. */
 typedef struct annc_bag_table {
   const float* table;          /* f32[rows, D]                         */
   int64_t rows;                /* table rows (bounds check)            */
