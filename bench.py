@@ -459,10 +459,11 @@ def run_gpu(args):
     it = iter(pairs)
 
     # Back-to-back batches may be issued in two orders: one step after the other (forward), or
-    # with the dense part of a step (interaction + top MLP; sharded: on a second stream) under the next
-    # step's embedding part and, under row sharding, the split of the next step under this
-    # step's pooling (DlrmPipeline.forward_pipelined).  Which one is faster depends on how much
-    # of the GPU the embedding part leaves free; five steps of each decide, the same on all ranks.
+    # DlrmPipeline.forward_pipelined.  On one GPU that is the same kernels on the same stream with two
+    # sets of buffers; on several, the dense part of a step (interaction + top MLP) runs on a second stream
+    # under the next step's embedding part and, under row sharding, the split of the next step under
+    # this step's pooling.  Which one is faster depends on how much of the GPU the embedding part
+    # leaves free; five steps of each decide, the same on all ranks.
     # Under row sharding there is a third order (forward_pipelined(split=True)): the sum of the
     # parts moves to the dense stream as well, so the pooling kernels, bound by their NVLink
     # stores, follow one another on the main stream; optionally with one block per SM fewer
@@ -470,7 +471,8 @@ def run_gpu(args):
     step_fn, issue_order, order_ms = pipe.forward, "none", {}
     if hasattr(pipe, "forward_pipelined"):
         rowex = getattr(getattr(pipe, "rowbags", None), "ex", None)
-        cands = [("none", pipe.forward, 0), ("dense_part_under_next_embedding", pipe.forward_pipelined, 0)]
+        pipelined = "two_buffer_sets" if world == 1 else "dense_part_under_next_embedding"
+        cands = [("none", pipe.forward, 0), (pipelined, pipe.forward_pipelined, 0)]
         if getattr(pipe, "split_finish", False) and rowex is not None:
             fs = lambda: pipe.forward_pipelined(split=True)
             cands += [("sum_and_dense_part_under_next_pooling", fs, 0),
