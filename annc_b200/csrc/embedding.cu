@@ -70,18 +70,22 @@ struct StreamShape {
 };
 
 static void launch_stream(StreamShape& shape, const BagParams& p, BagHeader* hdr, cudaStream_t s) {
+  static int sm_count[kMaxDevices] = {0};
   const int slot = device_slot();
+  if (!sm_count[slot]) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, slot);
+    sm_count[slot] = sms;
+  }
   if (!shape.per_sm[slot]) {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, shape.kernel, 256, 0) != cudaSuccess || n < 1) n = 2;
     shape.per_sm[slot] = n;
   }
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, slot);
   const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, shape.per_sm[slot])
                                             : std::max(1, shape.per_sm[slot] + t_stream_ctas_per_sm);
   const long long groups_per_block = (256 / 32) * (32 / shape.lanes);
-  const long long max_blocks = (long long)sms * ctas;
+  const long long max_blocks = (long long)sm_count[slot] * ctas;
   long long lookups = 0;
   for (int t = 0; t < p.num_tables; ++t) lookups += p.t[t].nnz;
   StreamChunks sc;

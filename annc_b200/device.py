@@ -85,7 +85,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, *, m: int, n: int, k
          stream: Optional[int] = None) -> str:
     """annc_gemm_run on the current stream (or the one whose handle is given); returns the name of
     the kernel family that ran."""
-    d = GemmDesc(int(trans_a), int(trans_b), m, n, k, batch,
+    d = GemmDesc(1 if trans_a else 0, 1 if trans_b else 0, m, n, k, batch,
                  (m if trans_a else k) if lda is None else lda,
                  (k if trans_b else n) if ldb is None else ldb,
                  n if ldc is None else ldc, n if ld_addend is None else ld_addend,
