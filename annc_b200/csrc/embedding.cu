@@ -39,12 +39,15 @@ static thread_local int t_stream_ctas_per_sm = 0;
 // to start a chunk and to follow its last bag past the end; the chunk that makes
 // rounds x (chunk + 16) smallest therefore spreads few lookups over all groups (one tile each)
 // and cuts a batch of a few rounds so that the last one is nearly full.  One table with 2,700
-// lookups: 90 us with chunks of 128 (one block), 15 us with chunks of 8.  Where the tables are
-// long enough that chunks of 128 in flight stay within four of them, longer ones would spread
-// over more tables and their rows no longer share L2: 17.9 M lookups of dim 64 over 26 tables
-// of 144 K rows 608 us with chunks up to 128, 645 us up to 256, 701 us up to 512, 659 us up to
-// 64.  With short tables the limit only costs: 64 tables x 50 K lookups of dim 128 199 us against
-// 183 us.
+// lookups: 90 us with chunks of 128 (one block), 15 us with chunks of 8.
+// Chunks are no longer than 128 where that many lookups for every group stay within the lookups of
+// four tables (of average length): longer ones reach over more tables at a time, whose rows then
+// share L2.  17.9 M lookups of dim 64 over 26 tables of 144 K rows, ids of Zipf 1.05: 608 us with chunks up to
+// 128, 645 us up to 256, 701 us up to 512, 659 us up to 64; with ids that repeat more, 494 us / 493 / 527 / 519.
+// Where the tables have few lookups the limit only costs (64 tables x 50 K of dim 128: 193 us / 176 us
+// without), and with few tables a little (4 tables x 690 K of dim 64 105 us / 97 us; 12 x 340 K of dim 128
+// 212 / 197).  Of 18 workloads (1 to 100 tables, dim 16 to 128, 0.6 to 18 M lookups) it took a length
+// within 10 % of the best of 64, 128, 256, 512 and 2048 for each.
 static int stream_chunk(long long lookups, int num_tables, int lanes, long long groups) {
   const int limit = groups * 128 <= 4 * (lookups / num_tables) ? 128 : 64 * lanes;
   int best = lanes;

@@ -357,7 +357,8 @@ bag_reduce_generic_kernel(BagParams p, BagHeader* hdr, int* offsets) {
 // batch 16384, 4.47 M lookups: 248 us with the former loop (two loads, then two adds; ids of a
 // tile fetched at its start), 189 us now; 26 x 2,100 lookups: 100 us -> 18 us.  Choices at
 // that size: DEPTH 2 with 64 registers 202 us, DEPTH 4 with 80 216 us, 64 bytes per lane 289 us,
-// groups that drift apart 414 us.
+// groups that drift apart 414 us.  The registers are its limit: at 64 it spills 54 bytes (dim 64; 68 at dim
+// 128).
 // The chunk length comes from the launch (stream_chunk): short for few lookups, so that they
 // spread over all SMs, long enough for a batch that fills the chip several times.
 //
