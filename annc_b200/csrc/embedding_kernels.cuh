@@ -20,7 +20,7 @@ constexpr int kMaxTables = 120;         // tables per grouped launch: BagParams 
 constexpr int kErrRow = 1;              // row index outside its table
 constexpr int kErrSegment = 2;          // segment id outside [0, batch)
 
-// Head of the bag workspace (256 bytes), then int32 offsets[num_tables][batch + 1].
+// Head of the bag workspace (512 bytes), then int32 offsets[num_tables][batch + 1].
 struct BagHeader {
   int err_bits;
   int any_unsorted;          // some table of the call is marked below
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(256, 4) bag_wide_kernel(BagParams p, StreamChu
   constexpr int LANES = 32, VPL = 2, INFLIGHT = 4, DIM = LANES * VPL * 4;
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kNoBag = -3;  // a lookup whose segment id is out of range is added nowhere
-  using Vec = RowVec<4>;
+  using Vec = RowVec;
   __shared__ int s_first[kMaxTables + 1];
   for (int i = threadIdx.x; i <= p.num_tables; i += blockDim.x) s_first[i] = sc.first[i];
   __syncthreads();
