@@ -112,14 +112,14 @@ static StreamShape& stream_shape(int vecs) {
   return vecs == LANES * VPL ? full : part;
 }
 
-// Rows of up to 128 floats for a caller that gave the kernel a share of two or more blocks per SM (0 and 1:
-// the faster shape).  The pooling kernel of the row exchange fits five times on an SM at these widths, and
+// Rows of up to 128 floats for a caller that gave the kernel a share of two to four blocks per SM (one leaves
+// room as it is, five are not beside anything: the faster shape).  The pooling kernel of the row exchange fits five times on an SM at these widths, and
 // shares of the two kernels that add up to five have to fit together: 48 registers, as that one has,
 // instead of 64 (three blocks of those leave room for one of the pooling kernel).  11 tables x 60 K rows of
 // dim 64, batch 16384, three blocks per SM, alone: 108 us, 79 us with 64 registers (two blocks 130 / 93).
 template <int LANES, int VPL>
 static StreamShape& stream_shape_beside(int vecs) {
-  return t_stream_ctas_per_sm >= 2 ? stream_shape<LANES, VPL, 2, 5>(vecs) : stream_shape<LANES, VPL, 2, 4>(vecs);
+  return t_stream_ctas_per_sm >= 2 && t_stream_ctas_per_sm <= 4 ? stream_shape<LANES, VPL, 2, 5>(vecs) : stream_shape<LANES, VPL, 2, 4>(vecs);
 }
 
 // The smallest shape whose LANES x VPL vectors hold a row; 32 bytes per lane from dim 64 on: fewer
