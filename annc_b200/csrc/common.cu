@@ -273,7 +273,7 @@ struct Mirror {
   bool valid = false;            // the mirror holds those contents
   bool pinned = false;           // registered with annc_register_constant: never evicted, never re-checked
   unsigned long long tick = 0;
-  int users = 0;                 // calls copying into the mirror right now: not to be evicted
+  int users = 0;                 // calls that were handed the mirror and have not ended: not to be evicted
   cudaEvent_t ready = nullptr;   // after the last write of the mirror
   cudaEvent_t used = nullptr;    // after the last read of the mirror
   std::unordered_map<long long, Relaid> derived;  // re-laid forms of a constant, by tag
@@ -420,6 +420,13 @@ void* Call::take_scratch(size_t bytes) {
 }
 
 Call::~Call() {
+  if (!held_.empty()) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    for (auto& k : held_) {
+      auto it = g_mirrors.find(Key{k.host, k.bytes, k.device});
+      if (it != g_mirrors.end() && it->second.users > 0) --it->second.users;
+    }
+  }
   if (used_scratch_ && !synced_) {
     if (!g_last_event[device_]) cudaEventCreateWithFlags(&g_last_event[device_], cudaEventDisableTiming);
     if (g_last_event[device_]) cudaEventRecord(g_last_event[device_], stream_);
@@ -475,6 +482,8 @@ void* Call::mirror(const void* p, size_t bytes, bool upload, bool role_constant,
     Mirror& m = it->second;
     mp = &m;  // stays where it is: entries are only erased by eviction, which skips `users`
     m.tick = ++g_tick;
+    ++m.users;
+    held_.push_back({key.host, key.bytes, key.device});
     may_reuse = !m.pinned && (g_mode == 2 || (g_mode == 1 && role_constant));
     if (upload) {
       need = true;
@@ -485,7 +494,6 @@ void* Call::mirror(const void* p, size_t bytes, bool upload, bool role_constant,
         need = !(m.valid && m.print == fp);
       }
       if (need) {
-        ++m.users;
         // writers wait for the readers and the writer before them
         cudaStreamWaitEvent(stream_, m.used, 0);
         cudaStreamWaitEvent(stream_, m.ready, 0);
@@ -505,7 +513,6 @@ void* Call::mirror(const void* p, size_t bytes, bool upload, bool role_constant,
   if (need) {  // the copy itself runs outside the lock: other threads' calls go on
     const cudaError_t e = staged_h2d(mp->dev, p, bytes, stream_);
     std::lock_guard<std::mutex> lk(g_mu);
-    --mp->users;
     if (e != cudaSuccess) {
       status_ = cuda_fail(e, "host-to-device copy");
       return nullptr;

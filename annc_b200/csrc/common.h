@@ -137,6 +137,7 @@ class Call {
   bool used_scratch_ = false;
   std::vector<Pending> pending_;
   std::vector<Touched> touched_;
+  std::vector<Touched> held_;  // mirrors this call was handed: kept until it ends
 };
 
 }  // namespace annc

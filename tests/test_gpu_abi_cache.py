@@ -216,6 +216,28 @@ def test_layout_matmul_constant_registered_again():
         assert lib.annc_unregister_constant(packed.ctypes.data) == 0
 
 
+@pytest.mark.parametrize("cap", [1, 1 << 20])
+def test_operands_beyond_the_cap_are_kept_for_their_call(cap):
+    """A call whose operands do not fit under the cap has them all on the device until it ends; the next
+    one uploads what was dropped since."""
+    rng = np.random.default_rng(4)
+    lib.annc_set_operand_cache(2, cap)
+    try:
+        for m, k, n in ((300, 512, 1024), (70, 2048, 516), (300, 512, 1024)):
+            x = rng.standard_normal((m, k)).astype(np.float32)
+            w = (rng.standard_normal((k, n)) / 16).astype(np.float32)
+            addend = rng.standard_normal((m, n)).astype(np.float32)
+            out = np.empty((m, n), np.float32)
+            info = [ops.shape_info(addend), ops.shape_info(addend), ops.shape_info(x), ops.shape_info(w)]
+            ops._call_custom("__matmul_add_relu", out, [addend, addend, x, w] + info)
+            assert nerr(out, oracle.matmul_add_relu(addend, x, w)) <= 2e-3
+            packed = oracle.kn4_pack(w)
+            ops._call_custom("__layout_matmul", out, [x, packed, ops.shape_info(x), ops.shape_info(packed)])
+            assert nerr(out, x.astype(np.float64) @ w) <= 2e-3
+    finally:
+        lib.annc_set_operand_cache(2, 24 << 30)
+
+
 def test_a_wait_that_ran_out_is_reported(capfd):
     rng = np.random.default_rng(3)
     a = rng.standard_normal((256, 256)).astype(np.float32)
