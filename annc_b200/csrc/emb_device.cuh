@@ -26,6 +26,12 @@ __device__ __forceinline__ unsigned long long fast_mod_u64(unsigned long long x,
   return r;
 }
 
+// The same for d below 2^31: the estimate leaves less than 2 d, so that 32 bits hold what is left.
+__device__ __forceinline__ unsigned fast_mod_u64_small(unsigned long long x, unsigned d, unsigned long long magic) {
+  const unsigned r = (unsigned)x - (unsigned)__umul64hi(x, magic) * d;
+  return r >= d ? r - d : r;
+}
+
 __device__ __forceinline__ long long load_row_id(const void* ids, int id_kind, long long i,
                                                  unsigned long long num_buckets,
                                                  unsigned long long magic) {
@@ -43,19 +49,6 @@ __device__ __forceinline__ void add4(float4& a, const float4& b) {
   a.z = __fadd_rn(a.z, b.z);
   a.w = __fadd_rn(a.w, b.w);
 }
-
-// Sixteen bytes of a row, loaded through the read-only path and added with round-to-nearest adds (no
-// contraction).
-struct RowVec {
-  float4 v;
-  __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ void load(const float* p) { v = ldg4(p); }
-  __device__ __forceinline__ void store(float* p) const { *reinterpret_cast<float4*>(p) = v; }
-  __device__ __forceinline__ void add(const RowVec& o) { add4(v, o.v); }
-  __device__ __forceinline__ void scale(float f) {
-    v.x = __fmul_rn(v.x, f); v.y = __fmul_rn(v.y, f); v.z = __fmul_rn(v.z, f); v.w = __fmul_rn(v.w, f);
-  }
-};
 
 // ---- exclusive scan of int32 (three passes, 2048 items per block) ---------------
 constexpr int kScanThreads = 512;

@@ -65,10 +65,34 @@ static int stream_chunk(long long lookups, int num_tables, int lanes, long long 
   return best;
 }
 
-// A lookup-granular kernel: lanes of a group, and its resident blocks per SM by device (0: not asked).
+// Lookups per chunk of the kernel by lists of bags: up to what a window holds, cut so that the last round of
+// a batch of a few rounds is nearly full, and short for few lookups, which then spread over all SMs.  A
+// warp pays about 64 lookups' worth of time to start a chunk (17.9 M lookups of dim 64: 478 us with
+// chunks of 224, 505 with 160, 549 with 96).  Warps of several groups take at least 24: a bag each for
+// their groups (26 x 2,100 lookups: 14.3 us with 8, 10.2 with 16, 9.1 with 24, 9.0 with 32; 1 x 2,100
+// 6.2 / 6.3 / 6.3 / 7.3).
+static int list_chunk(long long lookups, int num_tables, long long warps, int lanes) {
+  const int least = lanes == 32 ? 8 : 24;
+  int best = least;
+  long long best_cost = -1;
+  for (int chunk = least; chunk <= kBagChunk; chunk += 8) {
+    const long long chunks = lookups / chunk + num_tables / 2 + 1;
+    const long long rounds = (chunks + warps - 1) / warps;
+    const long long cost = rounds * (chunk + 64);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = chunk;
+    }
+  }
+  return best;
+}
+
+// A lookup-granular kernel: lanes of a group, whether it is the one by lists, and its resident blocks per SM
+// by device (0: not asked).
 struct StreamShape {
   void (*kernel)(BagParams, StreamChunks, BagHeader*);
   int lanes;
+  bool list;
   int per_sm[kMaxDevices];
 };
 
@@ -87,12 +111,14 @@ static void launch_stream(StreamShape& shape, const BagParams& p, BagHeader* hdr
   }
   const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, shape.per_sm[slot])
                                             : std::max(1, shape.per_sm[slot] + t_stream_ctas_per_sm);
-  const long long groups_per_block = (256 / 32) * (32 / shape.lanes);
+  // a chunk is a warp's, or a group's
+  const long long takers = shape.list ? 256 / 32 : 256 / shape.lanes;
   const long long max_blocks = (long long)sm_count[slot] * ctas;
   long long lookups = 0;
   for (int t = 0; t < p.num_tables; ++t) lookups += p.t[t].nnz;
   StreamChunks sc;
-  sc.chunk = stream_chunk(lookups, p.num_tables, shape.lanes, max_blocks * groups_per_block);
+  sc.chunk = shape.list ? list_chunk(lookups, p.num_tables, max_blocks * takers, shape.lanes)
+                        : stream_chunk(lookups, p.num_tables, shape.lanes, max_blocks * takers);
   long long total = 0;
   for (int t = 0; t < p.num_tables; ++t) {
     sc.first[t] = (int)total;
@@ -101,15 +127,21 @@ static void launch_stream(StreamShape& shape, const BagParams& p, BagHeader* hdr
   }
   sc.first[p.num_tables] = (int)total;
   // a persistent grid, no larger than the chunks there are
-  const long long blocks = std::min(max_blocks, (total + groups_per_block - 1) / groups_per_block);
+  const long long blocks = std::min(max_blocks, (total + takers - 1) / takers);
   shape.kernel<<<(unsigned)std::max<long long>(blocks, 1), 256, 0, s>>>(p, sc, hdr);
 }
 
-template <int LANES, int VPL, int DEPTH, int MINB>
+template <int LANES, int VPL, int MINB>
 static StreamShape& stream_shape(int vecs) {
-  static StreamShape full{bag_stream_kernel<LANES, VPL, DEPTH, true, MINB>, LANES, {}};
-  static StreamShape part{bag_stream_kernel<LANES, VPL, DEPTH, false, MINB>, LANES, {}};
+  static StreamShape full{bag_stream_kernel<LANES, VPL, 2, true, MINB>, LANES, false, {}};
+  static StreamShape part{bag_stream_kernel<LANES, VPL, 2, false, MINB>, LANES, false, {}};
   return vecs == LANES * VPL ? full : part;
+}
+
+template <int LANES, int F, int VPL, int Q, int MINB = 4>
+static StreamShape& list_shape() {
+  static StreamShape shape{bag_list_kernel<LANES, F, VPL, Q, MINB>, LANES, true, {}};
+  return shape;
 }
 
 // Rows of up to 128 floats for a caller that gave the kernel a share of two to four blocks per SM (one leaves
@@ -117,22 +149,34 @@ static StreamShape& stream_shape(int vecs) {
 // shares of the two kernels that add up to five have to fit together: 48 registers, as that one has,
 // instead of 64 (three blocks of those leave room for one of the pooling kernel).  11 tables x 60 K rows of
 // dim 64, batch 16384, three blocks per SM, alone: 108 us, 79 us with 64 registers (two blocks 130 / 93).
+static bool beside() { return t_stream_ctas_per_sm >= 2 && t_stream_ctas_per_sm <= 4; }
 template <int LANES, int VPL>
 static StreamShape& stream_shape_beside(int vecs) {
-  return t_stream_ctas_per_sm >= 2 && t_stream_ctas_per_sm <= 4 ? stream_shape<LANES, VPL, 2, 5>(vecs) : stream_shape<LANES, VPL, 2, 4>(vecs);
+  return beside() ? stream_shape<LANES, VPL, 5>(vecs) : stream_shape<LANES, VPL, 4>(vecs);
 }
 
-// The smallest shape whose LANES x VPL vectors hold a row; 32 bytes per lane from dim 64 on: fewer
-// lanes repeat the per-lookup control instructions.
-static StreamShape& stream_shape_for(int vecs, long long max_nnz) {
-  static StreamShape wide{bag_wide_kernel, 32, {}};
-  if (vecs <= 4) return stream_shape_beside<4, 1>(vecs);
-  if (vecs <= 8) return stream_shape_beside<8, 1>(vecs);
-  if (vecs <= 16) return stream_shape_beside<8, 2>(vecs);
-  if (vecs <= 32) return stream_shape_beside<16, 2>(vecs);
-  if (vecs == 64 && max_nnz < kWideLookups) return wide;
-  if (vecs <= 64) return stream_shape<32, 2, 2, 4>(vecs);
-  return stream_shape<32, 4, 2, 3>(vecs);
+// The smallest shape whose lanes hold a row, from dim 64 on 32 bytes each where rows are `wide`, 32-byte
+// aligned and a multiple of that long: fewer lanes repeat the control instructions, more bags go at a time.
+// mean_bag: lookups per bag, on average.  us for 11 tables x 60 K rows, bags of 1 to n lookups:
+//   * short bags stay with the pipeline, whose steps do not wait for a list; pipeline / list
+//       dim 16   n = 2 36 / 43, 4 44 / 46, 8 43 / 41, 20 45 / 40;   dim 32   2 62 / 71, 4 72 / 71, 8 64 / 62, 20 58 / 54
+//       dim 64   1 75 / 80, 2 85 / 88, 4 103 / 98, 20 82 / 73;      dim 128  1 132 / 141, 2 128 / 128, 4 103 / 100, 20 81 / 72
+//       dim 100 (not wide)  4 107 / 125, 8 91.3 / 91.5, 20 85 / 73
+//     dim 256  1 139 / 129 two rows at a time, 2 128 / 124, 20 74.1 / 74.0: by lists only
+//   * so does a share of the SM's slots, too few warps to hide the list's latencies: two blocks of dim 64
+//     152 / 164, of dim 128 137 / 150, three 126 / 126, 118 / 122
+//   * long bags are taken by groups twice as large, eight rows at a time: a chunk has too few of them for
+//     many groups.  dim 64, four / eight rows: 1 to 20 478 / 498 (26 tables up to 1 M rows), 1 to 30 72.1 / 72.5,
+//     20 to 40 73 / 69, 64 to 128 206 / 140
+static StreamShape& stream_shape_for(int vecs, bool wide, double mean_bag) {
+  const bool pipeline = beside() || mean_bag < (vecs <= 4 ? 3.5 : vecs > 8 && !wide ? 4.5 : 2.0);
+  const bool eight = mean_bag >= 18 || !wide;
+  if (vecs <= 4) return pipeline ? stream_shape_beside<4, 1>(vecs) : list_shape<4, 4, 1, 4>();
+  if (vecs <= 8) return pipeline ? stream_shape_beside<8, 1>(vecs) : list_shape<8, 4, 1, 4>();
+  if (vecs <= 16) return pipeline ? stream_shape_beside<8, 2>(vecs) : eight ? list_shape<16, 4, 1, 8>() : list_shape<8, 8, 1, 4>();
+  if (vecs <= 32) return pipeline ? stream_shape_beside<16, 2>(vecs) : eight ? list_shape<32, 4, 1, 8>() : list_shape<16, 8, 1, 4>();
+  if (vecs <= 64) return mean_bag < 2 ? list_shape<32, 4, 2, 2>() : wide ? list_shape<32, 8, 1, 4>() : list_shape<32, 4, 2, 4>();
+  return wide ? list_shape<32, 8, 2, 2, 3>() : list_shape<32, 4, 4, 2, 3>();
 }
 
 // Between two groups of tables of one call: the marks and the chunk counter start again.
@@ -168,8 +212,8 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
   p.batch = batch;
   p.dim = dim;
   p.out_stride = out_stride;
-  long long max_nnz = 0;
-  bool vec_ok = (dim % 4 == 0) && (out_stride % 4 == 0);
+  long long max_nnz = 0, lookups = 0;
+  bool vec_ok = (dim % 4 == 0) && (out_stride % 4 == 0), wide = dim % 8 == 0;
   for (int t = 0; t < num_tables; ++t) {
     if (tables[t].nnz >= (int64_t(1) << 31) - 1)
       return fail(ANNC_ERR_UNSUPPORTED, "more than 2^31-2 lookups in one table");
@@ -187,7 +231,9 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
     p.t[t].nnz = (int)tables[t].nnz;
     p.t[t].given_off = tables[t].offsets;
     max_nnz = std::max<long long>(max_nnz, tables[t].nnz);
+    lookups += tables[t].nnz;
     vec_ok = vec_ok && aligned16(tables[t].table) && aligned16(tables[t].out);
+    wide = wide && (reinterpret_cast<uintptr_t>(tables[t].table) & 31) == 0;
   }
   if (batch <= 0) return ANNC_OK;
 
@@ -211,7 +257,7 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
                       ncols < (1LL << 31) && out_stride < (1LL << 31);
   if (stream) {
     if (ev0) cudaEventRecord(ev0, s);
-    launch_stream(stream_shape_for(vecs, max_nnz), p, hdr, s);
+    launch_stream(stream_shape_for(vecs, wide, (double)lookups / ((double)num_tables * (double)batch)), p, hdr, s);
     if (ev1) cudaEventRecord(ev1, s);
     if (known_sorted) {
       ANNC_CUDA(cudaGetLastError());
@@ -331,7 +377,7 @@ int annc_embed_bag_stream_registers(int64_t dim, int* registers_per_thread) {
   ANNC_REQUIRE(registers_per_thread && dim >= 4 && dim <= 512 && dim % 4 == 0, ANNC_ERR_INVALID_ARGUMENT,
                "bag registers: dim must be a multiple of four up to 512");
   cudaFuncAttributes attr;
-  ANNC_CUDA(cudaFuncGetAttributes(&attr, stream_shape_for((int)(dim / 4), 0).kernel));
+  ANNC_CUDA(cudaFuncGetAttributes(&attr, stream_shape_for((int)(dim / 4), dim % 8 == 0, 10).kernel));
   *registers_per_thread = attr.numRegs;
   return ANNC_OK;
 }

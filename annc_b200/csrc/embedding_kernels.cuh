@@ -349,8 +349,10 @@ bag_reduce_generic_kernel(BagParams p, BagHeader* hdr, int* offsets) {
 // 0, the last bag's owner to the end).  A decrease of the segment ids marks the table unsorted:
 // bag_stream_reset_kernel then clears its output and the atomic route below redoes it.
 //
-// What bounds it: DRAM for tables beyond L2 (batch 65536 over 26 tables of 100 K rows moves
-// 3.4 GB, 0.67 ms), else the instructions per lookup and the latency of the row loads.  So the loop
+// For bags of a few lookups, and for callers that leave it a share of the SMs' block slots; bag_list_kernel
+// below takes the others (the line between them: stream_shape_for).
+//
+// What bounds it: the instructions per lookup and the latency of the row loads.  So the loop
 // is an unrolled pipeline: DEPTH - 1 row loads are out before a row is added, across tile borders
 // too, the ids of the next tile are already under way, and what only a bag's start needs (its
 // number, gaps of empty bags) is kept out of the loop.  Measured, 26 tables x 1 M rows x dim 64,
@@ -600,28 +602,118 @@ bag_stream_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
   pdl_trigger();
 }
 
-// The same for rows of 256 floats: a warp per chunk and two vectors per lane.  Row loads go out four at
-// a time and are added when they are back, without the pipeline above: of these long rows that keeps
-// only two on their way in 64 registers, and what it spills is reloaded from behind the rows that
-// stream through L1.  26 tables x 100 K rows, batch 2048: 63 us, 82 us in the pipeline (with four rows
-// on their way 108 us, with 80 registers 83 us); 10 tables x 1 M rows, batch 16384: 151 us / 186 us;
-// batch 100 over 26 tables 19 us / 23 us.  It lives at the edge of its registers (20 bytes spilled): with a
-// launch trigger at its end it spills 44 and the same three take 66, 163 and 21 us.
-// Tables of up to kWideLookups lookups, so that sums with a chunk fit an int.
-constexpr long long kWideLookups = (1LL << 31) - 8192;
-__global__ void __launch_bounds__(256, 4) bag_wide_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
-  constexpr int LANES = 32, VPL = 2, INFLIGHT = 4, DIM = LANES * VPL * 4;
+// ---- the same by lists of bags ---------------------------------------------------------
+// A warp takes a chunk of consecutive lookups of a table and
+// owns the bags whose first lookup lies in it; it follows its last bag past the chunk.
+//
+// First the whole warp decodes a window, the chunk and up to kBagAhead lookups behind it, one lookup
+// per lane: ids and segment ids by coalesced evict-first loads, the hash-bucket modulo, the rows'
+// addresses into shared memory; one ballot over the bag starts of a tile of 32 makes the list of the
+// chunk's bags.  Bags without lookups are zero-filled by the owner of the next bag (the first bag's
+// owner fills from 0, the last bag's owner to the end).  A decrease of the segment ids marks the table
+// unsorted: bag_stream_reset_kernel then clears its output and the atomic route below redoes it.
+//
+// Then the warp's groups of LANES lanes take bags from the list, each the next one when it has
+// finished its own: a round loads Q rows of every group's bag and adds them in lookup order into a
+// zero accumulator (the reference's order, bit-identical sums).  All groups run the same rounds; only
+// a finished bag's store and the fetch of the next one are conditional.
+//
+// What bounds it: the instructions per lookup and the latency of ids and rows; DRAM is at 40 to 55 %.
+// Hence: an address, not a row number, in shared memory (computed once, by the lane that decoded it);
+// a row of zeros for what is not to be added, so that loads and packed adds need no guards (predicated
+// packed adds are made of twice the instructions); rare ids behind one vote per tile.  The kernel above,
+// in which every step asks whether a bag begins, and this one, us:
+// 539 / 479 for 17.9 M lookups over 26 tables of up to 1 M rows of dim 64, 198 / 180 for 4.5 M over 26
+// x 1 M rows, 173 / 144 for 64 x 50 K rows of dim 128 in bags of 25, 12.0 / 9.1 for 26 tables x 2,100
+// lookups, 137 / 133 for 6 tables of dim 256.  Tried, us for 4.1 M lookups of dim 64 (this kernel: 127):
+// row copies into a ring in shared memory 168, and 358 past L1, whose hits keep the popular rows off their L2
+// slices; a warp per bag 179; groups over fixed shares of the chunk 167; windows of 160 lookups 140; two
+// 16-byte loads per row and lane instead of one of 32 138.  Ids of eight tiles at a time: 191 instead of 180.
+// Chunks are handed out as above.
+constexpr int kBagWindow = 256;                   // lookups decoded at a time
+constexpr int kBagAhead = 32;                     // of these behind the chunk: the end of its last bag
+constexpr int kBagChunk = kBagWindow - kBagAhead;
+
+// F floats of a row (4 or 8), one load of 16 or 32 aligned bytes, as packed pairs; each half of an add rounds
+// like __fadd_rn.
+template <int F>
+struct RowPiece {
+  static_assert(F == 4 || F == 8, "16 or 32 bytes");
+  unsigned long long v[F / 2];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int k = 0; k < F / 2; ++k) v[k] = 0ull;
+  }
+  __device__ __forceinline__ void load(const char* p) {
+    if (F == 8) {
+      asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+          : "=l"(v[0]), "=l"(v[1]), "=l"(v[F / 2 - 2]), "=l"(v[F / 2 - 1])
+          : "l"(p));
+    } else {
+      const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2*>(p));
+      v[0] = a.x;
+      v[1] = a.y;
+    }
+  }
+  __device__ __forceinline__ void add(const RowPiece& o) {
+#pragma unroll
+    for (int k = 0; k < F / 2; ++k) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v[k]) : "l"(o.v[k]));
+  }
+  __device__ __forceinline__ float4 four(int h) const {
+    float4 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v[2 * h]));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.z), "=f"(f.w) : "l"(v[2 * h + 1]));
+    return f;
+  }
+};
+
+// What stands for the rows that are not added, behind a bag's end or out of range: adding +0 changes no sum
+// that began at +0.
+__device__ __align__(32) float g_zero_row[512];
+
+template <int LANES, int F, int VPL, int Q, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+bag_list_kernel(BagParams p, StreamChunks sc, BagHeader* hdr) {
+  constexpr int GROUPS = 32 / LANES;
+  constexpr int TILES = 4;  // tiles of 32 lookups whose ids are on their way together
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kNoBag = -3;  // a lookup whose segment id is out of range is added nowhere
-  using Vec = RowVec;
+  using Vec = RowPiece<F>;
   __shared__ int s_first[kMaxTables + 1];
+  __shared__ unsigned long long s_row[8][kBagWindow + Q];  // where the rows of the decoded lookups are
+  // The chunk's bags: number, first lookup and the one behind the last, counted from the window's start
+  // (an entry before the first: the one whose end the first bag writes).
+  struct BagEntry {
+    int bag;
+    unsigned short first, end;
+  };
+  __shared__ __align__(8) BagEntry s_bag[8][kBagChunk + 2];
   for (int i = threadIdx.x; i <= p.num_tables; i += blockDim.x) s_first[i] = sc.first[i];
   __syncthreads();
   const int batch = (int)p.batch;
-  const int lane = threadIdx.x & 31;
-  const unsigned total_chunks = (unsigned)s_first[p.num_tables];
-  const unsigned warps = gridDim.x * (blockDim.x >> 5);
-  for (unsigned gc = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); gc < total_chunks; gc += warps) {
+  const unsigned pitch = (unsigned)p.dim * 4u;                                // bytes of a table row
+  const unsigned long long opitch = (unsigned long long)p.out_stride * 4ull;  // between two output rows
+  const unsigned long long spitch = (unsigned long long)p.ncols * 8ull;       // between two segment ids
+  const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31;
+  const int lane = wl % LANES, group = wl / LANES;
+  unsigned long long* const rows = s_row[warp];
+  const unsigned long long nothing = reinterpret_cast<unsigned long long>(g_zero_row);
+  BagEntry* const bags = s_bag[warp] + 1;
+  // Lane l holds the floats F l .. F l + F - 1 of every block of F * LANES; a lane past the row's end reads
+  // its start instead and writes nothing.  (dim is a multiple of F.)
+  bool col_ok[VPL];
+  int col[VPL];  // bytes
+#pragma unroll
+  for (int w = 0; w < VPL; ++w) {
+    const int c = (w * LANES + lane) * F;
+    col_ok[w] = c < (int)p.dim;
+    col[w] = col_ok[w] ? c * 4 : 0;
+  }
+
+  unsigned gc_next = blockIdx.x * 8 + warp;
+  while (gc_next < (unsigned)s_first[p.num_tables]) {
+    const unsigned gc = gc_next;
+    if (wl == 0) gc_next = gridDim.x * 8 + (unsigned)atomicAdd(&hdr->next_chunks, 1);
     int lo = 0, hi = p.num_tables - 1;  // table of chunk gc: last t with first[t] <= gc
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -629,124 +721,218 @@ __global__ void __launch_bounds__(256, 4) bag_wide_kernel(BagParams p, StreamChu
       else hi = mid - 1;
     }
     const int t = lo;
-    const unsigned chunk = gc - (unsigned)s_first[t];
     const BagTableDev& T = p.t[t];
     const int n = T.nnz;
-    const float* __restrict__ tab = T.table;
-    float* __restrict__ outp = T.out;
+    char* const outp = reinterpret_cast<char*>(T.out);
+    const unsigned long long tab = reinterpret_cast<unsigned long long>(T.table);
+    const char* const segs = reinterpret_cast<const char*>(T.seg + p.col);
 
-    // rows [a, b) of the output <- 0 (bags without lookups)
+    auto store = [&](char* o, const Vec& a, int w, bool mean, float inv) {
+#pragma unroll
+      for (int h = 0; h < F / 4; ++h) {
+        float4 f = a.four(h);
+        if (mean) {
+          f.x = __fmul_rn(f.x, inv);
+          f.y = __fmul_rn(f.y, inv);
+          f.z = __fmul_rn(f.z, inv);
+          f.w = __fmul_rn(f.w, inv);
+        }
+        if (col_ok[w]) __stcs(reinterpret_cast<float4*>(o + col[w] + 16 * h), f);
+      }
+    };
+    // rows [a, b) of the output <- 0 (bags without lookups), by the whole warp
     auto zero_fill = [&](int a, int b) {
       Vec z;
       z.zero();
-      for (int s = a; s < b; ++s) {
-        float* o = outp + (long long)s * p.out_stride;
+      for (int s = a + group; s < b; s += GROUPS) {
 #pragma unroll
-        for (int w = 0; w < VPL; ++w) z.store(o + (w * LANES + lane) * 4);
+        for (int w = 0; w < VPL; ++w) store(outp + (unsigned)s * opitch, z, w, false, 1.f);
       }
     };
+    const long long chunk = (long long)(gc - (unsigned)s_first[t]);
     if (n == 0) {  // a table without lookups: every bag is empty
-      zero_fill((int)min((long long)chunk * 1024, (long long)batch), (int)min((long long)(chunk + 1) * 1024, (long long)batch));
+      zero_fill((int)min(chunk * 1024, (long long)batch), (int)min((chunk + 1) * 1024, (long long)batch));
+      gc_next = __shfl_sync(kAll, gc_next, 0);
       continue;
+    }
+    const int base = (int)(chunk * sc.chunk);  // below nnz < 2^31
+    const int own = (int)min((long long)sc.chunk, (long long)n - base);
+
+    int before = -1;  // segment of the lookup before the next tile
+    if (base > 0) {
+      const unsigned long long ps = __ldcs(reinterpret_cast<const unsigned long long*>(segs + (unsigned)(base - 1) * spitch));
+      before = ps < (unsigned long long)batch ? (int)ps : kNoBag;
     }
     Vec acc[VPL];
 #pragma unroll
     for (int w = 0; w < VPL; ++w) acc[w].zero();
-    int cur = kNoBag;  // bag being summed
-    int count = 0;     // its lookups so far (for the mean)
-    bool open = false;
-    auto flush = [&]() {
-      if (open && cur >= 0) {
-        if (p.combiner == 1 && count > 0) {
-          const float inv = __fdiv_rn(1.0f, (float)count);
+    // The chunk's window, and then windows of the lookups behind it while its last bag goes on: one group
+    // (`holder`) has that bag and `counted` lookups of it in its accumulator.
+    int from = base, mine = own, window = min(own + kBagAhead, n - base);
+    int holder = -1, counted = 0, last = kNoBag;
+    int listed, end;  // bags in the list; lookup behind the last one, from the window's start
+    bool open;        // ... which goes on behind the window
+#pragma unroll 1
+    while (true) {
+      listed = 0;
+      end = -1;
+      const char* const seg0 = segs + ((unsigned)from + wl) * spitch;
+      const char* const id0 = reinterpret_cast<const char*>(T.ids) + (unsigned long long)((unsigned)from + wl) * (p.id_kind == 0 ? 4u : 8u);
+#pragma unroll 1
+      for (int t0 = 0; t0 < window; t0 += 32 * TILES) {
+        unsigned long long seg[TILES], id[TILES];
 #pragma unroll
-          for (int w = 0; w < VPL; ++w) acc[w].scale(inv);
+        for (int k = 0; k < TILES; ++k) seg[k] = id[k] = ~0ull;
+        // Ids and outputs pass through once: they leave L2 to the table rows (evict-first).
+#pragma unroll
+        for (int k = 0; k < TILES; ++k)
+          if (t0 + 32 * k + wl < window)
+            seg[k] = __ldcs(reinterpret_cast<const unsigned long long*>(seg0 + (unsigned)(t0 + 32 * k) * spitch));
+        if (p.id_kind == 0) {
+#pragma unroll
+          for (int k = 0; k < TILES; ++k)
+            if (t0 + 32 * k + wl < window) id[k] = (unsigned long long)(long long)__ldcs(reinterpret_cast<const int*>(id0) + (t0 + 32 * k));
+        } else {
+#pragma unroll
+          for (int k = 0; k < TILES; ++k)
+            if (t0 + 32 * k + wl < window) id[k] = __ldcs(reinterpret_cast<const unsigned long long*>(id0) + (t0 + 32 * k));
         }
-        float* o = outp + (long long)cur * p.out_stride;
+        if (p.id_kind == 2) {
+          if (T.num_buckets < (1ull << 31)) {
 #pragma unroll
-        for (int w = 0; w < VPL; ++w) acc[w].store(o + (w * LANES + lane) * 4);
+            for (int k = 0; k < TILES; ++k) id[k] = fast_mod_u64_small(id[k], (unsigned)T.num_buckets, T.magic);
+          } else {
+#pragma unroll
+            for (int k = 0; k < TILES; ++k) id[k] = fast_mod_u64(id[k], T.num_buckets, T.magic);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < TILES; ++k) {
+          if (t0 + 32 * k >= window) break;
+          const int j = t0 + 32 * k + wl;
+          const bool seg_ok = seg[k] < (unsigned long long)batch, row_ok = id[k] < (unsigned long long)T.rows;
+          const int key = seg_ok ? (int)seg[k] : kNoBag;
+          rows[j] = row_ok ? tab + (unsigned long long)(unsigned)id[k] * pitch : nothing;
+          int pk = __shfl_up_sync(kAll, key, 1);
+          if (wl == 0) pk = before;
+          before = __shfl_sync(kAll, key, 31);
+          const bool in = j < window, starts = in && key != pk;
+          const unsigned all = __ballot_sync(kAll, starts);
+          const int rest = mine - (t0 + 32 * k);  // lookups of the chunk from this tile on
+          const unsigned mask = rest >= 32 ? all : rest <= 0 ? 0u : all & ((1u << rest) - 1u);
+          const bool lists = (mask >> wl) & 1u;
+          if (lists) {
+            BagEntry* e = bags + listed + __popc(mask & ((1u << wl) - 1u));
+            e->bag = key;
+            e->first = (unsigned short)j;
+            e[-1].end = (unsigned short)j;
+          }
+          listed += __popc(mask);
+          if (all != mask && end < 0) end = t0 + 32 * k + __ffs(all ^ mask) - 1;
+          // Rare: ids out of range, and lookups whose segment id is not the previous one or its successor:
+          // unsorted segment ids, or empty bags in between.
+          if (__any_sync(kAll, in && (!seg_ok || !row_ok || (starts && key != pk + 1)))) {
+            if (in && !seg_ok) atomicOr(&hdr->err_bits, kErrSegment);
+            if (in && !row_ok) atomicOr(&hdr->err_bits, kErrRow);
+            const bool odd = lists && key != pk + 1 && key >= 0 && pk >= -1;
+            unsigned gaps = __ballot_sync(kAll, odd);
+            if (__any_sync(kAll, odd && key < pk)) {  // unsorted: its output is cleared and redone anyway
+              if (wl == 0) mark_unsorted(hdr, t);
+              gaps = 0;
+            }
+            while (gaps) {
+              const int src = __ffs(gaps) - 1;
+              gaps &= gaps - 1;
+              zero_fill(__shfl_sync(kAll, pk, src) + 1, __shfl_sync(kAll, key, src));
+            }
+          }
+        }
       }
-    };
+      open = end < 0 && from + window < n;  // the last bag goes on behind the window
+      if (end < 0) end = window;
+      if (holder >= 0) {
+        listed = 1;
+        if (wl == 0) {
+          bags[0].bag = last;
+          bags[0].first = 0;
+        }
+      }
+      if (listed == 0) break;  // the bag that crosses the chunk began before it
+      if (wl == 0) bags[listed - 1].end = (unsigned short)end;
+      if (wl < Q) rows[window + wl] = nothing;  // a round may read past the last lookup
+      __syncwarp();
 
-    const int chunk_end = min(n, (int)(chunk + 1) * sc.chunk);
-    for (int base = (int)chunk * sc.chunk; base < n; base += LANES) {
-      const int i = base + lane;
-      int key = kNoBag, row = -1;
-      if (i < n) {
-        const long long seg = T.seg[(long long)i * p.ncols + p.col];
-        const long long r64 = load_row_id(T.ids, p.id_kind, i, T.num_buckets, T.magic);
-        if (seg < 0 || seg >= batch) atomicOr(&hdr->err_bits, kErrSegment);
-        else key = (int)seg;
-        if (r64 < 0 || r64 >= T.rows) atomicOr(&hdr->err_bits, kErrRow);
-        else row = (int)r64;
+      // b: this group's bag in the list, e; next: the first one nobody has taken; r: where the rows of its
+      // next lookups are, `left` of them
+      int b = holder < 0 ? group : (group == holder ? 0 : 1);
+      int next = holder < 0 ? GROUPS : 1;
+      int left = 0;
+      BagEntry e{kNoBag, 0, 0};
+      const unsigned long long* r = rows;
+      bool holds = false;
+      if (b < listed) {
+        e = bags[b];
+        r = rows + e.first;
+        left = e.end - e.first;
       }
-      int prev_key = __shfl_up_sync(kAll, key, 1);
-      if (lane == 0) {
-        prev_key = -1;  // before the first lookup: bags 0 .. key - 1 are empty
-        if (base > 0) {
-          const long long ps = T.seg[(long long)(base - 1) * p.ncols + p.col];
-          prev_key = (ps < 0 || ps >= batch) ? kNoBag : (int)ps;
+#pragma unroll 1
+      while (__any_sync(kAll, b < listed)) {
+        Vec v[Q][VPL];
+        unsigned long long row[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) row[q] = r[q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          if (q >= left) row[q] = nothing;
+#pragma unroll
+          for (int w = 0; w < VPL; ++w) v[q][w].load(reinterpret_cast<const char*>(row[q]) + col[w]);
         }
-      }
-      const bool starts = i < n && key != prev_key;
-      if (starts && key >= 0 && prev_key >= 0 && key < prev_key) mark_unsorted(hdr, t);
-      const unsigned smask = __ballot_sync(kAll, starts);
-      const int tile_n = min(LANES, n - base);
-      int from = 0, to = tile_n;
-      const bool inside = base < chunk_end;
-      if (!open) {
-        if (!inside) break;
-        if (smask == 0) continue;
-        from = __ffs(smask) - 1;
-      } else if (!inside && smask != 0) {
-        to = __ffs(smask) - 1;
-      }
-      for (int j0 = from; j0 < to; j0 += INFLIGHT) {
-        Vec v[INFLIGHT][VPL];
-        bool has[INFLIGHT];
 #pragma unroll
-        for (int k = 0; k < INFLIGHT; ++k) {
-          const int j = j0 + k;
-          has[k] = false;
-          if (j < to) {
-            const int rw = __shfl_sync(kAll, row, j);
-            has[k] = rw >= 0;
-            if (has[k]) {
-              const float* src = tab + (long long)rw * DIM + lane * 4;
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
-              for (int w = 0; w < VPL; ++w) v[k][w].load(src + w * LANES * 4);
+          for (int w = 0; w < VPL; ++w) acc[w].add(v[q][w]);
+        left -= Q;
+        r += left > 0 ? Q : 0;
+        const bool done = left <= 0 && b < listed;
+        const unsigned mask = __ballot_sync(kAll, done);
+        if (done) {
+          holds = open && b == listed - 1;  // its bag stays in the accumulator
+          if (!holds) {
+            if (e.bag >= 0) {
+              char* o = outp + (unsigned)e.bag * opitch;
+              const bool mean = p.combiner == 1;
+              const float inv = mean ? __fdiv_rn(1.0f, (float)(counted + (int)e.end - (int)e.first)) : 1.0f;
+#pragma unroll
+              for (int w = 0; w < VPL; ++w) store(o, acc[w], w, mean, inv);
             }
+#pragma unroll
+            for (int w = 0; w < VPL; ++w) acc[w].zero();
+          }
+          b = next + __popc(mask & ((1u << (group * LANES)) - 1u)) / LANES;
+          if (b < listed) {
+            e = bags[b];
+            r = rows + e.first;
+            left = e.end - e.first;
           }
         }
-#pragma unroll
-        for (int k = 0; k < INFLIGHT; ++k) {
-          const int j = j0 + k;
-          if (j < to) {
-            if ((smask >> j) & 1u) {
-              flush();
-#pragma unroll
-              for (int w = 0; w < VPL; ++w) acc[w].zero();
-              cur = __shfl_sync(kAll, key, j);
-              const int before = __shfl_sync(kAll, prev_key, j);
-              // empty bags between the previous lookup's bag and this one (sorted input only)
-              if (cur >= 0 && before >= -1 && before < cur - 1) zero_fill(before + 1, cur);
-              count = 0;
-              open = true;
-            }
-            ++count;
-            if (has[k]) {
-#pragma unroll
-              for (int w = 0; w < VPL; ++w) acc[w].add(v[k][w]);
-            }
-          }
-        }
+        next += __popc(mask) / LANES;
       }
-      if (!inside && to < tile_n) break;
-      // the table's last lookup: bags after its bag are empty
-      if (base + tile_n >= n && to == tile_n && open && cur >= 0) zero_fill(cur + 1, batch);
+      last = bags[listed - 1].bag;
+      if (!open) break;
+      counted += end - (int)bags[listed - 1].first;
+      holder = (__ffs(__ballot_sync(kAll, holds)) - 1) / LANES;
+      before = last;
+      from += window;
+      window = min(32 * TILES, n - from);
+      mine = 0;
+      __syncwarp();
     }
-    flush();
+    // the table's last lookup: bags after its bag are empty
+    if (listed > 0 && last >= 0 && from + end == n) zero_fill(last + 1, batch);
+    __syncwarp();
+    gc_next = __shfl_sync(kAll, gc_next, 0);
   }
+  pdl_trigger();
 }
 
 // The kernels for tables marked unsorted.  They follow every call, sorted or not (the host does

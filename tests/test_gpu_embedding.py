@@ -434,6 +434,39 @@ def test_bag_plan_marks_unsorted_and_out_of_range(dim, combiner):
         assert plan.error_bits() == bit
 
 
+@pytest.mark.parametrize("dim", [4, 8, 40, 64, 72, 256, 512])
+@pytest.mark.parametrize("shift", [0, 4])
+@pytest.mark.parametrize("combiner", [0, 1])
+def test_bags_around_the_decoded_window(dim, shift, combiner):
+    """Bags that end at, just before and just behind the lookups a warp decodes at a time (chunk, look-ahead
+    and several windows), tables 32-byte aligned and not, rows out of range among them: the sums in lookup
+    order, bit for bit."""
+    rng = np.random.default_rng(dim + shift)
+    rows, lens = 300, []
+    for n in (1, 223, 1, 31, 32, 33, 224, 225, 255, 256, 257, 700, 127, 128, 129, 0, 0, 3, 1500, 1):
+        lens += [n] + list(rng.integers(0, 4, 5))
+    lens = np.array(lens * 12)
+    batch, n = len(lens), int(lens.sum())
+    seg = np.repeat(np.arange(batch), lens)
+    idx = rng.integers(0, rows, n)
+    idx[rng.integers(0, n, 5)] = rows + 3
+    base = torch.zeros(rows * dim + 4, device="cuda")
+    data = rng.standard_normal((rows, dim)).astype(np.float32)
+    table = base[shift:shift + rows * dim].view(rows, dim)
+    table.copy_(_dev(data))
+    out = torch.empty((batch, 1, dim), device="cuda")
+    plan = BagPlan([table], [_dev(idx)], [_dev(np.stack([seg, seg], 1).astype(np.int64))], out, 0, batch, id_kind=1,
+                   combiner=combiner)
+    plan.run()
+    want = np.zeros((batch, dim), np.float32)
+    ok = idx < rows
+    np.add.at(want, seg[ok], data[idx[ok]])  # in order, in fp32
+    if combiner:
+        want *= (np.float32(1) / np.maximum(lens, 1).astype(np.float32))[:, None]
+    assert plan.error_bits() == 1
+    np.testing.assert_array_equal(out.cpu().numpy()[:, 0], want)
+
+
 @pytest.mark.parametrize("dim", [16, 32, 64, 100, 128])
 def test_bag_share_fits_beside_the_pooling_kernel(dim):
     """A share of n blocks per SM leaves room for 5 - n blocks of the pooling kernel of the row exchange
