@@ -174,6 +174,8 @@ bool bounce_ready() {
 
 // Pinned destination of small device reads, one per thread (null when it cannot be had).
 constexpr size_t kMailboxBytes = 256;
+constexpr size_t kPostBytes = 64;  // behind it: the words kernels post results to (PostBox)
+thread_local unsigned long long g_post_ticket = 0;
 struct Mailbox {
   void* p = nullptr;
   bool tried = false;
@@ -190,7 +192,7 @@ void* mailbox() {
   if (!m.tried) {
     m.tried = true;
     OutsideCaptures relaxed;
-    if (cudaHostAlloc(&m.p, kMailboxBytes, cudaHostAllocPortable) != cudaSuccess) {
+    if (cudaHostAlloc(&m.p, kMailboxBytes + kPostBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
       m.p = nullptr;
     }
@@ -618,6 +620,32 @@ int Call::read_host(const void* p, size_t bytes, void* dst) {
   else if (via) memcpy(dst, via, bytes);
   synced_ = true;
   return status_;
+}
+
+PostBox Call::post_box() {
+  PostBox b;
+  if (void* m = mailbox()) {
+    b.words = reinterpret_cast<unsigned long long*>(static_cast<char*>(m) + kMailboxBytes);
+    b.ticket = ++g_post_ticket;
+  }
+  return b;
+}
+
+int Call::wait_posted(const PostBox& box, int* flags, long long* value) {
+  if (status_ != ANNC_OK) return status_;
+  const volatile unsigned long long* w = box.words;
+  auto posted = [&] { return w[0] >> 8 == box.ticket; };
+  for (unsigned spin = 1; !posted(); ++spin) {
+    if (spin % 4096 != 0) continue;
+    const cudaError_t e = cudaStreamQuery(stream_);  // ends with the kernels at the latest
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return status_ = cuda_fail(e, "wait_posted");
+    if (!posted()) return status_ = fail(ANNC_ERR_INTERNAL, "a kernel ended without posting its result");
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  *flags = (int)(w[0] & 0xff);
+  *value = (long long)w[1];
+  return ANNC_OK;
 }
 
 int Call::wait() {

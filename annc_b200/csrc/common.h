@@ -57,6 +57,20 @@ inline int64_t numel(const annc_tensor& t) {
 }
 size_t dtype_size(int32_t dtype);
 
+// Two words of pinned memory: {ticket << 8 | flags, value}, the first written last.
+struct PostBox {
+  unsigned long long* words = nullptr;
+  unsigned long long ticket = 0;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void post_result(const PostBox& box, int flags, long long value) {
+  volatile unsigned long long* w = box.words;
+  w[1] = (unsigned long long)value;
+  __threadfence_system();
+  w[0] = box.ticket << 8 | (unsigned)flags;
+}
+#endif
+
 // One entry-point invocation.  in()/out() turn caller pointers (host or device) into device
 // pointers.  A host operand is given a device mirror keyed by (pointer, bytes, device) that
 // persists between calls; an upload is skipped when a sampled fingerprint of the host contents
@@ -106,6 +120,12 @@ class Call {
                 const std::function<void(void*)>& fill);
   // Small host read of possibly-device memory (synchronous).
   int read_host(const void* p, size_t bytes, void* dst);
+  // For a small result that the host needs while the call's later kernels already run: a kernel posts it
+  // (post_result) into pinned memory of the thread and wait_posted() polls for it, where a copy and a
+  // synchronize would wait for everything queued so far and leave the device idle meanwhile.  `words` is
+  // null without pinned memory.  Every box handed to a launched kernel has to be waited for in the same call.
+  PostBox post_box();
+  int wait_posted(const PostBox& box, int* flags, long long* value);
   // Waits for the call's stream (an operator whose outputs are complete when it returns).
   int wait();
   // True when p is device (or managed) memory.

@@ -331,20 +331,23 @@ static int unique_first_appearance(Call& call, const int64_t* src, long long n, 
   auto* first = static_cast<int*>(call.scratch((cap + 1) * sizeof(int)));
   auto* slot_of = static_cast<int*>(call.scratch(n * sizeof(int)));
   auto* tiles = static_cast<int*>(call.scratch(scan_scratch_ints(n) * sizeof(int)));
-  auto* total_err = static_cast<int*>(call.scratch(3 * sizeof(int)));  // count, error bits, (scan total)
+  auto* total_err = static_cast<int*>(call.scratch(4 * sizeof(int)));  // count, error bits, blocks done, (scan total)
   if (call.status() != ANNC_OK) return call.status();
   unique_init_kernel<<<grid_for(cap + 1, 256), 256, 0, s>>>(keys, first, cap, total_err);
   const int g = grid_for(n, 256);
   unique_insert_kernel<<<g, 256, 0, s>>>(src, n, ncols, col, keys, first, cap, slot_of, rows, total_err + 1);
   const long long ntiles = (n + kScanTile - 1) / kScanTile;
-  unique_count_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(slot_of, first, n, tiles);
+  const PostBox box = call.post_box();
+  unique_count_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(slot_of, first, n, tiles, total_err, box);
   // every block adds up the tiles before it: up to 2048 tiles (4 M keys) that is at most four loads
   // a thread, cheaper than a pass of its own
   const int scanned = ntiles > 2048;
-  if (scanned) scan_tile_offsets_kernel<<<1, kScanThreads, 0, s>>>(tiles, ntiles, total_err + 2);
+  if (scanned) scan_tile_offsets_kernel<<<1, kScanThreads, 0, s>>>(tiles, ntiles, total_err + 3);
   unique_emit_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(src, n, ncols, col, slot_of, first, tiles, scanned,
-                                                               out_unique, total_err);
+                                                               out_unique);
   unique_inverse_kernel<<<g, 256, 0, s>>>(slot_of, first, n, inverse32, inverse64);
+  ANNC_CUDA(cudaGetLastError());
+  if (box.words) return call.wait_posted(box, &res->err_bits, &res->count);
   int h[2] = {0, 0};
   ANNC_TRY(call.read_host(total_err, sizeof(h), h));
   res->count = h[0];
@@ -633,7 +636,7 @@ int annc_KPFusedSparseSegmentReduce(const annc_tensor* data, const annc_tensor* 
   const float* d_data = call.in_constant((const float*)data->data, (size_t)numel(*data));
   const void* d_idx = call.in(indices->data, (size_t)nnz * dtype_size(indices->dtype));
   const int64_t* d_seg = call.in((const int64_t*)slice_input->data, (size_t)(nnz * ncols));
-  // the scan's result and the bag header side by side: one memset starts both
+  // the scan's result and the bag header side by side: one memset (or one block) starts both
   char* ctrl = static_cast<char*>(call.scratch(kHeaderBytes + sizeof(SegScan)));
   if (call.status() != ANNC_OK) return call.status();
   auto* hdr = reinterpret_cast<BagHeader*>(ctrl);
@@ -641,13 +644,23 @@ int annc_KPFusedSparseSegmentReduce(const annc_tensor* data, const annc_tensor* 
 
   // batch = max segment id + 1 (max starts at 0), needed on the host to size output 0.
   const int id_kind = indices->dtype == ANNC_I64 ? 1 : 0;
-  ANNC_CUDA(cudaMemsetAsync(ctrl, 0, kHeaderBytes + sizeof(SegScan), s));
-  if (nnz > 0)
-    seg_scan_kernel<<<grid_for(nnz, 256, 148 * 4), 256, 0, s>>>(d_seg, d_idx, id_kind, nnz, ncols, col, data->dims[0],
-                                                                d_scan);
-  SegScan scan;
-  ANNC_TRY(call.read_host(d_scan, sizeof(scan), &scan));
-  const int64_t batch = scan.max_seg + 1;
+  const bool one_block = nnz <= kSegScanOne;
+  if (!one_block) ANNC_CUDA(cudaMemsetAsync(ctrl, 0, kHeaderBytes + sizeof(SegScan), s));
+  const PostBox box = call.post_box();
+  seg_scan_kernel<<<one_block ? 1 : grid_for(nnz, kSegScanThreads, 148 * 2), kSegScanThreads, 0, s>>>(
+      d_seg, d_idx, id_kind, nnz, ncols, col, data->dims[0], hdr, d_scan, box);
+  ANNC_CUDA(cudaGetLastError());
+  long long max_seg = 0;
+  int flags = 0;
+  if (box.words) {
+    ANNC_TRY(call.wait_posted(box, &flags, &max_seg));
+  } else {
+    SegScan scan;
+    ANNC_TRY(call.read_host(d_scan, sizeof(scan), &scan));
+    max_seg = scan.max_seg;
+    flags = scan.flags;
+  }
+  const int64_t batch = max_seg + 1;
 
   const int64_t dims0[2] = {batch, dim};
   float* out0 = static_cast<float*>(alloc(ctx, 0, ANNC_F32, 2, dims0));
@@ -667,7 +680,7 @@ int annc_KPFusedSparseSegmentReduce(const annc_tensor* data, const annc_tensor* 
   tb.out = d_out;
   tb.offsets = nullptr;
   ANNC_TRY(run_bags(&tb, 1, dim, id_kind, ncols, col, combiner, batch, dim, hdr,
-                    reinterpret_cast<int*>(static_cast<char*>(ws) + kHeaderBytes), s, 1, 0, 0, !scan.unsorted));
+                    reinterpret_cast<int*>(static_cast<char*>(ws) + kHeaderBytes), s, 1, 0, 0, !(flags & kScanUnsorted)));
   // Second output: begin_1[0] == 0 ? batch : embedding size (reference :81-83).
   const int32_t slice_out = (b1 == 0) ? (int32_t)batch : (int32_t)dim;
   if (call.is_device(out1)) {
@@ -678,8 +691,8 @@ int annc_KPFusedSparseSegmentReduce(const annc_tensor* data, const annc_tensor* 
   }
   ANNC_TRY(call.wait());
   ANNC_TRY(call.finish());
-  if (scan.err_bits & kErrRow) return fail(ANNC_ERR_INVALID_ARGUMENT, "indices out of range of input rows");
-  if (scan.err_bits & kErrSegment) return fail(ANNC_ERR_INVALID_ARGUMENT, "segment ids must be >= 0");
+  if (flags & kErrRow) return fail(ANNC_ERR_INVALID_ARGUMENT, "indices out of range of input rows");
+  if (flags & kErrSegment) return fail(ANNC_ERR_INVALID_ARGUMENT, "segment ids must be >= 0");
   return ANNC_OK;
 }
 

@@ -529,3 +529,32 @@ def test_gather_and_reduce_report_rows_outside_the_table(bad):
         ops.kp_fused_sparse_segment_reduce(data, _dev(keys[:, 1].copy()), _dev(np.sort(keys.clip(0), axis=0)),
                                            np.zeros(2, np.int32), np.zeros(1, np.int32), 0)
     assert "indices out of range" in e.value.message
+
+
+@pytest.mark.parametrize("nnz", [0, 1, 511, 512, 4095, 4096, 4097, 9000])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_segment_reduce_at_the_edges_of_the_scan(nnz, shuffled):
+    """The scan for the output's size by one block and by several; its flags reach the host (unsorted ids,
+    rows out of range), call after call from the same thread."""
+    rng = np.random.default_rng(nnz)
+    data = rng.standard_normal((70, 8)).astype(np.float32)
+    seg = np.sort(rng.integers(0, nnz // 3 + 1, nnz))
+    if shuffled:
+        seg = rng.permutation(seg)
+    idx = rng.integers(0, 70, nnz)
+    pairs = np.stack([seg, seg], 1).astype(np.int64).reshape(nnz, 2)
+    b2, b1 = np.zeros(2, np.int32), np.zeros(1, np.int32)
+    for _ in range(3):
+        out, so = ops.kp_fused_sparse_segment_reduce(_dev(data), _dev(idx), _dev(pairs), b2, b1, 0)
+    batch = int(seg.max()) + 1 if nnz else 1
+    want = np.zeros((batch, 8), np.float32)
+    np.add.at(want, seg, data[idx])
+    assert int(so) == batch and tuple(out.shape) == (batch, 8)
+    if shuffled:  # sums of up to a few dozen rows in any order
+        np.testing.assert_allclose(out.cpu().numpy(), want, rtol=0, atol=1e-5)
+    else:
+        np.testing.assert_array_equal(out.cpu().numpy(), want)
+    if nnz:
+        idx[nnz - 1] = 70
+        with pytest.raises(AnncError):
+            ops.kp_fused_sparse_segment_reduce(_dev(data), _dev(idx), _dev(pairs), b2, b1, 0)
