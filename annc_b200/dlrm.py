@@ -37,6 +37,10 @@ from .synth import DlrmModel
 
 class DlrmPipeline:
     embed_first = True  # forward() queues the pooling kernel before the bottom MLP
+    # Up to this batch a step on one GPU stays on one stream.  The second one costs five event calls; what runs
+    # beside the pooling kernel there is worth less.  us a step, two streams / one (a step waited for):
+    # batch 64 79 / 66 (93 / 80), 200 80 / 71 (98 / 86), 512 79 / 77 (98 / 88), 1024 77 / 84 (102 / 96), 4096 123 / 137.
+    ONE_STREAM_BATCH = 512
     gemm_flags = 0
 
     def __init__(self, model: DlrmModel, device: torch.device, math: int = MATH_AUTO,
@@ -185,8 +189,17 @@ class DlrmPipeline:
                                   math=self.math, stream=stream, io_flags=self.gemm_flags))
             x = y
 
+    def _one_stream(self) -> bool:
+        return self.embed_first and self.batch <= self.ONE_STREAM_BATCH
+
     def _sparse_part(self, names, lookahead: bool = False) -> None:
-        """Bottom MLP (second stream) beside the embedding pooling; z is complete afterwards."""
+        """Bottom MLP (second stream, for larger batches) beside the embedding pooling; z is complete
+        afterwards."""
+        if self._one_stream():
+            self.embed_prefetch()
+            self.embed()
+            self._bottom_mlp(names, dev.raw_stream())
+            return
         main = torch.cuda.current_stream()
         self.embed_prefetch()
         self._forked.record(main)
@@ -227,7 +240,7 @@ class DlrmPipeline:
     def forward(self) -> torch.Tensor:
         if self._pstep:
             self.sync_pipeline()
-        else:  # nothing was ever queued on the dense stream
+        elif not self._one_stream():  # nothing was ever queued on the dense stream
             torch.cuda.current_stream().wait_event(self._side_done)
         self._select(0)
         names = []
