@@ -17,6 +17,10 @@ struct BiasBroadcast {
 // CUDA-core fp32 route; takes every shape, both transposes and the kn4 B format.
 int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb = nullptr);
 
+// Whether a product's blocks may take their places while the kernel before it on the stream drains (pdl.cuh).
+// Not beside another stream's kernel that needs the room, which is what ANNC_IO_SINGLE is for.
+inline bool early_launch(const annc_gemm_desc& d) { return !(d.io_flags & ANNC_IO_SINGLE); }
+
 // tcgen05 route: whether the descriptor fits, and the launch.
 bool tc_supported(const annc_gemm_desc& d, int math);
 int run_tc(const annc_gemm_desc& d, int math, cudaStream_t s);

@@ -5,6 +5,7 @@
 #include "common.h"
 #include "gemm.h"
 #include "kn4.h"
+#include "pdl.cuh"
 #include "tc_ptx.cuh"
 
 namespace annc {
@@ -252,6 +253,8 @@ __global__ void __launch_bounds__(BM * BN / (TM * TN), BM == 64 ? 4 : 8) sgemm_s
 
 // n == 1 with row-major A: one warp per output row (a GEMV with the GEMM epilogue).
 __global__ void __launch_bounds__(256) sgemm_n1_kernel(annc_gemm_desc d) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long i = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= d.m) return;
@@ -430,7 +433,9 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb) {
   if (d.m <= 0 || d.n <= 0 || d.batch <= 0) return ANNC_OK;
   if (d.n == 1 && d.batch == 1 && !d.trans_a && !bb && d.b_format == ANNC_B_PLAIN &&
       (d.trans_b || d.ldb == 1)) {
-    sgemm_n1_kernel<<<(unsigned)((d.m + 7) / 8), 256, 0, s>>>(d);
+    const dim3 grid((unsigned)((d.m + 7) / 8));
+    if (early_launch(d)) return launch_pdl(sgemm_n1_kernel, grid, dim3(256), 0, s, d) == cudaSuccess ? ANNC_OK : cuda_fail(cudaGetLastError(), "sgemm_n1_kernel");
+    sgemm_n1_kernel<<<grid, 256, 0, s>>>(d);
     ANNC_CUDA(cudaGetLastError());
     return ANNC_OK;
   }

@@ -32,6 +32,7 @@
 #include "common.h"
 #include "gemm.h"
 #include "kn4.h"
+#include "pdl.cuh"
 #include "tc_host.h"
 #include "tc_ptx.cuh"
 
@@ -101,10 +102,6 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + STAGES * STAGE_BYTES + 16 * STAGES + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  // A CTA of an earlier wave (or launch) gave up on a wait: do not start, fail fast.  (The
-  // CTAs of a split-K cluster always run to their cluster barriers.)
-  if (p.split <= 1 && *reinterpret_cast<volatile int*>(&g_gemm_error) != 0) return;
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   // Split K: cluster rank c of `split` takes the k-steps [it0, it0 + KT); every CTA keeps its
@@ -141,10 +138,18 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Launched while the kernel before it drains: what is above needs nothing of that kernel, what follows
+  // waits for its end.
+  pdl_trigger();
+  pdl_wait();
+  // A CTA of an earlier wave (or launch) gave up on a wait: do not start, fail fast.  (The
+  // CTAs of a split-K cluster always run to their cluster barriers.)
+  const bool poisoned = p.split <= 1 && *reinterpret_cast<volatile int*>(&g_gemm_error) != 0;
 
   bool done = false;  // warps 2..5: the accumulator is complete and sits in shared memory
   constexpr int LD = BN + 4;
-  if (warp == 0) {
+  if (poisoned) {
+  } else if (warp == 0) {
     // ---------------- TMA producer
     if (lane == 0) {
       for (int li = 0; li < KT; ++li) {
@@ -560,27 +565,26 @@ int run_tc(const annc_gemm_desc& d, int math, cudaStream_t s) {
     while (split < 8 && ctas <= max_clusters(split * 2) && kt_all / (split * 2) >= 2) split *= 2;
   }
   p.split = split;
+  if (split > 1) grid.z = (unsigned)split;
+  const bool deep = split > 1 || ctas <= 148 * 3 / 2;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = smem_bytes(deep ? 6 : 3);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
   if (split > 1) {
-    grid.z = (unsigned)split;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = smem_bytes(6);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = (unsigned)split;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    ANNC_CUDA(cudaLaunchKernelEx(&cfg, gemm_tf32_tcgen05_kernel<6>, ta, tb, p));
-  } else if (ctas <= 148 * 3 / 2) {
-    gemm_tf32_tcgen05_kernel<6><<<grid, NUM_THREADS, smem_bytes(6), s>>>(ta, tb, p);
-  } else {
-    gemm_tf32_tcgen05_kernel<3><<<grid, NUM_THREADS, smem_bytes(3), s>>>(ta, tb, p);
+    cudaLaunchAttribute& a = attr[cfg.numAttrs++];
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = 1;
+    a.val.clusterDim.y = 1;
+    a.val.clusterDim.z = (unsigned)split;
   }
+  if (early_launch(d)) attr[cfg.numAttrs++] = pdl_attribute();
+  ANNC_CUDA(deep ? cudaLaunchKernelEx(&cfg, gemm_tf32_tcgen05_kernel<6>, ta, tb, p)
+                 : cudaLaunchKernelEx(&cfg, gemm_tf32_tcgen05_kernel<3>, ta, tb, p));
   ANNC_CUDA(cudaGetLastError());
   return ANNC_OK;
 }

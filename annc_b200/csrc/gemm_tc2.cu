@@ -34,6 +34,7 @@
 
 #include "common.h"
 #include "gemm.h"
+#include "pdl.cuh"
 #include "tc_host.h"
 #include "tc_ptx.cuh"
 
@@ -127,8 +128,8 @@ __device__ __noinline__ float4 add_terms(float4 v, const void* c, int c_bf16, fl
   for (int e = 0; e < 4; ++e) {
     if (e >= cols) break;
     if (c) t[e] += beta * (c_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(c)[e]) : static_cast<const float*>(c)[e]);
-    if (addend) t[e] += __ldg(addend + e);
-    if (bias) t[e] += __ldg(bias + e);
+    if (addend) t[e] += *(addend + e);
+    if (bias) t[e] += *(bias + e);
   }
   return make_float4(t[0], t[1], t[2], t[3]);
 }
@@ -226,12 +227,12 @@ __device__ __forceinline__ void chunk_store_staged(const PairParams& p, float* s
       if (use_add) {
         const float* ap = p.addend + bz * p.stride_addend + grow * p.ld_addend + c;
         if (a_vec) {
-          ld_a[i] = __ldg(reinterpret_cast<const float4*>(ap));
+          ld_a[i] = *reinterpret_cast<const float4*>(ap);
         } else {
           float t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            if (c + e < p.N) t[e] = __ldg(ap + e);
+            if (c + e < p.N) t[e] = *(ap + e);
           ld_a[i] = make_float4(t[0], t[1], t[2], t[3]);
         }
       }
@@ -334,6 +335,10 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   cluster_sync_all();  // both CTAs' barriers exist before anything signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // As in the single-CTA kernel.  (What the kernel before may have written is read by plain loads: read-only
+  // ones need not stay behind the wait.)
+  pdl_trigger();
+  pdl_wait();
   const bool poisoned = *reinterpret_cast<volatile int*>(p.error_word) != 0;  // an earlier launch gave up
 
   if (!poisoned) {
@@ -441,12 +446,12 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (!SOFTMAX && p.bias) {
           const int c = nb + lane * 4;
           if (c + 3 < p.N && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
-            bias_w = __ldg(reinterpret_cast<const float4*>(p.bias + c));
+            bias_w = *reinterpret_cast<const float4*>(p.bias + c);
           } else {
-            if (c < p.N) bias_w.x = __ldg(p.bias + c);
-            if (c + 1 < p.N) bias_w.y = __ldg(p.bias + c + 1);
-            if (c + 2 < p.N) bias_w.z = __ldg(p.bias + c + 2);
-            if (c + 3 < p.N) bias_w.w = __ldg(p.bias + c + 3);
+            if (c < p.N) bias_w.x = *(p.bias + c);
+            if (c + 1 < p.N) bias_w.y = *(p.bias + c + 1);
+            if (c + 2 < p.N) bias_w.z = *(p.bias + c + 2);
+            if (c + 3 < p.N) bias_w.w = *(p.bias + c + 3);
           }
         }
         ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * acc, aph, abort_flag, p.error_word)) != 0;
@@ -472,7 +477,7 @@ gemm_pair_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const float* a = p.addend + bz * p.stride_addend + grow * p.ld_addend + c0;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              add[j] = row_ok && c0 + 4 * j < p.N ? __ldg(reinterpret_cast<const float4*>(a + 4 * j))
+              add[j] = row_ok && c0 + 4 * j < p.N ? *reinterpret_cast<const float4*>(a + 4 * j)
                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
           };
           auto finish = [&](const uint32_t (&r)[32], float (&v)[32], int first_lane) {
@@ -796,17 +801,18 @@ int run_pair(const annc_gemm_desc& d, int math, cudaStream_t s) {
   const long long pairs = p.items < max_pairs[bf16] ? p.items : max_pairs[bf16];
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1] = pdl_attribute();
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
   cfg.blockDim = dim3(P_THREADS, 1, 1);
   cfg.dynamicSmemBytes = P_SMEM;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early_launch(d) ? 2 : 1;
   ANNC_CUDA(cudaLaunchKernelEx(&cfg, kernels[bf16][cut][epi], ta, tb, tbh, tc, p));
   return ANNC_OK;
 }

@@ -24,6 +24,7 @@
 #include <cstring>
 
 #include "common.h"
+#include "pdl.cuh"
 #include "tc_host.h"
 #include "tc_ptx.cuh"
 
@@ -78,7 +79,6 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* epi_fail_all = reinterpret_cast<volatile int*>(tmem_slot + 2);  // one word per group
 
-  if (*reinterpret_cast<volatile int*>(&g_inter_error) != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -112,8 +112,12 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t box_bytes = (uint32_t)p.rows * 128u;
+  // Launched while the kernel before it drains: nothing above touches what that one reads or writes.
+  pdl_trigger();
+  pdl_wait();
 
-  if (warp == 0) {
+  if (*reinterpret_cast<volatile int*>(&g_inter_error) != 0) {  // an earlier launch gave up
+  } else if (warp == 0) {
     if (lane == 0) {
       long long li = 0;
       for (long long t = blockIdx.x; t < p.tiles; t += gridDim.x, ++li) {
@@ -176,7 +180,7 @@ dot_interaction_tc_kernel(const __grid_constant__ CUtensorMap tmap, InterParams 
       for (int r = 0; r < ROW0_PER_THREAD; ++r) {  // unrounded copy of Z[b, 0, :]
         const int idx = te + 128 * r;
         const int s = idx / ID, col = idx - s * ID;
-        row0[r] = s < samples ? __ldg(p.z + (b0 + s) * p.F * ID + col) : 0.f;
+        row0[r] = s < samples ? p.z[(b0 + s) * p.F * ID + col] : 0.f;
       }
       // All four warps leave together: a warp that gave up still joins the barrier.
       const bool ok = __all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * buf, tph, abort_flag,
@@ -285,9 +289,9 @@ int dot_interaction_tc(const float* z, int64_t batch, int F, int dim, int64_t z_
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const unsigned grid = (unsigned)(p.tiles < sms ? p.tiles : sms);
   const int need = (p.spt * ID + 127) / 128;
-  if (need <= 2) dot_interaction_tc_kernel<2><<<grid, I_THREADS, I_SMEM, s>>>(tm, p);
-  else if (need <= 8) dot_interaction_tc_kernel<8><<<grid, I_THREADS, I_SMEM, s>>>(tm, p);
-  else dot_interaction_tc_kernel<32><<<grid, I_THREADS, I_SMEM, s>>>(tm, p);
+  if (need <= 2) ANNC_CUDA(launch_pdl(dot_interaction_tc_kernel<2>, dim3(grid), dim3(I_THREADS), I_SMEM, s, tm, p));
+  else if (need <= 8) ANNC_CUDA(launch_pdl(dot_interaction_tc_kernel<8>, dim3(grid), dim3(I_THREADS), I_SMEM, s, tm, p));
+  else ANNC_CUDA(launch_pdl(dot_interaction_tc_kernel<32>, dim3(grid), dim3(I_THREADS), I_SMEM, s, tm, p));
   ANNC_CUDA(cudaGetLastError());
   return ANNC_OK;
 }
