@@ -13,6 +13,8 @@ shape-info vector [dims..., minor_to_major...] per operand
 from __future__ import annotations
 
 import ctypes as C
+import threading
+import weakref
 from functools import lru_cache
 from typing import List, Optional, Sequence
 
@@ -86,14 +88,25 @@ def as_tensor(x, dtype_code: Optional[int] = None) -> Tensor:
     return Tensor(_ptr(x), _code(x) if dtype_code is None else dtype_code, len(shape), shape)
 
 
+_calling = threading.local()  # .outputs: weak reference to the outputs of the call under way
+
+
+@ALLOC_FN
+def _allocate(ctx, index, dtype, rank, dims):
+    return _calling.outputs()._alloc(ctx, index, dtype, rank, dims)
+
+
 class _Outputs:
-    """allocate_output stand-in: numpy on the host, torch on the device."""
+    """allocate_output stand-in: numpy on the host, torch on the device.  One callback serves every call: one
+    per object would tie the object into a cycle with itself, and its arrays would stay allocated until
+    Python looks for cycles (outputs of 13 MB a call: device allocations of milliseconds now and then)."""
+    fn = _allocate
 
     def __init__(self, on_device: bool, device=None):
         self.on_device = on_device
         self.device = device
         self.arrays = {}
-        self.fn = ALLOC_FN(self._alloc)
+        _calling.outputs = weakref.ref(self)
 
     def _alloc(self, _ctx, index, dtype, rank, dims):
         shape = dims[:rank] if rank else ()
