@@ -434,7 +434,7 @@ def run_gpu(args):
                                  input_seed=(1000 + rank) if world > 1 else None)
         emb_bytes = model.emb.algorithmic_bytes()
         nnz = model.emb.nnz
-        bag_kernel = "bag_stream_kernel<8,2,2,true,4> (hash-bucket + gather + segment sum, 26 tables in one launch)"
+        bag_kernel = "bag_list_kernel<8,8,1,4,4> (hash-bucket + gather + segment sum, 26 tables in one launch)"
 
         def build(mode):
             if world == 1:
