@@ -354,3 +354,30 @@ def test_layout_matmul_beside_a_capture_of_another_thread():
     torch.cuda.synchronize()
     assert nerr(y, (x.double() @ x.double()).cpu().numpy()) <= 2e-3
     assert nerr(out, (a.double() @ w.double()).cpu().numpy()) <= 2e-3
+
+
+@pytest.mark.parametrize("m,n", [(64, 128), (200, 512), (2048, 512), (20000, 256), (4096, 1)])
+def test_back_to_back_products_wait_for_each_other(m, n):
+    """Kernels that are launched while the one before them drains read what that one wrote and overwrite what it
+    read: a chain of products over two buffers is the same, bit for bit, with the device idle between them."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w = torch.randn((512, 512), device="cuda", generator=g) * 512 ** -0.5
+    last = torch.randn((512, n), device="cuda", generator=g) * 512 ** -0.5
+    bias, tail = torch.randn(512, device="cuda", generator=g), torch.randn(n, device="cuda", generator=g)
+    x0 = torch.randn((m, 512), device="cuda", generator=g)
+
+    def chain(wait):
+        x, y, out = x0.clone(), torch.empty_like(x0), []
+        for _ in range(12):
+            for a, b in ((x, y), (y, x)):
+                device.gemm(a, w, b, m=m, n=512, k=512, bias=bias, activation=1)
+                if wait:
+                    torch.cuda.synchronize()
+            out.append(torch.empty((m, n), device="cuda"))
+            device.gemm(x, last, out[-1], m=m, n=n, k=512, bias=tail)
+            if wait:
+                torch.cuda.synchronize()
+        return out + [x]
+
+    for a, b in zip(chain(False), chain(True)):
+        assert torch.equal(a, b)
