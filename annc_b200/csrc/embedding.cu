@@ -334,18 +334,20 @@ static int unique_first_appearance(Call& call, const int64_t* src, long long n, 
   auto* total_err = static_cast<int*>(call.scratch(4 * sizeof(int)));  // count, error bits, blocks done, (scan total)
   if (call.status() != ANNC_OK) return call.status();
   unique_init_kernel<<<grid_for(cap + 1, 256), 256, 0, s>>>(keys, first, cap, total_err);
-  const int g = grid_for(n, 256);
-  unique_insert_kernel<<<g, 256, 0, s>>>(src, n, ncols, col, keys, first, cap, slot_of, rows, total_err + 1);
+  const dim3 g(grid_for(n, 256)), block(256), scan_block(kScanThreads);
+  ANNC_CUDA(launch_pdl(unique_insert_kernel, g, block, 0, s, src, n, ncols, col, keys, first, cap, slot_of, rows,
+                       total_err + 1));
   const long long ntiles = (n + kScanTile - 1) / kScanTile;
+  const dim3 tile_grid((unsigned)ntiles);
   const PostBox box = call.post_box();
-  unique_count_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(slot_of, first, n, tiles, total_err, box);
+  ANNC_CUDA(launch_pdl(unique_count_kernel, tile_grid, scan_block, 0, s, slot_of, first, n, tiles, total_err, box));
   // every block adds up the tiles before it: up to 2048 tiles (4 M keys) that is at most four loads
   // a thread, cheaper than a pass of its own
   const int scanned = ntiles > 2048;
   if (scanned) scan_tile_offsets_kernel<<<1, kScanThreads, 0, s>>>(tiles, ntiles, total_err + 3);
-  unique_emit_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(src, n, ncols, col, slot_of, first, tiles, scanned,
-                                                               out_unique);
-  unique_inverse_kernel<<<g, 256, 0, s>>>(slot_of, first, n, inverse32, inverse64);
+  ANNC_CUDA(launch_pdl(unique_emit_kernel, tile_grid, scan_block, 0, s, src, n, ncols, col, slot_of, first, tiles, scanned,
+                       out_unique));
+  ANNC_CUDA(launch_pdl(unique_inverse_kernel, g, block, 0, s, slot_of, first, n, inverse32, inverse64));
   ANNC_CUDA(cudaGetLastError());
   if (box.words) return call.wait_posted(box, &res->err_bits, &res->count);
   int h[2] = {0, 0};
