@@ -175,7 +175,9 @@ bool bounce_ready() {
 // Pinned destination of small device reads, one per thread (null when it cannot be had).
 constexpr size_t kMailboxBytes = 256;
 constexpr size_t kPostBytes = 64;  // behind it: the words kernels post results to (PostBox)
-thread_local unsigned long long g_post_ticket = 0;
+// Tickets of the whole process: a thread may be handed the pinned words of one that has ended, with what was
+// posted there last.
+std::atomic<unsigned long long> g_post_ticket{0};
 struct Mailbox {
   void* p = nullptr;
   bool tried = false;
@@ -196,6 +198,7 @@ void* mailbox() {
       cudaGetLastError();
       m.p = nullptr;
     }
+    if (m.p) memset(m.p, 0, kMailboxBytes + kPostBytes);  // no ticket is 0
   }
   return m.p;
 }

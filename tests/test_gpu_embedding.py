@@ -2,6 +2,7 @@
 known-answer tests, through the C ABI.  Bit-exact for ids, rows, COO indices and
 for sums over sorted segment ids; 1e-5 relative for the atomic (unsorted) route."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -558,3 +559,38 @@ def test_segment_reduce_at_the_edges_of_the_scan(nnz, shuffled):
         idx[nnz - 1] = 70
         with pytest.raises(AnncError):
             ops.kp_fused_sparse_segment_reduce(_dev(data), _dev(idx), _dev(pairs), b2, b1, 0)
+
+
+def test_one_operator_call_per_thread():
+    """Threads one after the other, each with a single call that waits for a posted size: a thread must not take
+    what was posted for one that has ended, whose pinned memory it may be given, for its own."""
+    rng = np.random.default_rng(5)
+    data = rng.standard_normal((50, 8)).astype(np.float32)
+    d_data, zeros = _dev(data), (np.zeros(2, np.int32), np.zeros(1, np.int32))
+    good = []
+
+    def call(i):
+        n = [9000, 40, 5000, 700][i // 2 % 4] + i
+        seg, idx = rng.integers(0, n // (2 + i // 4), n), rng.integers(0, 50, n)
+        if i % 3:
+            seg = np.sort(seg)
+        pairs = _dev(np.stack([idx, seg], 1).astype(np.int64))
+        if i % 2:
+            unique, inverse, rows = (o.cpu().numpy() for o in ops.kp_fused_gather(d_data, pairs, zeros[0]))
+            want = idx[np.sort(np.unique(idx, return_index=True)[1])]
+            assert np.array_equal(unique, want) and np.array_equal(want[inverse], idx)
+            assert np.array_equal(rows, data[want])
+        else:
+            out, so = ops.kp_fused_sparse_segment_reduce(d_data, _dev(idx), pairs, np.array([0, 1], np.int32), zeros[1], 0)
+            want, size = np.zeros((2, seg.max() + 1, 8)), np.bincount(seg)[:, None]
+            np.add.at(want[0], seg, data[idx])
+            np.add.at(want[1], seg, np.abs(data[idx]))
+            assert int(so) == len(size) == out.shape[0]
+            assert (np.abs(out.cpu().numpy() - want[0]) <= 2.0 ** -24 * size * want[1]).all()  # adds in any order
+        good.append(i)
+
+    for i in range(32):
+        t = threading.Thread(target=call, args=(i,))
+        t.start()
+        t.join()
+    assert good == list(range(32))
