@@ -416,6 +416,7 @@ Call::Call() : stream_(g_stream), device_(device_slot()) {
 // use the arena's scratch on another stream: a call that takes some is ordered after it.
 void* Call::take_scratch(size_t bytes) {
   void* d = g_arenas.per_device[device_].alloc(bytes);
+  synced_ = false;  // what the call waited for so far did not use this
   if (d && !used_scratch_) {
     if (g_unsynced[device_] && g_last_event[device_] && g_last_stream[device_] != stream_)
       cudaStreamWaitEvent(stream_, g_last_event[device_], 0);
@@ -425,6 +426,12 @@ void* Call::take_scratch(size_t bytes) {
 }
 
 Call::~Call() {
+  // A way out between a posted result and the call's own wait: kernels behind the one that posted still read the
+  // operands and write the outputs, and a box may not have been waited for.
+  if (posting_ && !synced_) {
+    cudaStreamSynchronize(stream_);
+    synced_ = true;
+  }
   if (!held_.empty()) {
     std::lock_guard<std::mutex> lk(g_mu);
     for (auto& k : held_) {
@@ -630,6 +637,8 @@ PostBox Call::post_box() {
   if (void* m = mailbox()) {
     b.words = reinterpret_cast<unsigned long long*>(static_cast<char*>(m) + kMailboxBytes);
     b.ticket = ++g_post_ticket;
+    posting_ = true;
+    synced_ = false;
   }
   return b;
 }

@@ -123,14 +123,15 @@ class Call {
   // For a small result that the host needs while the call's later kernels already run: a kernel posts it
   // (post_result) into pinned memory of the thread and wait_posted() polls for it, where a copy and a
   // synchronize would wait for everything queued so far and leave the device idle meanwhile.  `words` is
-  // null without pinned memory.  Every box handed to a launched kernel has to be waited for in the same call.
+  // null without pinned memory.  A call that ends after this without having waited for its stream (an error on
+  // the way) waits for it then: a kernel that posts late would write over the next call's result.
   PostBox post_box();
   int wait_posted(const PostBox& box, int* flags, long long* value);
   // Waits for the call's stream (an operator whose outputs are complete when it returns).
   int wait();
   // True when p is device (or managed) memory.
   bool is_device(const void* p);
-  // True when the call waited for its stream (then device-side error words can be read).
+  // True when the call waited for its stream and took no scratch since (then device-side error words can be read).
   bool synced() const { return synced_; }
 
   int finish();
@@ -155,6 +156,7 @@ class Call {
   bool staged_ = false;
   bool synced_ = false;
   bool used_scratch_ = false;
+  bool posting_ = false;  // a box was handed out
   std::vector<Pending> pending_;
   std::vector<Touched> touched_;
   std::vector<Touched> held_;  // mirrors this call was handed: kept until it ends

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 import torch
 from annc_b200 import ops  # noqa: E402  (no fallback: a missing library fails the collection)
 from annc_b200 import AnncError, synth  # noqa: E402
-from annc_b200._lib import lib  # noqa: E402
+from annc_b200._lib import ALLOC_FN, lib  # noqa: E402
 from annc_b200.device import BagPlan  # noqa: E402
 
 
@@ -594,3 +594,38 @@ def test_one_operator_call_per_thread():
         t.start()
         t.join()
     assert good == list(range(32))
+
+
+@pytest.mark.parametrize("refused", [0, 1, 2])
+@pytest.mark.parametrize("begin_on_device", [False, True])
+def test_calls_that_fail_between_their_kernels_leave_none_running(refused, begin_on_device):
+    """An output allocation that fails after the size was posted: the kernels behind the one that posted it write the
+    caller's other outputs, so the stream is idle when the call returns, and the next call is not disturbed."""
+    rng = np.random.default_rng(refused)
+    n, dim = 2_000_000, 8
+    data = _dev(rng.standard_normal((300_000, dim)).astype(np.float32))
+    key = rng.integers(0, 300_000, n)
+    keys, idx = _dev(np.stack([key, np.sort(key)], 1)), _dev(key)
+    begin = np.array([0, 1], np.int32)
+    want = [o.cpu().numpy() for o in ops.kp_fused_gather(data, keys, begin)]
+    total = ops.kp_fused_sparse_segment_reduce(data, idx, keys, begin, begin[:1], 0)[0].cpu().numpy()
+    if begin_on_device:
+        begin = _dev(begin)
+    outs = ops._outputs_for(data)
+
+    @ALLOC_FN
+    def alloc(ctx, index, dtype, rank, dims):
+        return None if index == refused else outs._alloc(ctx, index, dtype, rank, dims)
+
+    t, b = ops.as_tensor, C.byref
+    first = begin[:1]
+    for _ in range(5):
+        rc = lib.annc_KPFusedGather(b(t(data)), b(t(keys)), b(t(begin)), alloc, None)
+        assert rc != 0 and torch.cuda.current_stream().query()
+        if refused < 2:
+            rc = lib.annc_KPFusedSparseSegmentReduce(b(t(data)), b(t(idx)), b(t(keys)), b(t(begin)), b(t(first)), C.c_int(0),
+                                                     alloc, None)
+            assert rc != 0 and torch.cuda.current_stream().query()
+    for got, w in zip(ops.kp_fused_gather(data, keys, begin), want):
+        np.testing.assert_array_equal(got.cpu().numpy(), w)
+    np.testing.assert_array_equal(ops.kp_fused_sparse_segment_reduce(data, idx, keys, begin, first, 0)[0].cpu().numpy(), total)
