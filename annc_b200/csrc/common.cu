@@ -372,6 +372,7 @@ int fail(int code, const char* fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next call is not to find it again
   return fail(ANNC_ERR_CUDA, "CUDA error %d (%s) in %s", static_cast<int>(e),
               cudaGetErrorString(e), what);
 }

@@ -381,3 +381,26 @@ def test_back_to_back_products_wait_for_each_other(m, n):
 
     for a, b in zip(chain(False), chain(True)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m,n", [(64, 128), (20000, 512), (64, 1)])
+def test_a_refused_launch_is_reported_once(m, n):
+    """A product on a stream whose capture was ended by an error is refused; the one after it runs."""
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.12")
+    x, w = torch.randn((m, 128), device="cuda"), torch.randn((128, n), device="cuda")
+    y = torch.empty((m, n), device="cuda")
+    stream = torch.cuda.Stream()
+    handle, graph = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+    call = lambda: device.gemm(x, w, y, m=m, n=n, k=128, stream=stream.cuda_stream)
+    call()
+    stream.synchronize()
+    assert rt.cudaStreamBeginCapture(handle, 1) == 0  # of this thread only
+    assert rt.cudaStreamSynchronize(handle) != 0  # not permitted now: the capture is over
+    with pytest.raises(AnncError):
+        call()
+    assert rt.cudaStreamEndCapture(handle, ctypes.byref(graph)) != 0 and not graph
+    rt.cudaGetLastError()
+    call()
+    stream.synchronize()
+    assert nerr(y, (x.double() @ w.double()).cpu().numpy()) <= 2e-3
