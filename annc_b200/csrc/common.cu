@@ -648,9 +648,14 @@ int Call::wait_posted(const PostBox& box, int* flags, long long* value) {
   if (status_ != ANNC_OK) return status_;
   const volatile unsigned long long* w = box.words;
   auto posted = [&] { return w[0] >> 8 == box.ticket; };
+  unsigned mode = cudaDeviceScheduleAuto;  // how the application wants its threads to wait
   for (unsigned spin = 1; !posted(); ++spin) {
     if (spin % 4096 != 0) continue;
-    const cudaError_t e = cudaStreamQuery(stream_);  // ends with the kernels at the latest
+    if (spin == 4096 && cudaGetDeviceFlags(&mode) != cudaSuccess) cudaGetLastError();
+    mode &= cudaDeviceScheduleMask;
+    if (mode == cudaDeviceScheduleYield) std::this_thread::yield();
+    // ends with the kernels at the latest
+    const cudaError_t e = mode == cudaDeviceScheduleBlockingSync ? cudaStreamSynchronize(stream_) : cudaStreamQuery(stream_);
     if (e == cudaErrorNotReady) continue;
     if (e != cudaSuccess) return status_ = cuda_fail(e, "wait_posted");
     if (!posted()) return status_ = fail(ANNC_ERR_INTERNAL, "a kernel ended without posting its result");

@@ -2,6 +2,9 @@
 known-answer tests, through the C ABI.  Bit-exact for ids, rows, COO indices and
 for sums over sorted segment ids; 1e-5 relative for the atomic (unsorted) route."""
 import ctypes as C
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -17,6 +20,8 @@ from annc_b200 import ops  # noqa: E402  (no fallback: a missing library fails t
 from annc_b200 import AnncError, synth  # noqa: E402
 from annc_b200._lib import ALLOC_FN, lib  # noqa: E402
 from annc_b200.device import BagPlan  # noqa: E402
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _dev(a):
@@ -629,3 +634,33 @@ def test_calls_that_fail_between_their_kernels_leave_none_running(refused, begin
     for got, w in zip(ops.kp_fused_gather(data, keys, begin), want):
         np.testing.assert_array_equal(got.cpu().numpy(), w)
     np.testing.assert_array_equal(ops.kp_fused_sparse_segment_reduce(data, idx, keys, begin, first, 0)[0].cpu().numpy(), total)
+
+
+_BLOCKING = """
+import ctypes, time
+cuda = ctypes.CDLL("libcuda.so.1")
+assert cuda.cuInit(0) == 0 and cuda.cuDevicePrimaryCtxSetFlags_v2(0, 4) == 0  # CU_CTX_SCHED_BLOCKING_SYNC
+import numpy as np, torch
+from annc_b200 import ops
+data, begin = torch.randn((1000, 8), device="cuda"), np.array([0, 1], np.int32)
+key = torch.arange(20000, device="cuda") % 700
+keys = torch.stack([key, key.sort()[0]], 1)
+x = torch.randn((8192, 8192), device="cuda")
+calls = [lambda: ops.kp_fused_gather(data, keys, begin),
+         lambda: ops.kp_fused_sparse_segment_reduce(data, key, keys, begin, begin[:1], 0)]
+for call in calls:
+    call(), torch.mm(x, x)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        torch.mm(x, x)
+    wall, busy = time.perf_counter(), time.thread_time()
+    call()
+    wall, busy = time.perf_counter() - wall, time.thread_time() - busy
+    assert wall > 0.05 and busy < wall / 4, (wall, busy)  # tens of GFLOP of fp32 ahead: the thread sleeps
+"""
+
+
+def test_posted_results_are_waited_for_as_the_application_asked():
+    """With the device set to blocking waits, a call behind a long queue leaves its core to others."""
+    r = subprocess.run([sys.executable, "-c", _BLOCKING], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
