@@ -13,15 +13,13 @@ shape-info vector [dims..., minor_to_major...] per operand
 from __future__ import annotations
 
 import ctypes as C
-import threading
-import weakref
 from functools import lru_cache
 from typing import List, Optional, Sequence
 
 import numpy as np
 
 from . import _lib
-from ._lib import ALLOC_FN, ANNC_BOOL, ANNC_F32, ANNC_I32, ANNC_I64, ANNC_U64, Tensor, check, lib
+from ._lib import ANNC_BOOL, ANNC_F32, ANNC_I32, ANNC_I64, ANNC_U64, Tensor, check, lib
 
 try:  # torch is plumbing for device memory only
     import torch
@@ -88,25 +86,27 @@ def as_tensor(x, dtype_code: Optional[int] = None) -> Tensor:
     return Tensor(_ptr(x), _code(x) if dtype_code is None else dtype_code, len(shape), shape)
 
 
-_calling = threading.local()  # .outputs: weak reference to the outputs of the call under way
-
-
-@ALLOC_FN
-def _allocate(ctx, index, dtype, rank, dims):
-    return _calling.outputs()._alloc(ctx, index, dtype, rank, dims)
+# ALLOC_FN with the context as the Python object that the call passed.
+@C.CFUNCTYPE(C.c_void_p, C.py_object, C.c_int, C.c_int32, C.c_int32, C.POINTER(C.c_int64))
+def _allocate(outs, index, dtype, rank, dims):
+    return outs._alloc(None, index, dtype, rank, dims)
 
 
 class _Outputs:
-    """allocate_output stand-in: numpy on the host, torch on the device.  One callback serves every call: one
-    per object would tie the object into a cycle with itself, and its arrays would stay allocated until
-    Python looks for cycles (outputs of 13 MB a call: device allocations of milliseconds now and then)."""
+    """allocate_output stand-in: numpy on the host, torch on the device.  One callback serves every call, the
+    object is its context: a callback per object would tie the object into a cycle with itself, and its arrays
+    would stay allocated until Python looks for cycles (outputs of 13 MB a call: device allocations of
+    milliseconds now and then)."""
     fn = _allocate
+
+    @property
+    def ctx(self):
+        return C.py_object(self)
 
     def __init__(self, on_device: bool, device=None):
         self.on_device = on_device
         self.device = device
         self.arrays = {}
-        _calling.outputs = weakref.ref(self)
 
     def _alloc(self, _ctx, index, dtype, rank, dims):
         shape = dims[:rank] if rank else ()
@@ -142,7 +142,7 @@ def kp_fused_sparse_segment_reduce(data, indices, slice_input, begin, begin_1, c
     outs = _outputs_for(data)
     check(lib.annc_KPFusedSparseSegmentReduce(
         C.byref(as_tensor(data)), C.byref(as_tensor(indices)), C.byref(as_tensor(slice_input)),
-        C.byref(as_tensor(begin)), C.byref(as_tensor(begin_1)), C.c_int(combiner), outs.fn, None))
+        C.byref(as_tensor(begin)), C.byref(as_tensor(begin_1)), C.c_int(combiner), outs.fn, outs.ctx))
     return outs[0], outs[1]
 
 
@@ -153,7 +153,7 @@ def kp_fused_sparse_segment_reduce_nonzero(data, indices, slice_input, begin, co
     outs = _outputs_for(data)
     check(lib.annc_KPFusedSparseSegmentReduceNonzero(
         C.byref(as_tensor(data)), C.byref(as_tensor(indices)), C.byref(as_tensor(slice_input)),
-        C.byref(as_tensor(begin)), C.c_int(combiner), outs.fn, None))
+        C.byref(as_tensor(begin)), C.c_int(combiner), outs.fn, outs.ctx))
     return outs[0], outs[1], outs[2]
 
 
@@ -163,7 +163,7 @@ def kp_fused_gather(data, keys, begin):
     begin = _small_i32(begin)
     outs = _outputs_for(data)
     check(lib.annc_KPFusedGather(C.byref(as_tensor(data)), C.byref(as_tensor(keys)),
-                                 C.byref(as_tensor(begin)), outs.fn, None))
+                                 C.byref(as_tensor(begin)), outs.fn, outs.ctx))
     return outs[0], outs[1], outs[2]
 
 
@@ -174,7 +174,7 @@ def kp_fused_sparse_dynamic_stitch(x, tables: Sequence):
     arr = (Tensor * len(tabs))(*[as_tensor(t) for t in tabs])
     outs = _outputs_for(tabs[0])
     check(lib.annc_KPFusedSparseDynamicStitch(C.byref(as_tensor(x)), arr, C.c_int(len(tabs)),
-                                              outs.fn, None))
+                                              outs.fn, outs.ctx))
     return outs[0]
 
 
@@ -187,7 +187,7 @@ def kp_fused_embedding_with_hash_bucket(fingerprints, variable, num_buckets, emp
     e = C.byref(as_tensor(empty, ANNC_BOOL)) if empty is not None else None
     check(lib.annc_KPFusedEmbeddingWithHashBucket(
         C.byref(as_tensor(fingerprints, ANNC_U64)), e, C.byref(as_tensor(variable)),
-        C.c_int64(num_buckets), C.c_int(int(bounded)), outs.fn, None))
+        C.c_int64(num_buckets), C.c_int(int(bounded)), outs.fn, outs.ctx))
     return outs[0]
 
 
@@ -197,7 +197,7 @@ def kp_fused_sparse_embedding(fingerprints, num_buckets, empty=None):
     outs = _outputs_for(fingerprints)
     e = C.byref(as_tensor(empty, ANNC_BOOL)) if empty is not None else None
     check(lib.annc_KPFusedSparseEmbedding(C.byref(as_tensor(fingerprints, ANNC_U64)), e,
-                                          C.c_int64(num_buckets), outs.fn, None))
+                                          C.c_int64(num_buckets), outs.fn, outs.ctx))
     return outs[0], outs[1], outs[2], outs[3]
 
 
@@ -206,7 +206,7 @@ def kp_fused_batch_matmul_add_sigmoid(lhs, rhs, bias):
     lhs, rhs, bias = _contig(lhs), _contig(rhs), _contig(bias)
     outs = _outputs_for(lhs)
     check(lib.annc_KPFusedBatchMatMulAddSigmoid(C.byref(as_tensor(lhs)), C.byref(as_tensor(rhs)),
-                                                C.byref(as_tensor(bias)), outs.fn, None))
+                                                C.byref(as_tensor(bias)), outs.fn, outs.ctx))
     return outs[0]
 
 
@@ -426,7 +426,7 @@ def kp_fused_embedding_padding(origin_shape, input, input_rows, reshape_sizes, p
     pk = np.array(pack, dtype=np.int32)
     check(lib.annc_KPFusedEmbeddingPadding(C.byref(as_tensor(os_)), C.byref(as_tensor(input)),
                                            C.byref(as_tensor(ir)), C.byref(as_tensor(rs)),
-                                           C.byref(as_tensor(pk)), C.c_int(int(fast)), outs.fn, None))
+                                           C.byref(as_tensor(pk)), C.c_int(int(fast)), outs.fn, outs.ctx))
     return outs[0], outs[1]
 
 
@@ -438,7 +438,7 @@ def kp_fused_embedding_action_id_gather(indices1, params, indices2, pack_dim, pa
     pk = np.array(pack, dtype=np.int32)
     check(lib.annc_KPFusedEmbeddingActionIdGather(
         C.byref(as_tensor(indices1)), C.byref(as_tensor(params)), C.byref(as_tensor(indices2)),
-        C.byref(as_tensor(pd)), C.byref(as_tensor(pk)), outs.fn, None))
+        C.byref(as_tensor(pd)), C.byref(as_tensor(pk)), outs.fn, outs.ctx))
     return outs[0]
 
 
@@ -450,7 +450,7 @@ def kp_fused_sparse_reshape(slice_input, begin, new_shape, pack_const):
     ns = np.array(new_shape, dtype=np.int64)
     pc = np.array(pack_const, dtype=np.int64)
     check(lib.annc_KPFusedSparseReshape(C.byref(as_tensor(slice_input)), C.byref(as_tensor(bg)),
-                                        C.byref(as_tensor(ns)), C.byref(as_tensor(pc)), outs.fn, None))
+                                        C.byref(as_tensor(ns)), C.byref(as_tensor(pc)), outs.fn, outs.ctx))
     return outs[0], outs[1]
 
 
@@ -461,5 +461,5 @@ def kp_fused_sparse_select(a, b, c, greater, equal1, equal2, equal3=0):
     sc = [_scalar(v, np.int32) for v in (greater, equal1, equal2, equal3)]
     check(lib.annc_KPFusedSparseSelect(C.byref(as_tensor(a)), C.byref(as_tensor(b)),
                                        C.byref(as_tensor(c)), *[C.byref(as_tensor(v)) for v in sc],
-                                       outs.fn, None))
+                                       outs.fn, outs.ctx))
     return outs[0], outs[1], outs[2]

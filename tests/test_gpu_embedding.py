@@ -664,3 +664,25 @@ def test_posted_results_are_waited_for_as_the_application_asked():
     """With the device set to blocking waits, a call behind a long queue leaves its core to others."""
     r = subprocess.run([sys.executable, "-c", _BLOCKING], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("where", ["host", "device"])
+def test_an_operator_inside_the_allocation_of_another(monkeypatch, where):
+    """An operator that runs while another's output is allocated (an allocator's hook, a finalizer) leaves the outer
+    call its outputs."""
+    put = _dev if where == "device" else np.asarray
+    data = put(np.arange(40, dtype=np.float32).reshape(10, 4))
+    keys = put(np.array([[0, 3], [1, 7], [2, 3]], np.int64))
+    begin, inner = np.array([0, 1], np.int32), []
+    plain = ops._Outputs._alloc
+
+    def alloc(self, ctx, index, dtype, rank, dims):
+        if not inner:
+            inner.append(None)
+            inner[0] = ops.kp_fused_sparse_dynamic_stitch(put(np.array([1, 0], np.int64)), [data, data])
+        return plain(self, ctx, index, dtype, rank, dims)
+
+    monkeypatch.setattr(ops._Outputs, "_alloc", alloc)
+    unique, inverse, rows = ops.kp_fused_gather(data, keys, begin)
+    assert [int(v) for v in unique] == [3, 7] and [int(v) for v in inverse] == [0, 1, 0]
+    assert rows.tolist() == data[[3, 7]].tolist() and inner[0].tolist() == data[[0, 0]].tolist()
