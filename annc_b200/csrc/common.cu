@@ -77,6 +77,7 @@ thread_local Arenas g_arenas;
 thread_local cudaStream_t g_last_stream[kMaxDevices] = {nullptr};
 thread_local cudaEvent_t g_last_event[kMaxDevices] = {nullptr};
 thread_local bool g_unsynced[kMaxDevices] = {false};
+thread_local int g_calls = 0;  // under way: an output allocation may run another operator
 
 // ---- staged copies between pageable host memory and the device.
 // A large operand moves through a pinned two-half bounce buffer of the calling thread: while
@@ -410,7 +411,7 @@ static bool capturing(cudaStream_t s) {
 }
 
 Call::Call() : stream_(g_stream), device_(device_slot()) {
-  g_arenas.per_device[device_].reset();
+  if (g_calls++ == 0) g_arenas.per_device[device_].reset();
 }
 
 // A previous call of this thread that returned without synchronising (device pointers only) may still
@@ -427,6 +428,7 @@ void* Call::take_scratch(size_t bytes) {
 }
 
 Call::~Call() {
+  --g_calls;
   // A way out between a posted result and the call's own wait: kernels behind the one that posted still read the
   // operands and write the outputs, and a box may not have been waited for.
   if (posting_ && !synced_) {

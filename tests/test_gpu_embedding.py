@@ -673,16 +673,17 @@ def test_an_operator_inside_the_allocation_of_another(monkeypatch, where):
     put = _dev if where == "device" else np.asarray
     data = put(np.arange(40, dtype=np.float32).reshape(10, 4))
     keys = put(np.array([[0, 3], [1, 7], [2, 3]], np.int64))
-    begin, inner = np.array([0, 1], np.int32), []
+    begin, inner, outer = np.array([0, 1], np.int32), [], []
     plain = ops._Outputs._alloc
 
     def alloc(self, ctx, index, dtype, rank, dims):
-        if not inner:
-            inner.append(None)
-            inner[0] = ops.kp_fused_sparse_dynamic_stitch(put(np.array([1, 0], np.int64)), [data, data])
+        outer[:] = outer or [self]
+        if self is outer[0]:  # before each of its three outputs, in the middle of its scratch
+            inner.append(ops.kp_fused_gather(data, put(np.array([[0, 9], [1, 8], [2, 9]], np.int64)), begin))
         return plain(self, ctx, index, dtype, rank, dims)
 
     monkeypatch.setattr(ops._Outputs, "_alloc", alloc)
-    unique, inverse, rows = ops.kp_fused_gather(data, keys, begin)
-    assert [int(v) for v in unique] == [3, 7] and [int(v) for v in inverse] == [0, 1, 0]
-    assert rows.tolist() == data[[3, 7]].tolist() and inner[0].tolist() == data[[0, 0]].tolist()
+    calls = [ops.kp_fused_gather(data, keys, begin)] + inner
+    assert len(calls) == 4
+    for (unique, inverse, rows), want in zip(calls, ([3, 7], [9, 8], [9, 8], [9, 8])):
+        assert unique.tolist() == want and inverse.tolist() == [0, 1, 0] and rows.tolist() == data[want].tolist()
