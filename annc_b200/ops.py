@@ -275,7 +275,9 @@ def _call_custom(target: str, out, operands: List):
 
 def _new_like(x, shape):
     if _is_torch(x):
-        return x.new_empty(shape) if x.dtype is torch.float32 else torch.empty(shape, dtype=torch.float32, device=x.device)
+        if type(x) is torch.Tensor and x.dtype is torch.float32:  # a subclass would hand on its type
+            return x.new_empty(shape)
+        return torch.empty(shape, dtype=torch.float32, device=x.device)
     return np.empty(shape, np.float32)
 
 

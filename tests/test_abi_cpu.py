@@ -289,3 +289,18 @@ def test_gemm_takes_transposes_of_any_truth_type(annc, yes):
     t = torch.zeros(64, 64)
     with pytest.raises(annc.AnncError):
         device.gemm(t, t, t, m=-1, n=64, k=64, trans_a=yes, trans_b=yes, stream=0)
+
+
+def test_outputs_are_plain_tensors():
+    """Of a tensor subclass too, in float32 on its device."""
+    torch = pytest.importorskip("torch")
+    from annc_b200 import ops
+
+    class Named(torch.Tensor):
+        pass
+
+    x = torch.ones(3, 4)
+    for y in (x, x.as_subclass(Named), torch.nn.Parameter(x), x.double()):
+        out = ops._new_like(y, (2, 5))
+        assert type(out) is torch.Tensor and out.dtype is torch.float32 and tuple(out.shape) == (2, 5)
+        assert not out.requires_grad and out.device == x.device
