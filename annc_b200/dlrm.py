@@ -37,10 +37,16 @@ from .synth import DlrmModel
 
 class DlrmPipeline:
     embed_first = True  # forward() queues the pooling kernel before the bottom MLP
-    # Up to this batch a step on one GPU stays on one stream.  The second one costs five event calls; what runs
-    # beside the pooling kernel there is worth less.  us a step, two streams / one (a step waited for):
-    # batch 64 79 / 66 (93 / 80), 200 80 / 71 (98 / 86), 512 79 / 77 (98 / 88), 1024 77 / 84 (102 / 96), 4096 123 / 137.
+    # Small steps on one GPU stay on one stream.  The second one costs five event calls, and what runs beside the
+    # pooling kernel there is worth less: us a step, two streams / one (a step waited for), 26 tables of dim 64, bags
+    # of up to 20: batch 64 77 / 61 (86 / 70), 200 77 / 61 (87 / 72), 512 77 / 64 (89 / 75); batch 1024 77 / 84
+    # (102 / 96), 4096 123 / 137.  Not for many lookups, whose pooling the bottom MLP hides behind in steps issued
+    # back to back (8 tables, batch 512: 202 K lookups of dim 64 77 / 71, of dim 128 78 / 77, 365 K 78 / 80 and 78 / 86;
+    # batch 200 100 K 77 / 68, 281 K 77 / 87; 26 tables, batch 512 1.3 M 113 / 131), and not for long bags, whose
+    # lookups few warps pool (batch 64, 100 K lookups, mean bag 60 of 26 tables 78 / 63, 195 of 8 77 / 83).
     ONE_STREAM_BATCH = 512
+    ONE_STREAM_LOOKUPS = 150_000
+    ONE_STREAM_BAG = 64  # lookups per bag, on average
     gemm_flags = 0
 
     def __init__(self, model: DlrmModel, device: torch.device, math: int = MATH_AUTO,
@@ -190,10 +196,11 @@ class DlrmPipeline:
             x = y
 
     def _one_stream(self) -> bool:
-        return self.embed_first and self.batch <= self.ONE_STREAM_BATCH
+        return (self.embed_first and self.batch <= self.ONE_STREAM_BATCH and
+                self.nnz_total <= min(self.ONE_STREAM_LOOKUPS, self.ONE_STREAM_BAG * self.batch * self.T))
 
     def _sparse_part(self, names, lookahead: bool = False) -> None:
-        """Bottom MLP (second stream, for larger batches) beside the embedding pooling; z is complete
+        """Bottom MLP (on the second stream, but for small steps) beside the embedding pooling; z is complete
         afterwards."""
         if self._one_stream():
             self.embed_prefetch()

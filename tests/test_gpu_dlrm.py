@@ -52,6 +52,42 @@ def test_pipelined_steps_of_another_stream_are_waited_for():
             assert torch.equal(o, want)
 
 
+@pytest.mark.parametrize("batch,max_bag,one", [(1, 3, True), (64, 120, True), (64, 130, False), (512, 20, True), (513, 20, False),
+                                               (512, 24, False)])
+def test_small_steps_on_one_stream(batch, max_bag, one):
+    """Steps at either side of the lines between one stream and two (batch, lookups, mean bag): the oracle's predictions,
+    and the same ones whichever way the steps are issued."""
+    model = synth.dlrm_model(seed=6, batch=batch, max_rows=3e4, max_bag=max_bag)
+    pipe = DlrmPipeline(model, torch.device("cuda:0"), keep_host_inputs=True)
+    assert pipe._one_stream() is one
+    outs = [pipe.forward().clone() for _ in range(3)]
+    torch.cuda.synchronize()
+    if one:  # waits for nothing of another stream: it can be captured as it is
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = pipe.forward()
+        pipe.out.fill_(-1.0)
+        graph.replay()
+        outs.append(captured.clone())
+    outs += [pipe.forward_pipelined() for _ in range(4)][2:]
+    pipe.sync_pipeline()
+    outs = [o.clone() for o in outs]
+    outs.append(pipe.forward().clone())
+    for _ in range(3):  # from host inputs
+        for st in pipe.sets:
+            st["ids_all"].zero_()
+        torch.cuda.synchronize()
+        pipe._prefetched = [False, False]
+        host = pipe.forward_e2e()
+        torch.cuda.synchronize()
+        outs.append(host.cuda())
+    assert pipe.embed_error_bits() == 0
+    for o in outs:
+        assert torch.equal(o, outs[0])
+    want = oracle.dlrm_forward(model, threads=oracle.host_threads())
+    assert np.abs(outs[0].cpu().numpy() - want).max() <= 2e-3
+
+
 def test_smoke_entry():
     import __graft_entry__ as g
     g.smoke()
