@@ -87,12 +87,41 @@ static int list_chunk(long long lookups, int num_tables, long long warps, int la
   return best;
 }
 
-// A lookup-granular kernel: lanes of a group, whether it is the one by lists, and its resident blocks per SM
-// by device (0: not asked).
+// Rounds of `rows` rows per lookup that bags of this mean length take (its spread taken for wide).
+static float rounds_per_lookup(float mean_bag, int rows) {
+  const float len = std::max(mean_bag, 1.f);
+  return std::max(1.f, (len + 0.5f * (float)(rows - 1)) / (float)rows) / len;
+}
+
+// The chunks of the kernel by lists of bags, table by table.  A warp's time goes by rounds, and a round takes up
+// to four or eight rows of a bag or one: a table whose bags are shorter than the others' gets shorter chunks, of as
+// many rounds as a chunk of the call's average lookup (a chunk of 224 bags of one is 56 to 224 round trips to memory, one
+// after the other).  Its lookups count for as many more when the common length is chosen.  us, a fourth of the
+// tables with bags of 20 to 80, the others of one; one length for all / this (the pipeline kernel): 8 tables x 20,000 bags
+// of dim 64 131 / 95 (100), of dim 128 231 / 141 (162), of dim 256 419 / 254 (284); 26 x 2,048 of dim 256 157 / 110 (111).
+// Tables of nearly the same mean keep one length.
+static void list_chunks(const BagParams& p, long long lookups, long long warps, int lanes, int rows, StreamChunks* sc) {
+  float per[kMaxTables];
+  double rounds = 0, weight = 0;
+  for (int t = 0; t < p.num_tables; ++t) {
+    per[t] = rounds_per_lookup((float)p.t[t].nnz / (float)p.batch, rows);
+    rounds += (double)per[t] * p.t[t].nnz;
+  }
+  const float usual = lookups > 0 ? (float)(rounds / (double)lookups) : 1.f;
+  for (int t = 0; t < p.num_tables; ++t) {
+    per[t] = per[t] > 1.25f * usual ? per[t] / usual : 1.f;
+    weight += (double)per[t] * p.t[t].nnz;
+  }
+  const int chunk = list_chunk((long long)weight, p.num_tables, warps, lanes);
+  for (int t = 0; t < p.num_tables; ++t) sc->list_chunk[t] = std::max(8, (int)((float)chunk / per[t]) & ~7);
+}
+
+// A lookup-granular kernel: lanes of a group, the rows of a round of the one by lists (0: the other one), and
+// its resident blocks per SM by device (0: not asked).
 struct StreamShape {
   void (*kernel)(BagParams, StreamChunks, BagHeader*);
   int lanes;
-  bool list;
+  int list_rows;
   int per_sm[kMaxDevices];
 };
 
@@ -112,18 +141,19 @@ static void launch_stream(StreamShape& shape, const BagParams& p, BagHeader* hdr
   const int ctas = t_stream_ctas_per_sm > 0 ? std::min(t_stream_ctas_per_sm, shape.per_sm[slot])
                                             : std::max(1, shape.per_sm[slot] + t_stream_ctas_per_sm);
   // a chunk is a warp's, or a group's
-  const long long takers = shape.list ? 256 / 32 : 256 / shape.lanes;
+  const long long takers = shape.list_rows ? 256 / 32 : 256 / shape.lanes;
   const long long max_blocks = (long long)sm_count[slot] * ctas;
   long long lookups = 0;
   for (int t = 0; t < p.num_tables; ++t) lookups += p.t[t].nnz;
   StreamChunks sc;
-  sc.chunk = shape.list ? list_chunk(lookups, p.num_tables, max_blocks * takers, shape.lanes)
-                        : stream_chunk(lookups, p.num_tables, shape.lanes, max_blocks * takers);
+  if (shape.list_rows) list_chunks(p, lookups, max_blocks * takers, shape.lanes, shape.list_rows, &sc);
+  else sc.chunk = stream_chunk(lookups, p.num_tables, shape.lanes, max_blocks * takers);
   long long total = 0;
   for (int t = 0; t < p.num_tables; ++t) {
     sc.first[t] = (int)total;
     const long long n = p.t[t].nnz;
-    total += n > 0 ? (n + sc.chunk - 1) / sc.chunk : (p.batch + 1023) / 1024;
+    const int chunk = shape.list_rows ? sc.list_chunk[t] : sc.chunk;
+    total += n > 0 ? (n + chunk - 1) / chunk : (p.batch + 1023) / 1024;
   }
   sc.first[p.num_tables] = (int)total;
   // a persistent grid, no larger than the chunks there are
@@ -133,14 +163,14 @@ static void launch_stream(StreamShape& shape, const BagParams& p, BagHeader* hdr
 
 template <int LANES, int VPL, int MINB>
 static StreamShape& stream_shape(int vecs) {
-  static StreamShape full{bag_stream_kernel<LANES, VPL, 2, true, MINB>, LANES, false, {}};
-  static StreamShape part{bag_stream_kernel<LANES, VPL, 2, false, MINB>, LANES, false, {}};
+  static StreamShape full{bag_stream_kernel<LANES, VPL, 2, true, MINB>, LANES, 0, {}};
+  static StreamShape part{bag_stream_kernel<LANES, VPL, 2, false, MINB>, LANES, 0, {}};
   return vecs == LANES * VPL ? full : part;
 }
 
 template <int LANES, int F, int VPL, int Q, int MINB = 4>
 static StreamShape& list_shape() {
-  static StreamShape shape{bag_list_kernel<LANES, F, VPL, Q, MINB>, LANES, true, {}};
+  static StreamShape shape{bag_list_kernel<LANES, F, VPL, Q, MINB>, LANES, Q, {}};
   return shape;
 }
 
@@ -157,7 +187,7 @@ static StreamShape& stream_shape_beside(int vecs) {
 
 // The smallest shape whose lanes hold a row, from dim 64 on 32 bytes each where rows are `wide`, 32-byte
 // aligned and a multiple of that long: fewer lanes repeat the control instructions, more bags go at a time.
-// mean_bag: lookups per bag, on average.  us for 11 tables x 60 K rows, bags of 1 to n lookups:
+// us for 11 tables x 60 K rows, bags of 1 to n lookups:
 //   * short bags stay with the pipeline, whose steps do not wait for a list; pipeline / list
 //       dim 16   n = 2 36 / 43, 4 44 / 46, 8 43 / 41, 20 45 / 40;   dim 32   2 62 / 71, 4 72 / 71, 8 64 / 62, 20 58 / 54
 //       dim 64   1 75 / 80, 2 85 / 88, 4 103 / 98, 20 82 / 73;      dim 128  1 132 / 141, 2 128 / 128, 4 103 / 100, 20 81 / 72
@@ -165,16 +195,19 @@ static StreamShape& stream_shape_beside(int vecs) {
 //     dim 256  1 139 / 129 two rows at a time, 2 128 / 124, 20 74.1 / 74.0: by lists only
 //   * so does a share of the SM's slots, too few warps to hide the list's latencies: two blocks of dim 64
 //     152 / 164, of dim 128 137 / 150, three 126 / 126, 118 / 122
-//   * long bags are taken by groups twice as large, eight rows at a time: a chunk has too few of them for
-//     many groups.  dim 64, four / eight rows: 1 to 20 478 / 498 (26 tables up to 1 M rows), 1 to 30 72.1 / 72.5,
-//     20 to 40 73 / 69, 64 to 128 206 / 140
-static StreamShape& stream_shape_for(int vecs, bool wide, double mean_bag) {
+//   * long bags are taken eight rows at a time, wide rows by groups twice as large: a chunk has too few of them for many
+//     groups.  dim 64, four / eight rows: 1 to 20 478 / 498 (26 tables up to 1 M rows), 1 to 30 72.1 / 72.5,
+//     20 to 40 73 / 69, 64 to 128 206 / 140.  Where tables differ, the bag of the average lookup (`lookup_bag`) tells:
+//     8 tables x 20,000 bags, seven of bags of 1 and 2, one of 50 to 150, 146 / 104.  Rows that are not wide have one or
+//     two groups a warp either way; dim 100, 1 to 20 219 / 214, 26 tables x 2,048, every fourth with bags of one, the
+//     others of 1 to 20 52 / 70
+static StreamShape& stream_shape_for(int vecs, bool wide, double mean_bag, double lookup_bag) {
   const bool pipeline = beside() || mean_bag < (vecs <= 4 ? 3.5 : vecs > 8 && !wide ? 4.5 : 2.0);
-  const bool eight = mean_bag >= 18 || !wide;
+  const bool eight = lookup_bag >= 18;
   if (vecs <= 4) return pipeline ? stream_shape_beside<4, 1>(vecs) : list_shape<4, 4, 1, 4>();
   if (vecs <= 8) return pipeline ? stream_shape_beside<8, 1>(vecs) : list_shape<8, 4, 1, 4>();
-  if (vecs <= 16) return pipeline ? stream_shape_beside<8, 2>(vecs) : eight ? list_shape<16, 4, 1, 8>() : list_shape<8, 8, 1, 4>();
-  if (vecs <= 32) return pipeline ? stream_shape_beside<16, 2>(vecs) : eight ? list_shape<32, 4, 1, 8>() : list_shape<16, 8, 1, 4>();
+  if (vecs <= 16) return pipeline ? stream_shape_beside<8, 2>(vecs) : eight ? list_shape<16, 4, 1, 8>() : wide ? list_shape<8, 8, 1, 4>() : list_shape<16, 4, 1, 4>();
+  if (vecs <= 32) return pipeline ? stream_shape_beside<16, 2>(vecs) : eight ? list_shape<32, 4, 1, 8>() : wide ? list_shape<16, 8, 1, 4>() : list_shape<32, 4, 1, 4>();
   if (vecs <= 64) return mean_bag < 2 ? list_shape<32, 4, 2, 2>() : wide ? list_shape<32, 8, 1, 4>() : list_shape<32, 4, 2, 4>();
   return wide ? list_shape<32, 8, 2, 2, 3>() : list_shape<32, 4, 4, 2, 3>();
 }
@@ -213,6 +246,7 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
   p.dim = dim;
   p.out_stride = out_stride;
   long long max_nnz = 0, lookups = 0;
+  double squares = 0;
   bool vec_ok = (dim % 4 == 0) && (out_stride % 4 == 0), wide = dim % 8 == 0;
   for (int t = 0; t < num_tables; ++t) {
     if (tables[t].nnz >= (int64_t(1) << 31) - 1)
@@ -232,6 +266,7 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
     p.t[t].given_off = tables[t].offsets;
     max_nnz = std::max<long long>(max_nnz, tables[t].nnz);
     lookups += tables[t].nnz;
+    squares += (double)tables[t].nnz * (double)tables[t].nnz;
     vec_ok = vec_ok && aligned16(tables[t].table) && aligned16(tables[t].out);
     wide = wide && (reinterpret_cast<uintptr_t>(tables[t].table) & 31) == 0;
   }
@@ -257,7 +292,9 @@ static int run_bags(const annc_bag_table* tables, int num_tables, int64_t dim, i
                       ncols < (1LL << 31) && out_stride < (1LL << 31);
   if (stream) {
     if (ev0) cudaEventRecord(ev0, s);
-    launch_stream(stream_shape_for(vecs, wide, (double)lookups / ((double)num_tables * (double)batch)), p, hdr, s);
+    const double mean_bag = (double)lookups / ((double)num_tables * (double)batch);
+    const double lookup_bag = lookups > 0 ? squares / ((double)lookups * (double)batch) : 0.0;
+    launch_stream(stream_shape_for(vecs, wide, mean_bag, lookup_bag), p, hdr, s);
     if (ev1) cudaEventRecord(ev1, s);
     if (known_sorted) {
       ANNC_CUDA(cudaGetLastError());
@@ -382,7 +419,7 @@ int annc_embed_bag_stream_registers(int64_t dim, int* registers_per_thread) {
   ANNC_REQUIRE(registers_per_thread && dim >= 4 && dim <= 512 && dim % 4 == 0, ANNC_ERR_INVALID_ARGUMENT,
                "bag registers: dim must be a multiple of four up to 512");
   cudaFuncAttributes attr;
-  ANNC_CUDA(cudaFuncGetAttributes(&attr, stream_shape_for((int)(dim / 4), dim % 8 == 0, 10).kernel));
+  ANNC_CUDA(cudaFuncGetAttributes(&attr, stream_shape_for((int)(dim / 4), dim % 8 == 0, 10, 10).kernel));
   *registers_per_thread = attr.numRegs;
   return ANNC_OK;
 }

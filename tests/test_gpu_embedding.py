@@ -444,8 +444,8 @@ def test_bag_plan_marks_unsorted_and_out_of_range(dim, combiner):
 @pytest.mark.parametrize("shift", [0, 4])
 @pytest.mark.parametrize("combiner", [0, 1])
 def test_bags_around_the_decoded_window(dim, shift, combiner):
-    """Bags that end at, just before and just behind the lookups a warp decodes at a time (chunk, look-ahead
-    and several windows), tables 32-byte aligned and not, rows out of range among them: the sums in lookup
+    """Bags that end anywhere in the short windows of a call of few lookups (chunks of 16 or 24, then windows of 128) and
+    reach over several, tables 32-byte aligned and not, rows out of range among them: the sums in lookup
     order, bit for bit."""
     rng = np.random.default_rng(dim + shift)
     rows, lens = 300, []
@@ -471,6 +471,75 @@ def test_bags_around_the_decoded_window(dim, shift, combiner):
         want *= (np.float32(1) / np.maximum(lens, 1).astype(np.float32))[:, None]
     assert plan.error_bits() == 1
     np.testing.assert_array_equal(out.cpu().numpy()[:, 0], want)
+
+
+def _hash_bags(rng, lens):
+    """Raw ids and index matrix of one table's bags."""
+    seg = np.repeat(np.arange(len(lens)), lens)
+    ids = rng.integers(0, 1 << 62, len(seg))
+    return ids, np.stack([seg, seg], 1).astype(np.int64).reshape(-1, 2)
+
+
+def _oracle_bags(tables, ids, segs, batch, combiner):
+    want = np.full((batch, len(tables), tables[0].shape[1]), np.nan, np.float32)
+    oracle.embed_bags_tables(tables, [t.shape[0] for t in tables], ids, segs, batch, tables[0].shape[1], want, len(tables),
+                             0, combiner=combiner, threads=oracle.host_threads())
+    return want
+
+
+@pytest.mark.parametrize("dim", [12, 32, 40, 64, 100, 128, 160, 256, 512])
+@pytest.mark.parametrize("shift,id_kind", [(0, 2), (4, 1), (0, 0)])
+@pytest.mark.parametrize("bags", ["long", "short"])
+def test_bags_around_a_full_window(dim, shift, id_kind, bags):
+    """Enough lookups for the longest chunks (4736 resident warps of 224, 3552 above 256 floats): bags that end at, just
+    before and just behind the chunk, the 32 lookups behind it and the windows of 128 after that, in rows that
+    are 32-byte aligned and not, by four and by eight rows a round, every kind of id: the oracle's sums, bit for bit."""
+    rng = np.random.default_rng(dim + shift)
+    n_all = (3552 if dim > 256 else 4736) * 224
+    edges = [224] * 6 + [223, 1, 225, 31, 193, 32, 192, 33, 191, 255, 256, 257, 383, 384, 385, 512, 0, 0, 1500, 127, 128, 129]
+    lens = []
+    while sum(lens) < n_all // 8:  # an eighth of the lookups in bags that the edges are about
+        lens += edges + list(rng.integers(0, 5, rng.integers(0, 30)))
+    hi = 60 if bags == "long" else 9
+    fill = rng.integers(0, hi, 2 * (n_all - sum(lens)) // (hi - 1))
+    at = np.sort(rng.integers(0, len(fill), 40))
+    lens = np.concatenate([v for part in zip(np.array_split(np.array(lens), 41), np.split(fill, at)) for v in part])
+    batch, rows = len(lens), 3000
+    ids, pairs = _hash_bags(rng, lens)
+    data = rng.standard_normal((rows, dim)).astype(np.float32)
+    base = torch.zeros(rows * dim + 4, device="cuda")
+    table = base[shift:shift + rows * dim].view(rows, dim)
+    table.copy_(_dev(data))
+    out = torch.full((batch, 1, dim), np.nan, device="cuda")
+    given = ids if id_kind == 2 else ids.astype(np.uint64) % rows
+    plan = BagPlan([table], [_dev(given.astype(np.int32 if id_kind == 0 else np.int64))], [_dev(pairs)], out, 0, batch,
+                   id_kind=id_kind, combiner=id_kind == 1)
+    plan.run()
+    assert plan.error_bits() == 0
+    np.testing.assert_array_equal(out.cpu().numpy(), _oracle_bags([data], [ids], [pairs], batch, int(id_kind == 1)))
+
+
+@pytest.mark.parametrize("dim", [8, 16, 36, 64, 100, 128, 256, 512])
+@pytest.mark.parametrize("batch", [300, 12000])
+@pytest.mark.parametrize("share", [0, 3])
+def test_tables_of_different_bag_lengths(dim, batch, share):
+    """Tables of one call with bags of one, of a few, of many lookups, with very long ones among short ones and with none
+    at all: chunks of a length per table, the oracle's sums bit for bit; with a share of the SMs too."""
+    rng = np.random.default_rng(dim * batch)
+    u = lambda lo, hi: rng.integers(lo, hi + 1, batch)
+    lens = [np.ones(batch, int), u(20, 80), u(0, 1), np.zeros(batch, int), u(1, 3), np.where(u(0, 99) == 0, 400, 1), u(1, 20),
+            np.where(np.arange(batch) == batch - 1, 1, 0)]
+    ids, segs = zip(*(_hash_bags(rng, v) for v in lens))
+    tables = [rng.standard_normal((int(r), dim)).astype(np.float32) for r in rng.integers(1, 2000, len(lens))]
+    out = torch.full((batch, len(lens), dim), np.nan, device="cuda")
+    lib.annc_embed_bag_set_stream_ctas_per_sm(share)
+    try:
+        plan = BagPlan([_dev(t) for t in tables], [_dev(i) for i in ids], [_dev(s) for s in segs], out, 0, batch)
+        plan.run()
+        assert plan.error_bits() == 0
+    finally:
+        lib.annc_embed_bag_set_stream_ctas_per_sm(0)
+    np.testing.assert_array_equal(out.cpu().numpy(), _oracle_bags(tables, ids, segs, batch, 0))
 
 
 @pytest.mark.parametrize("dim", [16, 32, 64, 100, 128])
