@@ -756,3 +756,34 @@ def test_an_operator_inside_the_allocation_of_another(monkeypatch, where):
     assert len(calls) == 4
     for (unique, inverse, rows), want in zip(calls, ([3, 7], [9, 8], [9, 8], [9, 8])):
         assert unique.tolist() == want and inverse.tolist() == [0, 1, 0] and rows.tolist() == data[want].tolist()
+
+
+@pytest.mark.parametrize("n", [50, 5000, 400_000])
+def test_gather_and_reduce_behind_the_kernels_that_make_their_operands(n):
+    """Keys, segment ids and rows written by kernels that are still running when the operators are called, call after call
+    over the same buffers."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    heavy = torch.randn((4096, 4096), device="cuda", generator=g)
+    rows, zeros = 1000, np.zeros(2, np.int32)
+    data, pairs = torch.zeros((rows, 16), device="cuda"), torch.zeros((n, 2), dtype=torch.int64, device="cuda")
+    sources = [(torch.randn((rows, 16), device="cuda", generator=g),
+                torch.stack([torch.randint(0, hi, (n,), device="cuda", generator=g),
+                             torch.sort(torch.randint(0, n // hi + 1, (n,), device="cuda", generator=g))[0]], 1))
+               for hi in (7, rows, 300, 1)]
+
+    def calls(wait):
+        out = []
+        for d, p in sources:
+            torch.mm(heavy, heavy)
+            data.copy_(d)
+            pairs.copy_(p)
+            wait()
+            out += list(ops.kp_fused_gather(data, pairs, zeros))
+            out.append(ops.kp_fused_sparse_segment_reduce(data, pairs[:, 0].contiguous(), pairs, np.array([0, 1], np.int32),
+                                                          zeros[:1], 0)[0])
+        return out
+
+    want = calls(torch.cuda.synchronize)
+    for _ in range(3):
+        for a, b in zip(calls(lambda: None), want):
+            assert torch.equal(a, b)

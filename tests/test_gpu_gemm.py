@@ -383,6 +383,90 @@ def test_back_to_back_products_wait_for_each_other(m, n):
         assert torch.equal(a, b)
 
 
+def _same_with_and_without_waiting(chain):
+    """chain(wait) calls wait() after each of its steps; its outputs are those of the run that waits each time."""
+    want = chain(torch.cuda.synchronize)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = chain(lambda: None)
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m,bf16", [(128, False), (512, False), (1024, False), (4096, False), (256, True), (4096, True)])
+def test_a_product_reads_what_the_one_before_it_wrote(m, bf16):
+    """... as its A, its B, its bias or its addend, and overwrites what that one read: kernels of both tile sizes and of
+    split K, which are launched while the one before them drains."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    rnd = lambda *shape: torch.randn(shape, device="cuda", generator=g)
+    n = k = 512
+    a0, b0, t0, add0 = rnd(m, k), rnd(k, n) * k ** -0.5, rnd(n, n) * n ** -0.5, rnd(m, n)
+    bias0 = rnd(n)
+    if bf16:
+        a0, b0, t0 = a0.bfloat16(), (b0.t().contiguous()).bfloat16(), t0.bfloat16()
+
+    def chain(wait):
+        a, b, bias, add = a0.clone(), b0.clone(), bias0.clone(), add0.clone()
+        out = []
+
+        def mul(x, y, c, rows, **kw):
+            if bf16:
+                flags = _lib.IO_A_BF16 | _lib.IO_B_BF16 | (_lib.IO_C_BF16 if c.dtype is torch.bfloat16 else 0)
+                kw.update(trans_b=True, math=_lib.MATH_BF16, io_flags=flags)
+            device.gemm(x, y, c, m=rows, n=n, k=k, **kw)
+            wait()
+
+        for _ in range(6):
+            c = torch.empty((m, n), device="cuda")
+            nb = torch.empty_like(b)
+            mul(t0, b, nb, n)  # the next product's B ...
+            row = torch.empty((256, n), device="cuda")
+            mul(a[:128].repeat(2, 1), nb, row, 256, activation=1)  # ... and from it a bias
+            full = torch.empty((m, n), device="cuda")
+            mul(a, nb, full, m, addend=add, bias=row[3])
+            mul(a, b, c, m, addend=full, bias=row[5], activation=1)  # the addend of the launch before
+            mul(a, nb, full, m, bias=bias)  # over what that one read
+            bias = row[7]
+            na = torch.empty_like(a)
+            mul(a, b, na, m)
+            mul(na, nb, c, m, addend=full)
+            a, add = na, full
+            out += [c.clone(), full.clone(), row.clone()]
+        return out
+
+    _same_with_and_without_waiting(chain)
+
+
+@pytest.mark.parametrize("batch", [1, 100, 3000, 20000])
+def test_interaction_between_products(batch):
+    """z is written by the product before the interaction, what it wrote is read by the one behind it, and the next
+    round's first product overwrites z."""
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    F, D, H, pad = 27, 64, 256, 416
+    x0 = torch.randn((batch, H), device="cuda", generator=g)
+    w = torch.randn((H, D), device="cuda", generator=g) * H ** -0.5
+    top = torch.randn((pad, H), device="cuda", generator=g) * pad ** -0.5
+    last = torch.randn((H, 1), device="cuda", generator=g) * H ** -0.5
+    z0 = torch.randn((batch, F, D), device="cuda", generator=g)
+
+    def chain(wait):
+        x, z, inter, out = x0.clone(), z0.clone(), torch.full((batch, pad), -3.0, device="cuda"), []
+        for _ in range(8):
+            device.gemm(x, w, z, m=batch, n=D, k=H, ldc=F * D, activation=1)
+            wait()
+            device.dot_interaction(z, inter)
+            wait()
+            device.gemm(inter, top, x, m=batch, n=H, k=pad, activation=1)
+            wait()
+            out.append(torch.empty((batch, 1), device="cuda"))
+            device.gemm(x, last, out[-1], m=batch, n=1, k=H, activation=2)
+            wait()
+        return out + [x, z, inter]
+
+    _same_with_and_without_waiting(chain)
+
+
 @pytest.mark.parametrize("m,n", [(64, 128), (20000, 512), (64, 1)])
 def test_a_refused_launch_is_reported_once(m, n):
     """A product on a stream whose capture was ended by an error is refused; the one after it runs."""
