@@ -78,6 +78,8 @@ class DlrmPipeline:
         nnz = [b.raw_ids.shape[0] for b in emb.bags]
         self.nnz = nnz
         self.nnz_total = int(sum(nnz))
+        self._small = (B <= self.ONE_STREAM_BATCH and
+                       self.nnz_total <= min(self.ONE_STREAM_LOOKUPS, self.ONE_STREAM_BAG * B * T))
         ids_host = np.concatenate([b.raw_ids for b in emb.bags])
         seg_host = np.concatenate([b.slice_input for b in emb.bags])
         offs = np.concatenate([[0], np.cumsum(nnz)])
@@ -196,8 +198,7 @@ class DlrmPipeline:
             x = y
 
     def _one_stream(self) -> bool:
-        return (self.embed_first and self.batch <= self.ONE_STREAM_BATCH and
-                self.nnz_total <= min(self.ONE_STREAM_LOOKUPS, self.ONE_STREAM_BAG * self.batch * self.T))
+        return self._small and self.embed_first
 
     def _sparse_part(self, names, lookahead: bool = False) -> None:
         """Bottom MLP (on the second stream, but for small steps) beside the embedding pooling; z is complete
