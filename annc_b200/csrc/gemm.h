@@ -20,7 +20,9 @@ int run_simt(const annc_gemm_desc& d, cudaStream_t s, const BiasBroadcast* bb = 
 // Whether a product's blocks may take their places while the kernel before it on the stream drains (pdl.cuh).
 // us back to back, without / with: 200 x 512 x 256 7.3 / 6.3, 512 x 1024 x 1024 9.8 / 9.2, 4096 x 512 x 416 11.2 / 10.4,
 // 65536 x 64 x 256 23.7 / 22.2, 1024 x 2048 x 2048 28.3 / 27.3; to trigger behind the main loop instead of before
-// it is the same.  Not beside another stream's kernel that needs the room, which is what ANNC_IO_SINGLE is for, and
+// it is the same.  Less of it as a product gets longer, but none lost: 8192 x 4096 x 2048 254 / 251, BF16 256 x 1024 x 4096
+// 28.7 / 26.4, 16384 x 512 x 1024 26.6 / 23.5, 2048 x 1024 x 8192 51.8 / 49.3, 16384 x 1024 x 8192 253 / 247 (runs
+// of one side 1 % apart), and the three layers of which that is the first 283 / 276.  Not beside another stream's kernel that needs the room, which is what ANNC_IO_SINGLE is for, and
 // not where C is added to (600 x 2048 x 128 11.6 / 13.1, 256 x 5120 x 512 16.0 / 17.8, 1024 x 2048 x 2048 32.6 / 34.4).
 inline bool early_launch(const annc_gemm_desc& d) { return !(d.io_flags & ANNC_IO_SINGLE) && d.beta == 0.f; }
 

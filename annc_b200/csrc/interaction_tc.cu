@@ -288,6 +288,9 @@ int dot_interaction_tc(const float* z, int64_t batch, int F, int dim, int64_t z_
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const unsigned grid = (unsigned)(p.tiles < sms ? p.tiles : sms);
+  // Launched early at every size: us with the product that writes z before it, without / with, batch 200 12.1 / 11.6,
+  // 4096 18.8 / 16.5, 65536 125 / 121.  Row-sharded steps, whose pooling kernel runs beside it, lose nothing either:
+  // one rank, four issue orders, batch 65536 1327 to 1442 / 1323 to 1437, 16384 366 to 412 / 366 to 413.
   const int need = (p.spt * ID + 127) / 128;
   if (need <= 2) ANNC_CUDA(launch_pdl(dot_interaction_tc_kernel<2>, dim3(grid), dim3(I_THREADS), I_SMEM, s, tm, p));
   else if (need <= 8) ANNC_CUDA(launch_pdl(dot_interaction_tc_kernel<8>, dim3(grid), dim3(I_THREADS), I_SMEM, s, tm, p));

@@ -36,12 +36,10 @@ if ROOT not in sys.path:
 METRIC = "dlrm_inference_samples_per_s"
 UNIT = "samples/s"
 
-# DRAM bytes (read + write) of one bag-kernel launch: a constant, not measured by this run.  It is
-# the dram__bytes_read.sum + dram__bytes_write.sum of a profiler capture of the small case
-# (batch 16384, rows <= 1e6: 0.7148 GB for 4,472,660 lookups) scaled to this workload by the lookups
-# per launch (not checked against a capture of the full size).  Keyed by (batch, max_rows, seed); any other
-# workload reports null.
-NCU_BAG_TRAFFIC_BYTES = {(65536, 1e7, 0): 0.7148e9 * 17883957 / 4472660}
+# DRAM bytes (read + write) of one launch of bag_list_kernel: a constant, not measured by this run.  It is
+# the dram__bytes_read.sum + dram__bytes_write.sum (1.50 + 0.42 GB) of a one-pass profiler capture of this very
+# workload, 17,883,957 lookups.  Keyed by (batch, max_rows, seed); any other workload reports null.
+NCU_BAG_TRAFFIC_BYTES = {(65536, 1e7, 0): 1.92e9}
 
 
 def parse_args():
@@ -434,7 +432,7 @@ def run_gpu(args):
                                  input_seed=(1000 + rank) if world > 1 else None)
         emb_bytes = model.emb.algorithmic_bytes()
         nnz = model.emb.nnz
-        bag_kernel = "bag_list_kernel<8,8,1,4,4> (hash-bucket + gather + segment sum, 26 tables in one launch)"
+        bag_kernel = "bag_list_kernel (hash-bucket + gather + segment sum, 26 tables in one launch)"
 
         def build(mode):
             if world == 1:
@@ -605,8 +603,7 @@ def run_gpu(args):
                     "algorithmic_bytes_per_launch": emb_bytes, "lookups_per_launch": nnz,
                     "kernel_ms": bag_avg_ms, "traffic": traffic,
                     "traffic_source": "constant, not measured by this run: ncu dram__bytes_read.sum + "
-                                      "dram__bytes_write.sum of the small case (batch 16384, rows <= 1e6) scaled "
-                                      "by the lookups per launch" if traffic else None,
+                                      "dram__bytes_write.sum of bag_list_kernel on this workload" if traffic else None,
                     "dram_gbs": traffic / (bag_avg_ms / 1e3) / 1e9 if traffic else None,
                     "dram_frac": traffic / (bag_avg_ms / 1e3) / 1e9 / hbm_peak if traffic else None}
     else:

@@ -509,10 +509,12 @@ void annc_embed_bag_set_timing_events(void* start, void* stop);
  * (0 = as many as fit, the default; n > 0 = at most n; -n = n fewer than fit).  For a caller
  * that runs annc_embed_bags_dev on one stream beside another kernel of its own on a second
  * stream and wants both resident (see annc_row_exchange_set_pool_ctas_per_sm): shares of the two
- * kernels that add up to five per SM fit together for rows of up to 128 floats. */
+ * kernels that add up to five per SM fit together for rows of up to 128 floats.  A block also takes up to
+ * 32 KB of shared memory. */
 void annc_embed_bag_set_stream_ctas_per_sm(int ctas_per_sm);
 /* Registers per thread (256 threads a block) of that kernel for rows of dim floats (a multiple of
- * four up to 512), under the share set for this thread. */
+ * four up to 512), under the share set for this thread, for bags of ten lookups on average in tables that
+ * start on 32 bytes.  The builds for other bags and tables take at most 64, above 256 floats 85. */
 int annc_embed_bag_stream_registers(int64_t dim, int* registers_per_thread);
 
 /* GEMM core: C = act(alpha * op(A) * op(B) + beta * C + addend + bias), row-major. */
